@@ -188,7 +188,7 @@ int32_t setup_rve(RveDev& R, char* base, const e3d_rve_t& in, double e1, double 
     BCUDA(cudaMemcpyAsync(R.pix, scratch.data(), 4 * R.ns, cudaMemcpyHostToDevice, s));
   }
   BCUDA(cudaMemcpyAsync(R.mats, mats.data(), sizeof(PhaseMat) * mats.size(), cudaMemcpyHostToDevice, s));
-  batch_phase_kernel<<<R.nphase, 32, 0, s>>>(R.mats, R.nphase, R.cmod, R.cs64, R.cs32, R.dk, R.dkd);
+  batch_phase_kernel<<<R.nphase, 32, 0, s>>>(R.mats, R.nphase, R.cmod, R.cs64, R.cs32, R.dk, R.dkd, nullptr);
   GridDims G = job_dims(R.nx, R.ny, R.nz, 1);
   bjacobi_kernel<<<(unsigned)((R.ns + 255) / 256), 256, 0, s>>>(G, R.pix, R.dkd, nullptr, R.minv32);
   BCUDA(cudaGetLastError());

@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -98,7 +99,8 @@ bool e3d_encode_plane_maps(PlaneMaps* out, const float* h0, const float* h1, con
 
 struct e3d_handle {
   e3d_problem_t prob{};
-  GridDims G{};
+  GridDims G{};   // tiles of TILE_Y rows
+  GridDims Gx{};  // tiles of the fixed-point kernels (kFxRows rows)
   int device = 0;
   int num_sms = 0;
   cudaStream_t stream = nullptr;
@@ -134,6 +136,17 @@ struct e3d_handle {
   // TMA-fed FP32 stencil: tensor maps of h32a, h32b, z32, pix (null: per-thread loads)
   PlaneMaps* maps = nullptr;
   int pcg_grid32_tma = 0;
+  // fixed-point FP64 stencil (e3d_fixed.cuh): phase norms and integer tables,
+  // tile maxima of z (or of a stand-alone apply's x), h0 and h1
+  double* norms = nullptr;
+  int4* fxtab = nullptr;
+  unsigned* mz = nullptr;
+  unsigned* mh0 = nullptr;
+  unsigned* mh1 = nullptr;
+  int* fxleave = nullptr;
+  int fx_kc = 0;
+  bool fx_ok = false;   // the problem's tables allow it
+  bool fx_pcg = false;  // this solve runs in it (until a value leaves its range)
   double* hx = nullptr;
   double* hy = nullptr;
   double* hd = nullptr;
@@ -149,6 +162,7 @@ struct e3d_handle {
   double gg0 = 0.0;
   bool uploaded = false, femat_done = false, energy_done = false, solve_ready = false, minv_ready = false;
   int pcg_grid = 0;
+  int pcg_grid_fx = 0;
   int pcg_grid32 = 0;
   double ms_setup = 0.0, ms_iter = 0.0;
   JumpParams J{};
@@ -234,6 +248,15 @@ ApplyArgs<double> apply_args(e3d_handle* h, const double* x, double* y) {
 // y_partial = in-tile K x plus halos (not yet added).
 int32_t launch_apply_tiles(e3d_handle* h, const double* x, double* y) {
   ApplyArgs<double> A = apply_args(h, x, y);
+  if (h->fx_ok) {
+    A.g = h->Gx;
+    tile_max_kernel<<<(unsigned)h->Gx.ntiles, kFxThreads, 0, h->stream>>>(h->Gx, x, h->mz);
+    E3D_LAUNCHED(h);
+    apply_tiles_fx_kernel<<<(unsigned)h->Gx.ntiles, kFxThreads, sizeof(FxSmem<false>), h->stream>>>(
+        A, FxArgs{h->fxtab, h->fx_kc, h->mz, nullptr});
+    E3D_LAUNCHED(h);
+    return E3D_OK;
+  }
   apply_tiles_kernel<double><<<(unsigned)h->G.ntiles, NT, 0, h->stream>>>(A, nullptr);
   E3D_LAUNCHED(h);
   return E3D_OK;
@@ -242,20 +265,23 @@ int32_t launch_apply_tiles(e3d_handle* h, const double* x, double* y) {
 int32_t apply_device(e3d_handle* h, const double* d_x, double* d_y) {
   int32_t rc = launch_apply_tiles(h, d_x, h->Ah);
   if (rc) return rc;
-  apply_finish_kernel<double><<<blocks_for(h->G.ns, 256), 256, 0, h->stream>>>(h->G, h->Ah, h->hx, h->hy,
-                                                                                 h->hd, d_y);
+  const unsigned nb = blocks_for(h->G.ns, 256);
+  if (h->fx_ok)
+    apply_finish_kernel<double, kFxRows><<<nb, 256, 0, h->stream>>>(h->Gx, h->Ah, h->hx, h->hy, h->hd, d_y);
+  else
+    apply_finish_kernel<double><<<nb, 256, 0, h->stream>>>(h->G, h->Ah, h->hx, h->hy, h->hd, d_y);
   E3D_LAUNCHED(h);
   return E3D_OK;
 }
 
-GridDims make_dims(int nx, int ny, int nz, int num_sms) {
+GridDims make_dims(int nx, int ny, int nz, int num_sms, int tile_y) {
   GridDims G{};
   G.nx = nx;
   G.ny = ny;
   G.nz = nz;
   G.ns = (long long)nx * ny * nz;
   G.ntx = (nx + TILE_X - 1) / TILE_X;
-  G.nty = (ny + TILE_Y - 1) / TILE_Y;
+  G.nty = (ny + tile_y - 1) / tile_y;
   // z chunk: keep >= ~16 tiles per SM in flight (load balance) but long
   // enough that the one redundant element plane per chunk stays small.
   const long long cols = (long long)G.ntx * G.nty;
@@ -338,7 +364,8 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
   h->num_sms = prop.multiProcessorCount;
   if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess)
     return fail(cuda_fail(e, "cudaStreamCreate"));
-  h->G = make_dims(p->nx, p->ny, p->nz, h->num_sms);
+  h->G = make_dims(p->nx, p->ny, p->nz, h->num_sms, TILE_Y);
+  h->Gx = make_dims(p->nx, p->ny, p->nz, h->num_sms, kFxRows);
   const long long ns = h->G.ns, n3 = 3 * ns;
   const int np = p->nphase;
   // PCG grid: as many co-resident tile blocks as the device holds.
@@ -349,8 +376,18 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
       (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_persistent_kernel<double>, NT,
                                                          pcg_dyn_smem_bytes<double>())) != cudaSuccess)
     return fail(cuda_fail(e, "occupancy"));
-  if (per_sm < 1) return fail(E3D_ERR_CUDA);
+  int per_sm_fx = 0;
+  if ((e = cudaFuncSetAttribute(pcg_persistent_kernel<double, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                pcg_dyn_smem_bytes<double, true>())) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(apply_tiles_fx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(FxSmem<false>))) != cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_fx, pcg_persistent_kernel<double, false, true>,
+                                                         kFxThreads,
+                                                         pcg_dyn_smem_bytes<double, true>())) != cudaSuccess)
+    return fail(cuda_fail(e, "occupancy"));
+  if (per_sm < 1 || per_sm_fx < 1) return fail(E3D_ERR_CUDA);
   h->pcg_grid = per_sm * h->num_sms;
+  h->pcg_grid_fx = per_sm_fx * h->num_sms;
   int per_sm32 = 0;
   if ((e = cudaFuncSetAttribute(pcg_persistent_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 pcg_dyn_smem_bytes<float>())) != cudaSuccess ||
@@ -367,20 +404,24 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
                                                            kRingSmemBytes)) != cudaSuccess)
       return fail(cuda_fail(e, "occupancy (TMA)"));
   }
-  h->partial_n = std::max(std::max(h->pcg_grid, h->pcg_grid32), h->num_sms * 4) * 12;
-  const long long halo = h->G.ntiles * h->G.tz;
+  h->partial_n = std::max({h->pcg_grid, h->pcg_grid_fx, h->pcg_grid32, h->num_sms * 4}) * 12;
+  const long long halo = h->G.ntiles * h->G.tz, halo_x = h->Gx.ntiles * h->Gx.tz;
+  const size_t tile_rows = (size_t)h->Gx.ntiles * kFxRows;
   int32_t rc = E3D_OK;
   if ((rc = dalloc(h, &h->pix, ns)) || (rc = dalloc(h, &h->rod, 3 * (size_t)std::max(np - 1, 1))) ||
       (rc = dalloc(h, &h->cmod, 36 * (size_t)np)) || (rc = dalloc(h, &h->cs, kCsStride * (size_t)np)) ||
       (rc = dalloc(h, &h->cs32, kCs32Stride * (size_t)np)) || (rc = dalloc(h, &h->dk, 576 * (size_t)np)) ||
-      (rc = dalloc(h, &h->dkd, 72 * (size_t)np)) || (rc = dalloc(h, &h->u, n3)) || (rc = dalloc(h, &h->g, n3)) ||
+      (rc = dalloc(h, &h->dkd, 72 * (size_t)np)) || (rc = dalloc(h, &h->norms, 3 * (size_t)np)) ||
+      (rc = dalloc(h, &h->fxtab, kFxStride * (size_t)np)) || (rc = dalloc(h, &h->mz, tile_rows)) ||
+      (rc = dalloc(h, &h->mh0, tile_rows)) || (rc = dalloc(h, &h->mh1, tile_rows)) || (rc = dalloc(h, &h->u, n3)) || (rc = dalloc(h, &h->g, n3)) ||
       (rc = dalloc(h, &h->b, n3)) || (rc = dalloc(h, &h->z, n3)) || (rc = dalloc(h, &h->h0, n3)) ||
       (rc = dalloc(h, &h->h1, n3)) || (rc = dalloc(h, &h->Ah, n3)) || (rc = dalloc(h, &h->minv, 6 * ns)) ||
-      (rc = dalloc(h, &h->hx, 3 * halo * TILE_Y)) || (rc = dalloc(h, &h->hy, 3 * halo * TILE_X)) ||
-      (rc = dalloc(h, &h->hd, 3 * halo)) || (rc = dalloc(h, &h->partial, (size_t)h->partial_n)) ||
+      (rc = dalloc(h, &h->hx, 3 * std::max(halo * TILE_Y, halo_x * kFxRows))) ||
+      (rc = dalloc(h, &h->hy, 3 * std::max(halo, halo_x) * TILE_X)) ||
+      (rc = dalloc(h, &h->hd, 3 * std::max(halo, halo_x))) || (rc = dalloc(h, &h->partial, (size_t)h->partial_n)) ||
       (rc = dalloc(h, &h->scalars, 64)) ||
       (rc = dalloc(h, &h->history, (size_t)std::max(p->max_iter, 1))) || (rc = dalloc(h, &h->st, 1)) ||
-      (rc = dalloc(h, &h->bar, 1)) || (rc = dalloc(h, &h->err, 1)))
+      (rc = dalloc(h, &h->bar, 1)) || (rc = dalloc(h, &h->err, 1)) || (rc = dalloc(h, &h->fxleave, 1)))
     return fail(rc);
   if (p->precision == E3D_PREC_MIXED) {
     if ((rc = dalloc(h, &h->du32, n3)) || (rc = dalloc(h, &h->g32, n3)) || (rc = dalloc(h, &h->z32, n3)) ||
@@ -405,6 +446,10 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
   if ((e = cudaMemsetAsync(h->err, 0, sizeof(int), h->stream)) != cudaSuccess) return fail(cuda_fail(e, "memset"));
   if ((e = cudaMemsetAsync(h->bar, 0, sizeof(GridBarrier), h->stream)) != cudaSuccess)
     return fail(cuda_fail(e, "memset"));
+  // tile rows past the grid are never written: they stay zero
+  for (unsigned* q : {h->mz, h->mh0, h->mh1})
+    if ((e = cudaMemsetAsync(q, 0, sizeof(unsigned) * tile_rows, h->stream)) != cudaSuccess)
+      return fail(cuda_fail(e, "memset"));
   if ((e = cudaMemsetAsync(h->h0, 0, sizeof(double) * n3, h->stream)) != cudaSuccess)
     return fail(cuda_fail(e, "memset"));
   if ((e = cudaMemsetAsync(h->h1, 0, sizeof(double) * n3, h->stream)) != cudaSuccess)
@@ -521,7 +566,10 @@ int32_t e3d_femat(e3d_handle_t* h) {
     P.Km = E0 / 3.0 / (1.0 - 2.0 * nu0);
     P.Gm = E0 / 2.0 / (1.0 + nu0);
   }
-  femat_phase_kernel<<<p.nphase, 32, 0, h->stream>>>(P, h->rod, h->cmod, h->cs, h->cs32, h->dk, h->dkd);
+  femat_phase_kernel<<<p.nphase, 32, 0, h->stream>>>(P, h->rod, h->cmod, h->cs, h->cs32, h->dk, h->dkd, h->norms);
+  E3D_LAUNCHED(h);
+  fx_table_kernel<<<std::min(p.nphase, h->num_sms), 96, 0, h->stream>>>(p.nphase, h->norms, h->cs, h->fxtab,
+                                                                        h->scalars + 1);
   E3D_LAUNCHED(h);
   E3D_CUDA(cudaMemsetAsync(h->b, 0, sizeof(double) * 3 * h->G.ns, h->stream));  // interior nodes
   femat_b_kernel<<<blocks_for(boundary_node_count(h->G), 256), 256, 0, h->stream>>>(h->G, h->J, h->pix, h->dk,
@@ -530,10 +578,15 @@ int32_t e3d_femat(e3d_handle_t* h) {
   const int grid = reduction_grid(h);
   femat_c_kernel<<<grid, 256, 0, h->stream>>>(h->G, h->J, h->pix, h->dk, h->partial);
   E3D_LAUNCHED(h);
-  double C = 0.0;
-  int32_t rc = reduce_to_host(h, grid, 1, 1, &C);
+  reduce_partials_kernel<<<1, 256, 0, h->stream>>>(h->partial, grid, 1, 1, h->scalars);
+  E3D_LAUNCHED(h);
+  double out[3] = {0.0, 0.0, 0.0};  // C, and the table exponent with its flag
+  E3D_CUDA(cudaMemcpyAsync(out, h->scalars, sizeof out, cudaMemcpyDeviceToHost, h->stream));
+  int32_t rc = sync(h);
   if (rc) return rc;
-  h->C = C;
+  h->C = out[0];
+  h->fx_kc = (int)out[1];
+  h->fx_ok = out[2] != 0.0;
   h->femat_done = true;
   h->energy_done = h->solve_ready = h->minv_ready = false;
   return E3D_OK;
@@ -557,8 +610,12 @@ int32_t e3d_energy(e3d_handle_t* h, double* utot, double* gg) {
   int32_t rc = launch_apply_tiles(h, h->u, h->Ah);
   if (rc) return rc;
   const int grid = reduction_grid(h) / 2 > 0 ? std::min(reduction_grid(h), h->partial_n / 2) : 1;
-  energy_finish_kernel<<<grid, 256, 0, h->stream>>>(h->G, h->Ah, h->hx, h->hy, h->hd, h->u, h->b, h->g,
-                                                    h->partial);
+  if (h->fx_ok)
+    energy_finish_kernel<kFxRows><<<grid, 256, 0, h->stream>>>(h->Gx, h->Ah, h->hx, h->hy, h->hd, h->u, h->b, h->g,
+                                                               h->partial);
+  else
+    energy_finish_kernel<TILE_Y><<<grid, 256, 0, h->stream>>>(h->G, h->Ah, h->hx, h->hy, h->hd, h->u, h->b, h->g,
+                                                              h->partial);
   E3D_LAUNCHED(h);
   double out[2] = {0.0, 0.0};
   rc = reduce_to_host(h, grid, 2, 2, out);
@@ -615,6 +672,7 @@ int32_t e3d_solve_begin(e3d_handle_t* h) {
   h->since_replace = 0;
   h->minv_ready = true;
   h->solve_ready = true;
+  h->fx_pcg = h->fx_ok;
   return E3D_OK;
 }
 
@@ -665,6 +723,12 @@ PcgArgs<double> pcg_args<double>(e3d_handle* h) {
   P.z = h->z;
   P.Ah = h->Ah;
   P.minv = h->minv;
+  P.fxtab = h->fxtab;
+  P.fxkc = h->fx_kc;
+  P.mz = h->mz;
+  P.mh0 = h->mh0;
+  P.mh1 = h->mh1;
+  P.fxleave = h->fxleave;
   return P;
 }
 
@@ -692,7 +756,11 @@ PcgArgs<float> pcg_args<float>(e3d_handle* h) {
 template <typename T>
 int32_t launch_pcg(e3d_handle* h, int it_limit) {
   const bool tma = sizeof(T) == 4 && h->maps != nullptr;
-  const int grid = sizeof(T) == 8 ? h->pcg_grid : (tma ? h->pcg_grid32_tma : h->pcg_grid32);
+  const bool fx = sizeof(T) == 8 && h->fx_pcg;
+  const int grid = fx               ? h->pcg_grid_fx
+                   : sizeof(T) == 8 ? h->pcg_grid
+                   : tma            ? h->pcg_grid32_tma
+                                    : h->pcg_grid32;
   PcgArgs<T> P = pcg_args<T>(h);
   P.maps = h->maps;
   P.partA = h->partial;
@@ -704,10 +772,18 @@ int32_t launch_pcg(e3d_handle* h, int it_limit) {
   P.timeout_ns = 60ull * 1000000000ull;
   P.it_limit = it_limit;
   E3D_CUDA(cudaMemsetAsync(h->bar, 0, sizeof(GridBarrier), h->stream));
+  if (fx) E3D_CUDA(cudaMemsetAsync(h->fxleave, 0, sizeof(int), h->stream));
   void* args[] = {&P};
-  const void* fn = tma ? (const void*)pcg_persistent_kernel<float, true> : (const void*)pcg_persistent_kernel<T>;
-  cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(NT), args,
-                                              tma ? kRingSmemBytes : pcg_dyn_smem_bytes<T>(), h->stream);
+  const void* fn = tma ? (const void*)pcg_persistent_kernel<float, true>
+                   : fx ? (const void*)pcg_persistent_kernel<double, false, true>
+                                                : (const void*)pcg_persistent_kernel<T>;
+  if constexpr (sizeof(T) == 8)
+    if (fx) P.A.g = h->Gx;
+  cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(fx ? kFxThreads : NT), args,
+                                              tma  ? kRingSmemBytes
+                                              : fx ? pcg_dyn_smem_bytes<double, true>()
+                                                   : pcg_dyn_smem_bytes<T>(),
+                                              h->stream);
   h->launches++;
   if (e != cudaSuccess) return cuda_fail(e, "cudaLaunchCooperativeKernel(pcg)");
   return E3D_OK;
@@ -735,8 +811,12 @@ int32_t residual_replacement(e3d_handle* h) {
   if (rc) return rc;
   if ((rc = launch_apply_tiles(h, h->u, h->Ah))) return rc;
   const int grid = reduction_grid(h);
-  true_residual_kernel<<<grid, 256, 0, h->stream>>>(h->G, h->Ah, h->hx, h->hy, h->hd, h->b, h->minv32, h->g,
-                                                    h->g32, h->z32, h->partial);
+  if (h->fx_ok)
+    true_residual_kernel<kFxRows><<<grid, 256, 0, h->stream>>>(h->Gx, h->Ah, h->hx, h->hy, h->hd, h->b, h->minv32,
+                                                               h->g, h->g32, h->z32, h->partial);
+  else
+    true_residual_kernel<TILE_Y><<<grid, 256, 0, h->stream>>>(h->G, h->Ah, h->hx, h->hy, h->hd, h->b, h->minv32, h->g,
+                                                              h->g32, h->z32, h->partial);
   E3D_LAUNCHED(h);
   replace_scalars_kernel<<<1, 256, 0, h->stream>>>(h->partial, grid, h->st, h->history);
   E3D_LAUNCHED(h);
@@ -783,6 +863,10 @@ int32_t e3d_iterate(e3d_handle_t* h, int32_t n, e3d_solve_stats_t* st) {
         if ((rc = residual_replacement(h))) break;
         if ((rc = read_state(h, &S))) break;
       }
+    }
+    if (S.status == PCG_RUNNING && !mixed && h->fx_pcg && done < chunk) {
+      h->fx_pcg = false;  // values out of the fixed-point range: on in the FP64 form
+      continue;
     }
     if (done == 0 && S.status == PCG_RUNNING) break;  // nothing advanced: do not spin
   }
@@ -1275,6 +1359,7 @@ extern "C" int32_t e3d_checkpoint_load(e3d_handle_t* h, const char* path) {
   if (rc) return rc;
   h->gg0 = H.gg0;
   h->since_replace = S.since_replace;
+  h->fx_pcg = h->fx_ok;
   h->energy_done = true;
   h->minv_ready = true;
   h->solve_ready = true;

@@ -786,7 +786,7 @@ struct PhaseMat {
 
 static __global__ void batch_phase_kernel(const PhaseMat* __restrict__ mats, int nphase_total, double* __restrict__ cmod,
                                           double* __restrict__ cs, float* __restrict__ cs32, double* __restrict__ dk,
-                                          double* __restrict__ dkd) {
+                                          double* __restrict__ dkd, double* __restrict__ norms) {
   const int p = blockIdx.x;
   __shared__ double csh[kCsStride];
   __shared__ double col[24][24];
@@ -833,6 +833,7 @@ static __global__ void batch_phase_kernel(const PhaseMat* __restrict__ mats, int
     const int ra = r / 3, i = r % 3, cb = c / 3, j = c % 3;
     if (ra == cb) dkd[(long long)p * 72 + ra * 9 + i * 3 + j] = v;
   }
+  if (norms) fx_store_norms(col, csh, norms + 3 * p);
 }
 
 }  // namespace e3d

@@ -14,6 +14,7 @@
 
 #include "e3d_bounds.cuh"
 #include "e3d_device.cuh"
+#include "e3d_fixed.cuh"
 #include "e3d_tma.cuh"
 
 namespace e3d {
@@ -158,19 +159,19 @@ struct ApplyArgs {
   T lam_prev;
 };
 
-template <typename T, bool CARRY>
+template <typename T, bool CARRY, int TY = TILE_Y>
 struct ApplySmemT {
-  T node[2][3][(TILE_X + 1) * (TILE_Y + 1)];
-  T r[9][NT];
+  T node[2][3][(TILE_X + 1) * (TY + 1)];
+  T r[9][TILE_X * TY];
 };
-template <typename T>
-struct ApplySmemT<T, true> {
-  T node[2][3][(TILE_X + 1) * (TILE_Y + 1)];
-  T r[9][NT];
-  T carry[12][NT];
+template <typename T, int TY>
+struct ApplySmemT<T, true, TY> {
+  T node[2][3][(TILE_X + 1) * (TY + 1)];
+  T r[9][TILE_X * TY];
+  T carry[12][TILE_X * TY];
 };
-template <typename T>
-using ApplySmem = ApplySmemT<T, sizeof(T) == 4 && E3D_F32_CARRY_SMEM != 0>;
+template <typename T, int TY = TILE_Y>
+using ApplySmem = ApplySmemT<T, sizeof(T) == 4 && E3D_F32_CARRY_SMEM != 0, TY>;
 
 // ---------------------------------------------------------------------------
 // TMA plane ring of the fused FP32 stencil.  One stage holds one node plane of
@@ -364,10 +365,12 @@ __device__ __forceinline__ void ring_drain(PlaneRing& R) {
 // shared-memory slot one plane ahead (cp.async, two slots alternating by plane
 // parity in `tab`, 2 x 6 x NT float4), so the gather's latency is off the
 // element's critical path.
+// TY: rows of a tile (and warps of a block).
 template <typename T, bool FUSED, bool POLD_SMEM = (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), bool DEFER_U = false,
-          bool TAB_ASYNC = false>
-__device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T>& sm, double& hAh,
+          bool TAB_ASYNC = false, int TY = TILE_Y>
+__device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, TY>& sm, double& hAh,
                            float4* __restrict__ tab = nullptr) {
+  constexpr int TILE_Y = TY, NT = TILE_X * TY;
   static_assert(!TAB_ASYNC || sizeof(T) == 4, "the staged table rows are the FP32 ones");
   const GridDims& G = A.g;
   const int tid = threadIdx.x;
@@ -729,6 +732,362 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T>& 
   if constexpr (sizeof(T) == 4) hAh += (double)dot32;
 }
 
+__device__ __forceinline__ void cp_async_4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void cp_async_t(T* dst, const T* src) {
+  if constexpr (sizeof(T) == 4)
+    cp_async_4(dst, src);
+  else
+    cp_async_8(dst, src);
+}
+
+// ---------------------------------------------------------------------------
+// FP64 tile in fixed point (e3d_fixed.cuh).
+
+// Rows of a fixed-point tile, and blocks per SM.  What bounds the tile is the
+// heavy half of the FMA pipe (378 wide multiply-adds an element at 4 cycles a
+// warp) and how little of a warp's other work falls beside it: two blocks of 4
+// warps with 255 registers run their FP64, load and addition phases beside each
+// other's multiply-adds.  FP64 iteration at 300^3: 4.67 ms; one block of 8 warps
+// 4.89, two of 6 (168 registers) 5.04, one of 12 5.01, three of 4 5.08; and the
+// FP64 element form 14.5.
+constexpr int kFxRows = 4;
+constexpr int kFxThreads = TILE_X * kFxRows;
+constexpr int kFxBlocks = 2;
+
+// Largest |value| of each tile, kept as the high word of the double (sign
+// cleared) per warp row: word tile * kFxRows + ty.
+struct FxArgs {
+  const int4* __restrict__ tab;  // kFxStride int4 per phase
+  int kc;                        // table exponent
+  unsigned* mx;                  // tile maxima of A.x (written for h_new when fused)
+  unsigned* mz;                  // tile maxima of A.zv (fused only)
+};
+
+template <bool FUSED>
+struct FxSmem {
+  static constexpr int kHalo = TILE_X + kFxRows + 1;
+  long long node[3][3][(TILE_X + 1) * (kFxRows + 1)];  // plane k in one of three
+  long long r[2][9][kFxThreads];                       // by plane parity
+  // forces on the nodes past the tile's high edges (y row 0..31, x column
+  // 32.., corner last) by plane parity, and those nodes' values, plane k in k % 4
+  long long edge[2][3][kHalo];
+  long long edge_x[FUSED ? 4 : 1][3][kHalo];
+  // a thread's own slots: upper-plane forces of its last element, raw values of
+  // one plane in flight (x, then z; own node, halo node)
+  long long carry[12][kFxThreads];
+  double raw[FUSED ? 6 : 3][kFxThreads + kHalo];
+};
+
+__device__ __forceinline__ unsigned abs_hi(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
+
+constexpr int kFxGeneral = 0x7fffffff;
+
+// Exponent kx of a tile: 2^kx * |value| < 2^kFxNodeBits for every node that the
+// tile reads (its own and the surrounding tiles' maxima; for h_new = z + gamma
+// h_old the bound is max|z| + |gamma| max|h_old|).  kFxGeneral where a value is
+// not finite or the exponent leaves the range of exponent arithmetic: the tile
+// then takes the FP64 form.  All threads call it; every thread gets the result.
+static __device__ __forceinline__ int fx_tile_exponent(const GridDims& G, long long tile, const unsigned* mx,
+                                                       const unsigned* mz, double gamma, unsigned (&red)[2 * kFxRows]) {
+  const int tid = threadIdx.x;
+  static_assert(27 * kFxRows <= kFxThreads, "one load a thread");
+  unsigned bx = 0, bz = 0;
+  if (tid < 27 * kFxRows) {
+    const int nb = tid / kFxRows, row = tid % kFxRows;
+    const int tix = (int)(tile % G.ntx), tiy = (int)((tile / G.ntx) % G.nty),
+              tiz = (int)(tile / ((long long)G.ntx * G.nty));
+    const int ax = wrapi(tix + nb % 3 - 1, G.ntx), ay = wrapi(tiy + (nb / 3) % 3 - 1, G.nty),
+              az = wrapi(tiz + nb / 9 - 1, G.ntz);
+    const long long t = E3D_IDX((ax + (long long)G.ntx * (ay + (long long)G.nty * az)) * kFxRows + row,
+                                G.ntiles * kFxRows);
+    if (mx) bx = __ldcg(mx + t);
+    if (mz) bz = __ldcg(mz + t);
+  }
+  bx = __reduce_max_sync(0xffffffffu, bx);
+  bz = __reduce_max_sync(0xffffffffu, bz);
+  __syncthreads();  // the previous use of red is over
+  if ((tid & 31) == 0) {
+    red[tid >> 5] = bx;
+    red[kFxRows + (tid >> 5)] = bz;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kFxRows; ++i) {
+    bx = max(bx, red[i]);
+    bz = max(bz, red[kFxRows + i]);
+  }
+  if (bx >= 0x7ff00000u || bz >= 0x7ff00000u) return kFxGeneral;
+  const double vx = bx ? __hiloint2double((int)bx + 1, 0) : 0.0, vz = bz ? __hiloint2double((int)bz + 1, 0) : 0.0;
+  const double b = mz ? fma(fabs(gamma), vx, vz) : vx;
+  if (b == 0.0) return 0;
+  const int e = __double2hiint(b) >> 20;  // b < 2^(e - 1022)
+  if (e < 1023 - 400 || e > 1023 + 400) return kFxGeneral;
+  return kFxNodeBits - (e - 1022);
+}
+
+// apply_tile<double, FUSED> with the element products in fixed point: the same
+// march, halos and results; loads, h_new, the halos and K x are doubles.  One
+// block barrier a plane: between two of them a block sums the nodes of one
+// plane, forms the elements of the next, and converts the plane after that, so
+// that its warps need not be in the same phase.  Loads are in flight one plane
+// ahead without holding registers.  FP64 is left with the direction update, the
+// conversions of K x and the dot product.
+template <bool FUSED>
+static __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& A, const FxArgs& F, int kx, long long tile,
+                                                     FxSmem<FUSED>& sm, double& hAh) {
+  constexpr int TILE_Y = kFxRows, NT = kFxThreads;
+  const GridDims& G = A.g;
+  const int tid = threadIdx.x;
+  const int tx = tid % TILE_X, ty = tid / TILE_X;
+  const int tix = (int)(tile % G.ntx);
+  const int tiy = (int)((tile / G.ntx) % G.nty);
+  const int tiz = (int)(tile / ((long long)G.ntx * G.nty));
+  const int x0 = tix * TILE_X, y0 = tiy * TILE_Y, z0 = tiz * G.tz;
+  const int wx = min(TILE_X, G.nx - x0), wy = min(TILE_Y, G.ny - y0), wz = min(G.tz, G.nz - z0);
+  const bool active = (tx < wx) && (ty < wy);
+  const bool xedge = active && tx == wx - 1, yedge = active && ty == wy - 1;
+  const long long ns = G.ns;
+  const long long nxy = (long long)G.nx * G.ny;
+  const int nhalo = wx + wy + 1;
+  constexpr int cst = (TILE_X + 1) * (TILE_Y + 1);
+  constexpr int ed = TILE_X + TILE_Y + 1;
+  int hlx = wx, hly = wy;  // halo node of loader thread tid < nhalo
+  if (tid < wy)
+    hly = tid;
+  else if (tid < wy + wx)
+    hlx = tid - wy;
+  const long long own_col = (long long)(x0 + tx) + (long long)G.nx * (y0 + ty);
+  const long long halo_col = (long long)wrapi(x0 + hlx, G.nx) + (long long)G.nx * wrapi(y0 + hly, G.ny);
+  const int ko = 64 - kx - F.kc, ko20 = ko * (1 << 20);  // force unit 2^ko
+
+  // One node plane's loads are in flight while the previous element computes, in
+  // slots that the loading thread alone reads back: they hold no registers.
+  const bool need_x = !FUSED || !A.reset;
+  auto prefetch = [&](int zl) {
+    const long long zo = nxy * wrapi(zl, G.nz);
+    if (active) {
+      const long long m = E3D_IDX(own_col + zo, ns);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        if (need_x) cp_async_8(&sm.raw[c][tid], A.x + m + c * ns);
+        if (FUSED) cp_async_8(&sm.raw[FUSED ? 3 + c : c][tid], A.zv + m + c * ns);
+      }
+    }
+    if (tid < nhalo) {
+      const long long m = E3D_IDX(halo_col + zo, ns);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        if (need_x) cp_async_8(&sm.raw[c][NT + tid], A.x + m + c * ns);
+        if (FUSED) cp_async_8(&sm.raw[FUSED ? 3 + c : c][NT + tid], A.zv + m + c * ns);
+      }
+    }
+    cp_async_commit();
+  };
+  auto loaded = [&](int i, int c) {
+    if (!FUSED) return sm.raw[c][i];
+    const double z = sm.raw[FUSED ? 3 + c : c][i];
+    return A.reset ? z : fma(A.gamma, sm.raw[c][i], z);
+  };
+  unsigned hmax = 0;
+  // Plane zl's values from their slots: the node's own in X (stored to its plane
+  // buffer by commit), the halo's at once.
+  long long X[3];
+  int nb = (z0 + 2) % 3;  // z0 - 1 mod 3
+  auto convert = [&](int zl, int buf, bool own) {
+    cp_async_wait<0>();
+    if (active) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double v = loaded(tid, c);
+        if (FUSED) {
+          if (own) {
+            A.hnew[E3D_IDX(own_col + nxy * zl, ns) + c * ns] = v;
+            hmax = max(hmax, abs_hi(v));
+          }
+        }
+        X[c] = fx_from_double(v, kx);
+      }
+    }
+    if (tid < nhalo) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        sm.node[buf][c][E3D_IDX(hly * (TILE_X + 1) + hlx, cst)] = fx_from_double(loaded(NT + tid, c), kx);
+    }
+  };
+  auto commit = [&](int buf) {
+    if (active) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) sm.node[buf][c][ty * (TILE_X + 1) + tx] = X[c];
+    }
+  };
+  auto plane_transform = [&](int buf, long long (&P)[3][4]) {
+    const long long* b = sm.node[buf][0] + ty * (TILE_X + 1) + tx;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long v[4] = {b[c * cst], b[c * cst + 1], b[c * cst + TILE_X + 1], b[c * cst + TILE_X + 2]};
+      had_xy(v, P[c]);
+    }
+  };
+  double dot = 0.0, dot_edge = 0.0;
+  // Edge forces of plane k to the halo buffers, and their share of the dot
+  // product: the 3 * ed values in kFlush shares of 32, one a warp, rotating.
+  auto edge_flush = [&](int k, int share) {
+    const int v = share * 32 + (tid & 31);
+    if (v < 3 * ed) {
+      const int c = v / ed, e = v - c * ed;
+      const long long hb = tile * G.tz + (k - z0);
+      const long long per_c = G.ntiles * (long long)G.tz;
+      double* out = nullptr;
+      if (e < TILE_X) {
+        if (e < wx) out = A.hy + E3D_IDX((c * per_c + hb) * TILE_X + e, 3 * per_c * TILE_X);
+      } else if (e < ed - 1) {
+        if (e - TILE_X < wy) out = A.hx + E3D_IDX((c * per_c + hb) * TILE_Y + (e - TILE_X), 3 * per_c * TILE_Y);
+      } else {
+        out = A.hd + E3D_IDX(c * per_c + hb, 3 * per_c);
+      }
+      if (out) {
+        const double d = __ll2double_rn(sm.edge[k & 1][c][e]);
+        if (FUSED) dot_edge = fma(__ll2double_rn(sm.edge_x[FUSED ? k & 3 : 0][c][e]), d, dot_edge);
+        *out = fx_scale(d, ko20);
+      }
+    }
+  };
+  constexpr int kFlush = (3 * ed + 31) / 32;
+  static_assert(kFlush <= kFxRows, "a share for each of some of the warps");
+  long long acc0[3] = {0, 0, 0};  // own corner force of the last element
+  // node sums of plane k from the forces its elements left in sm.r; buf: the
+  // buffer whose own slot still holds the node's value there
+  auto node_sums = [&](int k, int buf) {
+    if (active) {
+      const long long m = E3D_IDX(own_col + nxy * k, ns);
+      const long long(*r)[NT] = sm.r[k & 1];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const long long left3 = tx > 0 ? r[3 * c + 2][tid - 1] : 0;
+        const long long below3 = ty > 0 ? r[3 * c + 2][tid - TILE_X] : 0;
+        long long acc = acc0[c];
+        if (tx > 0) acc += r[3 * c + 0][tid - 1];
+        if (ty > 0) acc += r[3 * c + 1][tid - TILE_X];
+        if (tx > 0 && ty > 0) acc += r[3 * c + 2][tid - TILE_X - 1];
+        const double d = __ll2double_rn(acc);
+        if (FUSED) dot = fma(__ll2double_rn(sm.node[buf][c][ty * (TILE_X + 1) + tx]), d, dot);
+        A.y[m + c * ns] = fx_scale(d, ko20);
+        if (xedge) sm.edge[k & 1][c][TILE_X + ty] = r[3 * c + 0][tid] + below3;
+        if (yedge) sm.edge[k & 1][c][tx] = r[3 * c + 1][tid] + left3;
+        if (xedge && yedge) sm.edge[k & 1][c][ed - 1] = r[3 * c + 2][tid];
+      }
+    }
+  };
+
+  // One barrier a plane.  Between barriers k-1 and k: node sums of plane k-1,
+  // the element of plane k (from plane k+1's buffer and the transform kept of
+  // plane k), conversion of plane k+2 into the buffer that held plane k-1, edge
+  // forces of plane k-2.
+  // (set here, or the threads outside the grid would carry them from tile to tile)
+  long long Pold[3][4] = {};
+  auto edge_share = [&](int k) { return ((tid >> 5) + k) % kFxRows; };
+  auto next = [](int b) { return b == 2 ? 0 : b + 1; };
+  prefetch(z0 - 1);
+  convert(z0 - 1, nb, false);
+  commit(nb);
+  prefetch(z0);
+  const int nb1 = next(nb);
+  convert(z0, nb1, true);
+  commit(nb1);
+  __syncthreads();
+  if (active) plane_transform(nb, Pold);
+  prefetch(z0 + 1);
+  int b0 = nb;  // buffer of plane k
+  int ph_cur = active ? __ldcs(A.pix + E3D_IDX(own_col + nxy * wrapi(z0 - 1, G.nz), ns)) : 0;
+  for (int k = z0 - 1; k < z0 + wz; ++k) {
+    const int b1 = next(b0), b2 = next(b1);  // of planes k + 1 and k + 2
+    const bool more = k + 2 <= z0 + wz;
+    if (more) convert(k + 2, b2, k + 2 < z0 + wz);
+    if (k + 3 <= z0 + wz) prefetch(k + 3);
+    const int ph_nxt = (active && k + 1 < z0 + wz) ? __ldcs(A.pix + E3D_IDX(own_col + nxy * (k + 1), ns)) : 0;
+    if (k > z0) node_sums(k - 1, b2);
+    if (k > z0 + 1 && edge_share(k) < kFlush) edge_flush(k - 2, edge_share(k));
+    if (active) {
+      long long h[3][8];
+      {
+        long long Pn[3][4];
+        plane_transform(b1, Pn);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            h[c][b] = Pn[c][b] + Pold[c][b];
+            h[c][b + 4] = Pn[c][b] - Pold[c][b];
+            Pold[c][b] = Pn[c][b];
+          }
+      }
+      long long f[3][8];
+      element_modal_fx(F.tab + E3D_IDX(ph_cur, A.ncs) * kFxStride, h, f);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        if (k >= z0) {
+          long long lo[4], rr[4];
+          lo[0] = sm.carry[4 * c][tid] - f[c][4];
+#pragma unroll
+          for (int b = 1; b < 4; ++b) lo[b] = (f[c][b] - f[c][b + 4]) + sm.carry[4 * c + b][tid];
+          had_xy_adj(lo, rr);
+          acc0[c] = rr[0];
+          sm.r[k & 1][3 * c + 0][tid] = rr[1];  // to node (x+1, y)
+          sm.r[k & 1][3 * c + 1][tid] = rr[2];  // to node (x, y+1)
+          sm.r[k & 1][3 * c + 2][tid] = rr[3];  // to node (x+1, y+1)
+        }
+        sm.carry[4 * c][tid] = f[c][4];
+#pragma unroll
+        for (int b = 1; b < 4; ++b) sm.carry[4 * c + b][tid] = f[c][b] + f[c][b + 4];
+      }
+      if (FUSED && k >= z0 && (xedge || yedge)) {  // plane k's values past the edges
+        const long long* b = sm.node[b0][0] + ty * (TILE_X + 1) + tx;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (yedge) sm.edge_x[FUSED ? k & 3 : 0][c][tx] = b[c * cst + TILE_X + 1];
+          if (xedge) sm.edge_x[FUSED ? k & 3 : 0][c][TILE_X + ty] = b[c * cst + 1];
+          if (xedge && yedge) sm.edge_x[FUSED ? k & 3 : 0][c][ed - 1] = b[c * cst + TILE_X + 2];
+        }
+      }
+    }
+    if (more) commit(b2);
+    __syncthreads();
+    ph_cur = ph_nxt;
+    b0 = b1;
+  }
+  const int kl = z0 + wz - 1;
+  node_sums(kl, b0 == 0 ? 2 : b0 - 1);
+  if (wz > 1 && edge_share(kl + 1) < kFlush) edge_flush(kl - 1, edge_share(kl + 1));
+  __syncthreads();
+  if (edge_share(kl + 2) < kFlush) edge_flush(kl, edge_share(kl + 2));
+  if (FUSED) {
+    hmax = __reduce_max_sync(0xffffffffu, hmax);
+    if ((tid & 31) == 0) F.mx[E3D_IDX(tile * kFxRows + ty, G.ntiles * kFxRows)] = hmax;
+    // ldexp, not exponent arithmetic: the sums may be zero or span any range
+    hAh += ldexp(dot + dot_edge, ko - kx);
+  }
+}
+
+// A tile that leaves the range of the fixed-point form: the FP64 form, out of line.
+static __device__ __noinline__ void apply_tile_general(const ApplyArgs<double>& A, long long tile,
+                                                       ApplySmem<double, kFxRows>& sm) {
+  double dot = 0.0;
+  apply_tile<double, false, false, false, false, kFxRows>(A, tile, sm, dot);
+}
+
 // Shared memory of apply_tile_ring: the in-plane force exchange of the ZS
 // planes of a step, double-buffered by step parity so one barrier per step
 // suffices.
@@ -932,10 +1291,11 @@ static __device__ void apply_tile_ring(const ApplyArgs<float>& A, long long tile
 }
 
 // Halo contribution for node (x, y, z) from the neighbouring tiles.
-template <typename T>
+template <typename T, int TY = TILE_Y>
 __device__ __forceinline__ void halo_add(const GridDims& G, const T* __restrict__ hx,
                                          const T* __restrict__ hy, const T* __restrict__ hd,
                                          int x, int y, int z, T (&v)[3]) {
+  constexpr int TILE_Y = TY;
   const int tix = x / TILE_X, lx = x - tix * TILE_X;
   const int tiy = y / TILE_Y, ly = y - tiy * TILE_Y;
   const int tiz = z / G.tz, lz = z - tiz * G.tz;
@@ -963,10 +1323,11 @@ __device__ __forceinline__ void halo_add(const GridDims& G, const T* __restrict_
 
 // halo_add for a node whose tile coordinates are known (no integer division);
 // same additions in the same order.
-template <typename T>
+template <typename T, int TY = TILE_Y>
 __device__ __forceinline__ void halo_add_tile(const GridDims& G, const T* __restrict__ hx,
                                               const T* __restrict__ hy, const T* __restrict__ hd,
                                               int tix, int tiy, int tiz, int lx, int ly, int lz, T (&v)[3]) {
+  constexpr int TILE_Y = TY;
   if (lx != 0 && ly != 0) return;
   const int txl = tix == 0 ? G.ntx - 1 : tix - 1;
   const int tyd = tiy == 0 ? G.nty - 1 : tiy - 1;
@@ -1001,7 +1362,53 @@ __global__ void __launch_bounds__(NT, 1) apply_tiles_kernel(ApplyArgs<T> A, doub
   if (partial && threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
-template <typename T>
+// Tile maxima of a nodal vector: one block per tile.
+template <int TY>
+__device__ __forceinline__ void tile_max(const GridDims& G, long long tile, const double* __restrict__ x,
+                                         unsigned* __restrict__ mx) {
+  const int tx = threadIdx.x % TILE_X, ty = threadIdx.x / TILE_X;
+  const int tix = (int)(tile % G.ntx), tiy = (int)((tile / G.ntx) % G.nty),
+            tiz = (int)(tile / ((long long)G.ntx * G.nty));
+  const int xg = tix * TILE_X + tx, yg = tiy * TY + ty, z0 = tiz * G.tz, z1 = min(G.nz, z0 + G.tz);
+  unsigned v = 0;
+  if (xg < G.nx && yg < G.ny) {
+    const long long nxy = (long long)G.nx * G.ny;
+    const double* col = x + E3D_IDX(xg + (long long)G.nx * yg + nxy * z0, G.ns);
+#pragma unroll 4
+    for (int z = z0; z < z1; ++z, col += nxy) {
+      const unsigned a = abs_hi(__ldcg(col)), b = abs_hi(__ldcg(col + G.ns)), c = abs_hi(__ldcg(col + 2 * G.ns));
+      v = max(v, max(a, max(b, c)));
+    }
+  }
+  v = __reduce_max_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) mx[E3D_IDX(tile * TY + ty, G.ntiles * TY)] = v;
+}
+
+static __global__ void __launch_bounds__(kFxThreads) tile_max_kernel(GridDims G, const double* __restrict__ x,
+                                                                     unsigned* __restrict__ mx) {
+  tile_max<kFxRows>(G, blockIdx.x, x, mx);
+}
+
+// The stand-alone FP64 apply in fixed point, one tile a block; F.mx holds the
+// tile maxima of A.x.
+static __global__ void __launch_bounds__(kFxThreads, kFxBlocks) apply_tiles_fx_kernel(ApplyArgs<double> A, FxArgs F) {
+  extern __shared__ __align__(128) unsigned char e3d_fx_dyn[];  // sizeof(FxSmem<false>)
+  FxSmem<false>& sm = *reinterpret_cast<FxSmem<false>*>(e3d_fx_dyn);
+  static_assert(sizeof(ApplySmem<double, kFxRows>) <= sizeof(FxSmem<false>), "the FP64 form shares the memory");
+  __shared__ unsigned mred[2 * kFxRows];
+  __shared__ ApplyArgs<double> sA;
+  double dummy = 0.0;
+  const int kx = fx_tile_exponent(A.g, blockIdx.x, F.mx, nullptr, 0.0, mred);
+  if (kx != kFxGeneral) {
+    apply_tile_fx<false>(A, F, kx, blockIdx.x, sm, dummy);
+  } else {
+    if (threadIdx.x == 0) sA = A;
+    __syncthreads();
+    apply_tile_general(sA, blockIdx.x, *reinterpret_cast<ApplySmem<double, kFxRows>*>(e3d_fx_dyn));
+  }
+}
+
+template <typename T, int TY = TILE_Y>
 __global__ void apply_finish_kernel(GridDims G, const T* __restrict__ yin, const T* __restrict__ hx,
                                     const T* __restrict__ hy, const T* __restrict__ hd,
                                     T* __restrict__ yout) {
@@ -1010,7 +1417,7 @@ __global__ void apply_finish_kernel(GridDims G, const T* __restrict__ yin, const
   int x, y, z;
   node_xyz(G, m, x, y, z);
   T v[3] = {yin[m], yin[m + G.ns], yin[m + 2 * G.ns]};
-  halo_add<T>(G, hx, hy, hd, x, y, z, v);
+  halo_add<T, TY>(G, hx, hy, hd, x, y, z, v);
   yout[m] = v[0];
   yout[m + G.ns] = v[1];
   yout[m + 2 * G.ns] = v[2];
@@ -1018,6 +1425,7 @@ __global__ void apply_finish_kernel(GridDims G, const T* __restrict__ yin, const
 
 // energy_OpenMP tail (src/elas3dxtal_pcg.f90:1332-1340): g = Ku + b,
 // partial sums of (u.Ku/2 + b.u) and of g.g (gg0, :452).
+template <int TY>
 static __global__ void __launch_bounds__(256) energy_finish_kernel(GridDims G, const double* __restrict__ ku,
                                                             const double* __restrict__ hx,
                                                             const double* __restrict__ hy,
@@ -1032,7 +1440,7 @@ static __global__ void __launch_bounds__(256) energy_finish_kernel(GridDims G, c
     int x, y, z;
     node_xyz(G, m, x, y, z);
     double v[3] = {ku[m], ku[m + G.ns], ku[m + 2 * G.ns]};
-    halo_add<double>(G, hx, hy, hd, x, y, z, v);
+    halo_add<double, TY>(G, hx, hy, hd, x, y, z, v);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const long long i = m + c * G.ns;
@@ -1173,9 +1581,38 @@ static __global__ void pix_to_zero_based_kernel(long long ns, int nphase, int32_
 // Reference local node r (1..8 -> 0..7) to corner index a = ox + 2oy + 4oz.
 static __constant__ int kRefToCorner[8] = {0, 1, 3, 2, 4, 5, 7, 6};
 
+// Norms of a phase (fx_phase_norms) from its element matrix in shared memory,
+// one warp.
+__device__ __forceinline__ double fx_max(double a, double b) { return b <= a ? a : b; }  // keeps a NaN in b
+static __device__ __forceinline__ void fx_store_norms(const double (&col)[24][24], const double* csh, double* out) {
+  const int lane = threadIdx.x;
+  double d = 0.0, rows = 0.0, entry = 0.0;
+  if (lane < 24)
+    for (int c = 0; c < 24; ++c) d += fabs(lane <= c ? col[c][lane] : col[lane][c]);
+  if (lane < 18) {
+    const int n = lane < 6 ? 6 : lane < 15 ? 9 : 3, r = lane < 6 ? lane : lane < 15 ? lane - 6 : lane - 15;
+    const double* m = csh + (lane < 6 ? 0 : lane < 15 ? kM2 : kM3) + n * r;
+    for (int c = 0; c < n; ++c) {
+      rows += fabs(m[c]);
+      entry = fx_max(entry, fabs(m[c]));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    d = fx_max(d, __shfl_xor_sync(0xffffffffu, d, o));
+    rows = fx_max(rows, __shfl_xor_sync(0xffffffffu, rows, o));
+    entry = fx_max(entry, __shfl_xor_sync(0xffffffffu, entry, o));
+  }
+  if (lane == 0) {
+    out[0] = d;
+    out[1] = rows;
+    out[2] = entry;
+  }
+}
+
 static __global__ void femat_phase_kernel(FematParams P, const double* __restrict__ rod, double* __restrict__ cmod,
                                    double* __restrict__ cs, float* __restrict__ cs32,
-                                   double* __restrict__ dk, double* __restrict__ dkd) {
+                                   double* __restrict__ dk, double* __restrict__ dkd, double* __restrict__ norms) {
   const int p = blockIdx.x;
   __shared__ double csh[kCsStride];
   __shared__ double col[24][24];  // col[c][r] = (K e_c)[r], c/r = refnode*3 + dof
@@ -1229,6 +1666,60 @@ static __global__ void femat_phase_kernel(FematParams P, const double* __restric
     const int ra = r / 3, i = r % 3, cb = c / 3, j = c % 3;
     if (ra == cb) dkd[(long long)p * 72 + ra * 9 + i * 3 + j] = v;
   }
+  fx_store_norms(col, csh, norms + 3 * p);
+}
+
+// Integer tables of the fixed-point stencil and their exponent, from all phases'
+// norms; every block reduces them itself.
+static __global__ void __launch_bounds__(96) fx_table_kernel(int nphase, const double* __restrict__ norms,
+                                                             const double* __restrict__ cs, int4* __restrict__ tab,
+                                                             double* __restrict__ info) {
+  __shared__ double red[4][3];
+  __shared__ FxInfo f;
+  double d = 0.0, dmin = 1e300, rows = 0.0, entry = 0.0;
+  for (int p = threadIdx.x; p < nphase; p += blockDim.x) {
+    const double a = norms[3 * p];
+    d = fx_max(d, a);
+    if (a > 0.0) dmin = fmin(dmin, a);
+    rows = fx_max(rows, norms[3 * p + 1]);
+    entry = fx_max(entry, norms[3 * p + 2]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    d = fx_max(d, __shfl_xor_sync(0xffffffffu, d, o));
+    dmin = fmin(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
+    rows = fx_max(rows, __shfl_xor_sync(0xffffffffu, rows, o));
+    entry = fx_max(entry, __shfl_xor_sync(0xffffffffu, entry, o));
+  }
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    red[0][w] = d;
+    red[1][w] = dmin;
+    red[2][w] = rows;
+    red[3][w] = entry;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 3; ++i) {
+      d = fx_max(d, red[0][i]);
+      dmin = fmin(dmin, red[1][i]);
+      rows = fx_max(rows, red[2][i]);
+      entry = fx_max(entry, red[3][i]);
+    }
+    f = fx_info(d, dmin, rows, entry);
+    if (blockIdx.x == 0) {
+      info[0] = f.kc;
+      info[1] = f.ok;
+    }
+  }
+  __syncthreads();
+  if (!f.ok) return;
+  for (int p = blockIdx.x; p < nphase; p += gridDim.x)
+    for (int e = threadIdx.x; e < kFxEntries; e += blockDim.x) {
+      int h, l;
+      fx_split(fx_source(cs + (long long)p * kCsStride, e), f.kc, h, l);
+      reinterpret_cast<int2*>(tab + (long long)p * kFxStride)[e] = make_int2(h, l);
+    }
 }
 
 // Periodic-jump force b (src/elas3dxtal_pcg.f90:815-1100), node-centric so
@@ -1637,52 +2128,33 @@ __device__ __forceinline__ double pcg_update_tiles(const GridDims& G, long long 
 // tile-edge halos (hx for lane 0 of each row, hy for row 0, hd for the corner
 // node) travel in the same stages.  Same additions in the same order as
 // pcg_update_tiles: the results are bitwise the same.
-__device__ __forceinline__ void cp_async_4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-template <typename T>
-__device__ __forceinline__ void cp_async_t(T* dst, const T* src) {
-  if constexpr (sizeof(T) == 4)
-    cp_async_4(dst, src);
-  else
-    cp_async_8(dst, src);
-}
-
 // Values of one stage: per thread Ah 3, g 3, Minv 6 (and h 3, u 3 when u is
 // updated here), then the halo slots hx[3][TILE_Y], hy[3][TILE_X], hd[3].
 template <bool UPD_U>
 __host__ __device__ constexpr int pb_fields() {
   return UPD_U ? 18 : 12;
 }
-template <bool UPD_U>
+template <bool UPD_U, int TY = TILE_Y>
 __host__ __device__ constexpr int pb_stage_len() {
-  return pb_fields<UPD_U>() * NT + 3 * TILE_Y + 3 * TILE_X + 3;
+  return pb_fields<UPD_U>() * TILE_X * TY + 3 * TY + 3 * TILE_X + 3;
 }
-template <typename T, int S, bool UPD_U>
+template <typename T, int S, bool UPD_U, int TY = TILE_Y>
 __host__ __device__ constexpr int pb_async_bytes() {
-  return S * pb_stage_len<UPD_U>() * (int)sizeof(T);
+  return S * pb_stage_len<UPD_U, TY>() * (int)sizeof(T);
 }
 
-template <typename T, int S, bool UPD_U = true>
+// ZMAX: the tile maxima of the new z go to mz (the next pass's fixed-point scale).
+template <typename T, int S, bool UPD_U = true, bool ZMAX = false, int TY = TILE_Y>
 __device__ __forceinline__ double pcg_update_tiles_async(const GridDims& G, long long first, long long stride, T lam,
                                                          const T* __restrict__ hc, const T* __restrict__ Ah,
                                                          const T* __restrict__ hx, const T* __restrict__ hy,
                                                          const T* __restrict__ hd, const T* __restrict__ minv,
                                                          T* __restrict__ u, T* __restrict__ g, T* __restrict__ z,
-                                                         T* __restrict__ stages) {
+                                                         T* __restrict__ stages, unsigned* __restrict__ mz = nullptr) {
   static_assert(S >= 2 && (S & (S - 1)) == 0, "stage count: a power of two");
+  constexpr int TILE_Y = TY, NT = TILE_X * TY;
   constexpr int F = pb_fields<UPD_U>();
-  constexpr int SL = pb_stage_len<UPD_U>();
+  constexpr int SL = pb_stage_len<UPD_U, TY>();
   const long long ns = G.ns;
   double zg_t = 0.0;
   const int tid = threadIdx.x;
@@ -1746,6 +2218,7 @@ __device__ __forceinline__ double pcg_update_tiles_async(const GridDims& G, long
       cp_async_commit();
     }
     float zg32 = 0.f;  // FP32: this column's z.g, added to the FP64 sum once per tile
+    unsigned zmax = 0;
     for (int lz = 0; lz < wz; ++lz) {
       if (lz + S - 1 < wz) issue(lz + S - 1);
       cp_async_commit();
@@ -1785,10 +2258,15 @@ __device__ __forceinline__ double pcg_update_tiles_async(const GridDims& G, long
       z[m] = z0v;
       z[m + ns] = z1v;
       z[m + 2 * ns] = z2v;
+      if constexpr (ZMAX) zmax = max(zmax, max(abs_hi(z0v), max(abs_hi(z1v), abs_hi(z2v))));
       if constexpr (sizeof(T) == 4)
         zg32 += z0v * gv[0] + z1v * gv[1] + z2v * gv[2];
       else
         zg_t += (double)(z0v * gv[0] + z1v * gv[1] + z2v * gv[2]);
+    }
+    if constexpr (ZMAX) {  // the row's lanes 0 .. wx-1 are here; rows past the grid keep their zero
+      zmax = __reduce_max_sync(wx == TILE_X ? 0xffffffffu : (1u << wx) - 1u, zmax);
+      if (tx == 0) mz[E3D_IDX(t * TY + ty, G.ntiles * TY)] = zmax;
     }
     if constexpr (sizeof(T) == 4) zg_t += (double)zg32;
   }
@@ -1885,6 +2363,7 @@ static __device__ bool grid_barrier(GridBarrier* gb, int* err, unsigned long lon
 }
 
 // Sum of n per-block partials in a fixed order, returned to every thread.
+template <int NT = e3d::NT>
 static __device__ double reduce_broadcast(const double* partial, int n, double* red) {
   __shared__ double s_val;
   double s = 0.0;
@@ -1897,13 +2376,14 @@ static __device__ double reduce_broadcast(const double* partial, int n, double* 
 
 // Dynamic shared memory of the per-thread-load persistent kernel: the phase-B
 // cp.async stages (0 when phase B keeps its loads in registers).
-template <typename T>
+template <typename T, bool FX = false>
 constexpr int pcg_dyn_smem_bytes() {
   constexpr bool defer_u = sizeof(T) == 4 && E3D_F32_DEFER_U != 0;
   constexpr int S = sizeof(T) == 4 ? E3D_PB_ASYNC_F32 : E3D_PB_ASYNC_F64;
-  constexpr int pb = S > 0 ? pb_async_bytes<T, (S > 0 ? S : 2), !defer_u>() : 0;
+  constexpr int pb = S > 0 ? pb_async_bytes<T, (S > 0 ? S : 2), !defer_u, FX ? kFxRows : TILE_Y>() : 0;
   // phase A's staged table rows use the same bytes (the phases never overlap)
-  constexpr int tab = (sizeof(T) == 4 && E3D_F32_TAB_ASYNC != 0) ? kTabAsyncBytes : 0;
+  // (staged table rows, or the fixed-point FP64 tile)
+  constexpr int tab = FX ? (int)sizeof(FxSmem<true>) : sizeof(T) == 4 && E3D_F32_TAB_ASYNC != 0 ? kTabAsyncBytes : 0;
   return pb > tab ? pb : tab;
 }
 
@@ -1930,15 +2410,28 @@ struct PcgArgs {
   int it_limit;
   unsigned long long timeout_ns;
   const PlaneMaps* maps;  // TMA form only
+  // fixed-point form only: tables, and the tile maxima of z, h0 and h1
+  const int4* fxtab;
+  int fxkc;
+  unsigned* mz;
+  unsigned* mh0;
+  unsigned* mh1;
+  int* fxleave;  // set by a tile whose values leave the fixed-point range
 };
 
 // TMA (FP32 only): phase A reads its node planes through the block's plane
-// ring (dynamic shared memory of kRingSmemBytes).
-template <typename T, bool TMA = false>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 ? 1 : E3D_F32_BLOCKS_PER_SM) : 1)
+// ring (dynamic shared memory of kRingSmemBytes).  FX (FP64 only): phase A in
+// fixed point, each tile scaled by its own values.
+template <typename T, bool TMA = false, bool FX = false>
+__global__ void __launch_bounds__(FX ? kFxThreads : NT,
+                                  FX               ? kFxBlocks
+                                  : sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 ? 1 : E3D_F32_BLOCKS_PER_SM)
+                                                   : 1)
     pcg_persistent_kernel(PcgArgs<T> P) {
+  constexpr int TY = FX ? kFxRows : TILE_Y, NT = TILE_X * TY;
   static_assert(!TMA || sizeof(T) == 4, "the plane ring feeds the FP32 stencil");
-  using Smem = std::conditional_t<TMA, RingApplySmem<E3D_RING_ZS>, ApplySmem<T>>;
+  static_assert(!FX || (sizeof(T) == 8 && E3D_PB_ASYNC_F64 > 0), "the fixed-point stencil is the FP64 one");
+  using Smem = std::conditional_t<TMA, RingApplySmem<E3D_RING_ZS>, std::conditional_t<FX, char, ApplySmem<T>>>;
   __shared__ Smem sm;
   __shared__ double red[NT / 32];
   __shared__ PcgState S0;
@@ -1970,6 +2463,20 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 
   constexpr bool kDeferU = sizeof(T) == 4 && !TMA && E3D_F32_DEFER_U != 0;
   T lam_pending = T(0);  // kDeferU: du -= lam_pending * h_pending not yet applied
   const T* h_pending = nullptr;
+  __shared__ unsigned mred[2 * kFxRows];
+  if constexpr (FX) {  // tile maxima of the vectors that this launch starts from
+    for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x) {
+      tile_max<TY>(G, t, P.z, P.mz);
+      if (!s.reset) tile_max<TY>(G, t, s.cur ? P.h1 : P.h0, s.cur ? P.mh1 : P.mh0);
+    }
+    if (!grid_barrier(P.bar, P.err, P.timeout_ns)) {
+      if (blockIdx.x == 0 && lead) {
+        s.status = PCG_TIMEOUT;
+        *P.st = s;
+      }
+      return;
+    }
+  }
   while (s.it < it_end) {
     // ---- phase A: fused direction update + stencil + h.Ah
     ApplyArgs<T> A = P.A;
@@ -1987,11 +2494,19 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 
     double hAh_t = 0.0;
     if constexpr (TMA) ring_begin(ring, G, cur ? P.maps->h1 : P.maps->h0, blockIdx.x, gridDim.x, G.ntiles);
     for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x) {
-      if constexpr (TMA)
+      if constexpr (TMA) {
         apply_tile_ring<E3D_RING_ZS>(A, t, sm, hAh_t, ring);
-      else
+      } else if constexpr (FX) {
+        const FxArgs F{P.fxtab, P.fxkc, cur ? P.mh0 : P.mh1, P.mz};
+        const int kx = fx_tile_exponent(G, t, A.reset ? nullptr : cur ? P.mh1 : P.mh0, P.mz, A.gamma, mred);
+        if (kx != kFxGeneral)
+          apply_tile_fx<true>(A, F, kx, t, *reinterpret_cast<FxSmem<true>*>(pb_stages), hAh_t);
+        else if (lead)
+          *P.fxleave = 1;
+      } else {
         apply_tile<T, true, (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), kDeferU, kTabAsync>(A, t, sm, hAh_t,
                                                                                            tab_slots);
+      }
       __syncthreads();
     }
     {
@@ -2003,8 +2518,13 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 
       if (lead) s.status = PCG_TIMEOUT;
       break;
     }
+    if constexpr (FX) {
+      // values that the fixed-point form cannot take: leave before anything but
+      // h_new and A h is written; the host goes on with the FP64 form
+      if (__ldcg(P.fxleave)) break;
+    }
     lam_pending = T(0);  // applied by this phase A
-    const double hAh = reduce_broadcast(P.partA, gridDim.x, red);
+    const double hAh = reduce_broadcast<NT>(P.partA, gridDim.x, red);
     if (lead) {
       s.it += 1;
       s.cur ^= 1;
@@ -2024,8 +2544,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 
     constexpr int U = TMA ? E3D_PB_UNROLL_RING : (sizeof(T) == 4 ? E3D_PB_UNROLL_F32 : E3D_PB_UNROLL_F64);
     double zg_t;
     if constexpr (kPbStages > 0)
-      zg_t = pcg_update_tiles_async<T, kPbStages, !kDeferU>(G, blockIdx.x, gridDim.x, lam, hc, P.Ah, P.A.hx, P.A.hy,
-                                                            P.A.hd, P.minv, P.u, P.g, P.z, pb_stages);
+      zg_t = pcg_update_tiles_async<T, kPbStages, !kDeferU, FX, TY>(G, blockIdx.x, gridDim.x, lam, hc, P.Ah, P.A.hx, P.A.hy,
+                                                                P.A.hd, P.minv, P.u, P.g, P.z, pb_stages, P.mz);
     else
       zg_t = pcg_update_tiles<T, U, !kDeferU>(G, blockIdx.x, gridDim.x, lam, hc, P.Ah, P.A.hx, P.A.hy, P.A.hd,
                                               P.minv, P.u, P.g, P.z);
@@ -2042,7 +2562,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 
       if (lead) s.status = PCG_TIMEOUT;
       break;
     }
-    const double gg_new = reduce_broadcast(P.partB, gridDim.x, red);
+    const double gg_new = reduce_broadcast<NT>(P.partB, gridDim.x, red);
     if (lead) {
       const double gglast = s.gg;
       s.gg = gg_new;
@@ -2147,6 +2667,7 @@ static __global__ void fold_correction_kernel(long long n3, const float* __restr
 
 // g = K u + b from the FP64 stencil (in-tile part + halos), stored in FP64 and
 // FP32; then z32 = Minv32 g32 and partial z.g for the replaced residual.
+template <int TY>
 static __global__ void __launch_bounds__(256) true_residual_kernel(GridDims G, const double* __restrict__ ku,
                                                             const double* __restrict__ hx,
                                                             const double* __restrict__ hy,
@@ -2161,7 +2682,7 @@ static __global__ void __launch_bounds__(256) true_residual_kernel(GridDims G, c
     int x, y, z;
     node_xyz(G, m, x, y, z);
     double v[3] = {ku[m], ku[m + G.ns], ku[m + 2 * G.ns]};
-    halo_add<double>(G, hx, hy, hd, x, y, z, v);
+    halo_add<double, TY>(G, hx, hy, hd, x, y, z, v);
     float gv[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
