@@ -274,7 +274,12 @@ int32_t apply_device(e3d_handle* h, const double* d_x, double* d_y) {
   return E3D_OK;
 }
 
-GridDims make_dims(int nx, int ny, int nz, int num_sms, int tile_y) {
+// Tiles of tile_y rows for a grid swept by `blocks` resident blocks.  The z chunk is
+// the one that ends first: waves of tiles times the planes a tile marches, its
+// one redundant element plane and about half a plane of start and end.  A small
+// grid is cut into tiles of one or two planes so that it reaches every SM (32^3:
+// 256 tiles instead of 16); a large one into chunks that fill the last wave.
+GridDims make_dims(int nx, int ny, int nz, int blocks, int tile_y) {
   GridDims G{};
   G.nx = nx;
   G.ny = ny;
@@ -282,15 +287,19 @@ GridDims make_dims(int nx, int ny, int nz, int num_sms, int tile_y) {
   G.ns = (long long)nx * ny * nz;
   G.ntx = (nx + TILE_X - 1) / TILE_X;
   G.nty = (ny + tile_y - 1) / tile_y;
-  // z chunk: keep >= ~16 tiles per SM in flight (load balance) but long
-  // enough that the one redundant element plane per chunk stays small.
   const long long cols = (long long)G.ntx * G.nty;
-  const long long want = std::max<long long>(1, (long long)num_sms * 16);
-  int ntz = (int)std::max<long long>(1, std::min<long long>(nz, (want + cols - 1) / cols));
-  int tz = (nz + ntz - 1) / ntz;
-  if (tz < 16) tz = std::min(nz, 16);
-  G.tz = tz;
-  G.ntz = (nz + tz - 1) / tz;
+  double best = 0.0;
+  for (int ntz = 1; ntz <= nz; ++ntz) {
+    const int tz = (nz + ntz - 1) / ntz;
+    const int n = (nz + tz - 1) / tz;
+    const double cost = (double)((cols * n + blocks - 1) / blocks) * (tz + 1.5);
+    if (ntz == 1 || cost < best) {
+      best = cost;
+      G.tz = tz;
+      G.ntz = n;
+    }
+    if (cols * n > 64LL * blocks) break;  // waves are even by now: shorter chunks only add redundant planes
+  }
   G.ntiles = cols * G.ntz;
   return G;
 }
@@ -364,8 +373,8 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
   h->num_sms = prop.multiProcessorCount;
   if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess)
     return fail(cuda_fail(e, "cudaStreamCreate"));
-  h->G = make_dims(p->nx, p->ny, p->nz, h->num_sms, TILE_Y);
-  h->Gx = make_dims(p->nx, p->ny, p->nz, h->num_sms, kFxRows);
+  h->G = make_dims(p->nx, p->ny, p->nz, E3D_F32_BLOCKS_PER_SM * h->num_sms, TILE_Y);
+  h->Gx = make_dims(p->nx, p->ny, p->nz, kFxBlocks * h->num_sms, kFxRows);
   const long long ns = h->G.ns, n3 = 3 * ns;
   const int np = p->nphase;
   // PCG grid: as many co-resident tile blocks as the device holds.
@@ -586,7 +595,11 @@ int32_t e3d_femat(e3d_handle_t* h) {
   if (rc) return rc;
   h->C = out[0];
   h->fx_kc = (int)out[1];
-  h->fx_ok = out[2] != 0.0;
+  // An indefinite stiffness (nu > 1/2, say) leaves PCG without a bound on what it
+  // makes of rounding, down to which iterations its divergence reset finds: such
+  // problems keep the FP64 form, whose rounding they were validated with.
+  const bool definite = P.K1 >= 0.0 && P.G1 >= 0.0 && P.Km >= 0.0 && P.Gm >= 0.0 && p.c11 >= p.c12 && p.c44 >= 0.0;
+  h->fx_ok = out[2] != 0.0 && definite;
   h->femat_done = true;
   h->energy_done = h->solve_ready = h->minv_ready = false;
   return E3D_OK;
