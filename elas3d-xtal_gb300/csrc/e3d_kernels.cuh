@@ -1871,33 +1871,25 @@ static __global__ void affine_kernel(GridDims G, JumpParams J, double* __restric
   u[m + 2 * G.ns] = x * exz + y * eyz + z * ezz;
 }
 
-// invert3x3 (src/elas3dxtal_pcg.f90:2046-2147); a is row-major a[i][j].
-__device__ __forceinline__ void invert3x3(const double a[3][3], double ai[3][3]) {
-  const double c11 = a[1][1] * a[2][2] - a[1][2] * a[2][1];
-  const double c21 = -a[1][0] * a[2][2] + a[1][2] * a[2][0];
-  const double c31 = a[1][0] * a[2][1] - a[1][1] * a[2][0];
-  const double det = a[0][0] * c11 + a[0][1] * c21 + a[0][2] * c31;
+// invert3x3 (src/elas3dxtal_pcg.f90:2046-2147) of a symmetric block: a and ai hold
+// 00 11 22 01 02 12.  Same products as there; the cofactors that symmetry makes
+// equal are formed once.
+__device__ __forceinline__ void invert3x3(const double (&a)[6], double (&ai)[6]) {
+  const double c00 = a[1] * a[2] - a[5] * a[5];
+  const double c01 = -a[3] * a[2] + a[5] * a[4];
+  const double c02 = a[3] * a[5] - a[1] * a[4];
+  const double det = a[0] * c00 + a[3] * c01 + a[4] * c02;
   if (fabs(det) < 1e-14) {
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) ai[i][j] = 0.0;
+    for (int i = 0; i < 6; ++i) ai[i] = 0.0;
     return;
   }
   const double inv_det = 1.0 / det;
-  const double c12 = -a[0][1] * a[2][2] + a[0][2] * a[2][1];
-  const double c22 = a[0][0] * a[2][2] - a[0][2] * a[2][0];
-  const double c32 = -a[0][0] * a[2][1] + a[0][1] * a[2][0];
-  const double c13 = a[0][1] * a[1][2] - a[0][2] * a[1][1];
-  const double c23 = -a[0][0] * a[1][2] + a[0][2] * a[1][0];
-  const double c33 = a[0][0] * a[1][1] - a[0][1] * a[1][0];
-  ai[0][0] = c11 * inv_det;
-  ai[1][0] = c21 * inv_det;
-  ai[2][0] = c31 * inv_det;
-  ai[0][1] = c12 * inv_det;
-  ai[1][1] = c22 * inv_det;
-  ai[2][1] = c32 * inv_det;
-  ai[0][2] = c13 * inv_det;
-  ai[1][2] = c23 * inv_det;
-  ai[2][2] = c33 * inv_det;
+  ai[0] = c00 * inv_det;
+  ai[1] = (a[0] * a[2] - a[4] * a[4]) * inv_det;
+  ai[2] = (a[0] * a[1] - a[3] * a[3]) * inv_det;
+  ai[3] = c01 * inv_det;
+  ai[4] = c02 * inv_det;
+  ai[5] = (-a[0] * a[5] + a[4] * a[3]) * inv_det;
 }
 
 // Block-Jacobi (src/elas3dxtal_pcg.f90:1498-1520): sum of the node's diagonal
@@ -1917,19 +1909,22 @@ static __global__ void bjacobi_kernel(GridDims G, const int32_t* __restrict__ pi
   }
   int x, y, z;
   node_xyz(G, m, x, y, z);
-  double M[3][3];
+  // FP64-issue-bound: the six distinct entries of the block and of its inverse,
+  // 73 FP64 instructions a node (103 with all nine); 300^3: 5.2 -> 3.45 ms
+  double M[6];
+#pragma unroll
   for (int ra = 0; ra < 8; ++ra) {
     const int a = kRefToCorner[ra];
     const int ex = wrapi(x - (a & 1), G.nx), ey = wrapi(y - ((a >> 1) & 1), G.ny),
               ez = wrapi(z - ((a >> 2) & 1), G.nz);
     const int ph = pix[E3D_IDX((long long)ex + (long long)G.nx * ey + (long long)G.nx * G.ny * ez, G.ns)];
     const double* D = dkd + (long long)ph * 72 + ra * 9;
-    for (int i = 0; i < 3; ++i)
-      for (int j = 0; j < 3; ++j) M[i][j] = (ra == 0) ? D[i * 3 + j] : M[i][j] + D[i * 3 + j];
+    const double d[6] = {__ldg(D), __ldg(D + 4), __ldg(D + 8), __ldg(D + 1), __ldg(D + 2), __ldg(D + 5)};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) M[i] = ra == 0 ? d[i] : M[i] + d[i];
   }
-  double Mi[3][3];
-  invert3x3(M, Mi);
-  const double s[6] = {Mi[0][0], Mi[1][1], Mi[2][2], Mi[0][1], Mi[0][2], Mi[1][2]};
+  double s[6];
+  invert3x3(M, s);
   for (int q = 0; q < 6; ++q) {
     if (minv) minv[m + q * G.ns] = s[q];
     if (minv32) minv32[m + q * G.ns] = (float)s[q];
@@ -1972,25 +1967,21 @@ __device__ __forceinline__ void voxel_strain(const GridDims& G, const JumpParams
     for (int a = 0; a < 8; ++a)
       if (a & 4)
         for (int c = 0; c < 3; ++c) v[c][a] += J.E[c][2] * (double)G.nz;
-  // centre strain = (1/4) x first-order Hadamard differences (engineering shear)
+  // centre strain = (1/4) x first-order Hadamard differences (engineering shear),
+  // differences before sums: neighbours differ little, so they are nearly exact
   double dX[3], dY[3], dZ[3];
+#pragma unroll
   for (int c = 0; c < 3; ++c) {
-    double sx = 0, sy = 0, sz = 0;
-    for (int a = 0; a < 8; ++a) {
-      sx += (a & 1) ? v[c][a] : -v[c][a];
-      sy += (a & 2) ? v[c][a] : -v[c][a];
-      sz += (a & 4) ? v[c][a] : -v[c][a];
-    }
-    dX[c] = 0.25 * sx;
-    dY[c] = 0.25 * sy;
-    dZ[c] = 0.25 * sz;
+    dX[c] = ((v[c][1] - v[c][0]) + (v[c][3] - v[c][2])) + ((v[c][5] - v[c][4]) + (v[c][7] - v[c][6]));
+    dY[c] = ((v[c][2] - v[c][0]) + (v[c][3] - v[c][1])) + ((v[c][6] - v[c][4]) + (v[c][7] - v[c][5]));
+    dZ[c] = ((v[c][4] - v[c][0]) + (v[c][5] - v[c][1])) + ((v[c][6] - v[c][2]) + (v[c][7] - v[c][3]));
   }
-  eps[0] = dX[0];
-  eps[1] = dY[1];
-  eps[2] = dZ[2];
-  eps[3] = dZ[0] + dX[2];
-  eps[4] = dZ[1] + dY[2];
-  eps[5] = dY[0] + dX[1];
+  eps[0] = 0.25 * dX[0];
+  eps[1] = 0.25 * dY[1];
+  eps[2] = 0.25 * dZ[2];
+  eps[3] = 0.25 * (dZ[0] + dX[2]);
+  eps[4] = 0.25 * (dZ[1] + dY[2]);
+  eps[5] = 0.25 * (dY[0] + dX[1]);
 }
 
 static __global__ void __launch_bounds__(256) stress_avg_kernel(GridDims G, JumpParams J, const int32_t* __restrict__ pix,
