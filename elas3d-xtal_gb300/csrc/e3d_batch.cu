@@ -33,20 +33,13 @@ namespace {
     }                                                \
   } while (0)
 
-constexpr int kPartChoices[] = {1, 2, 4, 8, 16, 32, 64};
-constexpr int kMaxParts = 64;
-// Tile depths along z the autotuner tries (0: the rule of job_dims).  Each
-// candidate costs two timed launches per size class and k.
-constexpr int kTzChoices[] = {0, 32};
+constexpr int kMaxParts = 152;  // blocks of one solve: one for each SM
 constexpr unsigned long long kTimeoutNs = 120ull * 1000000000ull;
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// Tiles of one solve run by k parts.  tz_req > 0: z chunks of that many planes
-// (the tile shape the autotuner picked); otherwise split z so that there are at
-// least ~4 tiles per part, keeping chunks of >= 16 planes (one redundant
-// element plane each).
-GridDims job_dims(int nx, int ny, int nz, int k, int tz_req = 0) {
+// Tiles of one solve in z chunks of tz element planes.
+GridDims chunk_dims(int nx, int ny, int nz, int tz) {
   GridDims G{};
   G.nx = nx;
   G.ny = ny;
@@ -54,24 +47,48 @@ GridDims job_dims(int nx, int ny, int nz, int k, int tz_req = 0) {
   G.ns = (long long)nx * ny * nz;
   G.ntx = (nx + TILE_X - 1) / TILE_X;
   G.nty = (ny + TILE_Y - 1) / TILE_Y;
-  const long long cols = (long long)G.ntx * G.nty;
-  const long long want = 4LL * k;
-  int ntz = (int)std::max<long long>(1, std::min<long long>(nz, (want + cols - 1) / cols));
-  int tz = (nz + ntz - 1) / ntz;
-  if (tz < 16) tz = std::min(nz, 16);
-  if (tz_req > 0) tz = std::min(nz, tz_req);
   G.tz = tz;
   G.ntz = (nz + tz - 1) / tz;
-  G.ntiles = cols * G.ntz;
+  G.ntiles = (long long)G.ntx * G.nty * G.ntz;
   return G;
 }
 
-long long halo_doubles(const GridDims& G) { return 3LL * G.ntiles * G.tz * (TILE_X + TILE_Y + 1); }
+// Tiles of one solve run by k parts, each two groups of threads with a tile of
+// its own: the z chunks that end first, by waves of tiles over the groups times
+// the planes a tile marches, its one redundant element plane and about half a
+// plane of start and end.
+GridDims job_dims(int nx, int ny, int nz, int k) {
+  const long long workers = 2LL * k;
+  GridDims best{};
+  double least = 0.0;
+  for (int ntz = 1; ntz <= nz; ++ntz) {
+    const GridDims G = chunk_dims(nx, ny, nz, (nz + ntz - 1) / ntz);
+    const double cost = (double)((G.ntiles + workers - 1) / workers) * (G.tz + 1.5);
+    if (ntz == 1 || cost < least) {
+      least = cost;
+      best = G;
+    }
+    if (G.ntiles > 16 * workers) break;  // waves are even by now
+  }
+  return best;
+}
 
+// The same z chunks in the fixed-point FP64 stencil's tiles.
+GridDims fx_dims(GridDims G) {
+  G.nty = (G.ny + kFxRows - 1) / kFxRows;
+  G.ntiles = (long long)G.ntx * G.nty * G.ntz;
+  return G;
+}
+
+long long halo_doubles(const GridDims& G) {
+  const GridDims X = fx_dims(G);
+  return std::max(3LL * G.ntiles * G.tz * (TILE_X + TILE_Y + 1), 3LL * X.ntiles * X.tz * (TILE_X + kFxRows + 1));
+}
+
+// Over every z chunk that job_dims may take, whatever the number of parts.
 long long max_halo_doubles(int nx, int ny, int nz) {
   long long m = 0;
-  for (int k = 1; k <= kMaxParts; ++k)
-    for (int tz : kTzChoices) m = std::max(m, halo_doubles(job_dims(nx, ny, nz, k, tz)));
+  for (int ntz = 1; ntz <= nz; ++ntz) m = std::max(m, halo_doubles(chunk_dims(nx, ny, nz, (nz + ntz - 1) / ntz)));
   return m;
 }
 
@@ -108,6 +125,9 @@ struct RveDev {
   int32_t* pix = nullptr;  // 0-based into this RVE's own tables
   double* cmod = nullptr;
   double* cs64 = nullptr;
+  int4* fxtab = nullptr;
+  double* fxinfo = nullptr;
+  double* norms = nullptr;
   float* cs32 = nullptr;
   double* dk = nullptr;
   double* dkd = nullptr;
@@ -124,7 +144,8 @@ struct JobDev {
 size_t rve_bytes(long long ns, int nphase) {
   return align256(4 * ns) + align256(8 * 36 * (size_t)nphase) + align256(8 * kCsStride * (size_t)nphase) +
          align256(4 * kCs32Stride * (size_t)nphase) + align256(8 * 576 * (size_t)nphase) +
-         align256(8 * 72 * (size_t)nphase) + align256(4 * 6 * ns) + align256(sizeof(PhaseMat) * (size_t)nphase);
+         align256(8 * 72 * (size_t)nphase) + align256(4 * 6 * ns) + align256(sizeof(PhaseMat) * (size_t)nphase) +
+         align256(sizeof(int4) * kFxStride * (size_t)nphase) + align256(8 * 2) + align256(8 * 3 * (size_t)nphase);
 }
 
 size_t job_bytes(int nx, int ny, int nz, int nphase) {
@@ -162,6 +183,9 @@ int32_t setup_rve(RveDev& R, char* base, const e3d_rve_t& in, double e1, double 
   R.dkd = carve<double>(p, 72 * (size_t)R.nphase);
   R.minv32 = carve<float>(p, 6 * R.ns);
   R.mats = carve<PhaseMat>(p, R.nphase);
+  R.fxtab = carve<int4>(p, kFxStride * (size_t)R.nphase);
+  R.fxinfo = carve<double>(p, 2);
+  R.norms = carve<double>(p, 3 * (size_t)R.nphase);
   if (!checked) {
     scratch.resize((size_t)R.ns);
     for (long long m = 0; m < R.ns; ++m) {
@@ -188,7 +212,11 @@ int32_t setup_rve(RveDev& R, char* base, const e3d_rve_t& in, double e1, double 
     BCUDA(cudaMemcpyAsync(R.pix, scratch.data(), 4 * R.ns, cudaMemcpyHostToDevice, s));
   }
   BCUDA(cudaMemcpyAsync(R.mats, mats.data(), sizeof(PhaseMat) * mats.size(), cudaMemcpyHostToDevice, s));
-  batch_phase_kernel<<<R.nphase, 32, 0, s>>>(R.mats, R.nphase, R.cmod, R.cs64, R.cs32, R.dk, R.dkd, nullptr);
+  batch_phase_kernel<<<R.nphase, 32, 0, s>>>(R.mats, R.nphase, R.cmod, R.cs64, R.cs32, R.dk, R.dkd, R.norms);
+  fx_table_kernel<<<std::min(R.nphase, 128), 96, 0, s>>>(R.nphase, R.norms, R.cs64, R.fxtab, R.fxinfo);
+  // an indefinite stiffness keeps the FP64 form (as e3d_femat does)
+  if (mats.back().K1 < 0.0 || mats.back().G1 < 0.0 || in.c11 < in.c12 || in.c44 < 0.0)
+    BCUDA(cudaMemsetAsync(R.fxinfo, 0, 2 * sizeof(double), s));
   GridDims G = job_dims(R.nx, R.ny, R.nz, 1);
   bjacobi_kernel<<<(unsigned)((R.ns + 255) / 256), 256, 0, s>>>(G, R.pix, R.dkd, nullptr, R.minv32);
   BCUDA(cudaGetLastError());
@@ -206,6 +234,8 @@ void fill_job(JobDev& J, const RveDev& R, char*& p, const double strain[6], int 
   d.pix = R.pix;
   d.cs32 = R.cs32;
   d.cs64 = R.cs64;
+  d.fxtab = R.fxtab;
+  d.fxinfo = R.fxinfo;
   d.dk = R.dk;
   d.cmod = R.cmod;
   d.nphase_total = R.nphase;
@@ -235,9 +265,10 @@ void fill_job(JobDev& J, const RveDev& R, char*& p, const double strain[6], int 
   d.tol = tol;
 }
 
-void set_parts(JobDev& J, const RveDev& R, int k, int tz_req = 0) {
+void set_parts(JobDev& J, const RveDev& R, int k) {
   JobDesc& d = J.d;
-  d.G = job_dims(R.nx, R.ny, R.nz, k, tz_req);
+  d.G = job_dims(R.nx, R.ny, R.nz, k);
+  d.Gx = fx_dims(d.G);
   d.nparts = k;
   const long long h = (long long)d.G.ntiles * d.G.tz;
   double* base = d.hx;
@@ -245,11 +276,14 @@ void set_parts(JobDev& J, const RveDev& R, int k, int tz_req = 0) {
   d.hd = d.hy + 3 * h * TILE_X;
 }
 
+// Nodes per block the serving loop splits a solve into: the longest solve of a
+// round sets its end, so few requests want many blocks each and a full queue few.
+// Seconds for 3, 9 and 40 requests of 48^3 to 160^3 nodes at 16384, 32768, 65536
+// and 131072: .18 .64 5.72, .33 .64 4.78, .50 .90 4.69, 1.39 1.72 5.62.
+constexpr long long kServeBlockNodes = 32768;
 int default_parts(long long ns) {
-  // about 128K nodes per block, at most kMaxParts blocks per solve
-  int k = 1;
-  while (k < kMaxParts && ns > (long long)k * 131072) k *= 2;
-  return k;
+  const long long k = (ns + kServeBlockNodes / 2) / kServeBlockNodes;
+  return (int)std::max(1LL, std::min<long long>(kMaxParts, k));
 }
 
 struct Engine {
@@ -357,18 +391,22 @@ struct e3d_batch {
 
 namespace {
 
-int32_t batch_time_job(e3d_batch* b, size_t j, int k, int tz_req, int iters, float* ms) {
-  JobDev J = b->jobs[j];
-  set_parts(J, b->rves[(size_t)J.rve], k, tz_req);
-  std::vector<JobDesc> one{J.d};
+// Every `step`-th solve with its blocks kjob: set-up and `iters` iterations.
+int32_t batch_time(e3d_batch* b, const std::vector<int>& kjob, size_t step, int iters, float* ms) {
+  std::vector<JobDesc> list;
+  for (size_t j = 0; j < b->jobs.size(); j += step) {
+    JobDev J = b->jobs[j];
+    set_parts(J, b->rves[(size_t)J.rve], kjob[j]);
+    list.push_back(J.d);
+  }
   int np = 0;
-  int32_t rc = b->eng.upload(one, b->stream, &np);
+  int32_t rc = b->eng.upload(list, b->stream, &np);
   if (rc) return rc;
   cudaEvent_t e0, e1;
   BCUDA(cudaEventCreate(&e0));
   BCUDA(cudaEventCreate(&e1));
   BCUDA(cudaEventRecord(e0, b->stream));
-  rc = b->eng.launch(1, np, iters, 1, b->stream);
+  rc = b->eng.launch((int)list.size(), np, iters, 1, b->stream);
   BCUDA(cudaEventRecord(e1, b->stream));
   BCUDA(cudaEventSynchronize(e1));
   float t = 0.f;
@@ -379,83 +417,51 @@ int32_t batch_time_job(e3d_batch* b, size_t j, int k, int tz_req, int iters, flo
   return rc;
 }
 
-// Autotuner: per size class (node count within a factor of two), time the
-// engine on one representative solve for each candidate schedule -- blocks per
-// solve k and tile shape (element planes per tile, kTzChoices) -- as set-up + 10
-// iterations minus set-up + 2; keep the fastest tile shape per k, then choose k
-// per class to minimise the estimated makespan max(total block-time / resident
-// blocks, longest solve).
-int32_t batch_autotune(e3d_batch* b, std::vector<int>& kjob, std::vector<int>& tzjob) {
-  std::map<int, std::vector<size_t>> cls;  // log2(ns) -> solves
-  for (size_t j = 0; j < b->jobs.size(); ++j) {
-    const long long ns = b->rves[(size_t)b->jobs[j].rve].ns;
-    cls[(int)std::floor(std::log2((double)ns))].push_back(j);
-  }
-  struct C {
-    std::vector<int> ks, tzs;  // per k: the fastest tile depth
-    std::vector<double> t;     // ms per iteration per solve
-    int pick = 0;
-    size_t n = 0;
+// Autotuner: times the batch itself (of a large one, evenly spaced solves enough
+// to fill the blocks four times) with the same number of blocks for every solve,
+// and with blocks by nodes, as set-up + 10 iterations minus set-up + 2, and keeps
+// the fastest.  A solve is never timed alone: it would have the L2, the memory
+// and the tail of the batch to itself.  A model of the batch from times of single
+// size classes took 0.81 s for ten ensembles of 32^3 to 88^3 nodes, where 8 blocks
+// for each takes 0.64.
+int32_t batch_autotune(e3d_batch* b, std::vector<int>& kjob) {
+  const size_t n = b->jobs.size();
+  const int B = b->eng.grid;
+  const size_t step = std::max<size_t>(1, n / (4 * (size_t)B));
+  auto limit = [&](size_t j, int k) {  // three in four groups of threads need a tile of their own
+    const RveDev& R = b->rves[(size_t)b->jobs[j].rve];
+    while (k > 1 && (k > B || 2 * job_dims(R.nx, R.ny, R.nz, k).ntiles < 3LL * k)) k /= 2;
+    return k;
   };
-  std::map<int, C> cc;
-  for (auto& kv : cls) {
-    C c;
-    c.n = kv.second.size();
-    const size_t rep = kv.second.front();
-    const RveDev& R = b->rves[(size_t)b->jobs[rep].rve];
-    for (int k : kPartChoices) {
-      const GridDims G = job_dims(R.nx, R.ny, R.nz, k);
-      if (k > 1 && G.ntiles < 2LL * k) break;  // too few tiles to share
-      double best_t = 1e300;
-      int best_tz = 0;
-      for (int tz : kTzChoices) {
-        const GridDims Gt = job_dims(R.nx, R.ny, R.nz, k, tz);
-        if (tz > 0 && (Gt.tz == G.tz || Gt.ntiles < (long long)k)) continue;  // same shape, or too few tiles
-        float t2 = 0.f, t10 = 0.f;
-        int32_t rc = batch_time_job(b, rep, k, tz, 2, &t2);
-        if (!rc) rc = batch_time_job(b, rep, k, tz, 10, &t10);
-        if (rc) return rc;
-        const double t = std::max(1e-6, (double)(t10 - t2) / 8.0);
-        if (t < best_t) {
-          best_t = t;
-          best_tz = tz;
-        }
-      }
-      c.ks.push_back(k);
-      c.tzs.push_back(best_tz);
-      c.t.push_back(best_t);
+  std::vector<std::vector<int>> plans;
+  auto add = [&](auto&& k_of) {
+    std::vector<int> p(n);
+    for (size_t j = 0; j < n; ++j) p[j] = limit(j, k_of(j));
+    if (std::find(plans.begin(), plans.end(), p) == plans.end()) plans.push_back(p);
+  };
+  for (int k = 1; k <= 64; k *= 2) add([&](size_t) { return k; });
+  // A few solves: an even share of the blocks each, beyond the powers of two that
+  // are close together (25 blocks, not 16 or 32, for six solves).
+  const int share = B / (int)n;
+  if (share > 16) add([&](size_t) { return std::min(share, kMaxParts); });
+  for (int per : {16384, 32768, 65536, 131072})
+    add([&](size_t j) {
+      const long long ns = b->rves[(size_t)b->jobs[j].rve].ns;
+      int k = 1;
+      while (k < 64 && (long long)per * k * 3 < ns * 2) k *= 2;  // nearest power of two
+      return k;
+    });
+  double best = 1e300;
+  for (const std::vector<int>& p : plans) {
+    float t2 = 0.f, t10 = 0.f;
+    int32_t rc = batch_time(b, p, step, 2, &t2);
+    if (!rc) rc = batch_time(b, p, step, 10, &t10);
+    if (rc) return rc;
+    if ((double)t10 - t2 < best) {
+      best = (double)t10 - t2;
+      kjob = p;
     }
-    // start from the most block-efficient choice
-    size_t best = 0;
-    for (size_t i = 1; i < c.ks.size(); ++i)
-      if (c.ks[i] * c.t[i] < c.ks[best] * c.t[best]) best = i;
-    c.pick = (int)best;
-    cc[kv.first] = c;
   }
-  const double B = b->eng.grid;
-  for (int guard = 0; guard < 64; ++guard) {
-    double total = 0.0, longest = 0.0;
-    int arg = -1;
-    for (auto& kv : cc) {
-      const C& c = kv.second;
-      total += c.n * c.ks[(size_t)c.pick] * c.t[(size_t)c.pick];
-      if (c.t[(size_t)c.pick] > longest) {
-        longest = c.t[(size_t)c.pick];
-        arg = kv.first;
-      }
-    }
-    C& c = cc[arg];
-    if (longest <= total / B || (size_t)c.pick + 1 >= c.ks.size()) break;
-    c.pick += 1;  // split the longest solves over more blocks
-  }
-  kjob.assign(b->jobs.size(), 1);
-  tzjob.assign(b->jobs.size(), 0);
-  for (auto& kv : cls)
-    for (size_t j : kv.second) {
-      const C& c = cc[kv.first];
-      kjob[j] = c.ks[(size_t)c.pick];
-      tzjob[j] = c.tzs[(size_t)c.pick];
-    }
   return E3D_OK;
 }
 
@@ -558,14 +564,14 @@ int32_t e3d_batch_create(e3d_batch_t** out, const e3d_rve_t* rves, int32_t n, co
     b->order.push_back(J.rve * (int)cases.size() + ci);
   }
   // blocks per solve
-  std::vector<int> kjob(b->jobs.size(), 1), tzjob(b->jobs.size(), 0);
+  std::vector<int> kjob(b->jobs.size(), 1);
   if (o->parts > 0) {
     for (size_t j = 0; j < b->jobs.size(); ++j) kjob[j] = std::min(o->parts, kMaxParts);
-  } else if ((rc = batch_autotune(b, kjob, tzjob))) {
+  } else if ((rc = batch_autotune(b, kjob))) {
     return fail(rc);
   }
   for (size_t j = 0; j < b->jobs.size(); ++j) {
-    set_parts(b->jobs[j], b->rves[(size_t)b->jobs[j].rve], std::min(kjob[j], b->eng.grid), tzjob[j]);
+    set_parts(b->jobs[j], b->rves[(size_t)b->jobs[j].rve], std::min(kjob[j], b->eng.grid));
     b->descs.push_back(b->jobs[j].d);
   }
   if ((rc = b->eng.upload(b->descs, b->stream, &b->nparts_total))) return fail(rc);
@@ -694,11 +700,6 @@ struct e3d_server {
   std::vector<int32_t> scratch;
 };
 
-// Nodes per block the serving loop aims at when it splits a solve into parts.
-#ifndef E3D_SERVE_BLOCK_NODES
-#define E3D_SERVE_BLOCK_NODES 131072
-#endif
-
 // Iterations per round of one solve: round_iters, or with round balancing
 // round_iters x (target nodes per block / this solve's nodes per block), within
 // [1, 8] x round_iters, so that a small solve's block is not left idle while
@@ -707,7 +708,7 @@ struct e3d_server {
 int serve_round_iters(const e3d_serve_opts_t& o, long long ns, int k) {
   if (!o.round_balance) return o.round_iters;
   const double per_block = (double)ns / k;
-  const double f = std::min(8.0, std::max(1.0, (double)E3D_SERVE_BLOCK_NODES / per_block));
+  const double f = std::min(8.0, std::max(1.0, (double)kServeBlockNodes / per_block));
   return (int)std::min<double>(2.0e9, std::floor(o.round_iters * f));
 }
 

@@ -5,9 +5,9 @@
 // 815-1100), affine guess (:423-438), energy (:1107-1353), PCG (:1356-2043) with
 // an FP32 inner loop and FP64 residual replacement, final energy and averaged
 // stress (:2149-2408).  A job is executed by k "parts" (thread blocks): part p
-// takes tiles p, p+k, ...; parts meet at job-local barriers and reduce through
-// per-job partial slots, exactly as the single-problem kernel does across the
-// whole grid.
+// takes tiles 2p, 2p+1, 2p+2k, ... (its two groups of threads one each); parts
+// meet at job-local barriers and reduce through per-job partial slots, exactly as
+// the single-problem kernel does across the whole grid.
 //
 // Scheduling: blocks pull parts from a global counter in order, so every part
 // of a job is handed out before any part of the next job; with k <= the number
@@ -35,12 +35,15 @@ struct JobResult {
 };
 
 struct JobDesc {
-  GridDims G;
+  GridDims G;   // tiles of TILE_Y rows
+  GridDims Gx;  // tiles of the fixed-point FP64 stencil (kFxRows rows, same z chunks)
   JumpParams J;
   // shared per RVE (read only)
   const int32_t* pix;  // global phase ids, 0-based into the batch tables
   const float* cs32;   // [phase][24] packed upper triangle of C/16
   const double* cs64;  // [phase][kCsStride], modal_table
+  const int4* fxtab;     // [phase][kFxStride], fixed-point tables
+  const double* fxinfo;  // their exponent, and whether they apply (fx_table_kernel)
   const double* dk;    // [phase][576]
   const double* cmod;  // cmod(nphase_total,6,6), Fortran layout
   int nphase_total;
@@ -85,6 +88,15 @@ struct EngineArgs {
   unsigned long long timeout_ns;
 };
 
+// A part is a block of 256 threads, which sweeps its tiles with two groups of 128
+// threads (e3d_f32x2.cuh, e3d_fixed.cuh): a part's tiles are 2 * part + group, then
+// every 2 * nparts.  One block holds an SM, so the groups are what runs beside
+// each other there.  Six solves of 64^3, 25 blocks each: 72 ms with one group of
+// 256 threads, an element and a node a thread, 44 with these; sixty of 32^3 to
+// 88^3, 8 blocks each, 770 and 559 ms.
+constexpr int kGroups = NT / kF2Threads;
+static_assert(kGroups == 2 && kFxThreads == kF2Threads, "two groups a block");
+
 // Barrier among the k parts of one job (same protocol as grid_barrier).
 static __device__ bool job_barrier(GridBarrier* gb, unsigned int k, int* err, unsigned long long timeout_ns) {
   __shared__ int s_ok;
@@ -125,8 +137,9 @@ static __device__ bool job_barrier(GridBarrier* gb, unsigned int k, int* err, un
 }
 
 // Slots of the per-job partial array.
-enum : int { SL_A = 0, SL_B = 1, SL_C = 2, SL_U = 3, SL_GG = 4, SL_ZG = 5, SL_S = 6 /* 6..17 */ };
-constexpr int kJobSlots = 18;
+enum : int { SL_A = 0, SL_B = 1, SL_C = 2, SL_U = 3, SL_GG = 4, SL_ZG = 5, SL_S = 6 /* 6..17 */, SL_MAX = 18 };
+constexpr int kJobSlots = 19;
+
 
 // Sum of the k partials of slot `slot`, same value in every part.
 static __device__ double job_reduce(const JobDesc& J, int slot, double* red) {
@@ -145,7 +158,10 @@ __device__ __forceinline__ void for_part_nodes(const JobDesc& J, int part, F&& f
   const GridDims& G = J.G;
   const int tx = threadIdx.x % TILE_X, ty = threadIdx.x / TILE_X;
   const long long nxy = (long long)G.nx * G.ny;
-  for (long long t = part; t < G.ntiles; t += J.nparts) {
+  // the same tiles as the part's two groups sweep, so that a part's own du, h and u
+  // need no barrier among parts
+  for (long long t = (long long)part * kGroups; t < G.ntiles;
+       t += t % kGroups == kGroups - 1 ? (long long)(J.nparts - 1) * kGroups + 1 : 1) {
     const int tix = (int)(t % G.ntx);
     const int tiy = (int)((t / G.ntx) % G.nty);
     const int tiz = (int)(t / ((long long)G.ntx * G.nty));
@@ -298,40 +314,68 @@ inline __device__ ApplyArgs<float> job_apply_args<float>(const JobDesc& J) {
 
 // FP64 K u into g (in-tile part + halos), all parts, then a job barrier.  The
 // apply arguments sit in shared memory (read there, not held in registers).
-static __device__ __noinline__ void job_fp64_apply_tiles(const JobDesc& J, int part, ApplySmem<double>& sm) {
+// Fixed point with one exponent for the whole of u (job_fold's maximum), in tiles
+// of Gx, where the tables and values allow it; returns whether it did (every part
+// decides alike).
+static __device__ __noinline__ bool job_fp64_apply_tiles(const JobDesc& J, int part, unsigned char* dyn) {
   __shared__ ApplyArgs<double> sA;
+  __shared__ int s_kx;
   if (threadIdx.x == 0) {
+    double m = 0.0;
+    for (int i = 0; i < J.nparts; ++i)
+      m = fx_max(m, __ldcg(J.partial + E3D_IDX((long long)SL_MAX * J.nparts + i, kJobSlots * (long long)J.nparts)));
+    s_kx = J.fxinfo[1] != 0.0 ? fx_exponent((unsigned)m) : kFxGeneral;
     ApplyArgs<double> A = job_apply_args<double>(J);
     A.x = J.u;
     A.y = J.g;
+    if (s_kx != kFxGeneral) {
+      const long long h = (long long)J.Gx.ntiles * J.Gx.tz;
+      A.g = J.Gx;
+      A.hy = J.hx + 3 * h * kFxRows;
+      A.hd = A.hy + 3 * h * TILE_X;
+    }
     sA = A;
   }
   __syncthreads();
+  const int kx = s_kx;
   double dummy = 0.0;
-  const long long nt = J.G.ntiles;
-  const int np = J.nparts;
-  for (long long t = part; t < nt; t += np) {
+  if (kx != kFxGeneral) {
+    const int group = threadIdx.x / kFxThreads;
+    FxSmem<false>& sm = reinterpret_cast<FxSmem<false>*>(dyn)[group];
+    const FxArgs F{J.fxtab, (int)J.fxinfo[0], nullptr, nullptr};
+    for (long long t = (long long)part * kGroups + group; t < J.Gx.ntiles; t += (long long)J.nparts * kGroups)
+      apply_tile_fx<false, true>(sA, F, kx, t, sm, dummy);
+    __syncthreads();
+    return true;
+  }
+  ApplySmem<double>& sm = *reinterpret_cast<ApplySmem<double>*>(dyn);
+  for (long long t = part; t < J.G.ntiles; t += J.nparts) {
     apply_tile<double, false>(sA, t, sm, dummy);
     __syncthreads();
   }
+  return false;
 }
 
-static __device__ bool job_fp64_apply_u(const JobDesc& J, int part, ApplySmem<double>& sm, int* err,
-                                 unsigned long long to) {
-  job_fp64_apply_tiles(J, part, sm);
+static __device__ bool job_fp64_apply_u(const JobDesc& J, int part, unsigned char* dyn, bool& fx, int* err,
+                                        unsigned long long to) {
+  fx = job_fp64_apply_tiles(J, part, dyn);
   return job_barrier(J.bar, J.nparts, err, to);
 }
 
 // After job_fp64_apply_u: g = Ku + b (+ halos), g32, z32 = Minv32 g32, partial z.g;
 // optionally the energy terms.  Ends with a barrier.
-static __device__ __noinline__ bool job_true_residual(const JobDesc& J, int part, bool energy, double* red, int* err,
-                                  unsigned long long to) {
+static __device__ __noinline__ bool job_true_residual(const JobDesc& J, int part, bool fx, bool energy, double* red,
+                                                      int* err, unsigned long long to) {
   const GridDims& G = J.G;
   const long long ns = G.ns;
   double zg = 0.0, eu = 0.0, gg = 0.0;
-  for_part_nodes(J, part, [&](long long m, int, int, int, int tix, int tiy, int tiz, int lx, int ly, int lz) {
+  const long long hfx = (long long)J.Gx.ntiles * J.Gx.tz;
+  for_part_nodes(J, part, [&](long long m, int x, int y, int z, int tix, int tiy, int tiz, int lx, int ly, int lz) {
     double v[3] = {J.g[m], J.g[m + ns], J.g[m + 2 * ns]};
-    halo_add_tile<double>(G, J.hx, J.hy, J.hd, tix, tiy, tiz, lx, ly, lz, v);
+    if (fx)
+      halo_add<double, kFxRows>(J.Gx, J.hx, J.hx + 3 * hfx * kFxRows, J.hx + 3 * hfx * (kFxRows + TILE_X), x, y, z, v);
+    else
+      halo_add_tile<double>(G, J.hx, J.hy, J.hd, tix, tiy, tiz, lx, ly, lz, v);
     float gv[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -388,21 +432,10 @@ static __device__ __noinline__ bool job_start_residual(const JobDesc& J, int par
 
 // One FP32 inner iteration's two sweeps, each kept out of line so that it gets
 // its own register allocation rather than the engine kernel's.
-// Fused direction update + stencil: returns this part's h.Ah.
-#ifndef E3D_ENGINE_SWEEP_ATTR
-#define E3D_ENGINE_SWEEP_ATTR __noinline__
-#endif
-#ifndef E3D_ENGINE_TAB_ASYNC
-#define E3D_ENGINE_TAB_ASYNC 0  // stiffness rows staged one plane ahead (E3D_F32_TAB_ASYNC; slower there)
-#endif
-#ifndef E3D_ENGINE_POLD_SMEM
-#define E3D_ENGINE_POLD_SMEM E3D_F32_POLD_SMEM  // lower node plane re-read from shared memory (1) or kept in registers (0)
-#endif
-#ifndef E3D_ENGINE_DEFER_U
-#define E3D_ENGINE_DEFER_U 0  // du -= lam h of iteration k applied in phase A of k+1 (as E3D_F32_DEFER_U)
-#endif
-static __device__ E3D_ENGINE_SWEEP_ATTR double job_fp32_apply(const JobDesc& J, int part, float gamma, int reset, int cur,
-                                                     float lam_prev, ApplySmem<float>& sm, float4* tab) {
+// Fused direction update + stencil + the previous iteration's du -= lam_prev h:
+// returns this thread's share of h.Ah.
+static __device__ __noinline__ double job_fp32_apply(const JobDesc& J, int part, float gamma, int reset, int cur,
+                                                     float lam_prev, unsigned char* dyn) {
   __shared__ ApplyArgs<float> sA;
   if (threadIdx.x == 0) {
     ApplyArgs<float> A = job_apply_args<float>(J);
@@ -418,50 +451,69 @@ static __device__ E3D_ENGINE_SWEEP_ATTR double job_fp32_apply(const JobDesc& J, 
   }
   __syncthreads();
   double hAh = 0.0;
-  const long long nt = J.G.ntiles;
-  const int np = J.nparts;
-  for (long long t = part; t < nt; t += np) {
-    apply_tile<float, true, E3D_ENGINE_POLD_SMEM != 0, E3D_ENGINE_DEFER_U != 0, E3D_ENGINE_TAB_ASYNC != 0>(sA, t, sm,
-                                                                                                         hAh, tab);
-    __syncthreads();
+  const int group = threadIdx.x / kF2Threads;
+  F2Smem& sm = reinterpret_cast<F2Smem*>(dyn)[group];
+  for (long long t = (long long)part * kGroups + group; t < J.G.ntiles; t += (long long)J.nparts * kGroups) {
+    if (tile_full(J.G, t))
+      apply_tile_f2<true, true, true>(sA, t, sm, hAh);
+    else
+      apply_tile_f2<true, false, true>(sA, t, sm, hAh);
   }
+  __syncthreads();
   return hAh;
 }
 
-// Phase-B planes in flight per thread through cp.async stages in the engine's
-// dynamic shared memory (0: the one-node register form).
-#ifndef E3D_ENGINE_PB_ASYNC
-#define E3D_ENGINE_PB_ASYNC 2
-#endif
-constexpr int kEnginePbBytes =
-    E3D_ENGINE_PB_ASYNC > 0 ? pb_async_bytes<float, (E3D_ENGINE_PB_ASYNC > 0 ? E3D_ENGINE_PB_ASYNC : 2), true>() : 0;
-// the FP32 stencil's staged table rows share these bytes (the sweeps never overlap)
-constexpr int kEngineDynSmem = (E3D_ENGINE_TAB_ASYNC && kTabAsyncBytes > kEnginePbBytes) ? kTabAsyncBytes : kEnginePbBytes;
-
-// du -= lam h, g -= lam Ah, z = Minv g: returns this part's z.g.
-static __device__ __noinline__ double job_fp32_update(const JobDesc& J, int part, float lam, int cur, float* stages) {
-  if constexpr (E3D_ENGINE_PB_ASYNC > 0)
-    return pcg_update_tiles_async<float, E3D_ENGINE_PB_ASYNC, E3D_ENGINE_DEFER_U == 0>(
-        J.G, part, J.nparts, lam, cur ? J.h0 : J.h1, J.Ah, reinterpret_cast<const float*>(J.hx),
-        reinterpret_cast<const float*>(J.hy), reinterpret_cast<const float*>(J.hd), J.minv32, J.du, J.g32, J.z32,
-        stages);
-  else
-    return pcg_update_tiles<float, E3D_PB_UNROLL_F32, E3D_ENGINE_DEFER_U == 0>(J.G, part, J.nparts, lam,
-                                                                                 cur ? J.h0 : J.h1, J.Ah,
-                                   reinterpret_cast<const float*>(J.hx), reinterpret_cast<const float*>(J.hy),
-                                   reinterpret_cast<const float*>(J.hd), J.minv32, J.du, J.g32, J.z32);
+// g -= lam Ah, z = Minv g (du waits for the next sweep): returns this thread's
+// share of z.g.  Nodes a thread takes at a time: what the rows' alignment allows.
+static __device__ __noinline__ double job_fp32_update(const JobDesc& J, int part, float lam, unsigned char* dyn) {
+  const int group = threadIdx.x / kF2Threads, tid = threadIdx.x % kF2Threads;
+  float* stages = reinterpret_cast<float*>(dyn + group * pv_bytes<false>());
+  const float *hx = reinterpret_cast<const float*>(J.hx), *hy = reinterpret_cast<const float*>(J.hy),
+              *hd = reinterpret_cast<const float*>(J.hd);
+  const long long first = (long long)part * kGroups + group, stride = (long long)J.nparts * kGroups;
+  if (J.G.nx % 4 == 0)
+    return pcg_update_tiles_v<4, false>(J.G, first, stride, lam, nullptr, J.Ah, hx, hy, hd, J.minv32, J.du, J.g32, J.z32,
+                                        stages, tid);
+  if (J.G.nx % 2 == 0)
+    return pcg_update_tiles_v<2, false>(J.G, first, stride, lam, nullptr, J.Ah, hx, hy, hd, J.minv32, J.du, J.g32, J.z32,
+                                        stages, tid);
+  return pcg_update_tiles_v<1, false>(J.G, first, stride, lam, nullptr, J.Ah, hx, hy, hd, J.minv32, J.du, J.g32, J.z32,
+                                      stages, tid);
 }
 
+// Shared memory of a part: the sweeps take it in turn.
+constexpr int kEngineDynSmem = [] {
+  int b = kGroups * (int)sizeof(F2Smem);
+  for (int c : {kGroups * (int)sizeof(FxSmem<false>), kGroups * pv_bytes<false>(), (int)sizeof(ApplySmem<double>)})
+    b = c > b ? c : b;
+  return b;
+}();
+static_assert(sizeof(F2Smem) % 8 == 0 && pv_bytes<false>() % 16 == 0 && sizeof(FxSmem<false>) % 8 == 0,
+              "the groups' parts stay aligned");
+
+// u += du, du = 0; the part's largest |u| (high word) to its slot, for the
+// fixed-point pass that follows.
 static __device__ void job_fold(const JobDesc& J, int part) {
   const long long ns = J.G.ns;
+  unsigned m_hi = 0;
   for_part_nodes(J, part, [&](long long m, int, int, int, int, int, int, int, int, int) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const long long i = m + c * ns;
-      J.u[i] += (double)J.du[i];
+      const double v = J.u[i] + (double)J.du[i];
+      J.u[i] = v;
       J.du[i] = 0.0f;
+      m_hi = max(m_hi, abs_hi(v));
     }
   });
+  __shared__ unsigned s_max[NT / 32];
+  m_hi = __reduce_max_sync(0xffffffffu, m_hi);
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m_hi;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < NT / 32; ++i) m_hi = max(m_hi, s_max[i]);
+    J.partial[E3D_IDX((long long)SL_MAX * J.nparts + part, kJobSlots * (long long)J.nparts)] = (double)m_hi;
+  }
 }
 
 // Residual drop after which the job engine replaces the FP32 recurrence's
@@ -481,16 +533,11 @@ constexpr double kRefineDrop = E3D_ENGINE_REFINE_DROP;
 // writes them, every thread reads them after a barrier, so neither occupies
 // registers during the sweeps.
 static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engine_kernel(EngineArgs E) {
-  static_assert(sizeof(ApplySmem<float>) <= sizeof(ApplySmem<double>), "the FP32 tile shares the FP64 tile's memory");
-  __shared__ __align__(16) unsigned char smraw[sizeof(ApplySmem<double>)];
   __shared__ double red[NT / 32];
   __shared__ int s_idx, s_part;
   __shared__ JobDesc sJ;
   __shared__ PcgState sS;
-  extern __shared__ __align__(128) unsigned char e3d_engine_dyn[];
-  float* pb_stages = reinterpret_cast<float*>(e3d_engine_dyn);  // kEngineDynSmem bytes
-  ApplySmem<double>& sm64 = *reinterpret_cast<ApplySmem<double>*>(smraw);
-  ApplySmem<float>& sm32 = *reinterpret_cast<ApplySmem<float>*>(smraw);
+  extern __shared__ __align__(128) unsigned char e3d_engine_dyn[];  // kEngineDynSmem bytes
   const unsigned long long to = E.timeout_ns;
   const bool lead = threadIdx.x == 0;
   const JobDesc& J = sJ;
@@ -596,18 +643,19 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
     // ---------------- FP32 inner iterations with FP64 residual replacement
     const int R = J.refine_every > 0 ? J.refine_every : 50;
     const int it_end = min(s.it + (J.it_round > 0 ? J.it_round : E.it_limit), s.max_iter);
-    // E3D_ENGINE_DEFER_U: du -= lam_pending * h_pending is still owed; the next
-    // phase A applies it, or flush_pending before du is read or the job yields
+    // du -= lam_pending * h_pending is still owed; the next sweep applies it, or
+    // flush_pending before du is read or the job yields
     float lam_pending = 0.f;
     const float* h_pending = nullptr;
     auto flush_pending = [&]() {
-      if (E3D_ENGINE_DEFER_U && lam_pending != 0.f) flush_u_tiles<float>(G, part, J.nparts, lam_pending, h_pending, J.du);
+      if (lam_pending != 0.f)
+        flush_u_tiles_f2(G, (long long)part * kGroups + threadIdx.x / kF2Threads, (long long)J.nparts * kGroups,
+                         lam_pending, h_pending, J.du, threadIdx.x % kF2Threads);
       lam_pending = 0.f;
     };
     while (ok && s.status == PCG_RUNNING && s.it < it_end) {
       const int cur = s.cur;
-      const double hAh_t = job_fp32_apply(J, part, (float)s.gamma, s.reset, cur, lam_pending, sm32,
-                                          reinterpret_cast<float4*>(e3d_engine_dyn));
+      const double hAh_t = job_fp32_apply(J, part, (float)s.gamma, s.reset, cur, lam_pending, e3d_engine_dyn);
       lam_pending = 0.f;  // applied by this phase A
       job_put(J, SL_A, part, hAh_t, red);
       if (!(ok = job_barrier(J.bar, J.nparts, E.err, to))) break;
@@ -624,11 +672,9 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
       __syncthreads();
       if (s.status != PCG_RUNNING) break;
       const float lam = (float)(s.gg / hAh);
-      const double zg = job_fp32_update(J, part, lam, cur, pb_stages);
-      if (E3D_ENGINE_DEFER_U) {
-        lam_pending = lam;
-        h_pending = cur ? J.h0 : J.h1;  // the h_new of this iteration's phase A
-      }
+      const double zg = job_fp32_update(J, part, lam, e3d_engine_dyn);
+      lam_pending = lam;
+      h_pending = cur ? J.h0 : J.h1;  // the h_new of this iteration's phase A
       job_put(J, SL_B, part, zg, red);
       if (!(ok = job_barrier(J.bar, J.nparts, E.err, to))) break;
       const double gg_new = job_reduce(J, SL_B, red);
@@ -667,12 +713,14 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
       if (s.status == PCG_CONVERGED || s.since_replace >= R || s.rel_res < kRefineDrop * s.rel_at_replace) {
         // FP64 residual replacement: u += du, g = K u + b, restart the FP32 recurrence
         flush_pending();
+        __syncthreads();  // du: flush_pending's owners are not the fold's
         job_fold(J, part);
         if (!(ok = job_barrier(J.bar, J.nparts, E.err, to))) break;
-        if (!(ok = job_fp64_apply_u(J, part, sm64, E.err, to))) break;
+        bool fx = false;
+        if (!(ok = job_fp64_apply_u(J, part, e3d_engine_dyn, fx, E.err, to))) break;
         // energy terms too: if this replacement ends the solve, the final
         // stage reuses them instead of another FP64 pass over the same u
-        if (!(ok = job_true_residual(J, part, true, red, E.err, to))) break;
+        if (!(ok = job_true_residual(J, part, fx, true, red, E.err, to))) break;
         const double ggt = job_reduce(J, SL_ZG, red);
         if (lead) {
           s.gg = ggt;
@@ -693,7 +741,7 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
         __syncthreads();
       }
     }
-    flush_pending();  // the part's own nodes, as phase A owns them: no barrier needed before the fold
+    flush_pending();
     __syncthreads();
     if (lead) {
       if (!ok) s.status = PCG_TIMEOUT;
@@ -718,8 +766,9 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
       job_fold(J, part);
       ok = job_barrier(J.bar, J.nparts, E.err, to);
     }
-    if (ok && !fresh) ok = job_fp64_apply_u(J, part, sm64, E.err, to);
-    if (ok && !fresh) ok = job_true_residual(J, part, true, red, E.err, to);
+    bool fx = false;
+    if (ok && !fresh) ok = job_fp64_apply_u(J, part, e3d_engine_dyn, fx, E.err, to);
+    if (ok && !fresh) ok = job_true_residual(J, part, fx, true, red, E.err, to);
     double sacc[12];
     for (int q = 0; q < 12; ++q) sacc[q] = 0.0;
     if (ok) {

@@ -14,6 +14,7 @@
 
 #include "e3d_bounds.cuh"
 #include "e3d_device.cuh"
+#include "e3d_f32x2.cuh"
 #include "e3d_fixed.cuh"
 #include "e3d_tma.cuh"
 
@@ -754,6 +755,331 @@ __device__ __forceinline__ void cp_async_t(T* dst, const T* src) {
 }
 
 // ---------------------------------------------------------------------------
+// FP32 tile with two elements a thread (e3d_f32x2.cuh): 32 x 8 columns, 128
+// threads; thread (tx, tr) has rows 2 tr and 2 tr + 1.
+constexpr int kF2Threads = TILE_X * TILE_Y / 2;
+
+struct F2Smem {
+  float node[3][3][(TILE_Y + 1) * (TILE_X + 1)];  // plane k in one of three, rows of TILE_X + 1
+  float r[2][6][kF2Threads];                      // forces to the row above, by plane parity
+  // a thread's own slots: one plane's values in flight (z, h_old, du; rows a and
+  // b; then the halo node's z and h_old), and what it carries up the column
+  float raw[18][kF2Threads];
+  float raw_halo[6][kF2Threads];
+  f2 carry[12][kF2Threads];
+  f2 pold[12][kF2Threads];
+};
+
+// The fused FP32 pass of apply_tile<float, true> over one tile: same results up
+// to the order of sums, same halos.  One barrier a plane: between two of them the
+// nodes of one plane are summed and the elements of the next formed, while the
+// loads of the plane after that are in flight.  The dot product h . K h is the
+// sum of the element energies, from values at hand in the element.  Byte offsets
+// into a component fit 32 bits: no device that holds a solve's state has 2^30
+// nodes.  DEFER_U: du -= lam_prev * h_old for the own nodes on the way.  FULL: the
+// tile has all its 32 x 8 columns, so that nothing is masked.
+__device__ __forceinline__ float* at_byte(float* p, unsigned o) {
+  return reinterpret_cast<float*>(reinterpret_cast<char*>(p) + o);
+}
+__device__ __forceinline__ const float* at_byte(const float* p, unsigned o) {
+  return reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + o);
+}
+
+// Whether a tile has all its 32 x 8 columns.
+__device__ __forceinline__ bool tile_full(const GridDims& G, long long tile) {
+  const long long txy = tile % ((long long)G.ntx * G.nty);
+  return (txy % G.ntx + 1) * TILE_X <= G.nx && (txy / G.ntx + 1) * TILE_Y <= G.ny;
+}
+
+// Barrier of the 128 threads that share a tile: the whole block, or, GROUPED,
+// one of the groups of 128 that make up a larger block.
+template <bool GROUPED>
+__device__ __forceinline__ void tile_sync() {
+  if constexpr (GROUPED)
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + (int)(threadIdx.x >> 7)) : "memory");
+  else
+    __syncthreads();
+}
+
+template <bool DEFER_U, bool FULL, bool GROUPED>
+static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, long long tile, F2Smem& sm,
+                                                     double& hAh) {
+  const GridDims& G = A.g;
+  const int tid = threadIdx.x % kF2Threads;
+  const int tx = tid % TILE_X, tr = tid / TILE_X, ya = 2 * tr;
+  const int tix = (int)(tile % G.ntx);
+  const int tiy = (int)((tile / G.ntx) % G.nty);
+  const int tiz = (int)(tile / ((long long)G.ntx * G.nty));
+  const int x0 = tix * TILE_X, y0 = tiy * TILE_Y, z0 = tiz * G.tz;
+  const int wx = FULL ? TILE_X : min(TILE_X, G.nx - x0), wy = FULL ? TILE_Y : min(TILE_Y, G.ny - y0);
+  const int wz = min(G.tz, G.nz - z0);
+  const bool act_a = FULL || (tx < wx && ya < wy), act_b = FULL || (tx < wx && ya + 1 < wy);
+  const unsigned nx = (unsigned)G.nx, nxy = nx * (unsigned)G.ny;
+  const long long ns = G.ns;
+  constexpr int kRow = TILE_X + 1;
+  const unsigned own = (unsigned)(x0 + tx) + nx * (unsigned)(y0 + ya);
+  // halo node of loader thread tid < wx + wy + 1
+  const int nhalo = wx + wy + 1;
+  int hlx = wx, hly = wy;
+  if (tid < wy)
+    hly = tid;
+  else if (tid < wy + wx)
+    hlx = tid - wy;
+  const unsigned halo = (unsigned)wrapi(x0 + hlx, G.nx) + nx * (unsigned)wrapi(y0 + hly, G.ny);
+  const bool reset = A.reset != 0, owe = DEFER_U && A.lam_prev != 0.f;
+  const int zend = z0 + wz;
+
+  // raw slot of field f (z 0, h_old 1, du 2), component c, row q
+  auto slot = [](int f, int c, int q) { return 6 * f + 2 * c + q; };
+  auto load = [&](int zl) {
+    const unsigned zo = nxy * (unsigned)wrapi(zl, G.nz);
+    const bool mine = DEFER_U && zl >= z0 && zl < zend, need_x = !reset || mine;
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (q ? act_b : act_a) {
+        const unsigned o = 4u * (unsigned)E3D_IDX(own + (q ? nx : 0u) + zo, ns);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[slot(0, c, q)][tid], at_byte(A.zv + c * ns, o));
+        if (need_x)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[slot(1, c, q)][tid], at_byte(A.x + c * ns, o));
+        if (mine)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[slot(2, c, q)][tid], at_byte(A.du + c * ns, o));
+      }
+    if (tid < nhalo) {
+      const unsigned o = 4u * (unsigned)E3D_IDX(halo + zo, ns);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw_halo[c][tid], at_byte(A.zv + c * ns, o));
+      if (!reset)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw_halo[3 + c][tid], at_byte(A.x + c * ns, o));
+    }
+    cp_async_commit();
+  };
+  auto commit = [&](int zl, float (&buf)[3][(TILE_Y + 1) * kRow]) {
+    cp_async_wait<0>();
+    const unsigned zo = nxy * (unsigned)zl;  // used on own planes only
+    const bool mine = zl >= z0 && zl < zend;
+    // every slot is read before anything is stored: a store in between would
+    // hold back the reads behind it
+    float z[6], x[6], du[6], zh[3], xh[3];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      z[i] = sm.raw[i][tid];
+      x[i] = sm.raw[6 + i][tid];
+      du[i] = DEFER_U ? sm.raw[12 + i][tid] : 0.f;
+    }
+    const bool halo_thread = tid < nhalo;
+    if (halo_thread) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        zh[c] = sm.raw_halo[c][tid];
+        xh[c] = sm.raw_halo[3 + c][tid];
+      }
+    }
+    float v[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) v[i] = reset ? z[i] : fmaf(A.gamma, x[i], z[i]);
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (q ? act_b : act_a) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) buf[c][(ya + q) * kRow + tx] = v[2 * c + q];
+      }
+    if (halo_thread) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        buf[c][E3D_IDX(hly * kRow + hlx, (TILE_Y + 1) * kRow)] = reset ? zh[c] : fmaf(A.gamma, xh[c], zh[c]);
+    }
+    if (mine) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (q ? act_b : act_a) {
+          const unsigned o = 4u * (unsigned)E3D_IDX(own + (q ? nx : 0u) + zo, ns);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) *at_byte(A.hnew + c * ns, o) = v[2 * c + q];
+          // nothing pending at the first step of a launch (lam_prev = 0): h_old
+          // may then hold another solve's direction and is not used
+          if (owe)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) *at_byte(A.du + c * ns, o) = du[2 * c + q] - A.lam_prev * x[2 * c + q];
+        }
+    }
+  };
+  // xy transform of a plane for both elements: P[by * 2 + bx]
+  auto plane_transform = [&](const float (&buf)[3][(TILE_Y + 1) * kRow], f2 (&P)[3][4]) {
+    float w[3][6];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < 6; ++i) w[c][i] = buf[c][(ya + i / 2) * kRow + tx + (i & 1)];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const f2 l = f2_pack(w[c][0], w[c][2]), r = f2_pack(w[c][1], w[c][3]);
+      const f2 s = f2_add(r, l), d = f2_sub(r, l);
+      const float s2 = w[c][5] + w[c][4], d2 = w[c][5] - w[c][4];
+      const f2 su = f2_pack(f2_hi(s), s2), du = f2_pack(f2_hi(d), d2);  // of the rows above
+      P[c][0] = f2_add(su, s);
+      P[c][2] = f2_sub(su, s);
+      P[c][1] = f2_add(du, d);
+      P[c][3] = f2_sub(du, d);
+    }
+  };
+  // sums of the last element plane that wait for the rows below and the lanes to the left
+  float e_a[3], g_a[3], e_b[3], g_b[3];  // (those of plane z0 - 1 are not used)
+  const bool top = tr == (wy - 1) / 2, odd = !FULL && (wy & 1) != 0;
+  const long long per_c = G.ntiles * (long long)G.tz;
+  auto node_sums = [&](int k) {
+    const float(*r)[kF2Threads] = sm.r[k & 1];
+    const unsigned o = 4u * (own + nxy * (unsigned)k);
+    const long long hb = tile * G.tz + (k - z0);
+    float ea[3], ga[3], rb[6], na[3], nb[3];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) rb[i] = tr > 0 ? r[i][tid - TILE_X] : 0.f;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      ea[c] = e_a[c] + rb[c];
+      ga[c] = g_a[c] + rb[3 + c];
+      const float gl = __shfl_up_sync(0xffffffffu, ga[c], 1), hl = __shfl_up_sync(0xffffffffu, g_b[c], 1);
+      na[c] = tx > 0 ? ea[c] + gl : ea[c];
+      nb[c] = tx > 0 ? e_b[c] + hl : e_b[c];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (act_a) *at_byte(A.y + E3D_IDX(c * ns, 3 * ns), o) = na[c];
+      if (act_b) *at_byte(A.y + E3D_IDX(c * ns, 3 * ns), o + 4u * nx) = nb[c];
+    }
+    if (tx == wx - 1) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        float* hx = A.hx + E3D_IDX((c * per_c + hb) * TILE_Y + ya, 3 * per_c * TILE_Y);
+        if (act_a) hx[0] = ga[c];
+        if (act_b) hx[1] = g_b[c];
+      }
+    }
+    if (top) {  // warp-uniform: the row past the tile, element b's rows above or, of an odd tile, b's own
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float gt = odd ? g_b[c] : r[3 + c][tid], et = odd ? e_b[c] : r[c][tid];
+        const float gtl = __shfl_up_sync(0xffffffffu, gt, 1);
+        if (tx < wx) A.hy[E3D_IDX((c * per_c + hb) * TILE_X + tx, 3 * per_c * TILE_X)] = tx > 0 ? et + gtl : et;
+        if (tx == wx - 1) A.hd[E3D_IDX(c * per_c + hb, 3 * per_c)] = gt;
+      }
+    }
+  };
+
+  f2 w1 = 0, w2 = 0, w3 = 0;  // element energies by Hadamard order
+  load(z0 - 1);
+  commit(z0 - 1, sm.node[0]);
+  load(z0);
+  commit(z0, sm.node[1]);
+  load(z0 + 1);
+  tile_sync<GROUPED>();
+  {
+    f2 P[3][4];
+    plane_transform(sm.node[0], P);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) sm.pold[4 * c + b][tid] = P[c][b];
+  }
+  int b0 = 0;  // buffer of plane k
+  const int32_t* pix = A.pix;
+  auto phase = [&](int z, int& pa, int& pb) {
+    const unsigned m = own + nxy * (unsigned)wrapi(z, G.nz);
+    pa = act_a ? __ldcs(pix + E3D_IDX(m, ns)) : 0;
+    pb = act_b ? __ldcs(pix + E3D_IDX(m + nx, ns)) : 0;
+  };
+  int pa, pb;
+  phase(z0 - 1, pa, pb);
+  for (int k = z0 - 1; k < zend; ++k) {
+    const int b1 = b0 == 2 ? 0 : b0 + 1, b2 = b1 == 2 ? 0 : b1 + 1;  // of planes k + 1 and k + 2
+    float4 qa[6], qb[6];
+    {
+      const float4* ra = reinterpret_cast<const float4*>(A.cs + E3D_IDX(pa, A.ncs) * kCs32Stride);
+      const float4* rb = reinterpret_cast<const float4*>(A.cs + E3D_IDX(pb, A.ncs) * kCs32Stride);
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        qa[i] = __ldg(ra + i);
+        qb[i] = __ldg(rb + i);
+      }
+    }
+    if (k + 2 <= zend) commit(k + 2, sm.node[b2]);
+    if (k + 3 <= zend) load(k + 3);
+    int na = 0, nb = 0;
+    if (k + 1 < zend) phase(k + 1, na, nb);
+    if (k > z0) node_sums(k - 1);
+    {
+      f2 h[3][8];
+      {
+        f2 Pn[3][4], Po[3][4];
+#pragma unroll
+        for (int i = 0; i < 12; ++i) Po[i / 4][i % 4] = sm.pold[i][tid];
+        plane_transform(sm.node[b1], Pn);
+#pragma unroll
+        for (int i = 0; i < 12; ++i) sm.pold[i][tid] = Pn[i / 4][i % 4];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            h[c][b] = f2_add(Pn[c][b], Po[c][b]);
+            h[c][b + 4] = f2_sub(Pn[c][b], Po[c][b]);
+          }
+      }
+      f2 t[21];
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        t[4 * i] = f2_pack(qa[i].x, qb[i].x);
+        if (i < 5) {
+          t[4 * i + 1] = f2_pack(qa[i].y, qb[i].y);
+          t[4 * i + 2] = f2_pack(qa[i].z, qb[i].z);
+          t[4 * i + 3] = f2_pack(qa[i].w, qb[i].w);
+        }
+      }
+      f2 f[3][8];
+      element_modal_f2(t, h, f, w1, w2, w3);
+      if (k < z0) w1 = w2 = w3 = 0;  // the redundant plane below the tile: its elements are another tile's
+      f2 cy[12];
+#pragma unroll
+      for (int i = 0; i < 12; ++i) cy[i] = sm.carry[i][tid];
+      float top_r[6];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        f2 lo[4];
+        lo[0] = f2_sub(cy[4 * c], f[c][4]);
+#pragma unroll
+        for (int b = 1; b < 4; ++b) lo[b] = f2_add(f2_sub(f[c][b], f[c][b + 4]), cy[4 * c + b]);
+        const f2 p0 = f2_sub(lo[0], lo[2]), p1 = f2_add(lo[0], lo[2]);
+        const f2 q0 = f2_sub(lo[1], lo[3]), q1 = f2_add(lo[1], lo[3]);
+        const f2 r0 = f2_sub(p0, q0), r1 = f2_add(p0, q0), r2 = f2_sub(p1, q1), r3 = f2_add(p1, q1);
+        e_a[c] = f2_lo(r0);
+        g_a[c] = f2_lo(r1);
+        e_b[c] = act_b ? f2_hi(r0) + f2_lo(r2) : f2_lo(r2);
+        g_b[c] = act_b ? f2_hi(r1) + f2_lo(r3) : f2_lo(r3);
+        top_r[c] = act_b ? f2_hi(r2) : 0.f;
+        top_r[3 + c] = act_b ? f2_hi(r3) : 0.f;
+        cy[4 * c] = f[c][4];
+#pragma unroll
+        for (int b = 1; b < 4; ++b) cy[4 * c + b] = f2_add(f[c][b], f[c][b + 4]);
+      }
+#pragma unroll
+      for (int i = 0; i < 12; ++i) sm.carry[i][tid] = cy[i];
+#pragma unroll
+      for (int i = 0; i < 6; ++i) sm.r[k & 1][i][tid] = top_r[i];
+    }
+    tile_sync<GROUPED>();
+    pa = na;
+    pb = nb;
+    b0 = b1;
+  }
+  node_sums(zend - 1);
+  const float ea = f2_lo(w1) + 3.f * f2_lo(w2) + 9.f * f2_lo(w3), eb = f2_hi(w1) + 3.f * f2_hi(w2) + 9.f * f2_hi(w3);
+  if (act_a) hAh += (double)ea;
+  if (act_b) hAh += (double)eb;
+}
+
+// ---------------------------------------------------------------------------
 // FP64 tile in fixed point (e3d_fixed.cuh).
 
 // Rows of a fixed-point tile, and blocks per SM.  What bounds the tile is the
@@ -791,9 +1117,24 @@ struct FxSmem {
   double raw[FUSED ? 6 : 3][kFxThreads + kHalo];
 };
 
+__device__ __forceinline__ double fx_max(double a, double b) { return b <= a ? a : b; }  // keeps a NaN in b
 __device__ __forceinline__ unsigned abs_hi(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
 
 constexpr int kFxGeneral = 0x7fffffff;
+
+// Exponent kx with 2^kx * b < 2^kFxNodeBits (b >= 0), or kFxGeneral where that
+// leaves the range of exponent arithmetic.
+__device__ __forceinline__ int fx_exponent_below(double b) {
+  if (b == 0.0) return 0;
+  const int e = __double2hiint(b) >> 20;  // b < 2^(e - 1022)
+  if (e < 1023 - 400 || e > 1023 + 400) return kFxGeneral;
+  return kFxNodeBits - (e - 1022);
+}
+// The same for values whose high words are at most hi.
+__device__ __forceinline__ int fx_exponent(unsigned hi) {
+  if (hi >= 0x7ff00000u) return kFxGeneral;
+  return fx_exponent_below(hi ? __hiloint2double((int)hi + 1, 0) : 0.0);
+}
 
 // Exponent kx of a tile: 2^kx * |value| < 2^kFxNodeBits for every node that the
 // tile reads (its own and the surrounding tiles' maxima; for h_new = z + gamma
@@ -829,13 +1170,10 @@ static __device__ __forceinline__ int fx_tile_exponent(const GridDims& G, long l
     bx = max(bx, red[i]);
     bz = max(bz, red[kFxRows + i]);
   }
+  if (!mz) return fx_exponent(bx);
   if (bx >= 0x7ff00000u || bz >= 0x7ff00000u) return kFxGeneral;
   const double vx = bx ? __hiloint2double((int)bx + 1, 0) : 0.0, vz = bz ? __hiloint2double((int)bz + 1, 0) : 0.0;
-  const double b = mz ? fma(fabs(gamma), vx, vz) : vx;
-  if (b == 0.0) return 0;
-  const int e = __double2hiint(b) >> 20;  // b < 2^(e - 1022)
-  if (e < 1023 - 400 || e > 1023 + 400) return kFxGeneral;
-  return kFxNodeBits - (e - 1022);
+  return fx_exponent_below(fma(fabs(gamma), vx, vz));
 }
 
 // apply_tile<double, FUSED> with the element products in fixed point: the same
@@ -845,12 +1183,12 @@ static __device__ __forceinline__ int fx_tile_exponent(const GridDims& G, long l
 // that its warps need not be in the same phase.  Loads are in flight one plane
 // ahead without holding registers.  FP64 is left with the direction update, the
 // conversions of K x and the dot product.
-template <bool FUSED>
+template <bool FUSED, bool GROUPED = false>
 static __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& A, const FxArgs& F, int kx, long long tile,
                                                      FxSmem<FUSED>& sm, double& hAh) {
   constexpr int TILE_Y = kFxRows, NT = kFxThreads;
   const GridDims& G = A.g;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x % kFxThreads;
   const int tx = tid % TILE_X, ty = tid / TILE_X;
   const int tix = (int)(tile % G.ntx);
   const int tiy = (int)((tile / G.ntx) % G.nty);
@@ -1007,7 +1345,7 @@ static __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& A,
   const int nb1 = next(nb);
   convert(z0, nb1, true);
   commit(nb1);
-  __syncthreads();
+  tile_sync<GROUPED>();
   if (active) plane_transform(nb, Pold);
   prefetch(z0 + 1);
   int b0 = nb;  // buffer of plane k
@@ -1064,14 +1402,14 @@ static __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& A,
       }
     }
     if (more) commit(b2);
-    __syncthreads();
+    tile_sync<GROUPED>();
     ph_cur = ph_nxt;
     b0 = b1;
   }
   const int kl = z0 + wz - 1;
   node_sums(kl, b0 == 0 ? 2 : b0 - 1);
   if (wz > 1 && edge_share(kl + 1) < kFlush) edge_flush(kl - 1, edge_share(kl + 1));
-  __syncthreads();
+  tile_sync<GROUPED>();
   if (edge_share(kl + 2) < kFlush) edge_flush(kl, edge_share(kl + 2));
   if (FUSED) {
     hmax = __reduce_max_sync(0xffffffffu, hmax);
@@ -1583,7 +1921,6 @@ static __constant__ int kRefToCorner[8] = {0, 1, 3, 2, 4, 5, 7, 6};
 
 // Norms of a phase (fx_phase_norms) from its element matrix in shared memory,
 // one warp.
-__device__ __forceinline__ double fx_max(double a, double b) { return b <= a ? a : b; }  // keeps a NaN in b
 static __device__ __forceinline__ void fx_store_norms(const double (&col)[24][24], const double* csh, double* out) {
   const int lane = threadIdx.x;
   double d = 0.0, rows = 0.0, entry = 0.0;
@@ -2263,6 +2600,222 @@ __device__ __forceinline__ double pcg_update_tiles_async(const GridDims& G, long
   }
   cp_async_wait<0>();
   return zg_t;
+}
+
+// ---------------------------------------------------------------------------
+// Phase B of the FP32 pass for 128-thread blocks, V consecutive nodes of a row a
+// thread (V = 4 or 2 where nx is a multiple of it, which aligns every row): g -=
+// lam Ah (+ halos), z = Minv g, share of z.g; du -= lam h too when UPD_U.  Loads
+// are in flight through cp.async stages of V * 4 bytes a field that the loading
+// thread alone reads back; S stages of them, about 51 KB a block for every V.  A quarter
+// of the load, store and address instructions of the one-node form.
+template <int N>
+__device__ __forceinline__ void cp_async_v(float* dst, const float* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if constexpr (N == 4)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+  else if constexpr (N == 2)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
+}
+template <int V>
+struct alignas(4 * V) FloatV {
+  float v[V];
+};
+
+template <int V, bool UPD_U>
+__host__ __device__ constexpr int pv_fields() {
+  return UPD_U ? 18 : 12;
+}
+// halo slots of a step: hy[3][planes][32], hx[3][rows], hd[3][planes]
+template <int V>
+__host__ __device__ constexpr int pv_planes() {
+  return V == 4 ? 2 : 1;
+}
+template <int V>
+__host__ __device__ constexpr int pv_halo() {
+  return 3 * (pv_planes<V>() * TILE_X + 4 * V + pv_planes<V>());
+}
+template <int V, bool UPD_U>
+__host__ __device__ constexpr int pv_stage() {  // floats, a multiple of 4
+  return pv_fields<V, UPD_U>() * kF2Threads * V + (pv_halo<V>() + 3) / 4 * 4;
+}
+template <bool UPD_U>
+__host__ __device__ constexpr int pv_bytes() {
+  // 8 / V stages (UPD_U: 4 / V, at least 2)
+  const int a = (UPD_U ? 4 : 8) * pv_stage<1, UPD_U>(), b = (UPD_U ? 2 : 4) * pv_stage<2, UPD_U>(),
+            c = 2 * pv_stage<4, UPD_U>();
+  return 4 * (a > b ? (a > c ? a : c) : (b > c ? b : c));
+}
+
+template <int V, bool UPD_U>
+__device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long long first, long long stride, float lam,
+                                                     const float* __restrict__ hc, const float* __restrict__ Ah,
+                                                     const float* __restrict__ hx, const float* __restrict__ hy,
+                                                     const float* __restrict__ hd, const float* __restrict__ minv,
+                                                     float* __restrict__ u, float* __restrict__ g,
+                                                     float* __restrict__ z, float* __restrict__ stages, int tid) {
+  constexpr int S = UPD_U ? (V == 4 ? 2 : 4 / V) : 8 / V;  // power of two
+  constexpr int F = pv_fields<V, UPD_U>(), SL = pv_stage<V, UPD_U>(), PL = pv_planes<V>(), R = 4 * V;
+  constexpr int kLanes = TILE_X / V;  // threads of a row
+  using Vec = FloatV<V>;
+  const unsigned ns = (unsigned)G.ns, nx = (unsigned)G.nx, nxy = nx * (unsigned)G.ny;
+  const int rs = tid / kLanes, tx = (tid % kLanes) * V;  // row slot of the step, first column
+  const long long per_c = G.ntiles * (long long)G.tz;
+  double zg_t = 0.0;
+  for (long long t = first; t < G.ntiles; t += stride) {
+    const int tix = (int)(t % G.ntx);
+    const int tiy = (int)((t / G.ntx) % G.nty);
+    const int tiz = (int)(t / ((long long)G.ntx * G.nty));
+    const int x0 = tix * TILE_X, y0 = tiy * TILE_Y, z0 = tiz * G.tz;
+    const int wx = min(TILE_X, G.nx - x0), wy = min(TILE_Y, G.ny - y0), wz = min(G.tz, G.nz - z0);
+    const int steps = (wz * TILE_Y + R - 1) / R;
+    const int txl = tix == 0 ? G.ntx - 1 : tix - 1;
+    const int tyd = tiy == 0 ? G.nty - 1 : tiy - 1;
+    const long long plane = (long long)tiz * G.nty;
+    const long long tX = (long long)txl + (long long)G.ntx * (tiy + plane);
+    const long long tY = (long long)tix + (long long)G.ntx * (tyd + plane);
+    const long long tD = (long long)txl + (long long)G.ntx * (tyd + plane);
+    // of step j: plane and row of this thread, and whether it has nodes
+    auto place = [&](int j, int& lz, int& row) {
+      const int s = j * R + rs;
+      lz = s / TILE_Y;
+      row = s % TILE_Y;
+      return tx < wx && row < wy && lz < wz;
+    };
+    const unsigned base = (unsigned)(x0 + tx) + nx * (unsigned)y0 + nxy * (unsigned)z0;
+    auto issue = [&](int j) {
+      int lz, row;
+      if (place(j, lz, row)) {
+        float* d = stages + (j & (S - 1)) * SL;
+        const unsigned m = base + nx * (unsigned)row + nxy * (unsigned)lz;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const unsigned i = (unsigned)E3D_IDX(m + c * ns, 3 * G.ns);
+          cp_async_v<V>(d + (c * kF2Threads + tid) * V, Ah + i);
+          cp_async_v<V>(d + ((3 + c) * kF2Threads + tid) * V, g + i);
+          if constexpr (UPD_U) {
+            cp_async_v<V>(d + ((12 + c) * kF2Threads + tid) * V, hc + i);
+            cp_async_v<V>(d + ((15 + c) * kF2Threads + tid) * V, u + i);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+          cp_async_v<V>(d + ((6 + q) * kF2Threads + tid) * V, minv + (unsigned long long)m + (unsigned long long)q * ns);
+        float* hs = d + F * kF2Threads * V;
+        const int pl = PL == 2 ? lz & 1 : 0;
+        if (row == 0) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            cp_async_v<V>(hs + (c * PL + pl) * TILE_X + tx,
+                          hy + E3D_IDX((c * per_c + tY * G.tz + lz) * TILE_X + tx, 3 * per_c * TILE_X));
+        }
+        if (tx == 0) {
+          float* hxs = hs + 3 * PL * TILE_X;
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            cp_async_4(hxs + c * R + rs, hx + E3D_IDX((c * per_c + tX * G.tz + lz) * TILE_Y + row, 3 * per_c * TILE_Y));
+          if (row == 0) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              cp_async_4(hxs + 3 * R + c * PL + pl, hd + E3D_IDX(c * per_c + tD * G.tz + lz, 3 * per_c));
+          }
+        }
+      }
+      cp_async_commit();
+    };
+#pragma unroll
+    for (int j = 0; j < S - 1; ++j) issue(j);
+    float zg32 = 0.f;  // this thread's z.g, added to the FP64 sum once per tile
+    for (int j = 0; j < steps; ++j) {
+      issue(j + S - 1);
+      cp_async_wait<S - 1>();  // step j has landed
+      int lz, row;
+      if (!place(j, lz, row)) continue;
+      const float* d = stages + (j & (S - 1)) * SL;
+      const float* hs = d + F * kF2Threads * V;
+      const int pl = PL == 2 ? lz & 1 : 0;
+      auto field = [&](int q) { return *reinterpret_cast<const Vec*>(d + (q * kF2Threads + tid) * V); };
+      Vec ah[3], gv[3], zv[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        ah[c] = field(c);
+        gv[c] = field(3 + c);
+      }
+      if (tx == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) ah[c].v[0] += hs[3 * PL * TILE_X + c * R + rs];
+      }
+      if (row == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const Vec a = *reinterpret_cast<const Vec*>(hs + (c * PL + pl) * TILE_X + tx);
+#pragma unroll
+          for (int i = 0; i < V; ++i) ah[c].v[i] += a.v[i];
+        }
+        if (tx == 0) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) ah[c].v[0] += hs[3 * PL * TILE_X + 3 * R + c * PL + pl];
+        }
+      }
+      const unsigned m = base + nx * (unsigned)row + nxy * (unsigned)lz;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) gv[c].v[i] -= lam * ah[c].v[i];
+        const unsigned o = (unsigned)E3D_IDX(m + c * ns, 3 * G.ns);
+        *reinterpret_cast<Vec*>(g + o) = gv[c];
+        if constexpr (UPD_U) {
+          const Vec hv = field(12 + c);
+          Vec uv = field(15 + c);
+#pragma unroll
+          for (int i = 0; i < V; ++i) uv.v[i] -= lam * hv.v[i];
+          *reinterpret_cast<Vec*>(u + o) = uv;
+        }
+      }
+      {
+        const Vec m00 = field(6), m11 = field(7), m22 = field(8), m01 = field(9), m02 = field(10), m12 = field(11);
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          const float a = gv[0].v[i], b = gv[1].v[i], c = gv[2].v[i];
+          zv[0].v[i] = m00.v[i] * a + m01.v[i] * b + m02.v[i] * c;
+          zv[1].v[i] = m01.v[i] * a + m11.v[i] * b + m12.v[i] * c;
+          zv[2].v[i] = m02.v[i] * a + m12.v[i] * b + m22.v[i] * c;
+          zg32 += zv[0].v[i] * a + zv[1].v[i] * b + zv[2].v[i] * c;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) *reinterpret_cast<Vec*>(z + (unsigned)E3D_IDX(m + c * ns, 3 * G.ns)) = zv[c];
+    }
+    zg_t += (double)zg32;
+    cp_async_wait<0>();
+  }
+  return zg_t;
+}
+
+// du -= lam h over the nodes that a thread owns in apply_tile_f2.
+static __device__ void flush_u_tiles_f2(const GridDims& G, long long first, long long stride, float lam,
+                                        const float* __restrict__ h, float* __restrict__ u, int tid) {
+  const unsigned ns = (unsigned)G.ns, nx = (unsigned)G.nx, nxy = nx * (unsigned)G.ny;
+  const int tx = tid % TILE_X, ya = 2 * (tid / TILE_X);
+  for (long long t = first; t < G.ntiles; t += stride) {
+    const int tix = (int)(t % G.ntx);
+    const int tiy = (int)((t / G.ntx) % G.nty);
+    const int tiz = (int)(t / ((long long)G.ntx * G.nty));
+    const int x0 = tix * TILE_X, y0 = tiy * TILE_Y, z0 = tiz * G.tz;
+    const int wx = min(TILE_X, G.nx - x0), wy = min(TILE_Y, G.ny - y0), wz = min(G.tz, G.nz - z0);
+    if (tx >= wx) continue;
+    for (int row = ya; row < min(wy, ya + 2); ++row)
+      for (int lz = 0; lz < wz; ++lz) {
+        const unsigned m = (unsigned)(x0 + tx) + nx * (unsigned)(y0 + row) + nxy * (unsigned)(z0 + lz);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const unsigned i = (unsigned)E3D_IDX(m + c * ns, 3 * G.ns);
+          u[i] = u[i] - lam * __ldcg(h + i);
+        }
+      }
+  }
 }
 
 // u -= lam h over the owned nodes of tiles first, first + stride, ... (the same

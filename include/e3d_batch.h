@@ -42,7 +42,7 @@ typedef struct e3d_batch_opts {
   int32_t divergence_reset; /* 1: h = z when rel_res grows > 10x                 */
   float tol;                /* single precision, as the reference's tol          */
   int32_t load_cases;       /* bitmask of the six unit load cases (0 = all six)  */
-  int32_t parts;            /* blocks per solve (<= 64): 0 = autotune            */
+  int32_t parts;            /* blocks per solve (<= 152): 0 = autotune           */
   int32_t pad;
   double strain;            /* magnitude of the unit load cases (1e-3)           */
   double e1, nu1;           /* inclusion phase modulus / Poisson ratio           */
@@ -54,7 +54,7 @@ typedef struct e3d_job_result {
   int32_t status;           /* E3D_EXIT_* of e3d_gpu.h                           */
   int32_t iterations, refinements, resets;
   int32_t parts;             /* blocks that ran the solve                         */
-  int32_t tile_z;            /* element planes per tile (autotuned tile shape)    */
+  int32_t tile_z;            /* element planes per tile                           */
   double utot0, utot;       /* initial / final energy                            */
   double rel_res, true_rel; /* criterion value and |g|/|g0| at exit              */
   double strav[6], epsav[6];
@@ -67,8 +67,8 @@ void e3d_batch_opts_defaults(e3d_batch_opts_t* o);
 
 /* Uploads the RVEs, builds every phase table (femat element part) and
  * block-Jacobi inverse, allocates all solve state (within hbm_budget), picks
- * the blocks per solve and the tile shape (autotuner when opts->parts == 0) and captures the
- * solve into a CUDA graph. */
+ * the blocks per solve (timed, when opts->parts == 0) and captures the solve
+ * into a CUDA graph. */
 int32_t e3d_batch_create(e3d_batch_t** b, const e3d_rve_t* rves, int32_t n, const e3d_batch_opts_t* opts);
 
 /* Runs every solve (one graph launch: one persistent kernel).  ceff receives
