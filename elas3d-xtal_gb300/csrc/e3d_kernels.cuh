@@ -759,13 +759,17 @@ __device__ __forceinline__ void cp_async_t(T* dst, const T* src) {
 // threads; thread (tx, tr) has rows 2 tr and 2 tr + 1.
 constexpr int kF2Threads = TILE_X * TILE_Y / 2;
 
+// Planes in flight: with one, half of the stalls were waits for it (sixty solves of
+// 32^3 to 88^3: 0.64 s; with two 0.60, with three the same).
+constexpr int kF2Depth = 2;
+
 struct F2Smem {
   float node[3][3][(TILE_Y + 1) * (TILE_X + 1)];  // plane k in one of three, rows of TILE_X + 1
   float r[2][6][kF2Threads];                      // forces to the row above, by plane parity
   // a thread's own slots: one plane's values in flight (z, h_old, du; rows a and
   // b; then the halo node's z and h_old), and what it carries up the column
-  float raw[18][kF2Threads];
-  float raw_halo[6][kF2Threads];
+  float raw[kF2Depth][18][kF2Threads];
+  float raw_halo[kF2Depth][6][kF2Threads];
   f2 carry[12][kF2Threads];
   f2 pold[12][kF2Threads];
 };
@@ -832,6 +836,8 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
   // raw slot of field f (z 0, h_old 1, du 2), component c, row q
   auto slot = [](int f, int c, int q) { return 6 * f + 2 * c + q; };
   auto load = [&](int zl) {
+    const int d = (zl - z0 + 1) % kF2Depth;
+    if (zl <= zend) {
     const unsigned zo = nxy * (unsigned)wrapi(zl, G.nz);
     const bool mine = DEFER_U && zl >= z0 && zl < zend, need_x = !reset || mine;
 #pragma unroll
@@ -839,26 +845,28 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
       if (q ? act_b : act_a) {
         const unsigned o = 4u * (unsigned)E3D_IDX(own + (q ? nx : 0u) + zo, ns);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[slot(0, c, q)][tid], at_byte(A.zv + c * ns, o));
+        for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[d][slot(0, c, q)][tid], at_byte(A.zv + c * ns, o));
         if (need_x)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[slot(1, c, q)][tid], at_byte(A.x + c * ns, o));
+          for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[d][slot(1, c, q)][tid], at_byte(A.x + c * ns, o));
         if (mine)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[slot(2, c, q)][tid], at_byte(A.du + c * ns, o));
+          for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[d][slot(2, c, q)][tid], at_byte(A.du + c * ns, o));
       }
     if (tid < nhalo) {
       const unsigned o = 4u * (unsigned)E3D_IDX(halo + zo, ns);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw_halo[c][tid], at_byte(A.zv + c * ns, o));
+      for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw_halo[d][c][tid], at_byte(A.zv + c * ns, o));
       if (!reset)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw_halo[3 + c][tid], at_byte(A.x + c * ns, o));
+        for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw_halo[d][3 + c][tid], at_byte(A.x + c * ns, o));
+    }
     }
     cp_async_commit();
   };
   auto commit = [&](int zl, float (&buf)[3][(TILE_Y + 1) * kRow]) {
-    cp_async_wait<0>();
+    const int d = (zl - z0 + 1) % kF2Depth;
+    cp_async_wait<kF2Depth - 1>();
     const unsigned zo = nxy * (unsigned)zl;  // used on own planes only
     const bool mine = zl >= z0 && zl < zend;
     // every slot is read before anything is stored: a store in between would
@@ -866,16 +874,16 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
     float z[6], x[6], du[6], zh[3], xh[3];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-      z[i] = sm.raw[i][tid];
-      x[i] = sm.raw[6 + i][tid];
-      du[i] = DEFER_U ? sm.raw[12 + i][tid] : 0.f;
+      z[i] = sm.raw[d][i][tid];
+      x[i] = sm.raw[d][6 + i][tid];
+      du[i] = DEFER_U ? sm.raw[d][12 + i][tid] : 0.f;
     }
     const bool halo_thread = tid < nhalo;
     if (halo_thread) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        zh[c] = sm.raw_halo[c][tid];
-        xh[c] = sm.raw_halo[3 + c][tid];
+        zh[c] = sm.raw_halo[d][c][tid];
+        xh[c] = sm.raw_halo[d][3 + c][tid];
       }
     }
     float v[6];
@@ -970,11 +978,12 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
   };
 
   f2 w1 = 0, w2 = 0, w3 = 0;  // element energies by Hadamard order
-  load(z0 - 1);
+#pragma unroll
+  for (int i = 0; i < kF2Depth; ++i) load(z0 - 1 + i);
   commit(z0 - 1, sm.node[0]);
-  load(z0);
+  load(z0 - 1 + kF2Depth);
   commit(z0, sm.node[1]);
-  load(z0 + 1);
+  load(z0 + kF2Depth);
   tile_sync<GROUPED>();
   {
     f2 P[3][4];
@@ -1006,7 +1015,7 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
       }
     }
     if (k + 2 <= zend) commit(k + 2, sm.node[b2]);
-    if (k + 3 <= zend) load(k + 3);
+    load(k + 2 + kF2Depth);
     int na = 0, nb = 0;
     if (k + 1 < zend) phase(k + 1, na, nb);
     if (k > z0) node_sums(k - 1);
