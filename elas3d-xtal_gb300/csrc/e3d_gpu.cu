@@ -227,6 +227,38 @@ int32_t reduce_to_host(e3d_handle* h, int n, int stride, int nfields, double* ou
   return sync(h);
 }
 
+// One form of the persistent kernel, with its launch shape.
+struct PcgForm {
+  const void* fn;
+  int threads, smem;
+};
+
+template <typename T, bool FX, int V>
+PcgForm pcg_form_of() {
+  return {(const void*)pcg_persistent_kernel<T, false, FX, V>, FX ? kFxThreads : NT, pcg_dyn_smem_bytes<T, FX, V>()};
+}
+
+// The form for a solve: phase B takes two nodes of a row at a time where every row
+// starts at an even node (FP32 iteration at 200^3 .389 ms, one node .414; FP64 300^3
+// 4.52, 4.60), else one.
+template <typename T>
+PcgForm pcg_form(const e3d_handle* h, bool fx) {
+  const int nx = h->prob.nx;
+  if constexpr (sizeof(T) == 4) {
+    return nx % 2 == 0 ? pcg_form_of<T, false, 2>() : pcg_form_of<T, false, 1>();
+  } else {
+    if (!fx) return pcg_form_of<T, false, 1>();
+    return nx % 2 == 0 ? pcg_form_of<T, true, 2>() : pcg_form_of<T, true, 1>();
+  }
+}
+
+PcgForm pcg_ring_form() { return {(const void*)pcg_persistent_kernel<float, true, false, 1>, NT, kRingSmemBytes}; }
+
+cudaError_t pcg_blocks_per_sm(const PcgForm& f, int* per_sm) {
+  const cudaError_t e = cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smem);
+  return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, f.fn, f.threads, f.smem);
+}
+
 ApplyArgs<double> apply_args(e3d_handle* h, const double* x, double* y) {
   ApplyArgs<double> A{};
   A.g = h->G;
@@ -378,41 +410,21 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
   const long long ns = h->G.ns, n3 = 3 * ns;
   const int np = p->nphase;
   // PCG grid: as many co-resident tile blocks as the device holds.
-  // (phase B of the per-thread-load kernels streams through dynamic shared memory)
-  int per_sm = 0;
-  if ((e = cudaFuncSetAttribute(pcg_persistent_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                pcg_dyn_smem_bytes<double>())) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_persistent_kernel<double>, NT,
-                                                         pcg_dyn_smem_bytes<double>())) != cudaSuccess)
+  if ((e = cudaFuncSetAttribute(apply_tiles_fx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(FxSmem<false>))) != cudaSuccess)
     return fail(cuda_fail(e, "occupancy"));
-  int per_sm_fx = 0;
-  if ((e = cudaFuncSetAttribute(pcg_persistent_kernel<double, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                pcg_dyn_smem_bytes<double, true>())) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(apply_tiles_fx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(FxSmem<false>))) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_fx, pcg_persistent_kernel<double, false, true>,
-                                                         kFxThreads,
-                                                         pcg_dyn_smem_bytes<double, true>())) != cudaSuccess)
-    return fail(cuda_fail(e, "occupancy"));
-  if (per_sm < 1 || per_sm_fx < 1) return fail(E3D_ERR_CUDA);
-  h->pcg_grid = per_sm * h->num_sms;
-  h->pcg_grid_fx = per_sm_fx * h->num_sms;
-  int per_sm32 = 0;
-  if ((e = cudaFuncSetAttribute(pcg_persistent_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                pcg_dyn_smem_bytes<float>())) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm32, pcg_persistent_kernel<float>, NT,
-                                                         pcg_dyn_smem_bytes<float>())) != cudaSuccess)
-    return fail(cuda_fail(e, "occupancy"));
-  if (per_sm32 < 1) return fail(E3D_ERR_CUDA);
-  h->pcg_grid32 = per_sm32 * h->num_sms;
-  int per_sm_tma = 0;
-  if (p->precision == E3D_PREC_MIXED) {
-    if ((e = cudaFuncSetAttribute(pcg_persistent_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kRingSmemBytes)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tma, pcg_persistent_kernel<float, true>, NT,
-                                                           kRingSmemBytes)) != cudaSuccess)
-      return fail(cuda_fail(e, "occupancy (TMA)"));
+  for (auto [form, grid] : {std::pair{pcg_form<double>(h, false), &h->pcg_grid},
+                            std::pair{pcg_form<double>(h, true), &h->pcg_grid_fx},
+                            std::pair{pcg_form<float>(h, false), &h->pcg_grid32}}) {
+    int per_sm = 0;
+    if ((e = pcg_blocks_per_sm(form, &per_sm)) != cudaSuccess) return fail(cuda_fail(e, "occupancy"));
+    if (per_sm < 1) return fail(E3D_ERR_CUDA);
+    *grid = per_sm * h->num_sms;
   }
+  int per_sm_tma = 0;
+  if (p->precision == E3D_PREC_MIXED &&
+      (e = pcg_blocks_per_sm(pcg_ring_form(), &per_sm_tma)) != cudaSuccess)
+    return fail(cuda_fail(e, "occupancy (TMA)"));
   h->partial_n = std::max({h->pcg_grid, h->pcg_grid_fx, h->pcg_grid32, h->num_sms * 4}) * 12;
   const long long halo = h->G.ntiles * h->G.tz, halo_x = h->Gx.ntiles * h->Gx.tz;
   const size_t tile_rows = (size_t)h->Gx.ntiles * kFxRows;
@@ -787,16 +799,10 @@ int32_t launch_pcg(e3d_handle* h, int it_limit) {
   E3D_CUDA(cudaMemsetAsync(h->bar, 0, sizeof(GridBarrier), h->stream));
   if (fx) E3D_CUDA(cudaMemsetAsync(h->fxleave, 0, sizeof(int), h->stream));
   void* args[] = {&P};
-  const void* fn = tma ? (const void*)pcg_persistent_kernel<float, true>
-                   : fx ? (const void*)pcg_persistent_kernel<double, false, true>
-                                                : (const void*)pcg_persistent_kernel<T>;
+  const PcgForm F = tma ? pcg_ring_form() : pcg_form<T>(h, fx);
   if constexpr (sizeof(T) == 8)
     if (fx) P.A.g = h->Gx;
-  cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(fx ? kFxThreads : NT), args,
-                                              tma  ? kRingSmemBytes
-                                              : fx ? pcg_dyn_smem_bytes<double, true>()
-                                                   : pcg_dyn_smem_bytes<T>(),
-                                              h->stream);
+  cudaError_t e = cudaLaunchCooperativeKernel(F.fn, dim3(grid), dim3(F.threads), args, F.smem, h->stream);
   h->launches++;
   if (e != cudaSuccess) return cuda_fail(e, "cudaLaunchCooperativeKernel(pcg)");
   return E3D_OK;

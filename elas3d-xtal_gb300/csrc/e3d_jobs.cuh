@@ -463,32 +463,36 @@ static __device__ __noinline__ double job_fp32_apply(const JobDesc& J, int part,
   return hAh;
 }
 
+// Stages of the update at four nodes a thread (more at one or two), and their bytes.
+constexpr int kJobPvStages = 2;
+constexpr int kJobPvBytes = pv_bytes<float, kF2Threads, TILE_Y, 4, kJobPvStages, false>();
+
 // g -= lam Ah, z = Minv g (du waits for the next sweep): returns this thread's
 // share of z.g.  Nodes a thread takes at a time: what the rows' alignment allows.
 static __device__ __noinline__ double job_fp32_update(const JobDesc& J, int part, float lam, unsigned char* dyn) {
   const int group = threadIdx.x / kF2Threads, tid = threadIdx.x % kF2Threads;
-  float* stages = reinterpret_cast<float*>(dyn + group * pv_bytes<false>());
+  float* stages = reinterpret_cast<float*>(dyn + group * kJobPvBytes);
   const float *hx = reinterpret_cast<const float*>(J.hx), *hy = reinterpret_cast<const float*>(J.hy),
               *hd = reinterpret_cast<const float*>(J.hd);
   const long long first = (long long)part * kGroups + group, stride = (long long)J.nparts * kGroups;
-  if (J.G.nx % 4 == 0)
-    return pcg_update_tiles_v<4, false>(J.G, first, stride, lam, nullptr, J.Ah, hx, hy, hd, J.minv32, J.du, J.g32, J.z32,
-                                        stages, tid);
-  if (J.G.nx % 2 == 0)
-    return pcg_update_tiles_v<2, false>(J.G, first, stride, lam, nullptr, J.Ah, hx, hy, hd, J.minv32, J.du, J.g32, J.z32,
-                                        stages, tid);
-  return pcg_update_tiles_v<1, false>(J.G, first, stride, lam, nullptr, J.Ah, hx, hy, hd, J.minv32, J.du, J.g32, J.z32,
-                                      stages, tid);
+  auto update = [&](auto v) {
+    constexpr int V = decltype(v)::value;
+    return pcg_update_tiles_v<float, kF2Threads, TILE_Y, V, 4 * kJobPvStages / V, false, false>(
+        J.G, first, stride, lam, nullptr, J.Ah, hx, hy, hd, J.minv32, J.du, J.g32, J.z32, stages, tid, nullptr);
+  };
+  if (J.G.nx % 4 == 0) return update(std::integral_constant<int, 4>{});
+  if (J.G.nx % 2 == 0) return update(std::integral_constant<int, 2>{});
+  return update(std::integral_constant<int, 1>{});
 }
 
 // Shared memory of a part: the sweeps take it in turn.
 constexpr int kEngineDynSmem = [] {
   int b = kGroups * (int)sizeof(F2Smem);
-  for (int c : {kGroups * (int)sizeof(FxSmem<false>), kGroups * pv_bytes<false>(), (int)sizeof(ApplySmem<double>)})
+  for (int c : {kGroups * (int)sizeof(FxSmem<false>), kGroups * kJobPvBytes, (int)sizeof(ApplySmem<double>)})
     b = c > b ? c : b;
   return b;
 }();
-static_assert(sizeof(F2Smem) % 8 == 0 && pv_bytes<false>() % 16 == 0 && sizeof(FxSmem<false>) % 8 == 0,
+static_assert(sizeof(F2Smem) % 8 == 0 && kJobPvBytes % 16 == 0 && sizeof(FxSmem<false>) % 8 == 0,
               "the groups' parts stay aligned");
 
 // u += du, du = 0; the part's largest |u| (high word) to its slot, for the

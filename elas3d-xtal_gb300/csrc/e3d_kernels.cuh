@@ -24,12 +24,6 @@ constexpr int TILE_X = 32;
 constexpr int TILE_Y = 8;
 
 // Tuning knobs of the persistent PCG kernel (set at build time).
-#ifndef E3D_PB_UNROLL_F32
-#define E3D_PB_UNROLL_F32 1  // phase-B nodes in flight per thread, FP32 form (2 spills under the 128-register cap)
-#endif
-#ifndef E3D_PB_UNROLL_F64
-#define E3D_PB_UNROLL_F64 1  // phase-B nodes in flight per thread, FP64 form
-#endif
 #ifndef E3D_F32_BLOCKS_PER_SM
 #define E3D_F32_BLOCKS_PER_SM 2  // resident 256-thread blocks per SM, FP32 form
 #endif
@@ -56,30 +50,6 @@ constexpr int TILE_Y = 8;
 #ifndef E3D_F32_CARRY_SMEM
 #define E3D_F32_CARRY_SMEM 0
 #endif
-// FP32 persistent kernel (per-thread loads): the correction update du -= lam*h
-// of iteration k is applied in phase A of iteration k+1, which loads h there
-// anyway, so phase B reads neither h nor du; the update still pending when the
-// launch ends is applied before it returns.
-#ifndef E3D_F32_DEFER_U
-#define E3D_F32_DEFER_U 1
-#endif
-// Phase-B planes in flight per thread through cp.async stages (a power of two;
-// 0 keeps the one-node register form of pcg_update_tiles).
-#ifndef E3D_PB_ASYNC_F32
-#define E3D_PB_ASYNC_F32 4
-#endif
-#ifndef E3D_PB_ASYNC_F64
-#define E3D_PB_ASYNC_F64 2
-#endif
-// FP32 stencil: each element's stiffness row staged in shared memory one plane
-// ahead through cp.async (per-thread-load persistent kernel).  Measured slower:
-// 500^3 inner iteration 8.41 ms against 5.68 ms with the rows read through the
-// read-only path, where a warp whose elements share a grain gets its row in
-// one broadcast access.
-#ifndef E3D_F32_TAB_ASYNC
-#define E3D_F32_TAB_ASYNC 0
-#endif
-constexpr int kTabAsyncBytes = 2 * 6 * 256 * 16;  // two slots of six float4 per thread (NT = 256)
 // FP64 stencil: node sums share the adjoint butterflies between neighbouring
 // elements (9 instead of 11 additions per component and node).
 #ifndef E3D_F64_SHARED_ADJ
@@ -362,17 +332,11 @@ __device__ __forceinline__ void ring_drain(PlaneRing& R) {
 // h_new is stored for the tile's own nodes.  Returns this thread's share of
 // h_new . (K h_new) through hAh.
 //
-// TAB_ASYNC (FP32): each element's stiffness row is copied into a per-thread
-// shared-memory slot one plane ahead (cp.async, two slots alternating by plane
-// parity in `tab`, 2 x 6 x NT float4), so the gather's latency is off the
-// element's critical path.
 // TY: rows of a tile (and warps of a block).
 template <typename T, bool FUSED, bool POLD_SMEM = (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), bool DEFER_U = false,
-          bool TAB_ASYNC = false, int TY = TILE_Y>
-__device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, TY>& sm, double& hAh,
-                           float4* __restrict__ tab = nullptr) {
+          int TY = TILE_Y>
+__device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, TY>& sm, double& hAh) {
   constexpr int TILE_Y = TY, NT = TILE_X * TY;
-  static_assert(!TAB_ASYNC || sizeof(T) == 4, "the staged table rows are the FP32 ones");
   const GridDims& G = A.g;
   const int tid = threadIdx.x;
   const int tx = tid % TILE_X, ty = tid / TILE_X;
@@ -505,43 +469,14 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
   }
   prefetch(z0);
   int ph_cur = active ? __ldcs(A.pix + E3D_IDX(ecol + nxy * wrapi(z0 - 1, G.nz), ns)) : 0;
-  // TAB_ASYNC: the row of element k sits in slot k & 1; ph_cur then holds the
-  // phase of element k + 1 (its row is copied during step k)
-  auto tab_issue = [&](int k, int ph) {
-    if constexpr (TAB_ASYNC) {
-      if (active) {
-        float4* d = tab + (k & 1) * 6 * NT + tid;
-        const float* src = reinterpret_cast<const float*>(A.cs) + E3D_IDX(ph, A.ncs) * kCs32Stride;
-#pragma unroll
-        for (int i = 0; i < 6; ++i)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(
-                           (unsigned)__cvta_generic_to_shared(d + i * NT)),
-                       "l"(src + 4 * i)
-                       : "memory");
-      }
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-  };
-  if constexpr (TAB_ASYNC) {
-    tab_issue(z0 - 1, ph_cur);
-    ph_cur = (active && z0 < z0 + wz) ? __ldcs(A.pix + E3D_IDX(ecol + nxy * wrapi(z0, G.nz), ns)) : 0;
-  }
   const int htiles_stride = G.tz;  // per-tile plane stride in halo buffers
   for (int k = z0 - 1; k < z0 + wz; ++k) {
     const bool own_next = (k + 1 >= z0) && (k + 1 < z0 + wz);
     commit(k + 1, own_next);
     __syncthreads();
     if (k + 2 <= z0 + wz) prefetch(k + 2);
-    int ph_nxt;
-    if constexpr (TAB_ASYNC) {
-      // row of element k + 1 now, phase of element k + 2 for the next step
-      if (k + 1 < z0 + wz) tab_issue(k + 1, ph_cur);
-      else asm volatile("cp.async.commit_group;\n" ::: "memory");
-      ph_nxt = (active && k + 2 < z0 + wz) ? __ldcs(A.pix + E3D_IDX(ecol + nxy * wrapi(k + 2, G.nz), ns)) : 0;
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // element k's row has landed
-    } else {
-      ph_nxt = (active && k + 1 < z0 + wz) ? __ldcs(A.pix + E3D_IDX(ecol + nxy * wrapi(k + 1, G.nz), ns)) : 0;
-    }
+    const int ph_nxt =
+        (active && k + 1 < z0 + wz) ? __ldcs(A.pix + E3D_IDX(ecol + nxy * wrapi(k + 1, G.nz), ns)) : 0;
     T rr[3][4];
     if (active) {
       T nxt[3][4];
@@ -564,10 +499,7 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
         }
       }
       T f[3][8];
-      if constexpr (TAB_ASYNC)
-        element_modal_f32<NT>(reinterpret_cast<const float*>(tab + (k & 1) * 6 * NT + tid), h[0], h[1], h[2], f[0],
-                              f[1], f[2]);
-      else if constexpr (sizeof(T) == 4)
+      if constexpr (sizeof(T) == 4)
         element_modal_f32(A.cs + E3D_IDX(ph_cur, A.ncs) * kCs32Stride, h[0], h[1], h[2], f[0], f[1], f[2]);
       else
         element_modal<T>(A.cs + E3D_IDX(ph_cur, A.ncs) * kCsStride, h[0], h[1], h[2], f[0], f[1], f[2]);
@@ -729,7 +661,6 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
     }
     ph_cur = ph_nxt;
   }
-  if constexpr (TAB_ASYNC) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   if constexpr (sizeof(T) == 4) hAh += (double)dot32;
 }
 
@@ -745,13 +676,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-template <typename T>
-__device__ __forceinline__ void cp_async_t(T* dst, const T* src) {
-  if constexpr (sizeof(T) == 4)
-    cp_async_4(dst, src);
-  else
-    cp_async_8(dst, src);
 }
 
 // ---------------------------------------------------------------------------
@@ -1432,7 +1356,7 @@ static __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& A,
 static __device__ __noinline__ void apply_tile_general(const ApplyArgs<double>& A, long long tile,
                                                        ApplySmem<double, kFxRows>& sm) {
   double dot = 0.0;
-  apply_tile<double, false, false, false, false, kFxRows>(A, tile, sm, dot);
+  apply_tile<double, false, false, false, kFxRows>(A, tile, sm, dot);
 }
 
 // Shared memory of apply_tile_ring: the in-plane force exchange of the ZS
@@ -2379,14 +2303,10 @@ static __global__ void stress_field_kernel(GridDims G, JumpParams J, const int32
   }
 }
 
-// Phase B of a PCG iteration over tiles first, first + stride, ... < ntiles,
-// node loop in tile order (no index division), U nodes of a column per thread
-// in flight (the defaults keep one: more spill under the register cap):
-// u -= lam h (unless UPD_U is false: the FP32 persistent kernel applies it in
-// the next phase A), g -= lam Ah (+ tile-edge halos), z = Minv g
-// (src/elas3dxtal_pcg.f90:1913-1932, symmetric Minv); returns this thread's
-// share of z.g (FP32: summed per tile column in FP32, then in FP64).
-template <typename T, int U = (sizeof(T) == 4 ? E3D_PB_UNROLL_F32 : E3D_PB_UNROLL_F64), bool UPD_U = true>
+// Phase B of the ring-fed kernel, whose shared memory the ring fills: as
+// pcg_update_tiles_v below, with U nodes of a column per thread in registers
+// (src/elas3dxtal_pcg.f90:1913-1932, symmetric Minv).
+template <typename T, int U>
 __device__ __forceinline__ double pcg_update_tiles(const GridDims& G, long long first, long long stride, T lam,
                                                    const T* __restrict__ hc, const T* __restrict__ Ah,
                                                    const T* __restrict__ hx, const T* __restrict__ hy,
@@ -2414,10 +2334,8 @@ __device__ __forceinline__ double pcg_update_tiles(const GridDims& G, long long 
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             ah[j][c] = __ldcg(Ah + m + c * ns);
-            if constexpr (UPD_U) {
-              hv[j][c] = __ldcg(hc + m + c * ns);
-              uv[j][c] = u[m + c * ns];
-            }
+            hv[j][c] = __ldcg(hc + m + c * ns);
+            uv[j][c] = u[m + c * ns];
             gv[j][c] = g[m + c * ns];
           }
 #pragma unroll
@@ -2431,7 +2349,7 @@ __device__ __forceinline__ double pcg_update_tiles(const GridDims& G, long long 
           halo_add_tile<T>(G, hx, hy, hd, tix, tiy, tiz, tx, ty, lz0 + j, ah[j]);
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            if constexpr (UPD_U) u[m + c * ns] = uv[j][c] - lam * hv[j][c];
+            u[m + c * ns] = uv[j][c] - lam * hv[j][c];
             gv[j][c] = gv[j][c] - lam * ah[j][c];
             g[m + c * ns] = gv[j][c];
           }
@@ -2454,232 +2372,87 @@ __device__ __forceinline__ double pcg_update_tiles(const GridDims& G, long long 
 }
 
 // ---------------------------------------------------------------------------
-// Phase B with its loads in flight through cp.async.  pcg_update_tiles keeps
-// one node's loads in registers at a time (the register cap set by the stencil
-// leaves nothing for more), so each thread waits a full memory latency per
-// node.  Here every thread streams its node column through S shared-memory
-// stages: the loads of plane lz + S - 1 are issued (cp.async, no registers held)
-// before plane lz is consumed, so S planes' worth of bytes stay in flight per
-// thread.  Each thread reads back only the slots it filled itself, so no block
-// barrier is needed: cp.async.wait_group orders a thread's own copies.  The
-// tile-edge halos (hx for lane 0 of each row, hy for row 0, hd for the corner
-// node) travel in the same stages.  Same additions in the same order as
-// pcg_update_tiles: the results are bitwise the same.
-// Values of one stage: per thread Ah 3, g 3, Minv 6 (and h 3, u 3 when u is
-// updated here), then the halo slots hx[3][TILE_Y], hy[3][TILE_X], hd[3].
-template <bool UPD_U>
-__host__ __device__ constexpr int pb_fields() {
-  return UPD_U ? 18 : 12;
-}
-template <bool UPD_U, int TY = TILE_Y>
-__host__ __device__ constexpr int pb_stage_len() {
-  return pb_fields<UPD_U>() * TILE_X * TY + 3 * TY + 3 * TILE_X + 3;
-}
-template <typename T, int S, bool UPD_U, int TY = TILE_Y>
-__host__ __device__ constexpr int pb_async_bytes() {
-  return S * pb_stage_len<UPD_U, TY>() * (int)sizeof(T);
-}
-
-// ZMAX: the tile maxima of the new z go to mz (the next pass's fixed-point scale).
-template <typename T, int S, bool UPD_U = true, bool ZMAX = false, int TY = TILE_Y>
-__device__ __forceinline__ double pcg_update_tiles_async(const GridDims& G, long long first, long long stride, T lam,
-                                                         const T* __restrict__ hc, const T* __restrict__ Ah,
-                                                         const T* __restrict__ hx, const T* __restrict__ hy,
-                                                         const T* __restrict__ hd, const T* __restrict__ minv,
-                                                         T* __restrict__ u, T* __restrict__ g, T* __restrict__ z,
-                                                         T* __restrict__ stages, unsigned* __restrict__ mz = nullptr) {
-  static_assert(S >= 2 && (S & (S - 1)) == 0, "stage count: a power of two");
-  constexpr int TILE_Y = TY, NT = TILE_X * TY;
-  constexpr int F = pb_fields<UPD_U>();
-  constexpr int SL = pb_stage_len<UPD_U, TY>();
-  const long long ns = G.ns;
-  double zg_t = 0.0;
-  const int tid = threadIdx.x;
-  const int tx = tid % TILE_X, ty = tid / TILE_X;
-  const long long nxy = (long long)G.nx * G.ny;
-  const long long per_c = G.ntiles * G.tz;
-  for (long long t = first; t < G.ntiles; t += stride) {
-    const int tix = (int)(t % G.ntx);
-    const int tiy = (int)((t / G.ntx) % G.nty);
-    const int tiz = (int)(t / ((long long)G.ntx * G.nty));
-    const int x0 = tix * TILE_X, y0 = tiy * TILE_Y, z0 = tiz * G.tz;
-    const int wx = min(TILE_X, G.nx - x0), wy = min(TILE_Y, G.ny - y0), wz = min(G.tz, G.nz - z0);
-    if (tx >= wx || ty >= wy) continue;
-    const long long col = (long long)(x0 + tx) + (long long)G.nx * (y0 + ty);
-    // halo sources (the tiles at -x, -y and -x-y), as in halo_add_tile
-    const bool hxn = tx == 0, hyn = ty == 0;
-    const int txl = tix == 0 ? G.ntx - 1 : tix - 1;
-    const int tyd = tiy == 0 ? G.nty - 1 : tiy - 1;
-    const long long plane = (long long)tiz * G.nty;
-    const long long tX = (long long)txl + (long long)G.ntx * (tiy + plane);
-    const long long tY = (long long)tix + (long long)G.ntx * (tyd + plane);
-    const long long tD = (long long)txl + (long long)G.ntx * (tyd + plane);
-    auto issue = [&](int lz) {
-      T* d = stages + (lz & (S - 1)) * SL;
-      const long long m = E3D_IDX(col + nxy * (z0 + lz), ns);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        cp_async_t<T>(d + c * NT + tid, Ah + m + c * ns);
-        cp_async_t<T>(d + (3 + c) * NT + tid, g + m + c * ns);
-      }
-#pragma unroll
-      for (int q = 0; q < 6; ++q) cp_async_t<T>(d + (6 + q) * NT + tid, minv + m + q * ns);
-      if constexpr (UPD_U) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          cp_async_t<T>(d + (12 + c) * NT + tid, hc + m + c * ns);
-          cp_async_t<T>(d + (15 + c) * NT + tid, u + m + c * ns);
-        }
-      }
-      T* hs = d + F * NT;
-      if (hxn) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          cp_async_t<T>(hs + c * TILE_Y + ty, hx + E3D_IDX((c * per_c + tX * G.tz + lz) * TILE_Y + ty, 3 * per_c * TILE_Y));
-      }
-      if (hyn) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          cp_async_t<T>(hs + 3 * TILE_Y + c * TILE_X + tx,
-                        hy + E3D_IDX((c * per_c + tY * G.tz + lz) * TILE_X + tx, 3 * per_c * TILE_X));
-      }
-      if (hxn && hyn) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          cp_async_t<T>(hs + 3 * TILE_Y + 3 * TILE_X + c, hd + E3D_IDX(c * per_c + tD * G.tz + lz, 3 * per_c));
-      }
-    };
-#pragma unroll
-    for (int j = 0; j < S - 1; ++j) {
-      if (j < wz) issue(j);
-      cp_async_commit();
-    }
-    float zg32 = 0.f;  // FP32: this column's z.g, added to the FP64 sum once per tile
-    unsigned zmax = 0;
-    for (int lz = 0; lz < wz; ++lz) {
-      if (lz + S - 1 < wz) issue(lz + S - 1);
-      cp_async_commit();
-      cp_async_wait<S - 1>();  // plane lz has landed
-      const T* d = stages + (lz & (S - 1)) * SL;
-      const T* hs = d + F * NT;
-      T ah[3], gv[3], mi[6];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        ah[c] = d[c * NT + tid];
-        gv[c] = d[(3 + c) * NT + tid];
-      }
-#pragma unroll
-      for (int q = 0; q < 6; ++q) mi[q] = d[(6 + q) * NT + tid];
-      if (hxn) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) ah[c] += hs[c * TILE_Y + ty];
-      }
-      if (hyn) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) ah[c] += hs[3 * TILE_Y + c * TILE_X + tx];
-      }
-      if (hxn && hyn) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) ah[c] += hs[3 * TILE_Y + 3 * TILE_X + c];
-      }
-      const long long m = E3D_IDX(col + nxy * (z0 + lz), ns);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        if constexpr (UPD_U) u[m + c * ns] = d[(15 + c) * NT + tid] - lam * d[(12 + c) * NT + tid];
-        gv[c] = gv[c] - lam * ah[c];
-        g[m + c * ns] = gv[c];
-      }
-      const T z0v = mi[0] * gv[0] + mi[3] * gv[1] + mi[4] * gv[2];
-      const T z1v = mi[3] * gv[0] + mi[1] * gv[1] + mi[5] * gv[2];
-      const T z2v = mi[4] * gv[0] + mi[5] * gv[1] + mi[2] * gv[2];
-      z[m] = z0v;
-      z[m + ns] = z1v;
-      z[m + 2 * ns] = z2v;
-      if constexpr (ZMAX) zmax = max(zmax, max(abs_hi(z0v), max(abs_hi(z1v), abs_hi(z2v))));
-      if constexpr (sizeof(T) == 4)
-        zg32 += z0v * gv[0] + z1v * gv[1] + z2v * gv[2];
-      else
-        zg_t += (double)(z0v * gv[0] + z1v * gv[1] + z2v * gv[2]);
-    }
-    if constexpr (ZMAX) {  // the row's lanes 0 .. wx-1 are here; rows past the grid keep their zero
-      zmax = __reduce_max_sync(wx == TILE_X ? 0xffffffffu : (1u << wx) - 1u, zmax);
-      if (tx == 0) mz[E3D_IDX(t * TY + ty, G.ntiles * TY)] = zmax;
-    }
-    if constexpr (sizeof(T) == 4) zg_t += (double)zg32;
-  }
-  cp_async_wait<0>();
-  return zg_t;
-}
-
-// ---------------------------------------------------------------------------
-// Phase B of the FP32 pass for 128-thread blocks, V consecutive nodes of a row a
-// thread (V = 4 or 2 where nx is a multiple of it, which aligns every row): g -=
-// lam Ah (+ halos), z = Minv g, share of z.g; du -= lam h too when UPD_U.  Loads
-// are in flight through cp.async stages of V * 4 bytes a field that the loading
-// thread alone reads back; S stages of them, about 51 KB a block for every V.  A quarter
-// of the load, store and address instructions of the one-node form.
-template <int N>
-__device__ __forceinline__ void cp_async_v(float* dst, const float* src) {
+// Phase B of a PCG iteration over tiles first, first + stride, ...: g -= lam Ah
+// (+ tile-edge halos), z = Minv g, u -= lam h too with UPD_U (else the next phase A
+// does it); returns this thread's share of z.g (FP32: summed per thread and tile in
+// FP32, then in FP64).  Bound by HBM in FP32, by the FP64 pipe as much in FP64.
+// NTH threads share a tile, V consecutive nodes of a row each, NTH * V / 32 rows a
+// step.  V = 4, 2 or 1 by the rows' alignment: a quarter or half of the load,
+// store and address instructions of the one-node form.  Loads are in flight
+// through S cp.async stages that the loading thread alone reads back, so that no
+// barrier is needed and they hold no registers.  Iteration with two nodes a thread
+// instead of one (four stages): FP32 500^3 6.00 -> 5.72 ms, 200^3 .414 -> .389, 100^3
+// .0757 -> .0716; FP64 300^3 4.63 -> 4.52.  Four nodes a thread: 500^3 6.29.  The
+// grid's warps side by side along memory instead of tile by tile: 8.0.
+// ZMAX: the tile's maxima of the new z, one a warp, go to mz (the next pass's
+// fixed-point scale).
+template <int BYTES>
+__device__ __forceinline__ void cp_async_n(void* dst, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (N == 4)
+  if constexpr (BYTES == 16)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-  else if constexpr (N == 2)
+  else if constexpr (BYTES == 8)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
-template <int V>
-struct alignas(4 * V) FloatV {
-  float v[V];
+template <typename T, int V>
+struct alignas(sizeof(T) * V) VecOf {
+  T v[V];
 };
 
-template <int V, bool UPD_U>
-__host__ __device__ constexpr int pv_fields() {
-  return UPD_U ? 18 : 12;
+// Values of one stage: per thread Ah 3, g 3, Minv 6 (and h 3, u 3 with UPD_U), V
+// each, then the halo slots of the step's rows and planes: hy[3][planes][32],
+// hx[3][rows], hd[3][planes].
+template <int NTH, int V>
+__host__ __device__ constexpr int pv_rows() {
+  return NTH * V / TILE_X;
 }
-// halo slots of a step: hy[3][planes][32], hx[3][rows], hd[3][planes]
-template <int V>
+template <int NTH, int TY, int V>
 __host__ __device__ constexpr int pv_planes() {
-  return V == 4 ? 2 : 1;
+  return pv_rows<NTH, V>() > TY ? pv_rows<NTH, V>() / TY : 1;
 }
-template <int V>
-__host__ __device__ constexpr int pv_halo() {
-  return 3 * (pv_planes<V>() * TILE_X + 4 * V + pv_planes<V>());
+template <typename T, int NTH, int TY, int V, bool UPD_U>
+__host__ __device__ constexpr int pv_stage() {  // a multiple of 16 bytes
+  const int halo = 3 * (pv_planes<NTH, TY, V>() * (TILE_X + 1) + pv_rows<NTH, V>()), a = 16 / (int)sizeof(T);
+  return (UPD_U ? 18 : 12) * NTH * V + (halo + a - 1) / a * a;
 }
-template <int V, bool UPD_U>
-__host__ __device__ constexpr int pv_stage() {  // floats, a multiple of 4
-  return pv_fields<V, UPD_U>() * kF2Threads * V + (pv_halo<V>() + 3) / 4 * 4;
-}
-template <bool UPD_U>
+// Bytes of S * VMAX / V stages, for every V up to VMAX.
+template <typename T, int NTH, int TY, int VMAX, int S, bool UPD_U>
 __host__ __device__ constexpr int pv_bytes() {
-  // 8 / V stages (UPD_U: 4 / V, at least 2)
-  const int a = (UPD_U ? 4 : 8) * pv_stage<1, UPD_U>(), b = (UPD_U ? 2 : 4) * pv_stage<2, UPD_U>(),
-            c = 2 * pv_stage<4, UPD_U>();
-  return 4 * (a > b ? (a > c ? a : c) : (b > c ? b : c));
+  int b = 0;
+  for (int c : {VMAX * S * pv_stage<T, NTH, TY, 1, UPD_U>(), VMAX / 2 * S * pv_stage<T, NTH, TY, 2, UPD_U>(),
+                VMAX == 4 ? S * pv_stage<T, NTH, TY, 4, UPD_U>() : 0})
+    b = b > c ? b : c;
+  return b * (int)sizeof(T);
 }
 
-template <int V, bool UPD_U>
-__device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long long first, long long stride, float lam,
-                                                     const float* __restrict__ hc, const float* __restrict__ Ah,
-                                                     const float* __restrict__ hx, const float* __restrict__ hy,
-                                                     const float* __restrict__ hd, const float* __restrict__ minv,
-                                                     float* __restrict__ u, float* __restrict__ g,
-                                                     float* __restrict__ z, float* __restrict__ stages, int tid) {
-  constexpr int S = UPD_U ? (V == 4 ? 2 : 4 / V) : 8 / V;  // power of two
-  constexpr int F = pv_fields<V, UPD_U>(), SL = pv_stage<V, UPD_U>(), PL = pv_planes<V>(), R = 4 * V;
+template <typename T, int NTH, int TY, int V, int S, bool UPD_U, bool ZMAX>
+__device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long long first, long long stride, T lam,
+                                                     const T* __restrict__ hc, const T* __restrict__ Ah,
+                                                     const T* __restrict__ hx, const T* __restrict__ hy,
+                                                     const T* __restrict__ hd, const T* __restrict__ minv,
+                                                     T* __restrict__ u, T* __restrict__ g, T* __restrict__ z,
+                                                     T* __restrict__ stages, int tid, unsigned* __restrict__ mz) {
+  static_assert((S & (S - 1)) == 0, "stage count: a power of two");
+  constexpr int F = UPD_U ? 18 : 12, SL = pv_stage<T, NTH, TY, V, UPD_U>(), R = pv_rows<NTH, V>(),
+                PL = pv_planes<NTH, TY, V>();
+  static_assert(R % TY == 0 || TY % R == 0, "whole planes a step, or whole steps a plane");
+  constexpr int B = V * (int)sizeof(T);
   constexpr int kLanes = TILE_X / V;  // threads of a row
-  using Vec = FloatV<V>;
+  using Vec = VecOf<T, V>;
   const unsigned ns = (unsigned)G.ns, nx = (unsigned)G.nx, nxy = nx * (unsigned)G.ny;
   const int rs = tid / kLanes, tx = (tid % kLanes) * V;  // row slot of the step, first column
+  const int pl = rs / TY;                                // plane of the step
   const long long per_c = G.ntiles * (long long)G.tz;
   double zg_t = 0.0;
   for (long long t = first; t < G.ntiles; t += stride) {
     const int tix = (int)(t % G.ntx);
     const int tiy = (int)((t / G.ntx) % G.nty);
     const int tiz = (int)(t / ((long long)G.ntx * G.nty));
-    const int x0 = tix * TILE_X, y0 = tiy * TILE_Y, z0 = tiz * G.tz;
-    const int wx = min(TILE_X, G.nx - x0), wy = min(TILE_Y, G.ny - y0), wz = min(G.tz, G.nz - z0);
-    const int steps = (wz * TILE_Y + R - 1) / R;
+    const int x0 = tix * TILE_X, y0 = tiy * TY, z0 = tiz * G.tz;
+    const int wx = min(TILE_X, G.nx - x0), wy = min(TY, G.ny - y0), wz = min(G.tz, G.nz - z0);
+    const int steps = (wz * TY + R - 1) / R;
     const int txl = tix == 0 ? G.ntx - 1 : tix - 1;
     const int tyd = tiy == 0 ? G.nty - 1 : tiy - 1;
     const long long plane = (long long)tiz * G.nty;
@@ -2688,47 +2461,46 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
     const long long tD = (long long)txl + (long long)G.ntx * (tyd + plane);
     // of step j: plane and row of this thread, and whether it has nodes
     auto place = [&](int j, int& lz, int& row) {
-      const int s = j * R + rs;
-      lz = s / TILE_Y;
-      row = s % TILE_Y;
+      lz = (j * R + rs) / TY;
+      row = R % TY == 0 ? rs % TY : (j * R + rs) % TY;
       return tx < wx && row < wy && lz < wz;
     };
     const unsigned base = (unsigned)(x0 + tx) + nx * (unsigned)y0 + nxy * (unsigned)z0;
     auto issue = [&](int j) {
       int lz, row;
       if (place(j, lz, row)) {
-        float* d = stages + (j & (S - 1)) * SL;
+        T* d = stages + (j & (S - 1)) * SL;
         const unsigned m = base + nx * (unsigned)row + nxy * (unsigned)lz;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           const unsigned i = (unsigned)E3D_IDX(m + c * ns, 3 * G.ns);
-          cp_async_v<V>(d + (c * kF2Threads + tid) * V, Ah + i);
-          cp_async_v<V>(d + ((3 + c) * kF2Threads + tid) * V, g + i);
+          cp_async_n<B>(d + (c * NTH + tid) * V, Ah + i);
+          cp_async_n<B>(d + ((3 + c) * NTH + tid) * V, g + i);
           if constexpr (UPD_U) {
-            cp_async_v<V>(d + ((12 + c) * kF2Threads + tid) * V, hc + i);
-            cp_async_v<V>(d + ((15 + c) * kF2Threads + tid) * V, u + i);
+            cp_async_n<B>(d + ((12 + c) * NTH + tid) * V, hc + i);
+            cp_async_n<B>(d + ((15 + c) * NTH + tid) * V, u + i);
           }
         }
 #pragma unroll
         for (int q = 0; q < 6; ++q)
-          cp_async_v<V>(d + ((6 + q) * kF2Threads + tid) * V, minv + (unsigned long long)m + (unsigned long long)q * ns);
-        float* hs = d + F * kF2Threads * V;
-        const int pl = PL == 2 ? lz & 1 : 0;
+          cp_async_n<B>(d + ((6 + q) * NTH + tid) * V, minv + (unsigned long long)m + (unsigned long long)q * ns);
+        T* hs = d + F * NTH * V;
         if (row == 0) {
 #pragma unroll
           for (int c = 0; c < 3; ++c)
-            cp_async_v<V>(hs + (c * PL + pl) * TILE_X + tx,
+            cp_async_n<B>(hs + (c * PL + pl) * TILE_X + tx,
                           hy + E3D_IDX((c * per_c + tY * G.tz + lz) * TILE_X + tx, 3 * per_c * TILE_X));
         }
         if (tx == 0) {
-          float* hxs = hs + 3 * PL * TILE_X;
+          T* hxs = hs + 3 * PL * TILE_X;
 #pragma unroll
           for (int c = 0; c < 3; ++c)
-            cp_async_4(hxs + c * R + rs, hx + E3D_IDX((c * per_c + tX * G.tz + lz) * TILE_Y + row, 3 * per_c * TILE_Y));
+            cp_async_n<sizeof(T)>(hxs + c * R + rs,
+                                  hx + E3D_IDX((c * per_c + tX * G.tz + lz) * TY + row, 3 * per_c * TY));
           if (row == 0) {
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-              cp_async_4(hxs + 3 * R + c * PL + pl, hd + E3D_IDX(c * per_c + tD * G.tz + lz, 3 * per_c));
+              cp_async_n<sizeof(T)>(hxs + 3 * R + c * PL + pl, hd + E3D_IDX(c * per_c + tD * G.tz + lz, 3 * per_c));
           }
         }
       }
@@ -2736,22 +2508,27 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
     };
 #pragma unroll
     for (int j = 0; j < S - 1; ++j) issue(j);
-    float zg32 = 0.f;  // this thread's z.g, added to the FP64 sum once per tile
+    float zg32 = 0.f;  // FP32: this thread's z.g, added to the FP64 sum once per tile
+    unsigned zmax = 0;
     for (int j = 0; j < steps; ++j) {
       issue(j + S - 1);
       cp_async_wait<S - 1>();  // step j has landed
       int lz, row;
       if (!place(j, lz, row)) continue;
-      const float* d = stages + (j & (S - 1)) * SL;
-      const float* hs = d + F * kF2Threads * V;
-      const int pl = PL == 2 ? lz & 1 : 0;
-      auto field = [&](int q) { return *reinterpret_cast<const Vec*>(d + (q * kF2Threads + tid) * V); };
-      Vec ah[3], gv[3], zv[3];
+      const T* d = stages + (j & (S - 1)) * SL;
+      const T* hs = d + F * NTH * V;
+      auto field = [&](int q) { return *reinterpret_cast<const Vec*>(d + (q * NTH + tid) * V); };
+      Vec ah[3], gv[3], zv[3], uv[3], hv[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         ah[c] = field(c);
         gv[c] = field(3 + c);
+        if constexpr (UPD_U) {
+          hv[c] = field(12 + c);
+          uv[c] = field(15 + c);
+        }
       }
+      const Vec m00 = field(6), m11 = field(7), m22 = field(8), m01 = field(9), m02 = field(10), m12 = field(11);
       if (tx == 0) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) ah[c].v[0] += hs[3 * PL * TILE_X + c * R + rs];
@@ -2776,28 +2553,33 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
         const unsigned o = (unsigned)E3D_IDX(m + c * ns, 3 * G.ns);
         *reinterpret_cast<Vec*>(g + o) = gv[c];
         if constexpr (UPD_U) {
-          const Vec hv = field(12 + c);
-          Vec uv = field(15 + c);
 #pragma unroll
-          for (int i = 0; i < V; ++i) uv.v[i] -= lam * hv.v[i];
-          *reinterpret_cast<Vec*>(u + o) = uv;
+          for (int i = 0; i < V; ++i) uv[c].v[i] -= lam * hv[c].v[i];
+          *reinterpret_cast<Vec*>(u + o) = uv[c];
         }
       }
-      {
-        const Vec m00 = field(6), m11 = field(7), m22 = field(8), m01 = field(9), m02 = field(10), m12 = field(11);
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-          const float a = gv[0].v[i], b = gv[1].v[i], c = gv[2].v[i];
-          zv[0].v[i] = m00.v[i] * a + m01.v[i] * b + m02.v[i] * c;
-          zv[1].v[i] = m01.v[i] * a + m11.v[i] * b + m12.v[i] * c;
-          zv[2].v[i] = m02.v[i] * a + m12.v[i] * b + m22.v[i] * c;
-          zg32 += zv[0].v[i] * a + zv[1].v[i] * b + zv[2].v[i] * c;
-        }
+      for (int i = 0; i < V; ++i) {
+        const T a = gv[0].v[i], b = gv[1].v[i], c = gv[2].v[i];
+        zv[0].v[i] = m00.v[i] * a + m01.v[i] * b + m02.v[i] * c;
+        zv[1].v[i] = m01.v[i] * a + m11.v[i] * b + m12.v[i] * c;
+        zv[2].v[i] = m02.v[i] * a + m12.v[i] * b + m22.v[i] * c;
+        const T zg = zv[0].v[i] * a + zv[1].v[i] * b + zv[2].v[i] * c;
+        if constexpr (sizeof(T) == 4)
+          zg32 += zg;
+        else
+          zg_t += zg;
+        if constexpr (ZMAX)
+          zmax = max(zmax, max(abs_hi(zv[0].v[i]), max(abs_hi(zv[1].v[i]), abs_hi(zv[2].v[i]))));
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) *reinterpret_cast<Vec*>(z + (unsigned)E3D_IDX(m + c * ns, 3 * G.ns)) = zv[c];
     }
-    zg_t += (double)zg32;
+    if constexpr (ZMAX) {
+      zmax = __reduce_max_sync(0xffffffffu, zmax);
+      if ((tid & 31) == 0) mz[E3D_IDX(t * (NTH / 32) + tid / 32, G.ntiles * (NTH / 32))] = zmax;
+    }
+    if constexpr (sizeof(T) == 4) zg_t += (double)zg32;
     cp_async_wait<0>();
   }
   return zg_t;
@@ -2927,17 +2709,17 @@ static __device__ double reduce_broadcast(const double* partial, int n, double* 
   return s_val;
 }
 
-// Dynamic shared memory of the per-thread-load persistent kernel: the phase-B
-// cp.async stages (0 when phase B keeps its loads in registers).
-template <typename T, bool FX = false>
+// Phase B's stages in the per-thread-load persistent kernels.  More take L1 from
+// phase A's loads: 500^3 FP32 iteration 5.72 ms with two, 8.0 with four at V = 4.
+constexpr int kPbStages = 2;
+
+// Dynamic shared memory of those kernels: phase B's stages, and in the same bytes
+// the fixed-point FP64 tile of phase A.
+template <typename T, bool FX, int V>
 constexpr int pcg_dyn_smem_bytes() {
-  constexpr bool defer_u = sizeof(T) == 4 && E3D_F32_DEFER_U != 0;
-  constexpr int S = sizeof(T) == 4 ? E3D_PB_ASYNC_F32 : E3D_PB_ASYNC_F64;
-  constexpr int pb = S > 0 ? pb_async_bytes<T, (S > 0 ? S : 2), !defer_u, FX ? kFxRows : TILE_Y>() : 0;
-  // phase A's staged table rows use the same bytes (the phases never overlap)
-  // (staged table rows, or the fixed-point FP64 tile)
-  constexpr int tab = FX ? (int)sizeof(FxSmem<true>) : sizeof(T) == 4 && E3D_F32_TAB_ASYNC != 0 ? kTabAsyncBytes : 0;
-  return pb > tab ? pb : tab;
+  constexpr int b = kPbStages * (int)sizeof(T) *
+                    pv_stage<T, FX ? kFxThreads : NT, FX ? kFxRows : TILE_Y, V, sizeof(T) == 8>();
+  return FX && b < (int)sizeof(FxSmem<true>) ? (int)sizeof(FxSmem<true>) : b;
 }
 
 // T = double: the plain FP64 solve (u is the solution).  T = float: the inner
@@ -2974,8 +2756,9 @@ struct PcgArgs {
 
 // TMA (FP32 only): phase A reads its node planes through the block's plane
 // ring (dynamic shared memory of kRingSmemBytes).  FX (FP64 only): phase A in
-// fixed point, each tile scaled by its own values.
-template <typename T, bool TMA = false, bool FX = false>
+// fixed point, each tile scaled by its own values.  V: nodes of a row a thread
+// takes at a time in phase B, what the rows' alignment allows.
+template <typename T, bool TMA, bool FX, int V>
 __global__ void __launch_bounds__(FX ? kFxThreads : NT,
                                   FX               ? kFxBlocks
                                   : sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 ? 1 : E3D_F32_BLOCKS_PER_SM)
@@ -2983,7 +2766,7 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
     pcg_persistent_kernel(PcgArgs<T> P) {
   constexpr int TY = FX ? kFxRows : TILE_Y, NT = TILE_X * TY;
   static_assert(!TMA || sizeof(T) == 4, "the plane ring feeds the FP32 stencil");
-  static_assert(!FX || (sizeof(T) == 8 && E3D_PB_ASYNC_F64 > 0), "the fixed-point stencil is the FP64 one");
+  static_assert(!FX || sizeof(T) == 8, "the fixed-point stencil is the FP64 one");
   using Smem = std::conditional_t<TMA, RingApplySmem<E3D_RING_ZS>, std::conditional_t<FX, char, ApplySmem<T>>>;
   __shared__ Smem sm;
   __shared__ double red[NT / 32];
@@ -2991,18 +2774,8 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
   __shared__ uint64_t ring_bars[E3D_TMA_STAGES];
   __shared__ RingCursor ring_cur;
   PlaneRing ring;
-  // per-thread-load form: phase B streams through cp.async stages in the
-  // dynamic shared memory (pcg_update_tiles_async)
-  constexpr int kPbStages = TMA ? 0 : (sizeof(T) == 4 ? E3D_PB_ASYNC_F32 : E3D_PB_ASYNC_F64);
-  constexpr bool kTabAsync = sizeof(T) == 4 && !TMA && E3D_F32_TAB_ASYNC != 0;
-  T* pb_stages = nullptr;
-  float4* tab_slots = nullptr;
-  {
-    extern __shared__ __align__(128) unsigned char e3d_ring_smem[];
-    if constexpr (TMA) ring_setup(ring, e3d_ring_smem, ring_bars, &ring_cur, P.maps, P.err, P.timeout_ns);
-    if constexpr (kPbStages > 0) pb_stages = reinterpret_cast<T*>(e3d_ring_smem);
-    if constexpr (kTabAsync) tab_slots = reinterpret_cast<float4*>(e3d_ring_smem);
-  }
+  extern __shared__ __align__(128) unsigned char e3d_pcg_smem[];  // the plane ring, or what pcg_dyn_smem_bytes says
+  if constexpr (TMA) ring_setup(ring, e3d_pcg_smem, ring_bars, &ring_cur, P.maps, P.err, P.timeout_ns);
   // The PCG scalars live in shared memory: every thread reads them after a
   // barrier, thread 0 alone updates them (all blocks compute the same values
   // from the same partials), so they hold no registers during the sweeps.
@@ -3013,7 +2786,7 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
   const bool lead = threadIdx.x == 0;
   const GridDims& G = P.A.g;
   const int it_end = min(s.it + P.it_limit, s.max_iter);
-  constexpr bool kDeferU = sizeof(T) == 4 && !TMA && E3D_F32_DEFER_U != 0;
+  constexpr bool kDeferU = sizeof(T) == 4 && !TMA;
   T lam_pending = T(0);  // kDeferU: du -= lam_pending * h_pending not yet applied
   const T* h_pending = nullptr;
   __shared__ unsigned mred[2 * kFxRows];
@@ -3053,12 +2826,11 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
         const FxArgs F{P.fxtab, P.fxkc, cur ? P.mh0 : P.mh1, P.mz};
         const int kx = fx_tile_exponent(G, t, A.reset ? nullptr : cur ? P.mh1 : P.mh0, P.mz, A.gamma, mred);
         if (kx != kFxGeneral)
-          apply_tile_fx<true>(A, F, kx, t, *reinterpret_cast<FxSmem<true>*>(pb_stages), hAh_t);
+          apply_tile_fx<true>(A, F, kx, t, *reinterpret_cast<FxSmem<true>*>(e3d_pcg_smem), hAh_t);
         else if (lead)
           *P.fxleave = 1;
       } else {
-        apply_tile<T, true, (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), kDeferU, kTabAsync>(A, t, sm, hAh_t,
-                                                                                           tab_slots);
+        apply_tile<T, true, (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), kDeferU>(A, t, sm, hAh_t);
       }
       __syncthreads();
     }
@@ -3094,14 +2866,15 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
     // ---- phase B: u, g update, preconditioner, z.g -- node loop in tile order
     // (no index division); with kDeferU the u update waits for the next phase A.
     const T* hc = cur ? P.h0 : P.h1;  // the h_new of phase A
-    constexpr int U = TMA ? E3D_PB_UNROLL_RING : (sizeof(T) == 4 ? E3D_PB_UNROLL_F32 : E3D_PB_UNROLL_F64);
     double zg_t;
-    if constexpr (kPbStages > 0)
-      zg_t = pcg_update_tiles_async<T, kPbStages, !kDeferU, FX, TY>(G, blockIdx.x, gridDim.x, lam, hc, P.Ah, P.A.hx, P.A.hy,
-                                                                P.A.hd, P.minv, P.u, P.g, P.z, pb_stages, P.mz);
-    else
-      zg_t = pcg_update_tiles<T, U, !kDeferU>(G, blockIdx.x, gridDim.x, lam, hc, P.Ah, P.A.hx, P.A.hy, P.A.hd,
-                                              P.minv, P.u, P.g, P.z);
+    if constexpr (TMA) {
+      zg_t = pcg_update_tiles<T, E3D_PB_UNROLL_RING>(G, blockIdx.x, gridDim.x, lam, hc, P.Ah, P.A.hx, P.A.hy, P.A.hd,
+                                                     P.minv, P.u, P.g, P.z);
+    } else {
+      zg_t = pcg_update_tiles_v<T, NT, TY, V, kPbStages, !kDeferU, FX>(
+          G, blockIdx.x, gridDim.x, lam, hc, P.Ah, P.A.hx, P.A.hy, P.A.hd, P.minv, P.u, P.g, P.z,
+          reinterpret_cast<T*>(e3d_pcg_smem), threadIdx.x, P.mz);
+    }
     if constexpr (kDeferU) {
       lam_pending = lam;
       h_pending = hc;
