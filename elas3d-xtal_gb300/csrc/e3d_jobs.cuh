@@ -97,43 +97,13 @@ struct EngineArgs {
 constexpr int kGroups = NT / kF2Threads;
 static_assert(kGroups == 2 && kFxThreads == kF2Threads, "two groups a block");
 
-// Barrier among the k parts of one job (same protocol as grid_barrier).
-static __device__ bool job_barrier(GridBarrier* gb, unsigned int k, int* err, unsigned long long timeout_ns) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    volatile unsigned int* vgen = &gb->gen;
-    const unsigned int g0 = *vgen;
-    __threadfence();
-    const unsigned int prev = atomicAdd(&gb->count, 1u);
-    if (prev == k - 1) {
-      atomicExch(&gb->count, 0u);
-      __threadfence();
-      atomicAdd(&gb->gen, 1u);
-    } else {
-      const unsigned long long t0 = global_timer_ns();
-      unsigned long long spins = 0;
-      while (*vgen == g0) {
-        if (*(volatile int*)err != DEV_OK) {
-          ok = 0;
-          break;
-        }
-        __nanosleep(128);
-        if (((++spins) & 255ull) == 0ull) {
-          if (global_timer_ns() - t0 > timeout_ns || spins > (1ull << 34)) {
-            atomicExch(err, DEV_TIMEOUT);
-            ok = 0;
-            break;
-          }
-        }
-      }
-    }
-    __threadfence();
-    s_ok = ok;
+// Barrier among the parts of one job.
+static __device__ bool job_barrier(const JobDesc& J, int part, int* err, unsigned long long timeout_ns) {
+  if (J.nparts == 1) {
+    __syncthreads();
+    return true;
   }
-  __syncthreads();
-  return s_ok != 0;
+  return barrier_among(J.bar, J.nparts, part == 0, err, timeout_ns);
 }
 
 // Slots of the per-job partial array.
@@ -359,7 +329,7 @@ static __device__ __noinline__ bool job_fp64_apply_tiles(const JobDesc& J, int p
 static __device__ bool job_fp64_apply_u(const JobDesc& J, int part, unsigned char* dyn, bool& fx, int* err,
                                         unsigned long long to) {
   fx = job_fp64_apply_tiles(J, part, dyn);
-  return job_barrier(J.bar, J.nparts, err, to);
+  return job_barrier(J, part, err, to);
 }
 
 // After job_fp64_apply_u: g = Ku + b (+ halos), g32, z32 = Minv32 g32, partial z.g;
@@ -397,7 +367,7 @@ static __device__ __noinline__ bool job_true_residual(const JobDesc& J, int part
   job_put(J, SL_ZG, part, zg, red);
   job_put(J, SL_U, part, eu, red);
   job_put(J, SL_GG, part, gg, red);
-  return job_barrier(J.bar, J.nparts, err, to);
+  return job_barrier(J, part, err, to);
 }
 
 // The set-up's counterpart of job_true_residual: g already holds the whole
@@ -427,7 +397,7 @@ static __device__ __noinline__ bool job_start_residual(const JobDesc& J, int par
   job_put(J, SL_ZG, part, zg, red);
   job_put(J, SL_U, part, eu, red);
   job_put(J, SL_GG, part, gg, red);
-  return job_barrier(J.bar, J.nparts, err, to);
+  return job_barrier(J, part, err, to);
 }
 
 // One FP32 inner iteration's two sweeps, each kept out of line so that it gets
@@ -569,7 +539,7 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
       const double exx = J.J.E[0][0], eyy = J.J.E[1][1], ezz = J.J.E[2][2];
       const double exy = J.J.E[0][1], exz = J.J.E[0][2], eyz = J.J.E[1][2];
       job_phase_stress(J, part);
-      ok = job_barrier(J.bar, J.nparts, E.err, to);
+      ok = job_barrier(J, part, E.err, to);
       if (ok)
         for_part_nodes(J, part, [&](long long m, int x, int y, int z, int, int, int, int, int, int) {
           if (!(x == 0 || x == G.nx - 1 || y == 0 || y == G.ny - 1 || z == 0 || z == G.nz - 1))
@@ -606,7 +576,7 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
         cpart += job_c_elem(J, i, j, k);
       }
       job_put(J, SL_C, part, cpart, red);
-      if (ok) ok = job_barrier(J.bar, J.nparts, E.err, to);
+      if (ok) ok = job_barrier(J, part, E.err, to);
       if (ok) ok = job_start_residual(J, part, red, E.err, to);
       if (ok) {
         const double C = job_reduce(J, SL_C, red);
@@ -662,7 +632,7 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
       const double hAh_t = job_fp32_apply(J, part, (float)s.gamma, s.reset, cur, lam_pending, e3d_engine_dyn);
       lam_pending = 0.f;  // applied by this phase A
       job_put(J, SL_A, part, hAh_t, red);
-      if (!(ok = job_barrier(J.bar, J.nparts, E.err, to))) break;
+      if (!(ok = job_barrier(J, part, E.err, to))) break;
       const double hAh = job_reduce(J, SL_A, red);
       if (lead) {
         s.it += 1;
@@ -680,7 +650,7 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
       lam_pending = lam;
       h_pending = cur ? J.h0 : J.h1;  // the h_new of this iteration's phase A
       job_put(J, SL_B, part, zg, red);
-      if (!(ok = job_barrier(J.bar, J.nparts, E.err, to))) break;
+      if (!(ok = job_barrier(J, part, E.err, to))) break;
       const double gg_new = job_reduce(J, SL_B, red);
       if (lead) {
         const double gglast = s.gg;
@@ -719,7 +689,7 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
         flush_pending();
         __syncthreads();  // du: flush_pending's owners are not the fold's
         job_fold(J, part);
-        if (!(ok = job_barrier(J.bar, J.nparts, E.err, to))) break;
+        if (!(ok = job_barrier(J, part, E.err, to))) break;
         bool fx = false;
         if (!(ok = job_fp64_apply_u(J, part, e3d_engine_dyn, fx, E.err, to))) break;
         // energy terms too: if this replacement ends the solve, the final
@@ -755,7 +725,7 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
     const bool finished = s.status != PCG_RUNNING;
     if (ok && !finished) {
       // out of iteration budget for this launch: persist and yield
-      if (!(ok = job_barrier(J.bar, J.nparts, E.err, to)) && lead) s.status = PCG_TIMEOUT;
+      if (!(ok = job_barrier(J, part, E.err, to)) && lead) s.status = PCG_TIMEOUT;
       if (part == 0 && lead) {
         *J.st = s;
         *J.stage = ok ? JOB_ITER : JOB_DONE;
@@ -768,7 +738,7 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
     const bool fresh = s.status == PCG_CONVERGED && s.final_ready;
     if (ok && !fresh) {
       job_fold(J, part);
-      ok = job_barrier(J.bar, J.nparts, E.err, to);
+      ok = job_barrier(J, part, E.err, to);
     }
     bool fx = false;
     if (ok && !fresh) ok = job_fp64_apply_u(J, part, e3d_engine_dyn, fx, E.err, to);
@@ -788,7 +758,7 @@ static __global__ void __launch_bounds__(NT, E3D_ENGINE_BLOCKS_PER_SM) job_engin
         }
       });
       for (int q = 0; q < 12; ++q) job_put(J, SL_S + q, part, sacc[q], red);
-      ok = job_barrier(J.bar, J.nparts, E.err, to);
+      ok = job_barrier(J, part, E.err, to);
     }
     if (ok) {
       const double C = J.out->C;
@@ -824,7 +794,6 @@ static __global__ void reset_jobs_kernel(const JobDesc* __restrict__ jobs, int n
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   jobs[j].bar->count = 0u;
-  jobs[j].bar->gen = 0u;
   if (reset_stage) *jobs[j].stage = JOB_NEW;
 }
 
