@@ -144,7 +144,7 @@ struct JobDev {
 size_t rve_bytes(long long ns, int nphase) {
   return align256(4 * ns) + align256(8 * 36 * (size_t)nphase) + align256(8 * kCsStride * (size_t)nphase) +
          align256(4 * kCs32Stride * (size_t)nphase) + align256(8 * 576 * (size_t)nphase) +
-         align256(8 * 72 * (size_t)nphase) + align256(4 * 6 * ns) + align256(sizeof(PhaseMat) * (size_t)nphase) +
+         align256(8 * kDkdStride * (size_t)nphase) + align256(4 * 6 * ns) + align256(sizeof(PhaseMat) * (size_t)nphase) +
          align256(sizeof(int4) * kFxStride * (size_t)nphase) + align256(8 * 2) + align256(8 * 3 * (size_t)nphase);
 }
 
@@ -180,7 +180,7 @@ int32_t setup_rve(RveDev& R, char* base, const e3d_rve_t& in, double e1, double 
   R.cs64 = carve<double>(p, kCsStride * (size_t)R.nphase);
   R.cs32 = carve<float>(p, kCs32Stride * (size_t)R.nphase);
   R.dk = carve<double>(p, 576 * (size_t)R.nphase);
-  R.dkd = carve<double>(p, 72 * (size_t)R.nphase);
+  R.dkd = carve<double>(p, kDkdStride * (size_t)R.nphase);
   R.minv32 = carve<float>(p, 6 * R.ns);
   R.mats = carve<PhaseMat>(p, R.nphase);
   R.fxtab = carve<int4>(p, kFxStride * (size_t)R.nphase);
@@ -218,7 +218,8 @@ int32_t setup_rve(RveDev& R, char* base, const e3d_rve_t& in, double e1, double 
   if (mats.back().K1 < 0.0 || mats.back().G1 < 0.0 || in.c11 < in.c12 || in.c44 < 0.0)
     BCUDA(cudaMemsetAsync(R.fxinfo, 0, 2 * sizeof(double), s));
   GridDims G = job_dims(R.nx, R.ny, R.nz, 1);
-  bjacobi_kernel<<<(unsigned)((R.ns + 255) / 256), 256, 0, s>>>(G, R.pix, R.dkd, nullptr, R.minv32);
+  const int per = bjacobi_per(R.ns, kMaxParts);
+  bjacobi_kernel<<<bjacobi_grid(R.ns, per), 256, 0, s>>>(G, per, R.pix, R.dkd, nullptr, R.minv32);
   BCUDA(cudaGetLastError());
   // the host copies above read `scratch`/`mats`: finish before they go away
   BCUDA(cudaStreamSynchronize(s));

@@ -140,6 +140,7 @@ struct e3d_handle {
   // tile maxima of z (or of a stand-alone apply's x), h0 and h1
   double* norms = nullptr;
   int4* fxtab = nullptr;
+  unsigned long long* phsums = nullptr;  // strain sums over each phase, then the exponent
   unsigned* mz = nullptr;
   unsigned* mh0 = nullptr;
   unsigned* mh1 = nullptr;
@@ -275,6 +276,17 @@ ApplyArgs<double> apply_args(e3d_handle* h, const double* x, double* y) {
   A.hy = h->hy;
   A.hd = h->hd;
   return A;
+}
+
+// Block-Jacobi (kkk == 1, src/elas3dxtal_pcg.f90:1498-1520); the mixed form keeps an
+// FP32 copy of the FP64 inverse.
+int32_t launch_bjacobi(e3d_handle* h) {
+  const int per = bjacobi_per(h->G.ns, h->num_sms);
+  bjacobi_kernel<<<bjacobi_grid(h->G.ns, per), 256, 0, h->stream>>>(
+      h->G, per, h->pix, h->dkd, h->minv, h->prob.precision == E3D_PREC_MIXED ? h->minv32 : nullptr,
+      h->prob.preconditioner == E3D_PRECOND_NONE);
+  E3D_LAUNCHED(h);
+  return E3D_OK;
 }
 
 // y_partial = in-tile K x plus halos (not yet added).
@@ -432,8 +444,9 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
   if ((rc = dalloc(h, &h->pix, ns)) || (rc = dalloc(h, &h->rod, 3 * (size_t)std::max(np - 1, 1))) ||
       (rc = dalloc(h, &h->cmod, 36 * (size_t)np)) || (rc = dalloc(h, &h->cs, kCsStride * (size_t)np)) ||
       (rc = dalloc(h, &h->cs32, kCs32Stride * (size_t)np)) || (rc = dalloc(h, &h->dk, 576 * (size_t)np)) ||
-      (rc = dalloc(h, &h->dkd, 72 * (size_t)np)) || (rc = dalloc(h, &h->norms, 3 * (size_t)np)) ||
+      (rc = dalloc(h, &h->dkd, kDkdStride * (size_t)np)) || (rc = dalloc(h, &h->norms, 3 * (size_t)np)) ||
       (rc = dalloc(h, &h->fxtab, kFxStride * (size_t)np)) || (rc = dalloc(h, &h->mz, tile_rows)) ||
+      (rc = dalloc(h, &h->phsums, 12 * (size_t)np + 1)) ||
       (rc = dalloc(h, &h->mh0, tile_rows)) || (rc = dalloc(h, &h->mh1, tile_rows)) || (rc = dalloc(h, &h->u, n3)) || (rc = dalloc(h, &h->g, n3)) ||
       (rc = dalloc(h, &h->b, n3)) || (rc = dalloc(h, &h->z, n3)) || (rc = dalloc(h, &h->h0, n3)) ||
       (rc = dalloc(h, &h->h1, n3)) || (rc = dalloc(h, &h->Ah, n3)) || (rc = dalloc(h, &h->minv, 6 * ns)) ||
@@ -663,11 +676,7 @@ int32_t e3d_solve_begin(e3d_handle_t* h) {
   E3D_CUDA(cudaEventCreate(&e0));
   E3D_CUDA(cudaEventCreate(&e1));
   E3D_CUDA(cudaEventRecord(e0, h->stream));
-  // block-Jacobi (kkk == 1, src/elas3dxtal_pcg.f90:1498-1520); the mixed form
-  // keeps an FP32 copy of the FP64 inverse.
-  bjacobi_kernel<<<blocks_for(h->G.ns, 256), 256, 0, h->stream>>>(
-      h->G, h->pix, h->dkd, h->minv, mixed ? h->minv32 : nullptr, h->prob.preconditioner == E3D_PRECOND_NONE);
-  E3D_LAUNCHED(h);
+  if (int32_t rc = launch_bjacobi(h)) return rc;
   const int grid = reduction_grid(h);
   if (mixed) {
     const long long n3 = 3 * h->G.ns;
@@ -924,11 +933,21 @@ int32_t e3d_stress(e3d_handle_t* h, double strav[6], double epsav[6]) {
   if (!h) return E3D_ERR_INPUT;
   if (!h->femat_done) return E3D_ERR_STATE;
   cudaSetDevice(h->device);
-  const int grid = std::max(1, std::min(reduction_grid(h), h->partial_n / 12));
-  stress_avg_kernel<<<grid, 256, 0, h->stream>>>(h->G, h->J, h->pix, h->cmod, h->prob.nphase, h->u, h->partial);
+  const int np = h->prob.nphase;
+  const unsigned tiles = (unsigned)h->Gx.ntiles;
+  const int pgrid = (int)std::min<long long>(std::min(reduction_grid(h), h->partial_n / 12), h->Gx.ntiles);
+  int* info = reinterpret_cast<int*>(h->phsums + 12 * (size_t)np);
+  E3D_CUDA(cudaMemsetAsync(h->phsums, 0, 12 * sizeof(unsigned long long) * np, h->stream));
+  tile_max_kernel<<<tiles, kFxThreads, 0, h->stream>>>(h->Gx, h->u, h->mz);
+  E3D_LAUNCHED(h);
+  stress_sums_kernel<<<tiles, kFxThreads, 0, h->stream>>>(h->Gx, h->J, h->pix, h->cmod, np, h->u, h->mz, h->phsums, info,
+                                                          h->partial, pgrid);
+  E3D_LAUNCHED(h);
+  stress_total_kernel<<<1, 256, 0, h->stream>>>(np, h->phsums, info, h->cmod, h->partial, pgrid, h->scalars);
   E3D_LAUNCHED(h);
   double out[12];
-  int32_t rc = reduce_to_host(h, grid, 12, 12, out);
+  E3D_CUDA(cudaMemcpyAsync(out, h->scalars, sizeof out, cudaMemcpyDeviceToHost, h->stream));
+  int32_t rc = sync(h);
   if (rc) return rc;
   const double ns = (double)h->G.ns;
   for (int r = 0; r < 6; ++r) {
@@ -1352,9 +1371,10 @@ extern "C" int32_t e3d_checkpoint_load(e3d_handle_t* h, const char* path) {
   }
   const bool mixed = h->prob.precision == E3D_PREC_MIXED;
   // preconditioner of this problem (deterministic, so it is rebuilt, not stored)
-  bjacobi_kernel<<<blocks_for(h->G.ns, 256), 256, 0, h->stream>>>(
-      h->G, h->pix, h->dkd, h->minv, mixed ? h->minv32 : nullptr, h->prob.preconditioner == E3D_PRECOND_NONE);
-  E3D_LAUNCHED(h);
+  if (int32_t rc = launch_bjacobi(h)) {
+    std::fclose(f);
+    return rc;
+  }
   const size_t n3 = 3 * (size_t)h->G.ns;
   PcgState S = H.st;
   int32_t rc = ckpt_read(f, h->u, n3, h->stream);

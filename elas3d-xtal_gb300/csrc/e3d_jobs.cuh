@@ -853,8 +853,9 @@ static __global__ void batch_phase_kernel(const PhaseMat* __restrict__ mats, int
     const double v = (r <= c) ? col[c][r] : col[r][c];
     dk[(long long)p * 576 + e] = v;
     const int ra = r / 3, i = r % 3, cb = c / 3, j = c % 3;
-    if (ra == cb) dkd[(long long)p * 72 + ra * 9 + i * 3 + j] = v;
+    if (ra == cb) dkd[(long long)p * kDkdStride + ra * 9 + i * 3 + j] = v;
   }
+  store_uniform_inverse(col, dkd + (long long)p * kDkdStride);
   if (norms) fx_store_norms(col, csh, norms + 3 * p);
 }
 

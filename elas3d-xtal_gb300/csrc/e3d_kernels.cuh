@@ -6,7 +6,7 @@
 //   cs                   : nphase*kCsStride FP64 stiffness tables (C/16 and the summed mode matrices)
 //   cs32                 : nphase*24, FP32 upper triangle of C/16 (element_modal_f32)
 //   dk                   : nphase*576, [p][a][i][b][j] (reference local order)
-//   dkd                  : nphase*72 diagonal 3x3 blocks [p][a][i][j]
+//   dkd                  : nphase*78: diagonal 3x3 blocks [a][i][j], then the inverse of their sum
 //   hx, hy, hd           : tile-edge force halos (see apply_tile)
 #pragma once
 #include <cstdint>
@@ -1880,6 +1880,47 @@ static __device__ __forceinline__ void fx_store_norms(const double (&col)[24][24
   }
 }
 
+// invert3x3 (src/elas3dxtal_pcg.f90:2046-2147) of a symmetric block: a and ai hold
+// 00 11 22 01 02 12.  Same products as there; the cofactors that symmetry makes
+// equal are formed once.
+__device__ __forceinline__ void invert3x3(const double (&a)[6], double (&ai)[6]) {
+  const double c00 = a[1] * a[2] - a[5] * a[5];
+  const double c01 = -a[3] * a[2] + a[5] * a[4];
+  const double c02 = a[3] * a[5] - a[1] * a[4];
+  const double det = a[0] * c00 + a[3] * c01 + a[4] * c02;
+  if (fabs(det) < 1e-14) {
+    for (int i = 0; i < 6; ++i) ai[i] = 0.0;
+    return;
+  }
+  const double inv_det = 1.0 / det;
+  ai[0] = c00 * inv_det;
+  ai[1] = (a[0] * a[2] - a[4] * a[4]) * inv_det;
+  ai[2] = (a[0] * a[1] - a[3] * a[3]) * inv_det;
+  ai[3] = c01 * inv_det;
+  ai[4] = c02 * inv_det;
+  ai[5] = (-a[0] * a[5] + a[4] * a[3]) * inv_det;
+}
+
+// Block-Jacobi (src/elas3dxtal_pcg.f90:1498-1520): sum of the node's diagonal
+// 3x3 blocks over its 8 elements (reference order), inverted.  Stores the
+// symmetric inverse as 6 SoA planes (00 11 22 01 02 12) in FP64 and FP32.
+
+// The diagonal blocks of a phase, and the inverse of their sum: the block of a node
+// whose eight elements are all of this phase (as bjacobi_kernel forms it).
+constexpr int kDkdStride = 78;
+static __device__ __forceinline__ void store_uniform_inverse(const double (&col)[24][24], double* __restrict__ dkd) {
+  if (threadIdx.x != 0) return;
+  double M[6], s[6];
+  for (int ra = 0; ra < 8; ++ra) {
+    const double(*b)[24] = col + 3 * ra;
+    const int o = 3 * ra;
+    const double d[6] = {b[0][o], b[1][o + 1], b[2][o + 2], b[1][o], b[2][o], b[2][o + 1]};
+    for (int i = 0; i < 6; ++i) M[i] = ra == 0 ? d[i] : M[i] + d[i];
+  }
+  invert3x3(M, s);
+  for (int q = 0; q < 6; ++q) dkd[72 + q] = s[q];
+}
+
 static __global__ void femat_phase_kernel(FematParams P, const double* __restrict__ rod, double* __restrict__ cmod,
                                    double* __restrict__ cs, float* __restrict__ cs32,
                                    double* __restrict__ dk, double* __restrict__ dkd, double* __restrict__ norms) {
@@ -1934,8 +1975,9 @@ static __global__ void femat_phase_kernel(FematParams P, const double* __restric
     const double v = (r <= c) ? col[c][r] : col[r][c];
     dk[(long long)p * 576 + e] = v;
     const int ra = r / 3, i = r % 3, cb = c / 3, j = c % 3;
-    if (ra == cb) dkd[(long long)p * 72 + ra * 9 + i * 3 + j] = v;
+    if (ra == cb) dkd[(long long)p * kDkdStride + ra * 9 + i * 3 + j] = v;
   }
+  store_uniform_inverse(col, dkd + (long long)p * kDkdStride);
   fx_store_norms(col, csh, norms + 3 * p);
 }
 
@@ -2140,66 +2182,82 @@ static __global__ void affine_kernel(GridDims G, JumpParams J, double* __restric
   u[m + G.ns] = x * exy + y * eyy + z * eyz;
   u[m + 2 * G.ns] = x * exz + y * eyz + z * ezz;
 }
-
-// invert3x3 (src/elas3dxtal_pcg.f90:2046-2147) of a symmetric block: a and ai hold
-// 00 11 22 01 02 12.  Same products as there; the cofactors that symmetry makes
-// equal are formed once.
-__device__ __forceinline__ void invert3x3(const double (&a)[6], double (&ai)[6]) {
-  const double c00 = a[1] * a[2] - a[5] * a[5];
-  const double c01 = -a[3] * a[2] + a[5] * a[4];
-  const double c02 = a[3] * a[5] - a[1] * a[4];
-  const double det = a[0] * c00 + a[3] * c01 + a[4] * c02;
-  if (fabs(det) < 1e-14) {
-    for (int i = 0; i < 6; ++i) ai[i] = 0.0;
-    return;
-  }
-  const double inv_det = 1.0 / det;
-  ai[0] = c00 * inv_det;
-  ai[1] = (a[0] * a[2] - a[4] * a[4]) * inv_det;
-  ai[2] = (a[0] * a[1] - a[3] * a[3]) * inv_det;
-  ai[3] = c01 * inv_det;
-  ai[4] = c02 * inv_det;
-  ai[5] = (-a[0] * a[5] + a[4] * a[3]) * inv_det;
-}
-
-// Block-Jacobi (src/elas3dxtal_pcg.f90:1498-1520): sum of the node's diagonal
-// 3x3 blocks over its 8 elements (reference order), inverted.  Stores the
-// symmetric inverse as 6 SoA planes (00 11 22 01 02 12) in FP64 and FP32.
-static __global__ void bjacobi_kernel(GridDims G, const int32_t* __restrict__ pix, const double* __restrict__ dkd,
-                               double* __restrict__ minv, float* __restrict__ minv32, int identity = 0) {
-  const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= G.ns) return;
-  if (identity) {  // plain CG: z = g
+constexpr int kBjacobiPer = 4;
+static __global__ void __launch_bounds__(256) bjacobi_kernel(GridDims G, int per, const int32_t* __restrict__ pix,
+                                                             const double* __restrict__ dkd, double* __restrict__ minv,
+                                                             float* __restrict__ minv32, int identity = 0) {
+  // FP64-issue-bound (73 instructions a node), so a block of 256 * per nodes first
+  // serves those inside a grain, whose eight elements are of one phase and whose
+  // inverse is in the phase's table, and then inverts for the others side by side.
+  // 300^3 polycrystal: 3.45 -> 0.81 ms.
+  __shared__ unsigned short todo[256 * kBjacobiPer];
+  __shared__ int n;
+  if (threadIdx.x == 0) n = 0;
+  __syncthreads();
+  const long long base = (long long)blockIdx.x * (256 * per);
+  auto store = [&](long long m, const double* s) {
+#pragma unroll
     for (int q = 0; q < 6; ++q) {
-      const double v = q < 3 ? 1.0 : 0.0;
-      if (minv) minv[m + q * G.ns] = v;
-      if (minv32) minv32[m + q * G.ns] = (float)v;
+      if (minv) minv[m + q * G.ns] = s[q];
+      if (minv32) minv32[m + q * G.ns] = (float)s[q];
     }
-    return;
-  }
-  int x, y, z;
-  node_xyz(G, m, x, y, z);
-  // FP64-issue-bound: the six distinct entries of the block and of its inverse,
-  // 73 FP64 instructions a node (103 with all nine); 300^3: 5.2 -> 3.45 ms
-  double M[6];
+  };
+  auto phases = [&](long long m, int (&ph)[8]) {  // of the elements around the node, by local node
+    int x, y, z;
+    node_xyz(G, m, x, y, z);
 #pragma unroll
-  for (int ra = 0; ra < 8; ++ra) {
-    const int a = kRefToCorner[ra];
-    const int ex = wrapi(x - (a & 1), G.nx), ey = wrapi(y - ((a >> 1) & 1), G.ny),
-              ez = wrapi(z - ((a >> 2) & 1), G.nz);
-    const int ph = pix[E3D_IDX((long long)ex + (long long)G.nx * ey + (long long)G.nx * G.ny * ez, G.ns)];
-    const double* D = dkd + (long long)ph * 72 + ra * 9;
-    const double d[6] = {__ldg(D), __ldg(D + 4), __ldg(D + 8), __ldg(D + 1), __ldg(D + 2), __ldg(D + 5)};
+    for (int ra = 0; ra < 8; ++ra) {
+      const int a = kRefToCorner[ra];
+      const int ex = wrapi(x - (a & 1), G.nx), ey = wrapi(y - ((a >> 1) & 1), G.ny),
+                ez = wrapi(z - ((a >> 2) & 1), G.nz);
+      ph[ra] = pix[E3D_IDX((long long)ex + (long long)G.nx * ey + (long long)G.nx * G.ny * ez, G.ns)];
+    }
+  };
+  for (int j = 0; j < per; ++j) {
+    const int i = j * 256 + threadIdx.x;
+    const long long m = base + i;
+    if (m >= G.ns) break;
+    if (identity) {  // plain CG: z = g
+      const double one[6] = {1.0, 1.0, 1.0, 0.0, 0.0, 0.0};
+      store(m, one);
+      continue;
+    }
+    int ph[8];
+    phases(m, ph);
+    bool same = true;
 #pragma unroll
-    for (int i = 0; i < 6; ++i) M[i] = ra == 0 ? d[i] : M[i] + d[i];
+    for (int ra = 1; ra < 8; ++ra) same = same && ph[ra] == ph[0];
+    if (same) {
+      double s[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) s[q] = __ldg(dkd + (long long)ph[0] * kDkdStride + 72 + q);
+      store(m, s);
+    } else {
+      todo[atomicAdd(&n, 1)] = (unsigned short)i;
+    }
   }
-  double s[6];
-  invert3x3(M, s);
-  for (int q = 0; q < 6; ++q) {
-    if (minv) minv[m + q * G.ns] = s[q];
-    if (minv32) minv32[m + q * G.ns] = (float)s[q];
+  __syncthreads();
+  for (int t = threadIdx.x; t < n; t += 256) {
+    const long long m = base + todo[t];
+    int ph[8];
+    phases(m, ph);
+    double M[6], s[6];  // the six distinct entries of the block, and of its inverse
+#pragma unroll
+    for (int ra = 0; ra < 8; ++ra) {
+      const double* D = dkd + (long long)ph[ra] * kDkdStride + ra * 9;
+      const double d[6] = {__ldg(D), __ldg(D + 4), __ldg(D + 8), __ldg(D + 1), __ldg(D + 2), __ldg(D + 5)};
+#pragma unroll
+      for (int i = 0; i < 6; ++i) M[i] = ra == 0 ? d[i] : M[i] + d[i];
+    }
+    invert3x3(M, s);
+    store(m, s);
   }
 }
+
+// `per` above: four once that leaves every SM eight blocks (more nodes to share the
+// few inversions among), else one.
+inline int bjacobi_per(long long ns, int sms) { return ns >= (long long)sms * 8 * 256 * kBjacobiPer ? kBjacobiPer : 1; }
+inline unsigned bjacobi_grid(long long ns, int per) { return (unsigned)((ns + 256 * per - 1) / (256 * per)); }
 
 template <typename T>
 __device__ __forceinline__ void precond3(const T* __restrict__ mi, long long m, long long ns, const T (&g)[3],
@@ -2254,14 +2312,25 @@ __device__ __forceinline__ void voxel_strain(const GridDims& G, const JumpParams
   eps[5] = 0.25 * (dY[0] + dX[1]);
 }
 
-static __global__ void __launch_bounds__(256) stress_avg_kernel(GridDims G, JumpParams J, const int32_t* __restrict__ pix,
-                                                         const double* __restrict__ cmod, int nphase,
-                                                         const double* __restrict__ u, double* partial) {
-  __shared__ double red[8];
+// Volume sums of stress and strain (src/elas3dxtal_pcg.f90:2149-2408).  The stress
+// of a voxel is C(phase) . strain, so only the strains are summed over the voxels,
+// phase by phase: 72 additions a voxel instead of 130 FP64 operations.  They are
+// 64-bit integers as in the fixed-point stencil, with one exponent for the whole of
+// u (maxima in mx) and the periodic jumps, and their sums, in two words of 64 bits,
+// are exact and so do not depend on the order in which threads add a run of voxels
+// of one phase to its sums.  300^3: 6.55 ms voxel by voxel in FP64, 0.85 with the
+// maxima and the final sums.
+// sums[12 p + 2 i]: low halves of component i (first-order Hadamard sum, four times
+// the strain) over phase p; sums[12 p + 2 i + 1]: high halves.  info: the exponent.
+// Values that are not finite or out of the exponents' range: FP64, voxel by voxel,
+// to the partials of pgrid blocks.
+static __device__ __noinline__ void stress_general(const GridDims& G, const JumpParams& J, const int32_t* __restrict__ pix,
+                                                   const double* __restrict__ cmod, int nphase,
+                                                   const double* __restrict__ u, double* partial, int pgrid, double* red) {
+  if ((int)blockIdx.x >= pgrid) return;
   double acc[12];
   for (int t = 0; t < 12; ++t) acc[t] = 0.0;
-  for (long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x; m < G.ns;
-       m += (long long)gridDim.x * blockDim.x) {
+  for (long long m = (long long)blockIdx.x * kFxThreads + threadIdx.x; m < G.ns; m += (long long)pgrid * kFxThreads) {
     int x, y, z;
     node_xyz(G, m, x, y, z);
     double eps[6];
@@ -2275,8 +2344,180 @@ static __global__ void __launch_bounds__(256) stress_avg_kernel(GridDims G, Jump
     }
   }
   for (int t = 0; t < 12; ++t) {
-    const double s = block_sum<256>(acc[t], red);
+    const double s = block_sum<kFxThreads>(acc[t], red);
     if (threadIdx.x == 0) partial[12 * (long long)blockIdx.x + t] = s;
+  }
+}
+
+static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
+    GridDims G, JumpParams J, const int32_t* __restrict__ pix, const double* __restrict__ cmod, int nphase,
+    const double* __restrict__ u, const unsigned* __restrict__ mx, unsigned long long* __restrict__ sums,
+    int* __restrict__ info, double* partial, int pgrid) {
+  constexpr int kHalo = TILE_X + kFxRows + 1, kRow = TILE_X + 1, cst = kRow * (kFxRows + 1);
+  __shared__ long long node[2][3][cst];
+  __shared__ double raw[3][kFxThreads + kHalo];
+  __shared__ double red[kFxThreads / 32];
+  __shared__ unsigned mred[kFxThreads / 32];
+  const int tid = threadIdx.x;
+  unsigned b = 0;
+  for (long long i = tid; i < G.ntiles * kFxRows; i += kFxThreads) b = max(b, mx[i]);
+  b = __reduce_max_sync(0xffffffffu, b);
+  if ((tid & 31) == 0) mred[tid >> 5] = b;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kFxThreads / 32; ++i) b = max(b, mred[i]);
+  const double n3[3] = {(double)G.nx, (double)G.ny, (double)G.nz};
+  double big = b ? __hiloint2double((int)b + 1, 0) : 0.0;
+  for (int c = 0; c < 3; ++c)
+    for (int d = 0; d < 3; ++d) big = fx_max(big, fabs(J.E[c][d] * n3[d]));
+  const int kx = b >= 0x7ff00000u ? kFxGeneral : fx_exponent_below(big);
+  if (blockIdx.x == 0 && tid == 0) *info = kx;
+  if (kx == kFxGeneral) {
+    stress_general(G, J, pix, cmod, nphase, u, partial, pgrid, red);
+    return;
+  }
+  const int tx = tid % TILE_X, ty = tid / TILE_X;
+  const long long tile = blockIdx.x;
+  const int tix = (int)(tile % G.ntx), tiy = (int)((tile / G.ntx) % G.nty),
+            tiz = (int)(tile / ((long long)G.ntx * G.nty));
+  const int x0 = tix * TILE_X, y0 = tiy * kFxRows, z0 = tiz * G.tz;
+  const int wx = min(TILE_X, G.nx - x0), wy = min(kFxRows, G.ny - y0), zend = min(G.nz, z0 + G.tz);
+  const bool active = tx < wx && ty < wy;
+  const int nhalo = wx + wy + 1;
+  int hlx = wx, hly = wy;  // halo node of loader thread tid < nhalo
+  if (tid < wy)
+    hly = tid;
+  else if (tid < wy + wx)
+    hlx = tid - wy;
+  const long long ns = G.ns, nxy = (long long)G.nx * G.ny;
+  const long long own = (long long)(x0 + tx) + (long long)G.nx * (y0 + ty);
+  const long long halo = (long long)wrapi(x0 + hlx, G.nx) + (long long)G.nx * wrapi(y0 + hly, G.ny);
+  auto load = [&](int zl) {
+    const long long zo = nxy * wrapi(zl, G.nz);
+    if (active) {
+      const long long m = E3D_IDX(own + zo, ns);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) cp_async_8(&raw[c][tid], u + m + c * ns);
+    }
+    if (tid < nhalo) {
+      const long long m = E3D_IDX(halo + zo, ns);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) cp_async_8(&raw[c][kFxThreads + tid], u + m + c * ns);
+    }
+    cp_async_commit();
+  };
+  auto convert = [&](int buf) {
+    cp_async_wait<0>();
+    if (active) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) node[buf][c][ty * kRow + tx] = fx_from_double(raw[c][tid], kx);
+    }
+    if (tid < nhalo) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        node[buf][c][E3D_IDX(hly * kRow + hlx, cst)] = fx_from_double(raw[c][kFxThreads + tid], kx);
+    }
+  };
+  // sum, x and y difference of the voxel's four nodes of a plane
+  auto plane = [&](int buf, long long (&P)[3][3]) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long* v = node[buf][c] + ty * kRow + tx;
+      const long long v0 = v[0], v1 = v[1], v2 = v[kRow], v3 = v[kRow + 1];
+      const long long s0 = v0 + v1, s1 = v2 + v3;
+      P[c][0] = s0 + s1;
+      P[c][1] = (v1 - v0) + (v3 - v2);
+      P[c][2] = s1 - s0;
+    }
+  };
+  // what the periodic jumps add at the last voxel of x, y and z
+  const bool jx = active && x0 + tx == G.nx - 1, jy = active && y0 + ty == G.ny - 1;
+  auto jump = [&](int c, int d) { return 4 * fx_from_double(J.E[c][d] * n3[d], kx); };
+  unsigned long long lo[6] = {};
+  long long hi[6] = {};
+  int cur = -1;
+  auto flush = [&] {
+    unsigned long long* s = sums + 12 * (long long)E3D_IDX(cur, nphase);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      atomicAdd(s + 2 * i, lo[i]);
+      atomicAdd(s + 2 * i + 1, (unsigned long long)hi[i]);
+      lo[i] = 0;
+      hi[i] = 0;
+    }
+  };
+  load(z0);
+  convert(0);
+  load(z0 + 1);
+  __syncthreads();
+  long long Po[3][3] = {};
+  if (active) plane(0, Po);
+  for (int k = z0; k < zend; ++k) {
+    const int ph = active ? __ldcs(pix + E3D_IDX(own + nxy * k, ns)) : -1;
+    const int buf = (k + 1 - z0) & 1;
+    convert(buf);
+    if (k + 2 <= zend) load(k + 2);
+    __syncthreads();
+    if (!active) continue;
+    long long Pn[3][3], X[3], Y[3], Z[3];
+    plane(buf, Pn);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      X[c] = Pn[c][1] + Po[c][1];
+      Y[c] = Pn[c][2] + Po[c][2];
+      Z[c] = Pn[c][0] - Po[c][0];
+      if (jx) X[c] += jump(c, 0);
+      if (jy) Y[c] += jump(c, 1);
+      if (k == G.nz - 1) Z[c] += jump(c, 2);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) Po[c][q] = Pn[c][q];
+    }
+    if (ph != cur) {
+      if (cur >= 0) flush();
+      cur = ph;
+    }
+    const long long e[6] = {X[0], Y[1], Z[2], Z[0] + X[2], Z[1] + Y[2], Y[0] + X[1]};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      lo[i] += (unsigned)e[i];
+      hi[i] += e[i] >> 32;
+    }
+  }
+  if (cur >= 0) flush();
+}
+
+// The six sums of stress and of strain, from the sums over the phases.
+static __global__ void __launch_bounds__(256) stress_total_kernel(int nphase, const unsigned long long* __restrict__ sums,
+                                                                  const int* __restrict__ info,
+                                                                  const double* __restrict__ cmod,
+                                                                  const double* __restrict__ partial, int pgrid,
+                                                                  double* __restrict__ out) {
+  __shared__ double red[8];
+  const int kx = *info;
+  double acc[12];
+  for (int t = 0; t < 12; ++t) acc[t] = 0.0;
+  if (kx == kFxGeneral) {
+    for (int i = threadIdx.x; i < pgrid; i += 256)
+      for (int t = 0; t < 12; ++t) acc[t] += partial[12 * (long long)i + t];
+  } else {
+    for (int p = threadIdx.x; p < nphase; p += 256) {
+      double eps[6];
+      for (int c = 0; c < 6; ++c) {
+        const unsigned long long* s = sums + 12 * (long long)p + 2 * c;
+        const __int128 t = ((__int128)(long long)s[1] << 32) + s[0];
+        eps[c] = ldexp(ldexp((double)(long long)(t >> 32), 32) + (double)(unsigned)t, -kx - 2);
+        acc[6 + c] += eps[c];
+      }
+      for (int r = 0; r < 6; ++r) {
+        double s = 0.0;
+        for (int c = 0; c < 6; ++c) s += cmod[p + (long long)nphase * (r + 6 * c)] * eps[c];
+        acc[r] += s;
+      }
+    }
+  }
+  for (int t = 0; t < 12; ++t) {
+    const double s = block_sum<256>(acc[t], red);
+    if (threadIdx.x == 0) out[t] = s;
   }
 }
 
