@@ -606,11 +606,11 @@ int32_t e3d_femat(e3d_handle_t* h) {
                                                                         h->scalars + 1);
   E3D_LAUNCHED(h);
   E3D_CUDA(cudaMemsetAsync(h->b, 0, sizeof(double) * 3 * h->G.ns, h->stream));  // interior nodes
-  femat_b_kernel<<<blocks_for(boundary_node_count(h->G), 256), 256, 0, h->stream>>>(h->G, h->J, h->pix, h->dk,
-                                                                                         h->b);
+  femat_b_kernel<<<blocks_for(boundary_node_count(h->G), kFematThreads), kFematThreads, 0, h->stream>>>(
+      h->G, h->J, h->pix, h->dk, h->b);
   E3D_LAUNCHED(h);
-  const int grid = reduction_grid(h);
-  femat_c_kernel<<<grid, 256, 0, h->stream>>>(h->G, h->J, h->pix, h->dk, h->partial);
+  const int grid = (int)std::min<unsigned>((unsigned)reduction_grid(h), blocks_for(boundary_node_count(h->G), kFematThreads));
+  femat_c_kernel<<<grid, kFematThreads, 0, h->stream>>>(h->G, h->J, h->pix, h->dk, h->partial);
   E3D_LAUNCHED(h);
   reduce_partials_kernel<<<1, 256, 0, h->stream>>>(h->partial, grid, 1, 1, h->scalars);
   E3D_LAUNCHED(h);

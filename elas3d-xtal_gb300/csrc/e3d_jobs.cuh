@@ -149,40 +149,28 @@ static __device__ __noinline__ void job_b_node(const JobDesc& J, int x, int y, i
   const GridDims& G = J.G;
   acc[0] = acc[1] = acc[2] = 0.0;
   if (!(x == 0 || x == G.nx - 1 || y == 0 || y == G.ny - 1 || z == 0 || z == G.nz - 1)) return;
+  ElementJump jump;
+  for (int q = 1; q < 8; ++q) jump.fill(G, J.J, q);
   for (int ra = 0; ra < 8; ++ra) {
     const int a = kRefToCorner[ra];
     const int ex = wrapi(x - (a & 1), G.nx), ey = wrapi(y - ((a >> 1) & 1), G.ny),
               ez = wrapi(z - ((a >> 2) & 1), G.nz);
-    double d[8][3];
-    bool any;
-    element_delta(G, J.J, ex, ey, ez, d, any);
-    if (!any) continue;
+    const int w = ElementJump::crossing(G, ex, ey, ez);
+    if (!w) continue;
     const int ph = J.pix[E3D_IDX((long long)ex + (long long)G.nx * ey + (long long)G.nx * G.ny * ez, G.ns)];
     const double* D = J.dk + E3D_IDX(ph, J.nphase_total) * 576;
-    for (int i = 0; i < 3; ++i) {
-      double s = 0.0;
-      for (int rb = 0; rb < 8; ++rb)
-        for (int jj = 0; jj < 3; ++jj) s += D[(ra * 3 + i) * 24 + rb * 3 + jj] * d[rb][jj];
-      acc[i] += s;
-    }
+    for (int i = 0; i < 3; ++i) acc[i] += jump.row(D, ra * 3 + i, w);
   }
 }
 
 static __device__ __noinline__ double job_c_elem(const JobDesc& J, int x, int y, int z) {
   const GridDims& G = J.G;
   if (!(x == G.nx - 1 || y == G.ny - 1 || z == G.nz - 1)) return 0.0;
-  double d[8][3];
-  bool any;
-  element_delta(G, J.J, x, y, z, d, any);
+  ElementJump jump;
+  for (int q = 1; q < 8; ++q) jump.fill(G, J.J, q);
   const int ph = J.pix[E3D_IDX((long long)x + (long long)G.nx * y + (long long)G.nx * G.ny * z, G.ns)];
   const double* D = J.dk + E3D_IDX(ph, J.nphase_total) * 576;
-  double e = 0.0;
-  for (int r = 0; r < 24; ++r) {
-    double s = 0.0;
-    for (int c = 0; c < 24; ++c) s += D[r * 24 + c] * d[c / 3][c % 3];
-    e += d[r / 3][r % 3] * s;
-  }
-  return 0.5 * e;
+  return jump.energy(D, ElementJump::crossing(G, x, y, z));
 }
 
 // Elements with a corner across a high face (i = nx-1, j = ny-1 or k = nz-1),
@@ -812,25 +800,14 @@ static __global__ void batch_phase_kernel(const PhaseMat* __restrict__ mats, int
   const int p = blockIdx.x;
   __shared__ double csh[kCsStride];
   __shared__ double col[24][24];
-  if (threadIdx.x == 0) {
-    const PhaseMat M = mats[p];
-    double C6[6][6];
-    if (M.pore) {
-      for (int i = 0; i < 6; ++i)
-        for (int j = 0; j < 6; ++j) {
-          const double ck = (i < 3 && j < 3) ? 1.0 : 0.0;
-          double cmu = 0.0;
-          if (i < 3 && j < 3) cmu = (i == j) ? 4.0 / 3.0 : -2.0 / 3.0;
-          if (i >= 3 && i == j) cmu = 1.0;
-          C6[i][j] = M.K1 * ck + M.G1 * cmu;
-        }
-    } else {
-      bond_rotate(M.r, M.c11, M.c12, M.c44, C6);
-    }
-    for (int i = 0; i < 6; ++i)
-      for (int j = 0; j < 6; ++j) cmod[p + (long long)nphase_total * (i + 6 * j)] = C6[i][j];
-    modal_table(C6, csh);
-  }
+  __shared__ double C6[6][6], w1[6][6], w2[6][6];
+  const PhaseMat M = mats[p];
+  if (M.pore)
+    isotropic_warp(M.K1, M.G1, C6);
+  else
+    bond_rotate_warp(M.r, M.c11, M.c12, M.c44, w1, w2, C6);
+  for (int e = threadIdx.x; e < 36; e += 32) cmod[p + (long long)nphase_total * (e / 6 + 6 * (e % 6))] = C6[e / 6][e % 6];
+  modal_table_warp(C6, csh, w1, w2);
   __syncthreads();
   for (int i = threadIdx.x; i < kCsStride; i += blockDim.x) cs[(long long)p * kCsStride + i] = csh[i];
   for (int r = threadIdx.x; r < 6; r += blockDim.x)  // FP32: upper triangle of C/16

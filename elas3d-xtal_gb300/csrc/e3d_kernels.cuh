@@ -1749,14 +1749,8 @@ struct FematParams {
   double c11, c12, c44, K1, G1, Km, Gm;
 };
 
-// rotatestiffnessby (src/elas3dxtal_pcg.f90:2535-2633) for one grain.
-static __device__ void bond_rotate(const double r[3], double c11, double c12, double c44, double out[6][6]) {
-  double Cc[6][6];
-  for (int i = 0; i < 6; ++i)
-    for (int j = 0; j < 6; ++j) Cc[i][j] = 0.0;
-  Cc[0][0] = Cc[1][1] = Cc[2][2] = c11;
-  Cc[0][1] = Cc[0][2] = Cc[1][2] = Cc[1][0] = Cc[2][0] = Cc[2][1] = c12;
-  Cc[3][3] = Cc[4][4] = Cc[5][5] = c44;
+// rotatestiffnessby (src/elas3dxtal_pcg.f90:2535-2633) for one grain: the Bond matrix.
+static __device__ void bond_matrix(const double (&r)[3], double (&N)[6][6]) {
   const double rdotr = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
   const double term1 = 1.0 - rdotr;
   double term2 = 1.0 + rdotr;
@@ -1777,7 +1771,6 @@ static __device__ void bond_rotate(const double r[3], double c11, double c12, do
     for (int i = 0; i < 3; ++i)
       for (int j = 0; j < 3; ++j) Q[i][j] = (i == j) ? 1.0 : 0.0;
   }
-  double N[6][6];
   for (int row = 0; row < 3; ++row) {
     N[row][0] = Q[row][0] * Q[row][0];
     N[row][1] = Q[row][1] * Q[row][1];
@@ -1804,19 +1797,68 @@ static __device__ void bond_rotate(const double r[3], double c11, double c12, do
   N[5][3] = Q[0][1] * Q[1][2] + Q[0][2] * Q[1][1];
   N[5][4] = Q[0][2] * Q[1][0] + Q[0][0] * Q[1][2];
   N[5][5] = Q[0][0] * Q[1][1] + Q[0][1] * Q[1][0];
-  double Tm[6][6];
-  for (int i = 0; i < 6; ++i)
-    for (int j = 0; j < 6; ++j) {
-      double s = 0.0;
-      for (int k = 0; k < 6; ++k) s += N[k][i] * Cc[k][j];
-      Tm[i][j] = s;
-    }
-  for (int i = 0; i < 6; ++i)
-    for (int j = 0; j < 6; ++j) {
-      double s = 0.0;
-      for (int k = 0; k < 6; ++k) s += Tm[i][k] * N[k][j];
-      out[i][j] = s;
-    }
+}
+
+// N^T C N for the cubic C, by the 32 threads of a warp, an entry of the 6 x 6 products
+// each; every array is in shared memory.  A lane's FP64 instructions cost as much as
+// a warp's: with one thread at work here and in modal_table_warp (72 divisions) the
+// tables of seven phases took 97 us, so 31; those of 300^3's phases 331, so 89.
+static __device__ void bond_rotate_warp(const double (&r)[3], double c11, double c12, double c44, double (&N)[6][6],
+                                        double (&Tm)[6][6], double (&out)[6][6]) {
+  const int lane = threadIdx.x;
+  if (lane == 0) bond_matrix(r, N);
+  __syncwarp();
+  for (int e = lane; e < 36; e += 32) {
+    const int i = e / 6, j = e % 6;
+    double s = 0.0;
+    for (int k = 0; k < 6; ++k) s += N[k][i] * (k < 3 && j < 3 ? (k == j ? c11 : c12) : k == j ? c44 : 0.0);
+    Tm[i][j] = s;
+  }
+  __syncwarp();
+  for (int e = lane; e < 36; e += 32) {
+    const int i = e / 6, j = e % 6;
+    double s = 0.0;
+    for (int k = 0; k < 6; ++k) s += Tm[i][k] * N[k][j];
+    out[i][j] = s;
+  }
+  __syncwarp();
+}
+
+// modal_table by the threads of a warp; C1 and C2: scratch, in shared memory as the rest.
+static __device__ void modal_table_warp(const double (&C6)[6][6], double* tab, double (&C1)[6][6], double (&C2)[6][6]) {
+  const int lane = threadIdx.x;
+  for (int e = lane; e < 36; e += 32) {
+    const double v = C6[e / 6][e % 6];
+    tab[e] = v / 16.0;
+    C1[e / 6][e % 6] = v / 48.0;
+    C2[e / 6][e % 6] = v / 144.0;
+  }
+  __syncwarp();
+  if (lane < 9) {  // column of M2: the response to a unit component
+    double in[9], out[9];
+    for (int r = 0; r < 9; ++r) in[r] = r == lane ? 1.0 : 0.0;
+    second_order_modes(&C1[0][0], in, out);
+    for (int r = 0; r < 9; ++r) tab[kM2 + 9 * r + lane] = out[r];
+  } else if (lane < 12) {
+    double in[3], out[3];
+    for (int r = 0; r < 3; ++r) in[r] = r == lane - 9 ? 1.0 : 0.0;
+    third_order_modes(&C2[0][0], in, out);
+    for (int r = 0; r < 3; ++r) tab[kM3 + 3 * r + lane - 9] = out[r];
+  }
+  __syncwarp();
+}
+
+// K ck + G cmu of an isotropic phase (src/elas3dxtal_pcg.f90:655-664, 680-682, 701-705).
+static __device__ void isotropic_warp(double K, double G, double (&C6)[6][6]) {
+  for (int e = threadIdx.x; e < 36; e += 32) {
+    const int i = e / 6, j = e % 6;
+    const double ck = (i < 3 && j < 3) ? 1.0 : 0.0;
+    double cmu = 0.0;
+    if (i < 3 && j < 3) cmu = (i == j) ? 4.0 / 3.0 : -2.0 / 3.0;
+    if (i >= 3 && i == j) cmu = 1.0;
+    C6[i][j] = K * ck + G * cmu;
+  }
+  __syncwarp();
 }
 
 // Phase ids from device memory: 1-based with the range check of ppixel_hdf5
@@ -1927,29 +1969,17 @@ static __global__ void femat_phase_kernel(FematParams P, const double* __restric
   const int p = blockIdx.x;
   __shared__ double csh[kCsStride];
   __shared__ double col[24][24];  // col[c][r] = (K e_c)[r], c/r = refnode*3 + dof
-  if (threadIdx.x == 0) {
-    double C6[6][6];
-    const bool iso_phase = (p == P.nphase - 1) || (P.flag_m == 0);
-    if (iso_phase) {
-      // K*ck + G*cmu (src/elas3dxtal_pcg.f90:655-664, 680-682, 701-705)
-      const double K = (p == P.nphase - 1) ? P.K1 : P.Km;
-      const double Gs = (p == P.nphase - 1) ? P.G1 : P.Gm;
-      for (int i = 0; i < 6; ++i)
-        for (int j = 0; j < 6; ++j) {
-          const double ck = (i < 3 && j < 3) ? 1.0 : 0.0;
-          double cmu = 0.0;
-          if (i < 3 && j < 3) cmu = (i == j) ? 4.0 / 3.0 : -2.0 / 3.0;
-          if (i >= 3 && i == j) cmu = 1.0;
-          C6[i][j] = K * ck + Gs * cmu;
-        }
-    } else {
-      const double r[3] = {rod[3 * p], rod[3 * p + 1], rod[3 * p + 2]};
-      bond_rotate(r, P.c11, P.c12, P.c44, C6);
-    }
-    for (int i = 0; i < 6; ++i)
-      for (int j = 0; j < 6; ++j) cmod[p + (long long)P.nphase * (i + 6 * j)] = C6[i][j];
-    modal_table(C6, csh);
+  __shared__ double C6[6][6], w1[6][6], w2[6][6];
+  if (p == P.nphase - 1) {
+    isotropic_warp(P.K1, P.G1, C6);
+  } else if (P.flag_m == 0) {
+    isotropic_warp(P.Km, P.Gm, C6);
+  } else {
+    const double r[3] = {rod[3 * p], rod[3 * p + 1], rod[3 * p + 2]};
+    bond_rotate_warp(r, P.c11, P.c12, P.c44, w1, w2, C6);
   }
+  for (int e = threadIdx.x; e < 36; e += 32) cmod[p + (long long)P.nphase * (e / 6 + 6 * (e % 6))] = C6[e / 6][e % 6];
+  modal_table_warp(C6, csh, w1, w2);
   __syncthreads();
   for (int i = threadIdx.x; i < kCsStride; i += blockDim.x) cs[(long long)p * kCsStride + i] = csh[i];
   for (int r = threadIdx.x; r < 6; r += blockDim.x)  // FP32: upper triangle of C/16
@@ -2042,22 +2072,41 @@ struct JumpParams {
   double E[3][3];  // symmetric strain tensor
 };
 
-__device__ __forceinline__ void element_delta(const GridDims& G, const JumpParams& J, int i, int j, int k,
-                                              double (&d)[8][3], bool& any) {
-  const bool wx = (i == G.nx - 1), wy = (j == G.ny - 1), wz = (k == G.nz - 1);
-  any = wx || wy || wz;
-  for (int ra = 0; ra < 8; ++ra) {
-    const int a = kRefToCorner[ra];
-    const int ox = a & 1, oy = (a >> 1) & 1, oz = (a >> 2) & 1;
+struct ElementJump {
+  double T[8][3];  // jump of a corner by the directions in which it crosses (bits x, y, z)
+  __device__ __forceinline__ void fill(const GridDims& G, const JumpParams& J, int m) {
+    const double n[3] = {(double)G.nx, (double)G.ny, (double)G.nz};
     for (int c = 0; c < 3; ++c) {
       double v = 0.0;
-      if (wx && ox) v += J.E[c][0] * (double)G.nx;
-      if (wy && oy) v += J.E[c][1] * (double)G.ny;
-      if (wz && oz) v += J.E[c][2] * (double)G.nz;
-      d[ra][c] = v;
+      for (int d = 0; d < 3; ++d)
+        if (m >> d & 1) v += J.E[c][d] * n[d];
+      T[m][c] = v;
     }
   }
-}
+  // directions in which element (x, y, z) crosses a high face
+  static __device__ __forceinline__ int crossing(const GridDims& G, int x, int y, int z) {
+    return (x == G.nx - 1 ? 1 : 0) | (y == G.ny - 1 ? 2 : 0) | (z == G.nz - 1 ? 4 : 0);
+  }
+  // row r of D delta over the corners that cross (the others' terms are zero)
+  __device__ __forceinline__ double row(const double* __restrict__ D, int r, int w) const {
+    double s = 0.0;
+#pragma unroll
+    for (int rb = 0; rb < 8; ++rb)
+      if (kRefToCorner[rb] & w)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) s += D[r * 24 + rb * 3 + c] * T[kRefToCorner[rb] & w][c];
+    return s;
+  }
+  __device__ __forceinline__ double energy(const double* __restrict__ D, int w) const {  // delta . D delta / 2
+    double e = 0.0;
+#pragma unroll 1
+    for (int ra = 0; ra < 8; ++ra)
+      if (kRefToCorner[ra] & w)
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) e += T[kRefToCorner[ra] & w][c] * row(D, 3 * ra + c, w);
+    return 0.5 * e;
+  }
+};
 
 // Boundary nodes (x, y or z on a face of the box), each once: the two x faces
 // whole, then the y faces at interior x, then the z faces at interior x and y.
@@ -2093,8 +2142,15 @@ __device__ __forceinline__ void boundary_node(const GridDims& G, long long t, in
 
 // b over the boundary nodes listed by boundary_node (b is zero elsewhere and
 // cleared beforehand): one thread per boundary node.
+// Few nodes, much FP64 work each: small blocks, which reach every SM on small grids,
+// and no terms of corners that do not cross.  b 70 -> 32 us and C 47 -> 29 at 32^3,
+// 672 -> 424 and 337 -> 166 at 300^3.
+constexpr int kFematThreads = 64;
 static __global__ void femat_b_kernel(GridDims G, JumpParams J, const int32_t* __restrict__ pix,
                                const double* __restrict__ dk, double* __restrict__ b) {
+  __shared__ ElementJump jump;
+  if (threadIdx.x < 8) jump.fill(G, J, threadIdx.x);
+  __syncthreads();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= boundary_node_count(G)) return;
   int x, y, z;
@@ -2106,18 +2162,11 @@ static __global__ void femat_b_kernel(GridDims G, JumpParams J, const int32_t* _
     const int a = kRefToCorner[ra];
     const int ex = wrapi(x - (a & 1), G.nx), ey = wrapi(y - ((a >> 1) & 1), G.ny),
               ez = wrapi(z - ((a >> 2) & 1), G.nz);
-    double d[8][3];
-    bool any;
-    element_delta(G, J, ex, ey, ez, d, any);
-    if (!any) continue;
+    const int w = ElementJump::crossing(G, ex, ey, ez);
+    if (!w) continue;
     const int ph = pix[E3D_IDX((long long)ex + (long long)G.nx * ey + (long long)G.nx * G.ny * ez, G.ns)];
     const double* D = dk + (long long)ph * 576;
-    for (int i = 0; i < 3; ++i) {
-      double s = 0.0;
-      for (int rb = 0; rb < 8; ++rb)
-        for (int jj = 0; jj < 3; ++jj) s += D[(ra * 3 + i) * 24 + rb * 3 + jj] * d[rb][jj];
-      acc[i] += s;
-    }
+    for (int i = 0; i < 3; ++i) acc[i] += jump.row(D, ra * 3 + i, w);
   }
   b[m] = acc[0];
   b[m + G.ns] = acc[1];
@@ -2125,10 +2174,13 @@ static __global__ void femat_b_kernel(GridDims G, JumpParams J, const int32_t* _
 }
 
 // Constant C = 1/2 sum_e delta_e^T K_e delta_e over boundary elements.
-static __global__ void __launch_bounds__(256) femat_c_kernel(GridDims G, JumpParams J, const int32_t* __restrict__ pix,
+static __global__ void __launch_bounds__(kFematThreads) femat_c_kernel(GridDims G, JumpParams J, const int32_t* __restrict__ pix,
                                                       const double* __restrict__ dk, double* partial) {
-  __shared__ double red[8];
+  __shared__ double red[kFematThreads / 32];
   double acc = 0.0;
+  __shared__ ElementJump jump;
+  if (threadIdx.x < 8) jump.fill(G, J, threadIdx.x);
+  __syncthreads();
   // boundary elements: enumerate the three high faces without double counting
   const long long nfx = (long long)G.ny * G.nz;                        // i = nx-1
   const long long nfy = (long long)(G.nx - 1) * G.nz;                  // j = ny-1, i < nx-1
@@ -2152,20 +2204,11 @@ static __global__ void __launch_bounds__(256) femat_c_kernel(GridDims G, JumpPar
       i = (int)(s % (G.nx - 1));
       j = (int)(s / (G.nx - 1));
     }
-    double d[8][3];
-    bool any;
-    element_delta(G, J, i, j, k, d, any);
     const int ph = pix[E3D_IDX((long long)i + (long long)G.nx * j + (long long)G.nx * G.ny * k, G.ns)];
     const double* D = dk + (long long)ph * 576;
-    double e = 0.0;
-    for (int r = 0; r < 24; ++r) {
-      double s = 0.0;
-      for (int c = 0; c < 24; ++c) s += D[r * 24 + c] * d[c / 3][c % 3];
-      e += d[r / 3][r % 3] * s;
-    }
-    acc += 0.5 * e;
+    acc += jump.energy(D, ElementJump::crossing(G, i, j, k));
   }
-  const double s = block_sum<256>(acc, red);
+  const double s = block_sum<kFematThreads>(acc, red);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
@@ -2436,14 +2479,35 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
   unsigned long long lo[6] = {};
   long long hi[6] = {};
   int cur = -1;
-  auto flush = [&] {
-    unsigned long long* s = sums + 12 * (long long)E3D_IDX(cur, nphase);
+  // Adds the runs of the lanes with `ends` to their phases' sums and clears them.  The
+  // lanes of one phase are added up first (in pieces of 26 bits, whose sums fit 32),
+  // and twelve lanes then add a word each: every thread by itself, all to the words
+  // of a few phases, took 158 us on a grid of 32^3, where this takes 9.5.
+  auto flush = [&](bool ends) {
+    const int lane = tid & 31;
+    unsigned left = __ballot_sync(0xffffffffu, ends);
+    while (left) {
+      const int p = __shfl_sync(0xffffffffu, cur, __ffs(left) - 1);
+      const bool in = ends && cur == p;
+      unsigned long long word = 0;
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      atomicAdd(s + 2 * i, lo[i]);
-      atomicAdd(s + 2 * i + 1, (unsigned long long)hi[i]);
-      lo[i] = 0;
-      hi[i] = 0;
+      for (int i = 0; i < 6; ++i) {
+        const unsigned l0 = __reduce_add_sync(0xffffffffu, in ? (unsigned)lo[i] & 0x3ffffffu : 0u),
+                       l1 = __reduce_add_sync(0xffffffffu, in ? (unsigned)(lo[i] >> 26) : 0u),
+                       h0 = __reduce_add_sync(0xffffffffu, in ? (unsigned)hi[i] & 0x3ffffffu : 0u);
+        const int h1 = __reduce_add_sync(0xffffffffu, in ? (int)(hi[i] >> 26) : 0);
+        if (lane == 2 * i) word = l0 + ((unsigned long long)l1 << 26);
+        if (lane == 2 * i + 1) word = h0 + (unsigned long long)((long long)h1 * (1 << 26));
+      }
+      if (lane < 12) atomicAdd(sums + 12 * (long long)E3D_IDX(p, nphase) + lane, word);
+      left &= ~__ballot_sync(0xffffffffu, in);
+    }
+    if (ends) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        lo[i] = 0;
+        hi[i] = 0;
+      }
     }
   };
   load(z0);
@@ -2458,6 +2522,8 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
     convert(buf);
     if (k + 2 <= zend) load(k + 2);
     __syncthreads();
+    if (__any_sync(0xffffffffu, ph != cur && cur >= 0)) flush(ph != cur && cur >= 0);
+    cur = ph;
     if (!active) continue;
     long long Pn[3][3], X[3], Y[3], Z[3];
     plane(buf, Pn);
@@ -2472,10 +2538,6 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
 #pragma unroll
       for (int q = 0; q < 3; ++q) Po[c][q] = Pn[c][q];
     }
-    if (ph != cur) {
-      if (cur >= 0) flush();
-      cur = ph;
-    }
     const long long e[6] = {X[0], Y[1], Z[2], Z[0] + X[2], Z[1] + Y[2], Y[0] + X[1]};
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
@@ -2483,7 +2545,7 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
       hi[i] += e[i] >> 32;
     }
   }
-  if (cur >= 0) flush();
+  flush(cur >= 0);
 }
 
 // The six sums of stress and of strain, from the sums over the phases.
