@@ -634,7 +634,10 @@ int32_t e3d_init_affine(e3d_handle_t* h) {
   E3D_TRACE("e3d_init_affine");
   if (!h) return E3D_ERR_INPUT;
   cudaSetDevice(h->device);
-  affine_kernel<<<blocks_for(h->G.ns, 256), 256, 0, h->stream>>>(h->G, h->J, h->u);
+  // z chunks as long as that leaves every SM eight blocks
+  const int chunk = (int)std::clamp<long long>(h->G.ns / (256ll * 8 * h->num_sms), 1, 16);
+  const unsigned cols = blocks_for((long long)h->G.nx * h->G.ny, 256), chunks = blocks_for(h->G.nz, chunk);
+  affine_kernel<<<cols * chunks, 256, 0, h->stream>>>(h->G, h->J, chunk, h->u);
   E3D_LAUNCHED(h);
   h->energy_done = h->solve_ready = false;
   return sync(h);

@@ -2213,17 +2213,24 @@ static __global__ void __launch_bounds__(kFematThreads) femat_c_kernel(GridDims 
 }
 
 // Affine initial guess (src/elas3dxtal_pcg.f90:423-438).
-static __global__ void affine_kernel(GridDims G, JumpParams J, double* __restrict__ u) {
-  const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= G.ns) return;
-  int xi, yi, zi;
-  node_xyz(G, m, xi, yi, zi);
-  const double x = xi, y = yi, z = zi;
+// FP64-issue-bound: a thread takes `chunk` nodes of a z column, whose x and y terms
+// are one sum, 4 FP64 instructions a node instead of 12 (AFFINE_FIGURES).
+static __global__ void __launch_bounds__(256) affine_kernel(GridDims G, JumpParams J, int chunk, double* __restrict__ u) {
+  const unsigned nxy = (unsigned)G.nx * (unsigned)G.ny, cols = (nxy + 255u) / 256u;
+  const unsigned col = blockIdx.x % cols * 256u + threadIdx.x;
+  if (col >= nxy) return;
+  const double x = (int)(col % (unsigned)G.nx), y = (int)(col / (unsigned)G.nx);
   const double exx = J.E[0][0], eyy = J.E[1][1], ezz = J.E[2][2];
   const double exy = J.E[0][1], exz = J.E[0][2], eyz = J.E[1][2];
-  u[m] = x * exx + y * exy + z * exz;
-  u[m + G.ns] = x * exy + y * eyy + z * eyz;
-  u[m + 2 * G.ns] = x * exz + y * eyz + z * ezz;
+  const double c0 = x * exx + y * exy, c1 = x * exy + y * eyy, c2 = x * exz + y * eyz;
+  const int z0 = (int)(blockIdx.x / cols) * chunk, z1 = min(G.nz, z0 + chunk);
+  for (int zi = z0; zi < z1; ++zi) {
+    const double z = zi;
+    const long long m = (long long)col + (long long)nxy * zi;
+    u[m] = c0 + z * exz;
+    u[m + G.ns] = c1 + z * eyz;
+    u[m + 2 * G.ns] = c2 + z * ezz;
+  }
 }
 constexpr int kBjacobiPer = 4;
 static __global__ void __launch_bounds__(256) bjacobi_kernel(GridDims G, int per, const int32_t* __restrict__ pix,
