@@ -1015,13 +1015,14 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
 // ---------------------------------------------------------------------------
 // FP64 tile in fixed point (e3d_fixed.cuh).
 
-// Rows of a fixed-point tile, and blocks per SM.  What bounds the tile is the
-// heavy half of the FMA pipe (378 wide multiply-adds an element at 4 cycles a
-// warp) and how little of a warp's other work falls beside it: two blocks of 4
-// warps with 255 registers run their FP64, load and addition phases beside each
-// other's multiply-adds.  FP64 iteration at 300^3: 4.67 ms; one block of 8 warps
-// 4.89, two of 6 (168 registers) 5.04, one of 12 5.01, three of 4 5.08; and the
-// FP64 element form 14.5.
+// Rows of a fixed-point tile, and blocks per SM.  What bounds the tile is integer
+// issue: 378 wide multiply-adds an element at two cycles of a scheduler each, which
+// its other integer instructions (some 1200 a warp and plane) do not overlap, and
+// the latency of their chains with two warps a scheduler.  Two blocks of 4 warps
+// with 255 registers run their FP64 and load phases beside each other's products.
+// FP64 iteration at 300^3 as first built: 4.67 ms; one block of 8 warps 4.89, two of
+// 6 (168 registers) 5.04, one of 12 5.01, three of 4 5.08; the FP64 element form 14.5.
+// Now 4.52.
 constexpr int kFxRows = 4;
 constexpr int kFxThreads = TILE_X * kFxRows;
 constexpr int kFxBlocks = 2;
