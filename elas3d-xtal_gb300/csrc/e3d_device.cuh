@@ -214,10 +214,7 @@ __device__ __forceinline__ void matvec_sym(const float (&t)[kCs32Stride], const 
   }
 }
 
-// The table row comes from global memory (tstride == 0: six consecutive float4,
-// read through the read-only path) or from a shared-memory slot whose six
-// float4 lie tstride float4 apart (staged there ahead of use).
-template <int TSTRIDE = 0>
+// The table row is six consecutive float4, read through the read-only path.
 __device__ __forceinline__ void element_modal_f32(const float* __restrict__ cs, const float (&hu)[8],
                                                   const float (&hv)[8], const float (&hw)[8], float (&fu)[8],
                                                   float (&fv)[8], float (&fw)[8]) {
@@ -225,7 +222,7 @@ __device__ __forceinline__ void element_modal_f32(const float* __restrict__ cs, 
   const float4* t4 = reinterpret_cast<const float4*>(cs);
 #pragma unroll
   for (int i = 0; i < kCs32Stride / 4; ++i) {
-    const float4 q = TSTRIDE == 0 ? __ldg(t4 + i) : t4[i * TSTRIDE];
+    const float4 q = __ldg(t4 + i);
     t[4 * i] = q.x;
     t[4 * i + 1] = q.y;
     t[4 * i + 2] = q.z;

@@ -336,7 +336,7 @@ __device__ __forceinline__ void ring_drain(PlaneRing& R) {
 template <typename T, bool FUSED, bool POLD_SMEM = (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), bool DEFER_U = false,
           int TY = TILE_Y>
 __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, TY>& sm, double& hAh) {
-  constexpr int TILE_Y = TY, NT = TILE_X * TY;
+  constexpr int TILE_Y = TY;
   const GridDims& G = A.g;
   const int tid = threadIdx.x;
   const int tx = tid % TILE_X, ty = tid / TILE_X;
