@@ -1051,7 +1051,9 @@ struct FxSmem {
   double raw[FUSED ? 6 : 3][kFxThreads + kHalo];
 };
 
-__device__ __forceinline__ double fx_max(double a, double b) { return b <= a ? a : b; }  // keeps a NaN in b
+// Larger of the two, or a NaN where either is one: in a reduction, which meets its
+// values in any order, a NaN must reach the result.
+__host__ __device__ __forceinline__ double fx_max(double a, double b) { return a != a || b <= a ? a : b; }
 __device__ __forceinline__ unsigned abs_hi(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
 
 constexpr int kFxGeneral = 0x7fffffff;
