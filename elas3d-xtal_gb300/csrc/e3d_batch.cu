@@ -15,6 +15,7 @@
 #include "e3d_batch.h"
 #include "e3d_gpu.h"
 #include "e3d_jobs.cuh"
+#include "e3d_rounds.h"
 #include "e3d_trace.h"
 
 using namespace e3d;
@@ -685,7 +686,7 @@ int32_t e3d_batch_parts(e3d_batch_t* b, int32_t* parts, int32_t capacity) {
 struct ServeJob {
   int64_t id = 0;
   int parts = 1;  // blocks per solve, fixed at admission
-  int rounds = 0; // it took part in
+  long long last = 0;  // round it ran in last (new: the one before its first)
   e3d_rve_t rve{};
   std::vector<int32_t> pix;
   std::vector<double> rod;
@@ -705,6 +706,7 @@ struct e3d_server {
   cudaStream_t stream = nullptr;
   Engine eng;
   int64_t next_id = 1;
+  long long round = 0;  // of the next step
   std::deque<ServeJob*> queue;
   std::vector<ServeJob*> active;
   std::map<int64_t, ServeJob*> finished;
@@ -722,28 +724,6 @@ int serve_round_iters(const e3d_serve_opts_t& o, long long ns, int k) {
   const double per_block = (double)ns / k;
   const double f = std::min(8.0, std::max(1.0, (double)kServeBlockNodes / per_block));
   return (int)std::min<double>(2.0e9, std::floor(o.round_iters * f));
-}
-
-// The active requests of the next round, in the order of `active`.  Once they ask for
-// more blocks than there are, a last wave of blocks that is mostly empty would take
-// as long as a full one, so a round runs whole waves: the requests that ran least
-// often first, the others wait for the next round.  A request's own iterations are
-// the same in whichever rounds they run.  Nine requests
-// that ask for 172 blocks: .595 -> .529 s; forty for some 1500: the same.
-static std::vector<ServeJob*> serve_round(const e3d_server& s) {
-  long long total = 0;
-  for (const ServeJob* j : s.active) total += j->parts;
-  if (total <= s.eng.grid) return s.active;
-  std::vector<ServeJob*> order = s.active, take;
-  std::stable_sort(order.begin(), order.end(), [](const ServeJob* a, const ServeJob* c) { return a->rounds < c->rounds; });
-  long long room = total / s.eng.grid * s.eng.grid;
-  for (ServeJob* j : order)
-    if (j->parts <= room) {
-      room -= j->parts;
-      take.push_back(j);
-    }
-  std::stable_sort(take.begin(), take.end(), [](const ServeJob* a, const ServeJob* c) { return a->R.ns > c->R.ns; });
-  return take;
 }
 
 extern "C" {
@@ -873,6 +853,7 @@ int32_t e3d_serve_step(e3d_server_t* s, int32_t* pending) {
     set_parts(j->J, j->R, j->parts);
     j->J.d.it_round = serve_round_iters(s->opts, ns, j->parts);
     BCUDA(cudaMemsetAsync(j->J.d.stage, 0, 4, s->stream));
+    j->last = s->round - 1;
     s->active.push_back(j);
   }
   if (!s->active.empty()) {
@@ -880,11 +861,19 @@ int32_t e3d_serve_step(e3d_server_t* s, int32_t* pending) {
     // filled with small ones
     std::stable_sort(s->active.begin(), s->active.end(),
                      [](const ServeJob* a, const ServeJob* c) { return a->R.ns > c->R.ns; });
+    std::vector<int> parts;
+    std::vector<long long> last;
+    for (const ServeJob* j : s->active) {
+      parts.push_back(j->parts);
+      last.push_back(j->last);
+    }
     std::vector<JobDesc> descs;
-    for (ServeJob* j : serve_round(*s)) {
-      ++j->rounds;
+    for (int i : round_requests(parts, last, s->eng.grid)) {
+      ServeJob* j = s->active[(size_t)i];
+      j->last = s->round;
       descs.push_back(j->J.d);
     }
+    ++s->round;
     int np = 0;
     int32_t rc = s->eng.upload(descs, s->stream, &np);
     if (rc) return rc;

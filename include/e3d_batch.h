@@ -111,8 +111,10 @@ int32_t e3d_serve_create(e3d_server_t** s, const e3d_serve_opts_t* opts);
 int32_t e3d_serve_submit(e3d_server_t* s, const e3d_rve_t* rve, const double strain[6], int64_t* id);
 
 /* One scheduling round: admits queued requests while slots and HBM allow,
- * advances every active solve by round_iters iterations in one engine launch,
- * and retires finished solves (their memory is freed for the next admission).
+ * advances the active solves by round_iters iterations in one engine launch, and
+ * retires finished solves (their memory is freed for the next admission).  Where
+ * the solves ask for more blocks than the device has, some may wait for the next
+ * round; none waits twice in a row, whatever is submitted meanwhile.
  * Returns the number of requests still queued or active through *pending. */
 int32_t e3d_serve_step(e3d_server_t* s, int32_t* pending);
 
