@@ -16,6 +16,7 @@
 #include "e3d_device.cuh"
 #include "e3d_f32x2.cuh"
 #include "e3d_fixed.cuh"
+#include "e3d_index.h"
 #include "e3d_tma.cuh"
 
 namespace e3d {
@@ -702,14 +703,13 @@ struct F2Smem {
 // to the order of sums, same halos.  One barrier a plane: between two of them the
 // nodes of one plane are summed and the elements of the next formed, while the
 // loads of the plane after that are in flight.  The dot product h . K h is the
-// sum of the element energies, from values at hand in the element.  Byte offsets
-// into a component fit 32 bits: no device that holds a solve's state has 2^30
-// nodes.  DEFER_U: du -= lam_prev * h_old for the own nodes on the way.  FULL: the
-// tile has all its 32 x 8 columns, so that nothing is masked.
-__device__ __forceinline__ float* at_byte(float* p, unsigned o) {
+// sum of the element energies, from values at hand in the element.  DEFER_U: du -=
+// lam_prev * h_old for the own nodes on the way.  FULL: the tile has all its 32 x 8
+// columns, so that nothing is masked.
+__device__ __forceinline__ float* at_byte(float* p, unsigned long long o) {
   return reinterpret_cast<float*>(reinterpret_cast<char*>(p) + o);
 }
-__device__ __forceinline__ const float* at_byte(const float* p, unsigned o) {
+__device__ __forceinline__ const float* at_byte(const float* p, unsigned long long o) {
   return reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + o);
 }
 
@@ -762,12 +762,12 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
   auto load = [&](int zl) {
     const int d = (zl - z0 + 1) % kF2Depth;
     if (zl <= zend) {
-    const unsigned zo = nxy * (unsigned)wrapi(zl, G.nz);
+    const int zw = wrapi(zl, G.nz);
     const bool mine = DEFER_U && zl >= z0 && zl < zend, need_x = !reset || mine;
 #pragma unroll
     for (int q = 0; q < 2; ++q)
       if (q ? act_b : act_a) {
-        const unsigned o = 4u * (unsigned)E3D_IDX(own + (q ? nx : 0u) + zo, ns);
+        const unsigned long long o = node_bytes4(E3D_IDX(node_of(own + (q ? nx : 0u), nxy, zw), ns));
 #pragma unroll
         for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[d][slot(0, c, q)][tid], at_byte(A.zv + c * ns, o));
         if (need_x)
@@ -778,7 +778,7 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
           for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw[d][slot(2, c, q)][tid], at_byte(A.du + c * ns, o));
       }
     if (tid < nhalo) {
-      const unsigned o = 4u * (unsigned)E3D_IDX(halo + zo, ns);
+      const unsigned long long o = node_bytes4(E3D_IDX(node_of(halo, nxy, zw), ns));
 #pragma unroll
       for (int c = 0; c < 3; ++c) cp_async_4(&sm.raw_halo[d][c][tid], at_byte(A.zv + c * ns, o));
       if (!reset)
@@ -791,7 +791,6 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
   auto commit = [&](int zl, float (&buf)[3][(TILE_Y + 1) * kRow]) {
     const int d = (zl - z0 + 1) % kF2Depth;
     cp_async_wait<kF2Depth - 1>();
-    const unsigned zo = nxy * (unsigned)zl;  // used on own planes only
     const bool mine = zl >= z0 && zl < zend;
     // every slot is read before anything is stored: a store in between would
     // hold back the reads behind it
@@ -828,7 +827,7 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
 #pragma unroll
       for (int q = 0; q < 2; ++q)
         if (q ? act_b : act_a) {
-          const unsigned o = 4u * (unsigned)E3D_IDX(own + (q ? nx : 0u) + zo, ns);
+          const unsigned long long o = node_bytes4(E3D_IDX(node_of(own + (q ? nx : 0u), nxy, zl), ns));
 #pragma unroll
           for (int c = 0; c < 3; ++c) *at_byte(A.hnew + c * ns, o) = v[2 * c + q];
           // nothing pending at the first step of a launch (lam_prev = 0): h_old
@@ -864,7 +863,7 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
   const long long per_c = G.ntiles * (long long)G.tz;
   auto node_sums = [&](int k) {
     const float(*r)[kF2Threads] = sm.r[k & 1];
-    const unsigned o = 4u * (own + nxy * (unsigned)k);
+    const unsigned long long o = node_bytes4(node_of(own, nxy, k));
     const long long hb = tile * G.tz + (k - z0);
     float ea[3], ga[3], rb[6], na[3], nb[3];
 #pragma unroll
@@ -880,7 +879,7 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       if (act_a) *at_byte(A.y + E3D_IDX(c * ns, 3 * ns), o) = na[c];
-      if (act_b) *at_byte(A.y + E3D_IDX(c * ns, 3 * ns), o + 4u * nx) = nb[c];
+      if (act_b) *at_byte(A.y + E3D_IDX(c * ns, 3 * ns), o + node_bytes4(nx)) = nb[c];
     }
     if (tx == wx - 1) {
 #pragma unroll
@@ -920,7 +919,7 @@ static __device__ __forceinline__ void apply_tile_f2(const ApplyArgs<float>& A, 
   int b0 = 0;  // buffer of plane k
   const int32_t* pix = A.pix;
   auto phase = [&](int z, int& pa, int& pb) {
-    const unsigned m = own + nxy * (unsigned)wrapi(z, G.nz);
+    const unsigned m = node_of(own, nxy, wrapi(z, G.nz));
     pa = act_a ? __ldcs(pix + E3D_IDX(m, ns)) : 0;
     pb = act_b ? __ldcs(pix + E3D_IDX(m + nx, ns)) : 0;
   };
@@ -2754,7 +2753,8 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
   constexpr int B = V * (int)sizeof(T);
   constexpr int kLanes = TILE_X / V;  // threads of a row
   using Vec = VecOf<T, V>;
-  const unsigned ns = (unsigned)G.ns, nx = (unsigned)G.nx, nxy = nx * (unsigned)G.ny;
+  const long long ns = G.ns;  // in a register: G may lie in shared memory, read again after every copy issued
+  const unsigned nx = (unsigned)G.nx, nxy = nx * (unsigned)G.ny;
   const int rs = tid / kLanes, tx = (tid % kLanes) * V;  // row slot of the step, first column
   const int pl = rs / TY;                                // plane of the step
   const long long per_c = G.ntiles * (long long)G.tz;
@@ -2786,7 +2786,7 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
         const unsigned m = base + nx * (unsigned)row + nxy * (unsigned)lz;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const unsigned i = (unsigned)E3D_IDX(m + c * ns, 3 * G.ns);
+          const unsigned long long i = E3D_IDX(value_of(m, c, ns), 3 * ns);
           cp_async_n<B>(d + (c * NTH + tid) * V, Ah + i);
           cp_async_n<B>(d + ((3 + c) * NTH + tid) * V, g + i);
           if constexpr (UPD_U) {
@@ -2796,7 +2796,7 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
         }
 #pragma unroll
         for (int q = 0; q < 6; ++q)
-          cp_async_n<B>(d + ((6 + q) * NTH + tid) * V, minv + (unsigned long long)m + (unsigned long long)q * ns);
+          cp_async_n<B>(d + ((6 + q) * NTH + tid) * V, minv + E3D_IDX(value_of(m, q, ns), 6 * ns));
         T* hs = d + F * NTH * V;
         if (row == 0) {
 #pragma unroll
@@ -2863,7 +2863,7 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
       for (int c = 0; c < 3; ++c) {
 #pragma unroll
         for (int i = 0; i < V; ++i) gv[c].v[i] -= lam * ah[c].v[i];
-        const unsigned o = (unsigned)E3D_IDX(m + c * ns, 3 * G.ns);
+        const unsigned long long o = E3D_IDX(value_of(m, c, ns), 3 * ns);
         *reinterpret_cast<Vec*>(g + o) = gv[c];
         if constexpr (UPD_U) {
 #pragma unroll
@@ -2886,7 +2886,7 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
           zmax = max(zmax, max(abs_hi(zv[0].v[i]), max(abs_hi(zv[1].v[i]), abs_hi(zv[2].v[i]))));
       }
 #pragma unroll
-      for (int c = 0; c < 3; ++c) *reinterpret_cast<Vec*>(z + (unsigned)E3D_IDX(m + c * ns, 3 * G.ns)) = zv[c];
+      for (int c = 0; c < 3; ++c) *reinterpret_cast<Vec*>(z + E3D_IDX(value_of(m, c, ns), 3 * ns)) = zv[c];
     }
     if constexpr (ZMAX) {
       zmax = __reduce_max_sync(0xffffffffu, zmax);
@@ -2901,7 +2901,7 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
 // du -= lam h over the nodes that a thread owns in apply_tile_f2.
 static __device__ void flush_u_tiles_f2(const GridDims& G, long long first, long long stride, float lam,
                                         const float* __restrict__ h, float* __restrict__ u, int tid) {
-  const unsigned ns = (unsigned)G.ns, nx = (unsigned)G.nx, nxy = nx * (unsigned)G.ny;
+  const unsigned nx = (unsigned)G.nx, nxy = nx * (unsigned)G.ny;
   const int tx = tid % TILE_X, ya = 2 * (tid / TILE_X);
   for (long long t = first; t < G.ntiles; t += stride) {
     const int tix = (int)(t % G.ntx);
@@ -2915,7 +2915,7 @@ static __device__ void flush_u_tiles_f2(const GridDims& G, long long first, long
         const unsigned m = (unsigned)(x0 + tx) + nx * (unsigned)(y0 + row) + nxy * (unsigned)(z0 + lz);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const unsigned i = (unsigned)E3D_IDX(m + c * ns, 3 * G.ns);
+          const unsigned long long i = E3D_IDX(value_of(m, c, G.ns), 3 * G.ns);
           u[i] = u[i] - lam * __ldcg(h + i);
         }
       }
