@@ -15,6 +15,7 @@
 #include "e3d_batch.h"
 #include "e3d_gpu.h"
 #include "e3d_jobs.cuh"
+#include "e3d_material.h"
 #include "e3d_rounds.h"
 #include "e3d_trace.h"
 
@@ -216,7 +217,7 @@ int32_t setup_rve(RveDev& R, char* base, const e3d_rve_t& in, double e1, double 
   batch_phase_kernel<<<R.nphase, 32, 0, s>>>(R.mats, R.nphase, R.cmod, R.cs64, R.cs32, R.dk, R.dkd, R.norms);
   fx_table_kernel<<<std::min(R.nphase, 128), 96, 0, s>>>(R.nphase, R.norms, R.cs64, R.fxtab, R.fxinfo);
   // an indefinite stiffness keeps the FP64 form (as e3d_femat does)
-  if (mats.back().K1 < 0.0 || mats.back().G1 < 0.0 || in.c11 < in.c12 || in.c44 < 0.0)
+  if (!semidefinite(mats.back().K1, mats.back().G1) || !semidefinite_cubic(in.c11, in.c12, in.c44))
     BCUDA(cudaMemsetAsync(R.fxinfo, 0, 2 * sizeof(double), s));
   GridDims G = job_dims(R.nx, R.ny, R.nz, 1);
   const int per = bjacobi_per(R.ns, kMaxParts);

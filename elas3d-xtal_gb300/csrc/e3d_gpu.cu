@@ -17,6 +17,7 @@
 
 #include "e3d_gpu.h"
 #include "e3d_kernels.cuh"
+#include "e3d_material.h"
 #include "e3d_trace.h"
 
 using namespace e3d;
@@ -623,7 +624,8 @@ int32_t e3d_femat(e3d_handle_t* h) {
   // An indefinite stiffness (nu > 1/2, say) leaves PCG without a bound on what it
   // makes of rounding, down to which iterations its divergence reset finds: such
   // problems keep the FP64 form, whose rounding they were validated with.
-  const bool definite = P.K1 >= 0.0 && P.G1 >= 0.0 && P.Km >= 0.0 && P.Gm >= 0.0 && p.c11 >= p.c12 && p.c44 >= 0.0;
+  const bool definite =
+      semidefinite(P.K1, P.G1) && semidefinite(P.Km, P.Gm) && semidefinite_cubic(p.c11, p.c12, p.c44);
   h->fx_ok = out[2] != 0.0 && definite;
   h->femat_done = true;
   h->energy_done = h->solve_ready = h->minv_ready = false;
