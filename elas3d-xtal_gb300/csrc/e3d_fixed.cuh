@@ -5,8 +5,9 @@
 // the FP64 element product is formed in 64-bit integers with the precision of
 // FP64 or better:
 //
-//   - a tile's nodal values become X = rint(x * 2^kx), |X| <= 2^57, with kx from
-//     the largest value of the tile and its neighbours (tile_exponent);
+//   - a tile's nodal values become X = rint(x * 2^kx), |X| <= 2^57, with kx from the
+//     largest value that the tile reads (fx_tile_exponent, which sends tiles whose
+//     values are uneven to the FP64 form);
 //   - the Walsh-Hadamard transform and every sum of forces are integer
 //     additions, exact (and modular: only final sums have to fit 64 bits);
 //   - the stiffness entries are integers c = ch * 2^32 + cl of up to 63 bits with

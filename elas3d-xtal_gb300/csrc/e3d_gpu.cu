@@ -138,7 +138,7 @@ struct e3d_handle {
   PlaneMaps* maps = nullptr;
   int pcg_grid32_tma = 0;
   // fixed-point FP64 stencil (e3d_fixed.cuh): phase norms and integer tables,
-  // tile maxima of z (or of a stand-alone apply's x), h0 and h1
+  // row maxima of z, h0 and h1 (a stand-alone apply's x: in the last two)
   double* norms = nullptr;
   int4* fxtab = nullptr;
   unsigned long long* phsums = nullptr;  // strain sums over each phase, then the exponent
@@ -148,7 +148,12 @@ struct e3d_handle {
   int* fxleave = nullptr;
   int fx_kc = 0;
   bool fx_ok = false;   // the problem's tables allow it
-  bool fx_pcg = false;  // this solve runs in it (until a value leaves its range)
+  // Whether the solve goes on in the form for uneven tiles, and how many iterations
+  // without one, in a row, end that; twice as many after each return to it.  A
+  // direction is uneven until it has spread from the grains' boundaries over the
+  // grid, some five iterations, or, in a problem that stays so, always.
+  bool fx_uneven = false;
+  int fx_even = 1;
   double* hx = nullptr;
   double* hy = nullptr;
   double* hd = nullptr;
@@ -164,7 +169,7 @@ struct e3d_handle {
   double gg0 = 0.0;
   bool uploaded = false, femat_done = false, energy_done = false, solve_ready = false, minv_ready = false;
   int pcg_grid = 0;
-  int pcg_grid_fx = 0;
+  int pcg_grid_fx = 0, pcg_grid_uneven = 0;
   int pcg_grid32 = 0;
   double ms_setup = 0.0, ms_iter = 0.0;
   JumpParams J{};
@@ -235,9 +240,9 @@ struct PcgForm {
   int threads, smem;
 };
 
-template <typename T, bool FX, int V>
+template <typename T, bool FX, int V, bool UNEVEN = false>
 PcgForm pcg_form_of() {
-  return {(const void*)pcg_persistent_kernel<T, false, FX, V>, FX ? kFxThreads : NT, pcg_dyn_smem_bytes<T, FX, V>()};
+  return {(const void*)pcg_persistent_kernel<T, false, FX, V, UNEVEN>, FX ? kFxThreads : NT, pcg_dyn_smem_bytes<T, FX, V>()};
 }
 
 // The form for a solve: phase B takes two nodes of a row at a time where every row
@@ -253,6 +258,8 @@ PcgForm pcg_form(const e3d_handle* h, bool fx) {
     return nx % 2 == 0 ? pcg_form_of<T, true, 2>() : pcg_form_of<T, true, 1>();
   }
 }
+
+PcgForm pcg_uneven_form() { return pcg_form_of<double, true, 1, true>(); }
 
 PcgForm pcg_ring_form() { return {(const void*)pcg_persistent_kernel<float, true, false, 1>, NT, kRingSmemBytes}; }
 
@@ -295,10 +302,11 @@ int32_t launch_apply_tiles(e3d_handle* h, const double* x, double* y) {
   ApplyArgs<double> A = apply_args(h, x, y);
   if (h->fx_ok) {
     A.g = h->Gx;
-    tile_max_kernel<<<(unsigned)h->Gx.ntiles, kFxThreads, 0, h->stream>>>(h->Gx, x, h->mz);
+    // (a solve finds its own row maxima again when it goes on)
+    tile_max_kernel<<<(unsigned)h->Gx.ntiles, kFxThreads, 0, h->stream>>>(h->Gx, x, h->mh0, h->mh1);
     E3D_LAUNCHED(h);
     apply_tiles_fx_kernel<<<(unsigned)h->Gx.ntiles, kFxThreads, sizeof(FxSmem<false>), h->stream>>>(
-        A, FxArgs{h->fxtab, h->fx_kc, h->mz, nullptr});
+        A, FxArgs{h->fxtab, h->fx_kc, nullptr}, FxRowMax{h->mh0, h->mh1});
     E3D_LAUNCHED(h);
     return E3D_OK;
   }
@@ -428,6 +436,7 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
     return fail(cuda_fail(e, "occupancy"));
   for (auto [form, grid] : {std::pair{pcg_form<double>(h, false), &h->pcg_grid},
                             std::pair{pcg_form<double>(h, true), &h->pcg_grid_fx},
+                            std::pair{pcg_uneven_form(), &h->pcg_grid_uneven},
                             std::pair{pcg_form<float>(h, false), &h->pcg_grid32}}) {
     int per_sm = 0;
     if ((e = pcg_blocks_per_sm(form, &per_sm)) != cudaSuccess) return fail(cuda_fail(e, "occupancy"));
@@ -438,7 +447,7 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
   if (p->precision == E3D_PREC_MIXED &&
       (e = pcg_blocks_per_sm(pcg_ring_form(), &per_sm_tma)) != cudaSuccess)
     return fail(cuda_fail(e, "occupancy (TMA)"));
-  h->partial_n = std::max({h->pcg_grid, h->pcg_grid_fx, h->pcg_grid32, h->num_sms * 4}) * 12;
+  h->partial_n = std::max({h->pcg_grid, h->pcg_grid_fx, h->pcg_grid_uneven, h->pcg_grid32, h->num_sms * 4}) * 12;
   const long long halo = h->G.ntiles * h->G.tz, halo_x = h->Gx.ntiles * h->Gx.tz;
   const size_t tile_rows = (size_t)h->Gx.ntiles * kFxRows;
   int32_t rc = E3D_OK;
@@ -446,7 +455,7 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
       (rc = dalloc(h, &h->cmod, 36 * (size_t)np)) || (rc = dalloc(h, &h->cs, kCsStride * (size_t)np)) ||
       (rc = dalloc(h, &h->cs32, kCs32Stride * (size_t)np)) || (rc = dalloc(h, &h->dk, 576 * (size_t)np)) ||
       (rc = dalloc(h, &h->dkd, kDkdStride * (size_t)np)) || (rc = dalloc(h, &h->norms, 3 * (size_t)np)) ||
-      (rc = dalloc(h, &h->fxtab, kFxStride * (size_t)np)) || (rc = dalloc(h, &h->mz, tile_rows)) ||
+      (rc = dalloc(h, &h->fxtab, kFxStride * (size_t)np)) || (rc = dalloc(h, &h->mz, 2 * tile_rows)) ||
       (rc = dalloc(h, &h->phsums, 12 * (size_t)np + 1)) ||
       (rc = dalloc(h, &h->mh0, tile_rows)) || (rc = dalloc(h, &h->mh1, tile_rows)) || (rc = dalloc(h, &h->u, n3)) || (rc = dalloc(h, &h->g, n3)) ||
       (rc = dalloc(h, &h->b, n3)) || (rc = dalloc(h, &h->z, n3)) || (rc = dalloc(h, &h->h0, n3)) ||
@@ -481,10 +490,6 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
   if ((e = cudaMemsetAsync(h->err, 0, sizeof(int), h->stream)) != cudaSuccess) return fail(cuda_fail(e, "memset"));
   if ((e = cudaMemsetAsync(h->bar, 0, sizeof(GridBarrier), h->stream)) != cudaSuccess)
     return fail(cuda_fail(e, "memset"));
-  // tile rows past the grid are never written: they stay zero
-  for (unsigned* q : {h->mz, h->mh0, h->mh1})
-    if ((e = cudaMemsetAsync(q, 0, sizeof(unsigned) * tile_rows, h->stream)) != cudaSuccess)
-      return fail(cuda_fail(e, "memset"));
   if ((e = cudaMemsetAsync(h->h0, 0, sizeof(double) * n3, h->stream)) != cudaSuccess)
     return fail(cuda_fail(e, "memset"));
   if ((e = cudaMemsetAsync(h->h1, 0, sizeof(double) * n3, h->stream)) != cudaSuccess)
@@ -711,7 +716,8 @@ int32_t e3d_solve_begin(e3d_handle_t* h) {
   h->since_replace = 0;
   h->minv_ready = true;
   h->solve_ready = true;
-  h->fx_pcg = h->fx_ok;
+  h->fx_uneven = false;
+  h->fx_even = 1;
   return E3D_OK;
 }
 
@@ -768,6 +774,7 @@ PcgArgs<double> pcg_args<double>(e3d_handle* h) {
   P.mh0 = h->mh0;
   P.mh1 = h->mh1;
   P.fxleave = h->fxleave;
+  P.fxeven = h->fx_even;
   return P;
 }
 
@@ -795,8 +802,10 @@ PcgArgs<float> pcg_args<float>(e3d_handle* h) {
 template <typename T>
 int32_t launch_pcg(e3d_handle* h, int it_limit) {
   const bool tma = sizeof(T) == 4 && h->maps != nullptr;
-  const bool fx = sizeof(T) == 8 && h->fx_pcg;
-  const int grid = fx               ? h->pcg_grid_fx
+  const bool fx = sizeof(T) == 8 && h->fx_ok;
+  const bool uneven = fx && h->fx_uneven;
+  const int grid = uneven           ? h->pcg_grid_uneven
+                   : fx             ? h->pcg_grid_fx
                    : sizeof(T) == 8 ? h->pcg_grid
                    : tma            ? h->pcg_grid32_tma
                                     : h->pcg_grid32;
@@ -813,7 +822,7 @@ int32_t launch_pcg(e3d_handle* h, int it_limit) {
   E3D_CUDA(cudaMemsetAsync(h->bar, 0, sizeof(GridBarrier), h->stream));
   if (fx) E3D_CUDA(cudaMemsetAsync(h->fxleave, 0, sizeof(int), h->stream));
   void* args[] = {&P};
-  const PcgForm F = tma ? pcg_ring_form() : pcg_form<T>(h, fx);
+  const PcgForm F = tma ? pcg_ring_form() : uneven ? pcg_uneven_form() : pcg_form<T>(h, fx);
   if constexpr (sizeof(T) == 8)
     if (fx) P.A.g = h->Gx;
   cudaError_t e = cudaLaunchCooperativeKernel(F.fn, dim3(grid), dim3(F.threads), args, F.smem, h->stream);
@@ -881,6 +890,7 @@ int32_t e3d_iterate(e3d_handle_t* h, int32_t n, e3d_solve_stats_t* st) {
   while (remaining > 0 && S.status == PCG_RUNNING) {
     int chunk = std::min(remaining, 256);
     if (mixed) chunk = std::min(chunk, R - h->since_replace);
+    const bool fx = !mixed && h->fx_ok;
     const int it0 = S.it;
     rc = mixed ? launch_pcg<float>(h, chunk) : launch_pcg<double>(h, chunk);
     if (rc) break;
@@ -897,8 +907,11 @@ int32_t e3d_iterate(e3d_handle_t* h, int32_t n, e3d_solve_stats_t* st) {
         if ((rc = read_state(h, &S))) break;
       }
     }
-    if (S.status == PCG_RUNNING && !mixed && h->fx_pcg && done < chunk) {
-      h->fx_pcg = false;  // values out of the fixed-point range: on in the FP64 form
+    if (fx && h->fx_uneven) {
+      h->fx_uneven = S.since_replace < h->fx_even;
+    } else if (fx && S.status == PCG_RUNNING && done < chunk) {  // it left at an uneven tile
+      h->fx_uneven = true;
+      h->fx_even = std::min(2 * h->fx_even, 64);
       continue;
     }
     if (done == 0 && S.status == PCG_RUNNING) break;  // nothing advanced: do not spin
@@ -943,9 +956,9 @@ int32_t e3d_stress(e3d_handle_t* h, double strav[6], double epsav[6]) {
   const int pgrid = (int)std::min<long long>(std::min(reduction_grid(h), h->partial_n / 12), h->Gx.ntiles);
   int* info = reinterpret_cast<int*>(h->phsums + 12 * (size_t)np);
   E3D_CUDA(cudaMemsetAsync(h->phsums, 0, 12 * sizeof(unsigned long long) * np, h->stream));
-  tile_max_kernel<<<tiles, kFxThreads, 0, h->stream>>>(h->Gx, h->u, h->mz);
+  tile_max_kernel<<<tiles, kFxThreads, 0, h->stream>>>(h->Gx, h->u, h->mh0, h->mh1);
   E3D_LAUNCHED(h);
-  stress_sums_kernel<<<tiles, kFxThreads, 0, h->stream>>>(h->Gx, h->J, h->pix, h->cmod, np, h->u, h->mz, h->phsums, info,
+  stress_sums_kernel<<<tiles, kFxThreads, 0, h->stream>>>(h->Gx, h->J, h->pix, h->cmod, np, h->u, h->mh0, h->phsums, info,
                                                           h->partial, pgrid);
   E3D_LAUNCHED(h);
   stress_total_kernel<<<1, 256, 0, h->stream>>>(np, h->phsums, info, h->cmod, h->partial, pgrid, h->scalars);
@@ -1339,7 +1352,10 @@ extern "C" int32_t e3d_checkpoint_save(e3d_handle_t* h, const char* path) {
   H.gg0 = h->gg0;
   E3D_CUDA(cudaMemcpyAsync(&H.st, h->st, sizeof(PcgState), cudaMemcpyDeviceToHost, h->stream));
   E3D_CUDA(cudaStreamSynchronize(h->stream));
-  H.st.since_replace = h->since_replace;
+  if (mixed)
+    H.st.since_replace = h->since_replace;
+  else  // a field that this form has no other use for
+    H.st.final_ready = 2 * h->fx_even + h->fx_uneven;
   FILE* f = std::fopen(path, "wb");
   if (!f) return E3D_ERR_INPUT;
   const size_t n3 = 3 * (size_t)h->G.ns;
@@ -1382,6 +1398,7 @@ extern "C" int32_t e3d_checkpoint_load(e3d_handle_t* h, const char* path) {
   }
   const size_t n3 = 3 * (size_t)h->G.ns;
   PcgState S = H.st;
+  S.final_ready = 0;
   int32_t rc = ckpt_read(f, h->u, n3, h->stream);
   if (!rc) rc = ckpt_read(f, h->g, n3, h->stream);
   if (!mixed) {
@@ -1402,8 +1419,9 @@ extern "C" int32_t e3d_checkpoint_load(e3d_handle_t* h, const char* path) {
   rc = sync(h);
   if (rc) return rc;
   h->gg0 = H.gg0;
-  h->since_replace = S.since_replace;
-  h->fx_pcg = h->fx_ok;
+  h->since_replace = mixed ? S.since_replace : 0;
+  h->fx_uneven = !mixed && (H.st.final_ready & 1);
+  h->fx_even = std::clamp(H.st.final_ready / 2, 1, 64);  // (zero in older files)
   h->energy_done = true;
   h->minv_ready = true;
   h->solve_ready = true;

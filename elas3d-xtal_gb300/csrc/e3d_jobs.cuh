@@ -300,7 +300,7 @@ static __device__ __noinline__ bool job_fp64_apply_tiles(const JobDesc& J, int p
   if (kx != kFxGeneral) {
     const int group = threadIdx.x / kFxThreads;
     FxSmem<false>& sm = reinterpret_cast<FxSmem<false>*>(dyn)[group];
-    const FxArgs F{J.fxtab, (int)J.fxinfo[0], nullptr, nullptr};
+    const FxArgs F{J.fxtab, (int)J.fxinfo[0], nullptr};
     for (long long t = (long long)part * kGroups + group; t < J.Gx.ntiles; t += (long long)J.nparts * kGroups)
       apply_tile_fx<false, true>(sA, F, kx, t, sm, dummy);
     __syncthreads();

@@ -1026,13 +1026,10 @@ constexpr int kFxRows = 4;
 constexpr int kFxThreads = TILE_X * kFxRows;
 constexpr int kFxBlocks = 2;
 
-// Largest |value| of each tile, kept as the high word of the double (sign
-// cleared) per warp row: word tile * kFxRows + ty.
 struct FxArgs {
   const int4* __restrict__ tab;  // kFxStride int4 per phase
   int kc;                        // table exponent
-  unsigned* mx;                  // tile maxima of A.x (written for h_new when fused)
-  unsigned* mz;                  // tile maxima of A.zv (fused only)
+  unsigned* mx;                  // fused: row maxima of h_new, written here
 };
 
 template <bool FUSED>
@@ -1071,44 +1068,66 @@ __device__ __forceinline__ int fx_exponent(unsigned hi) {
   return fx_exponent_below(hi ? __hiloint2double((int)hi + 1, 0) : 0.0);
 }
 
-// Exponent kx of a tile: 2^kx * |value| < 2^kFxNodeBits for every node that the
-// tile reads (its own and the surrounding tiles' maxima; for h_new = z + gamma
-// h_old the bound is max|z| + |gamma| max|h_old|).  kFxGeneral where a value is
-// not finite or the exponent leaves the range of exponent arithmetic: the tile
-// then takes the FP64 form.  All threads call it; every thread gets the result.
-static __device__ __forceinline__ int fx_tile_exponent(const GridDims& G, long long tile, const unsigned* mx,
-                                                       const unsigned* mz, double gamma, unsigned (&red)[2 * kFxRows]) {
-  const int tid = threadIdx.x;
-  static_assert(27 * kFxRows <= kFxThreads, "one load a thread");
-  unsigned bx = 0, bz = 0;
-  if (tid < 27 * kFxRows) {
-    const int nb = tid / kFxRows, row = tid % kFxRows;
+// How much smaller than the largest value that a tile reads its parts may be, in
+// powers of two.  A tile's values share one exponent, so that a part 2^s smaller is
+// held to 2^-(56 - s) of itself.  Error of K.x there over that of the FP64 form,
+// measured with s from the typical size to the peak: 0.6 at s = 2, 1 at 4, 7 at 7, 57
+// at 10 (1.6e-15 of the part's own size).  Random vectors, the directions of a
+// solve from its fifth iteration on and displacements stay within these; a few
+// entries far above the rest, a direction that has not reached all of the grid
+// yet, and a rigid offset of one component do not: such a tile takes the FP64 form.
+constexpr unsigned kFxRow = 5;         // a row of the tile over all its planes
+constexpr unsigned kFxSegment = 8;     // a row of one plane (stand-alone pass only)
+constexpr unsigned kFxComponent = 10;  // one component of a row (stand-alone pass only)
+
+// What fx_tile_exponent asks of the rows of a tile, per row of 32 nodes over all
+// planes, words tile * kFxRows + row: m, the largest |value| as the high word of the
+// double; lim, the largest exponent that the tile's scale may have by the
+// limits above.
+struct FxRowMax {
+  const unsigned* m;
+  const unsigned* lim;
+};
+// The same of h_new = z + gamma h_old before it is formed: the largest |h_old| (null: a
+// reset) and |z| (two words a row, tile * 2 * kFxRows + row and + kFxRows).
+struct FxRowMaxFused {
+  const unsigned* h;
+  const unsigned* z;
+  double gamma;
+};
+
+// Exponent kx of a tile: 2^kx * |value| < 2^kFxNodeBits for every node that the tile
+// reads: its own rows, those of the next tile in x, the first of the next in y, and
+// of all these the planes above and below.  kFxGeneral where a value is not finite,
+// the exponent leaves the range of exponent arithmetic or the values are uneven.
+// Every warp finds it by itself, a row a lane.
+template <typename Rows>
+static __device__ __forceinline__ int fx_tile_exponent(const GridDims& G, long long tile, const Rows& R) {
+  const int lane = threadIdx.x & 31;
+  unsigned w = 0, limit = 0xffffffffu;  // bound of the row's values, and the largest exponent it allows
+  if (lane < 30) {
+    const int row = lane % 5, nb = lane / 5;
     const int tix = (int)(tile % G.ntx), tiy = (int)((tile / G.ntx) % G.nty),
               tiz = (int)(tile / ((long long)G.ntx * G.nty));
-    const int ax = wrapi(tix + nb % 3 - 1, G.ntx), ay = wrapi(tiy + (nb / 3) % 3 - 1, G.nty),
-              az = wrapi(tiz + nb / 9 - 1, G.ntz);
-    const long long t = E3D_IDX((ax + (long long)G.ntx * (ay + (long long)G.nty * az)) * kFxRows + row,
-                                G.ntiles * kFxRows);
-    if (mx) bx = __ldcg(mx + t);
-    if (mz) bz = __ldcg(mz + t);
+    const int ax = wrapi(tix + nb / 3, G.ntx), ay = wrapi(tiy + row / 4, G.nty), az = wrapi(tiz + nb % 3 - 1, G.ntz);
+    const long long t = E3D_IDX(ax + (long long)G.ntx * (ay + (long long)G.nty * az), G.ntiles);
+    const int r = row % 4;
+    if constexpr (std::is_same_v<Rows, FxRowMaxFused>) {
+      const unsigned bx = R.h ? __ldcg(R.h + t * kFxRows + r) : 0u;
+      const unsigned bz = max(__ldcg(R.z + t * 2 * kFxRows + r), __ldcg(R.z + t * 2 * kFxRows + kFxRows + r));
+      const double vx = bx ? __hiloint2double((int)bx + 1, 0) : 0.0, vz = bz ? __hiloint2double((int)bz + 1, 0) : 0.0;
+      w = max(bx, bz) >= 0x7ff00000u ? 0x7ff00000u : abs_hi(fma(fabs(R.gamma), vx, vz));
+      if (w) limit = (w >> 20) + kFxRow;
+    } else {
+      w = __ldcg(R.m + t * kFxRows + r);
+      limit = __ldcg(R.lim + t * kFxRows + r);
+    }
   }
-  bx = __reduce_max_sync(0xffffffffu, bx);
-  bz = __reduce_max_sync(0xffffffffu, bz);
-  __syncthreads();  // the previous use of red is over
-  if ((tid & 31) == 0) {
-    red[tid >> 5] = bx;
-    red[kFxRows + (tid >> 5)] = bz;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < kFxRows; ++i) {
-    bx = max(bx, red[i]);
-    bz = max(bz, red[kFxRows + i]);
-  }
-  if (!mz) return fx_exponent(bx);
-  if (bx >= 0x7ff00000u || bz >= 0x7ff00000u) return kFxGeneral;
-  const double vx = bx ? __hiloint2double((int)bx + 1, 0) : 0.0, vz = bz ? __hiloint2double((int)bz + 1, 0) : 0.0;
-  return fx_exponent_below(fma(fabs(gamma), vx, vz));
+  static_assert(kFxRows == 4, "30 rows: a tile's, times two in x and three in z, and the next one's first");
+  w = __reduce_max_sync(0xffffffffu, w);
+  limit = __reduce_min_sync(0xffffffffu, limit);
+  if ((w + 1) >> 20 > limit) return kFxGeneral;
+  return fx_exponent(w);
 }
 
 // apply_tile<double, FUSED> with the element products in fixed point: the same
@@ -1354,11 +1373,21 @@ static __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& A,
   }
 }
 
-// A tile that leaves the range of the fixed-point form: the FP64 form, out of line.
+// A tile that the fixed-point form does not take: the FP64 form, out of line.
 static __device__ __noinline__ void apply_tile_general(const ApplyArgs<double>& A, long long tile,
                                                        ApplySmem<double, kFxRows>& sm) {
   double dot = 0.0;
   apply_tile<double, false, false, false, kFxRows>(A, tile, sm, dot);
+}
+__device__ __forceinline__ unsigned tile_row_max(const GridDims& G, long long tile, const double* x);
+// The same, fused, with the row maxima of h_new; returns the thread's share of h . A h.
+static __device__ __noinline__ double apply_tile_general_fused(const ApplyArgs<double>& A, long long tile,
+                                                               ApplySmem<double, kFxRows>& sm, unsigned* mx) {
+  double dot = 0.0;
+  apply_tile<double, true, false, false, kFxRows>(A, tile, sm, dot);
+  const unsigned v = tile_row_max(A.g, tile, A.hnew);  // the thread's own stores
+  if (threadIdx.x % TILE_X == 0) mx[E3D_IDX(tile * kFxRows + threadIdx.x / TILE_X, A.g.ntiles * kFxRows)] = v;
+  return dot;
 }
 
 // Shared memory of apply_tile_ring: the in-plane force exchange of the ZS
@@ -1635,14 +1664,40 @@ __global__ void __launch_bounds__(NT, 1) apply_tiles_kernel(ApplyArgs<T> A, doub
   if (partial && threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
-// Tile maxima of a nodal vector: one block per tile.
-template <int TY>
-__device__ __forceinline__ void tile_max(const GridDims& G, long long tile, const double* __restrict__ x,
-                                         unsigned* __restrict__ mx) {
+// Bound of |v| as FxRowMax keeps it: zero for zero alone.
+__device__ __forceinline__ unsigned size_word(double v) { return abs_hi(v) | (__double2loint(v) != 0 ? 1u : 0u); }
+
+// Row maxima of a warp's row of nodes, plane by plane (FxRowMax); all lanes take part.
+struct FxRowScan {
+  unsigned comp[3] = {0, 0, 0}, segment = 0xffffffffu;
+  __device__ __forceinline__ void plane(unsigned a, unsigned b, unsigned c) {
+    comp[0] = max(comp[0], a);
+    comp[1] = max(comp[1], b);
+    comp[2] = max(comp[2], c);
+    const unsigned seg = __reduce_max_sync(0xffffffffu, max(a, max(b, c)));
+    if (seg) segment = min(segment, seg);
+  }
+  // The row's words, the same in every lane.
+  __device__ __forceinline__ void finish(unsigned& m, unsigned& lim) {
+    m = 0;
+    lim = segment == 0xffffffffu ? segment : (segment >> 20) + kFxSegment;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const unsigned v = __reduce_max_sync(0xffffffffu, comp[c]);
+      m = max(m, v);
+      if (v) lim = min(lim, (v >> 20) + kFxComponent);
+    }
+    if (m) lim = min(lim, (m >> 20) + kFxRow);
+  }
+};
+
+// Row maxima of a tile of a nodal vector, one block a tile: the largest |value|
+// alone, for a solve's own vectors.
+__device__ __forceinline__ unsigned tile_row_max(const GridDims& G, long long tile, const double* x) {
   const int tx = threadIdx.x % TILE_X, ty = threadIdx.x / TILE_X;
   const int tix = (int)(tile % G.ntx), tiy = (int)((tile / G.ntx) % G.nty),
             tiz = (int)(tile / ((long long)G.ntx * G.nty));
-  const int xg = tix * TILE_X + tx, yg = tiy * TY + ty, z0 = tiz * G.tz, z1 = min(G.nz, z0 + G.tz);
+  const int xg = tix * TILE_X + tx, yg = tiy * kFxRows + ty, z0 = tiz * G.tz, z1 = min(G.nz, z0 + G.tz);
   unsigned v = 0;
   if (xg < G.nx && yg < G.ny) {
     const long long nxy = (long long)G.nx * G.ny;
@@ -1653,25 +1708,47 @@ __device__ __forceinline__ void tile_max(const GridDims& G, long long tile, cons
       v = max(v, max(a, max(b, c)));
     }
   }
-  v = __reduce_max_sync(0xffffffffu, v);
-  if ((threadIdx.x & 31) == 0) mx[E3D_IDX(tile * TY + ty, G.ntiles * TY)] = v;
+  return __reduce_max_sync(0xffffffffu, v);
 }
 
 static __global__ void __launch_bounds__(kFxThreads) tile_max_kernel(GridDims G, const double* __restrict__ x,
-                                                                     unsigned* __restrict__ mx) {
-  tile_max<kFxRows>(G, blockIdx.x, x, mx);
+                                                                     unsigned* __restrict__ m, unsigned* __restrict__ lim) {
+  const long long tile = blockIdx.x;
+  const int tx = threadIdx.x % TILE_X, ty = threadIdx.x / TILE_X;
+  const int tix = (int)(tile % G.ntx), tiy = (int)((tile / G.ntx) % G.nty),
+            tiz = (int)(tile / ((long long)G.ntx * G.nty));
+  const int xg = tix * TILE_X + tx, yg = tiy * kFxRows + ty, z0 = tiz * G.tz, z1 = min(G.nz, z0 + G.tz);
+  const bool active = xg < G.nx && yg < G.ny;
+  const long long nxy = (long long)G.nx * G.ny;
+  const double* col = x + E3D_IDX(active ? xg + (long long)G.nx * yg + nxy * z0 : 0, G.ns);
+  FxRowScan scan;
+#pragma unroll 4
+  for (int z = z0; z < z1; ++z, col += nxy) {
+    unsigned a = 0, b = 0, c = 0;
+    if (active) {
+      a = size_word(__ldcg(col));
+      b = size_word(__ldcg(col + G.ns));
+      c = size_word(__ldcg(col + 2 * G.ns));
+    }
+    scan.plane(a, b, c);
+  }
+  unsigned vm, vl;
+  scan.finish(vm, vl);
+  if (tx == 0) {
+    m[E3D_IDX(tile * kFxRows + ty, G.ntiles * kFxRows)] = vm;
+    lim[E3D_IDX(tile * kFxRows + ty, G.ntiles * kFxRows)] = vl;
+  }
 }
 
-// The stand-alone FP64 apply in fixed point, one tile a block; F.mx holds the
-// tile maxima of A.x.
-static __global__ void __launch_bounds__(kFxThreads, kFxBlocks) apply_tiles_fx_kernel(ApplyArgs<double> A, FxArgs F) {
+// The stand-alone FP64 apply in fixed point, one tile a block; R: of A.x.
+static __global__ void __launch_bounds__(kFxThreads, kFxBlocks) apply_tiles_fx_kernel(ApplyArgs<double> A, FxArgs F,
+                                                                                      FxRowMax R) {
   extern __shared__ __align__(128) unsigned char e3d_fx_dyn[];  // sizeof(FxSmem<false>)
   FxSmem<false>& sm = *reinterpret_cast<FxSmem<false>*>(e3d_fx_dyn);
   static_assert(sizeof(ApplySmem<double, kFxRows>) <= sizeof(FxSmem<false>), "the FP64 form shares the memory");
-  __shared__ unsigned mred[2 * kFxRows];
   __shared__ ApplyArgs<double> sA;
   double dummy = 0.0;
-  const int kx = fx_tile_exponent(A.g, blockIdx.x, F.mx, nullptr, 0.0, mred);
+  const int kx = fx_tile_exponent(A.g, blockIdx.x, R);
   if (kx != kFxGeneral) {
     apply_tile_fx<false>(A, F, kx, blockIdx.x, sm, dummy);
   } else {
@@ -2696,8 +2773,7 @@ __device__ __forceinline__ double pcg_update_tiles(const GridDims& G, long long 
 // instead of one (four stages): FP32 500^3 6.00 -> 5.72 ms, 200^3 .414 -> .389, 100^3
 // .0757 -> .0716; FP64 300^3 4.63 -> 4.52.  Four nodes a thread: 500^3 6.29.  The
 // grid's warps side by side along memory instead of tile by tile: 8.0.
-// ZMAX: the tile's maxima of the new z, one a warp, go to mz (the next pass's
-// fixed-point scale).
+// ZMAX: the row maxima of the new z go to mz (FxRowMaxFused, for the next pass).
 template <int BYTES>
 __device__ __forceinline__ void cp_async_n(void* dst, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -2888,9 +2964,12 @@ __device__ __forceinline__ double pcg_update_tiles_v(const GridDims& G, long lon
 #pragma unroll
       for (int c = 0; c < 3; ++c) *reinterpret_cast<Vec*>(z + E3D_IDX(value_of(m, c, ns), 3 * ns)) = zv[c];
     }
-    if constexpr (ZMAX) {
-      zmax = __reduce_max_sync(0xffffffffu, zmax);
-      if ((tid & 31) == 0) mz[E3D_IDX(t * (NTH / 32) + tid / 32, G.ntiles * (NTH / 32))] = zmax;
+    if constexpr (ZMAX) {  // a thread's nodes lie in one row; slots rs and rs + TY are of the same
+      static_assert(R == TY || R == 2 * TY, "one slot a row, or two");
+      const int half = V == 2 ? (tid & 31) / kLanes : 0;
+      const unsigned a = __reduce_max_sync(0xffffffffu, half ? 0u : zmax),
+                     b = V == 2 ? __reduce_max_sync(0xffffffffu, half ? zmax : 0u) : 0u;
+      if (tid % kLanes == 0) mz[E3D_IDX(t * 2 * TY + rs, G.ntiles * 2 * TY)] = half ? b : a;
     }
     if constexpr (sizeof(T) == 4) zg_t += (double)zg32;
     cp_async_wait<0>();
@@ -2961,7 +3040,9 @@ struct PcgState {
   double rel_at_replace;  // mixed form: rel_res of the last FP64 residual (set-up or replacement)
   double refine_drop;     // mixed form: replace once rel_res < refine_drop * rel_at_replace (0: never)
   int it, status, reset, resets, cur, max_iter, divergence_reset, refinements;
-  int since_replace, final_ready;  // final_ready: the job engine ended on a converged FP64 replacement
+  // FP32 forms: iterations since the last replacement; FP64: see UNEVEN below
+  int since_replace;
+  int final_ready;  // the job engine ended on a converged FP64 replacement
 };
 
 struct GridBarrier {
@@ -3065,20 +3146,26 @@ struct PcgArgs {
   int it_limit;
   unsigned long long timeout_ns;
   const PlaneMaps* maps;  // TMA form only
-  // fixed-point form only: tables, and the tile maxima of z, h0 and h1
+  // fixed-point form only: tables, and the row maxima of z, h0 and h1
   const int4* fxtab;
   int fxkc;
   unsigned* mz;
   unsigned* mh0;
   unsigned* mh1;
-  int* fxleave;  // set by a tile whose values leave the fixed-point range
+  int* fxleave;  // set where a tile needs the FP64 form (UNEVEN: to the iteration)
+  int fxeven;    // UNEVEN: iterations without such a tile, in a row, that end the launch
 };
 
 // TMA (FP32 only): phase A reads its node planes through the block's plane
 // ring (dynamic shared memory of kRingSmemBytes).  FX (FP64 only): phase A in
 // fixed point, each tile scaled by its own values.  V: nodes of a row a thread
 // takes at a time in phase B, what the rows' alignment allows.
-template <typename T, bool TMA, bool FX, int V>
+// UNEVEN (with FX): tiles that fixed point does not take go through the FP64 form,
+// instead of ending the launch, until there is none for some iterations (counted in
+// PcgState::since_replace).  A form of its own: with the FP64 form in the kernel,
+// in line or called, the fixed-point sweep has too few registers (an iteration at
+// 300^3 4.5 ms without, 6.6 with).
+template <typename T, bool TMA, bool FX, int V, bool UNEVEN = false>
 __global__ void __launch_bounds__(FX ? kFxThreads : NT,
                                   FX               ? kFxBlocks
                                   : sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 ? 1 : E3D_F32_BLOCKS_PER_SM)
@@ -3109,11 +3196,16 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
   constexpr bool kDeferU = sizeof(T) == 4 && !TMA;
   T lam_pending = T(0);  // kDeferU: du -= lam_pending * h_pending not yet applied
   const T* h_pending = nullptr;
-  __shared__ unsigned mred[2 * kFxRows];
-  if constexpr (FX) {  // tile maxima of the vectors that this launch starts from
+  if constexpr (FX) {  // row maxima of the vectors that this launch starts from
     for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x) {
-      tile_max<TY>(G, t, P.z, P.mz);
-      if (!s.reset) tile_max<TY>(G, t, s.cur ? P.h1 : P.h0, s.cur ? P.mh1 : P.mh0);
+      const unsigned z = tile_row_max(G, t, P.z);
+      const unsigned h = s.reset ? 0u : tile_row_max(G, t, s.cur ? P.h1 : P.h0);
+      if (threadIdx.x % TILE_X == 0) {
+        const int row = threadIdx.x / TILE_X;
+        P.mz[E3D_IDX(t * 2 * TY + row, G.ntiles * 2 * TY)] = z;
+        P.mz[E3D_IDX(t * 2 * TY + TY + row, G.ntiles * 2 * TY)] = 0u;
+        (s.cur ? P.mh1 : P.mh0)[E3D_IDX(t * TY + row, G.ntiles * TY)] = h;
+      }
     }
     if (!grid_barrier(P.bar, P.err, P.timeout_ns)) {
       if (blockIdx.x == 0 && lead) {
@@ -3139,20 +3231,40 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
     }
     double hAh_t = 0.0;
     if constexpr (TMA) ring_begin(ring, G, cur ? P.maps->h1 : P.maps->h0, blockIdx.x, gridDim.x, G.ntiles);
+    bool general = false;  // UNEVEN: tiles left to the FP64 form
     for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x) {
       if constexpr (TMA) {
         apply_tile_ring<E3D_RING_ZS>(A, t, sm, hAh_t, ring);
       } else if constexpr (FX) {
-        const FxArgs F{P.fxtab, P.fxkc, cur ? P.mh0 : P.mh1, P.mz};
-        const int kx = fx_tile_exponent(G, t, A.reset ? nullptr : cur ? P.mh1 : P.mh0, P.mz, A.gamma, mred);
+        const FxArgs F{P.fxtab, P.fxkc, cur ? P.mh0 : P.mh1};
+        const int kx = fx_tile_exponent(G, t, FxRowMaxFused{A.reset ? nullptr : cur ? P.mh1 : P.mh0, P.mz, A.gamma});
         if (kx != kFxGeneral)
           apply_tile_fx<true>(A, F, kx, t, *reinterpret_cast<FxSmem<true>*>(e3d_pcg_smem), hAh_t);
+        else if constexpr (UNEVEN)
+          general = true;
         else if (lead)
           *P.fxleave = 1;
       } else {
         apply_tile<T, true, (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), kDeferU>(A, t, sm, hAh_t);
       }
       __syncthreads();
+    }
+    if constexpr (UNEVEN) {
+      if (general) {
+        __shared__ ApplyArgs<double> sA;
+        if (lead) {
+          sA = A;
+          *P.fxleave = s.it + 1;
+        }
+        __syncthreads();
+        const FxRowMaxFused R{sA.reset ? nullptr : cur ? P.mh1 : P.mh0, P.mz, sA.gamma};
+        for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x)
+          if (fx_tile_exponent(G, t, R) == kFxGeneral) {
+            hAh_t += apply_tile_general_fused(sA, t, *reinterpret_cast<ApplySmem<double, TY>*>(e3d_pcg_smem),
+                                              cur ? P.mh0 : P.mh1);
+            __syncthreads();
+          }
+      }
     }
     {
       const double bs = block_sum<NT>(hAh_t, red);
@@ -3163,11 +3275,16 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
       if (lead) s.status = PCG_TIMEOUT;
       break;
     }
-    if constexpr (FX) {
-      // values that the fixed-point form cannot take: leave before anything but
-      // h_new and A h is written; the host goes on with the FP64 form
-      if (__ldcg(P.fxleave)) break;
+    if constexpr (FX && !UNEVEN) {
+      // a tile that needs the FP64 form: leave before anything but h_new and A h is
+      // written; the host goes on with the UNEVEN form
+      if (__ldcg(P.fxleave)) {
+        if (lead) s.since_replace = 0;
+        break;
+      }
     }
+    if constexpr (UNEVEN)
+      if (lead) s.since_replace = __ldcg(P.fxleave) == s.it + 1 ? 0 : s.since_replace + 1;
     lam_pending = T(0);  // applied by this phase A
     const double hAh = reduce_broadcast<NT>(P.partA, gridDim.x, red);
     if (lead) {
@@ -3235,6 +3352,8 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
     }
     __syncthreads();
     if (s.status != PCG_RUNNING) break;
+    if constexpr (UNEVEN)
+      if (s.since_replace >= P.fxeven) break;
   }
   __syncthreads();
   if (lead && s.status == PCG_RUNNING && s.it >= s.max_iter) s.status = PCG_MAXITER;

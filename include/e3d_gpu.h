@@ -162,7 +162,14 @@ int32_t e3d_stress_field(e3d_handle_t* h, double* sigma, double* vm);
 int32_t e3d_run(e3d_handle_t* h, double utot[2], double out12[12], e3d_solve_stats_t* st);
 
 /* Matrix-free y = K x (the stencil of :1585-1883 without b), host buffers of
- * 3*ns doubles.  e3d_apply_device takes device pointers instead. */
+ * 3*ns doubles.  e3d_apply_device takes device pointers instead.
+ * Products are formed in FP64, or in 64-bit fixed point with one exponent for the
+ * values that a tile of 32 x 4 columns reads, whose error is below FP64's where
+ * these are of one order.  A tile takes FP64 where a row of it is more than 2^5
+ * below its largest value, a row of one plane more than 2^8 or one component of a
+ * row more than 2^10, and where values are not finite or beyond 2^+-400; so does
+ * the whole problem where the phases' stiffnesses differ by more than a factor 8 or
+ * are indefinite. */
 int32_t e3d_apply(e3d_handle_t* h, const double* x, double* y);
 int32_t e3d_apply_device(e3d_handle_t* h, const double* d_x, double* d_y);
 
