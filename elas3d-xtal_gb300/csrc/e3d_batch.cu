@@ -82,12 +82,14 @@ GridDims fx_dims(GridDims G) {
   return G;
 }
 
+// Halos of the tiles of G, and what the fixed-point pass needs beyond Ah, which its
+// scratch starts at (FxScratch); over every z chunk that job_dims may take, whatever
+// the number of parts.
 long long halo_doubles(const GridDims& G) {
-  const GridDims X = fx_dims(G);
-  return std::max(3LL * G.ntiles * G.tz * (TILE_X + TILE_Y + 1), 3LL * X.ntiles * X.tz * (TILE_X + kFxRows + 1));
+  const long long fx = fx_scratch_bytes(fx_dims(G)) - (long long)align256(4 * 3 * G.ns);
+  return std::max(3LL * G.ntiles * G.tz * (TILE_X + TILE_Y + 1), (fx + 7) / 8);
 }
 
-// Over every z chunk that job_dims may take, whatever the number of parts.
 long long max_halo_doubles(int nx, int ny, int nz) {
   long long m = 0;
   for (int ntz = 1; ntz <= nz; ++ntz) m = std::max(m, halo_doubles(chunk_dims(nx, ny, nz, (nz + ntz - 1) / ntz)));
@@ -251,8 +253,8 @@ void fill_job(JobDev& J, const RveDev& R, char*& p, const double strain[6], int 
   d.z32 = carve<float>(p, n3);
   d.h0 = carve<float>(p, n3);
   d.h1 = carve<float>(p, n3);
-  d.Ah = carve<float>(p, n3);
   d.sig = carve<double>(p, 6 * (size_t)R.nphase);
+  d.Ah = carve<float>(p, n3);  // with the halos behind it: FxScratch
   J.halo_cap = max_halo_doubles(R.nx, R.ny, R.nz);
   double* halo = carve<double>(p, (size_t)J.halo_cap);
   d.hx = halo;  // split per k in set_parts

@@ -107,9 +107,8 @@ static __device__ bool job_barrier(const JobDesc& J, int part, int* err, unsigne
 }
 
 // Slots of the per-job partial array.
-enum : int { SL_A = 0, SL_B = 1, SL_C = 2, SL_U = 3, SL_GG = 4, SL_ZG = 5, SL_S = 6 /* 6..17 */, SL_MAX = 18 };
-constexpr int kJobSlots = 19;
-
+enum : int { SL_A = 0, SL_B = 1, SL_C = 2, SL_U = 3, SL_GG = 4, SL_ZG = 5, SL_S = 6 /* 6..17 */ };
+constexpr int kJobSlots = 18;
 
 // Sum of the k partials of slot `slot`, same value in every part.
 static __device__ double job_reduce(const JobDesc& J, int slot, double* red) {
@@ -269,40 +268,72 @@ inline __device__ ApplyArgs<float> job_apply_args<float>(const JobDesc& J) {
   return A;
 }
 
+// Scratch of the fixed-point FP64 pass: its halos, then the row maxima of u
+// (FxRowMax).  It starts at Ah, whose values phase B has used up by then, and may go
+// on into the halos behind it, which are the FP32 sweep's.
+struct FxScratch {
+  double *hx, *hy, *hd;
+  unsigned *m, *lim;
+};
+__host__ __device__ inline long long fx_scratch_bytes(const GridDims& X) {
+  return 8 * (3 * X.ntiles * X.tz * (TILE_X + kFxRows + 1)) + 4 * (2 * X.ntiles * kFxRows);
+}
+static __device__ __forceinline__ FxScratch job_fx_scratch(const JobDesc& J) {
+  const long long h = 3 * J.Gx.ntiles * J.Gx.tz, rows = J.Gx.ntiles * kFxRows;
+  FxScratch S;
+  S.hx = reinterpret_cast<double*>(J.Ah);
+  S.hy = S.hx + h * kFxRows;
+  S.hd = S.hy + h * TILE_X;
+  S.m = reinterpret_cast<unsigned*>(S.hd + h);
+  S.lim = S.m + rows;
+  return S;
+}
 
 // FP64 K u into g (in-tile part + halos), all parts, then a job barrier.  The
 // apply arguments sit in shared memory (read there, not held in registers).
-// Fixed point with one exponent for the whole of u (job_fold's maximum), in tiles
-// of Gx, where the tables and values allow it; returns whether it did (every part
-// decides alike).
+// Fixed point in tiles of Gx, each with its own exponent by job_fold's row maxima,
+// where the tables allow it (uneven tiles in the FP64 form); returns whether they did
+// (every part decides alike).
 static __device__ __noinline__ bool job_fp64_apply_tiles(const JobDesc& J, int part, unsigned char* dyn) {
   __shared__ ApplyArgs<double> sA;
-  __shared__ int s_kx;
+  __shared__ bool s_fx;
   if (threadIdx.x == 0) {
-    double m = 0.0;
-    for (int i = 0; i < J.nparts; ++i)
-      m = fx_max(m, __ldcg(J.partial + E3D_IDX((long long)SL_MAX * J.nparts + i, kJobSlots * (long long)J.nparts)));
-    s_kx = J.fxinfo[1] != 0.0 ? fx_exponent((unsigned)m) : kFxGeneral;
+    s_fx = J.fxinfo[1] != 0.0;
     ApplyArgs<double> A = job_apply_args<double>(J);
     A.x = J.u;
     A.y = J.g;
-    if (s_kx != kFxGeneral) {
-      const long long h = (long long)J.Gx.ntiles * J.Gx.tz;
+    if (s_fx) {
       A.g = J.Gx;
-      A.hy = J.hx + 3 * h * kFxRows;
-      A.hd = A.hy + 3 * h * TILE_X;
+      const FxScratch S = job_fx_scratch(J);
+      A.hx = S.hx;
+      A.hy = S.hy;
+      A.hd = S.hd;
     }
     sA = A;
   }
   __syncthreads();
-  const int kx = s_kx;
   double dummy = 0.0;
-  if (kx != kFxGeneral) {
+  if (s_fx) {
     const int group = threadIdx.x / kFxThreads;
-    FxSmem<false>& sm = reinterpret_cast<FxSmem<false>*>(dyn)[group];
+    unsigned char* smem = dyn + group * sizeof(FxSmem<false>);
     const FxArgs F{J.fxtab, (int)J.fxinfo[0], nullptr};
-    for (long long t = (long long)part * kGroups + group; t < J.Gx.ntiles; t += (long long)J.nparts * kGroups)
-      apply_tile_fx<false, true>(sA, F, kx, t, sm, dummy);
+    const FxScratch S = job_fx_scratch(J);
+    const FxRowMax R{S.m, S.lim};
+    const long long first = (long long)part * kGroups + group, stride = (long long)J.nparts * kGroups;
+    bool general = false;
+    for (long long t = first; t < J.Gx.ntiles; t += stride) {
+      const int kx = fx_tile_exponent(J.Gx, t, R);
+      if (kx != kFxGeneral)
+        apply_tile_fx<false, true>(sA, F, kx, t, *reinterpret_cast<FxSmem<false>*>(smem), dummy);
+      else
+        general = true;
+    }
+    if (general)
+      for (long long t = first; t < J.Gx.ntiles; t += stride)
+        if (fx_tile_exponent(J.Gx, t, R) == kFxGeneral) {
+          tile_sync<true>();  // the memory is another tile's until here
+          apply_tile_general<true>(sA, t, *reinterpret_cast<ApplySmem<double, kFxRows>*>(smem));
+        }
     __syncthreads();
     return true;
   }
@@ -327,11 +358,11 @@ static __device__ __noinline__ bool job_true_residual(const JobDesc& J, int part
   const GridDims& G = J.G;
   const long long ns = G.ns;
   double zg = 0.0, eu = 0.0, gg = 0.0;
-  const long long hfx = (long long)J.Gx.ntiles * J.Gx.tz;
+  const FxScratch S = job_fx_scratch(J);
   for_part_nodes(J, part, [&](long long m, int x, int y, int z, int tix, int tiy, int tiz, int lx, int ly, int lz) {
     double v[3] = {J.g[m], J.g[m + ns], J.g[m + 2 * ns]};
     if (fx)
-      halo_add<double, kFxRows>(J.Gx, J.hx, J.hx + 3 * hfx * kFxRows, J.hx + 3 * hfx * (kFxRows + TILE_X), x, y, z, v);
+      halo_add<double, kFxRows>(J.Gx, S.hx, S.hy, S.hd, x, y, z, v);
     else
       halo_add_tile<double>(G, J.hx, J.hy, J.hd, tix, tiy, tiz, lx, ly, lz, v);
     float gv[3];
@@ -453,28 +484,45 @@ constexpr int kEngineDynSmem = [] {
 static_assert(sizeof(F2Smem) % 8 == 0 && kJobPvBytes % 16 == 0 && sizeof(FxSmem<false>) % 8 == 0,
               "the groups' parts stay aligned");
 
-// u += du, du = 0; the part's largest |u| (high word) to its slot, for the
-// fixed-point pass that follows.
-static __device__ void job_fold(const JobDesc& J, int part) {
-  const long long ns = J.G.ns;
-  unsigned m_hi = 0;
-  for_part_nodes(J, part, [&](long long m, int, int, int, int, int, int, int, int, int) {
+// u += du, du = 0, and the row maxima of u for the fixed-point pass that follows: a warp
+// has a row of a tile of G, which is a row of one of the two tiles of Gx in its place.
+// The tiles are those of for_part_nodes.
+static __device__ __noinline__ void job_fold(const JobDesc& J, int part) {
+  const GridDims &G = J.G, &X = J.Gx;
+  const int tx = threadIdx.x % TILE_X, ty = threadIdx.x / TILE_X;
+  const long long ns = G.ns, nxy = (long long)G.nx * G.ny;
+  const FxScratch S = job_fx_scratch(J);
+  double* const u = J.u;
+  float* const du = J.du;
+  for (long long t = (long long)part * kGroups; t < G.ntiles;
+       t += t % kGroups == kGroups - 1 ? (long long)(J.nparts - 1) * kGroups + 1 : 1) {
+    const int tix = (int)(t % G.ntx), tiy = (int)((t / G.ntx) % G.nty), tiz = (int)(t / ((long long)G.ntx * G.nty));
+    const int x = tix * TILE_X + tx, y = tiy * TILE_Y + ty, z0 = tiz * G.tz, z1 = min(G.nz, z0 + G.tz);
+    const bool active = x < G.nx && y < G.ny;
+    FxRowScan scan;
+    for (int z = z0; z < z1; ++z) {
+      unsigned w[3] = {0, 0, 0};
+      if (active) {
+        const long long m = E3D_IDX(x + (long long)G.nx * y + nxy * z, ns);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const long long i = m + c * ns;
-      const double v = J.u[i] + (double)J.du[i];
-      J.u[i] = v;
-      J.du[i] = 0.0f;
-      m_hi = max(m_hi, abs_hi(v));
+        for (int c = 0; c < 3; ++c) {
+          const double v = u[m + c * ns] + (double)du[m + c * ns];
+          u[m + c * ns] = v;
+          du[m + c * ns] = 0.0f;
+          w[c] = size_word(v);
+        }
+      }
+      scan.plane(w[0], w[1], w[2]);
     }
-  });
-  __shared__ unsigned s_max[NT / 32];
-  m_hi = __reduce_max_sync(0xffffffffu, m_hi);
-  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m_hi;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < NT / 32; ++i) m_hi = max(m_hi, s_max[i]);
-    J.partial[E3D_IDX((long long)SL_MAX * J.nparts + part, kJobSlots * (long long)J.nparts)] = (double)m_hi;
+    unsigned m, lim;
+    scan.finish(m, lim);
+    const int fy = tiy * (TILE_Y / kFxRows) + ty / kFxRows;
+    if (tx == 0 && fy < X.nty) {
+      const long long o = E3D_IDX((tix + (long long)X.ntx * (fy + (long long)X.nty * tiz)) * kFxRows + ty % kFxRows,
+                                  X.ntiles * kFxRows);
+      S.m[o] = m;
+      S.lim[o] = lim;
+    }
   }
 }
 

@@ -321,6 +321,16 @@ __device__ __forceinline__ void ring_drain(PlaneRing& R) {
   }
 }
 
+// Barrier of the 128 threads that share a tile: the whole block, or, GROUPED,
+// one of the groups of 128 that make up a larger block.
+template <bool GROUPED>
+__device__ __forceinline__ void tile_sync() {
+  if constexpr (GROUPED)
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + (int)(threadIdx.x >> 7)) : "memory");
+  else
+    __syncthreads();
+}
+
 // One tile: TILE_X x TILE_Y element columns marching through tz element planes
 // (plus one redundant plane below).  Each thread owns node column (x0+tx,
 // y0+ty) and the element whose lower corner it is.  Element forces are summed
@@ -333,13 +343,14 @@ __device__ __forceinline__ void ring_drain(PlaneRing& R) {
 // h_new is stored for the tile's own nodes.  Returns this thread's share of
 // h_new . (K h_new) through hAh.
 //
-// TY: rows of a tile (and warps of a block).
+// TY: rows of a tile (and warps of a block, or, GROUPED, of a group of 128 threads).
 template <typename T, bool FUSED, bool POLD_SMEM = (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), bool DEFER_U = false,
-          int TY = TILE_Y>
+          int TY = TILE_Y, bool GROUPED = false>
 __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, TY>& sm, double& hAh) {
   constexpr int TILE_Y = TY;
+  static_assert(!GROUPED || TILE_X * TY == 128, "a group is 128 threads");
   const GridDims& G = A.g;
-  const int tid = threadIdx.x;
+  const int tid = GROUPED ? threadIdx.x % (TILE_X * TY) : threadIdx.x;
   const int tx = tid % TILE_X, ty = tid / TILE_X;
   const int tix = (int)(tile % G.ntx);
   const int tiy = (int)((tile / G.ntx) % G.nty);
@@ -461,7 +472,7 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
   const long long ecol = (long long)xg + (long long)G.nx * yg;  // element column
   prefetch(z0 - 1);
   commit(z0 - 1, false);
-  __syncthreads();
+  tile_sync<GROUPED>();
   if (!kPoldSmem && active) {
     T v0[3][4];
     read_corners(z0 - 1, v0);
@@ -474,7 +485,7 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
   for (int k = z0 - 1; k < z0 + wz; ++k) {
     const bool own_next = (k + 1 >= z0) && (k + 1 < z0 + wz);
     commit(k + 1, own_next);
-    __syncthreads();
+    tile_sync<GROUPED>();
     if (k + 2 <= z0 + wz) prefetch(k + 2);
     const int ph_nxt =
         (active && k + 1 < z0 + wz) ? __ldcs(A.pix + E3D_IDX(ecol + nxy * wrapi(k + 1, G.nz), ns)) : 0;
@@ -565,7 +576,7 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
           sm.r[2 * c + 1][tid] = rr[c][3];  // g1
         }
       }
-      __syncthreads();
+      tile_sync<GROUPED>();
       if (ty < wy) {  // warp-uniform: every lane of the row takes part in the shuffles
         const int lz = k - z0;
         T acc[3], pxv[3], hyv[3];
@@ -623,7 +634,7 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
           sm.r[3 * c + 2][tid] = rr[c][3];  // to node (x+1, y+1)
         }
       }
-      __syncthreads();
+      tile_sync<GROUPED>();
       if (active) {
         const int lz = k - z0;
         const long long m = E3D_IDX((long long)xg + (long long)G.nx * yg + nxy * wrapi(k, G.nz), ns);
@@ -658,7 +669,7 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
         }
       }
     } else if constexpr (kPoldSmem) {
-      __syncthreads();  // plane z0-1 was re-read: the next step refills its buffer
+      tile_sync<GROUPED>();  // plane z0-1 was re-read: the next step refills its buffer
     }
     ph_cur = ph_nxt;
   }
@@ -717,16 +728,6 @@ __device__ __forceinline__ const float* at_byte(const float* p, unsigned long lo
 __device__ __forceinline__ bool tile_full(const GridDims& G, long long tile) {
   const long long txy = tile % ((long long)G.ntx * G.nty);
   return (txy % G.ntx + 1) * TILE_X <= G.nx && (txy / G.ntx + 1) * TILE_Y <= G.ny;
-}
-
-// Barrier of the 128 threads that share a tile: the whole block, or, GROUPED,
-// one of the groups of 128 that make up a larger block.
-template <bool GROUPED>
-__device__ __forceinline__ void tile_sync() {
-  if constexpr (GROUPED)
-    asm volatile("bar.sync %0, 128;" ::"r"(1 + (int)(threadIdx.x >> 7)) : "memory");
-  else
-    __syncthreads();
 }
 
 template <bool DEFER_U, bool FULL, bool GROUPED>
@@ -1374,10 +1375,11 @@ static __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& A,
 }
 
 // A tile that the fixed-point form does not take: the FP64 form, out of line.
+template <bool GROUPED>
 static __device__ __noinline__ void apply_tile_general(const ApplyArgs<double>& A, long long tile,
                                                        ApplySmem<double, kFxRows>& sm) {
   double dot = 0.0;
-  apply_tile<double, false, false, false, kFxRows>(A, tile, sm, dot);
+  apply_tile<double, false, false, false, kFxRows, GROUPED>(A, tile, sm, dot);
 }
 __device__ __forceinline__ unsigned tile_row_max(const GridDims& G, long long tile, const double* x);
 // The same, fused, with the row maxima of h_new; returns the thread's share of h . A h.
@@ -1754,7 +1756,7 @@ static __global__ void __launch_bounds__(kFxThreads, kFxBlocks) apply_tiles_fx_k
   } else {
     if (threadIdx.x == 0) sA = A;
     __syncthreads();
-    apply_tile_general(sA, blockIdx.x, *reinterpret_cast<ApplySmem<double, kFxRows>*>(e3d_fx_dyn));
+    apply_tile_general<false>(sA, blockIdx.x, *reinterpret_cast<ApplySmem<double, kFxRows>*>(e3d_fx_dyn));
   }
 }
 
