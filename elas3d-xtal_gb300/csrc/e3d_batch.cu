@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 
+#include "e3d_autotune.h"
 #include "e3d_batch.h"
 #include "e3d_gpu.h"
 #include "e3d_jobs.cuh"
@@ -438,46 +439,16 @@ int32_t batch_autotune(e3d_batch* b, std::vector<int>& kjob) {
     while (k > 1 && (k > B || 2 * job_dims(R.nx, R.ny, R.nz, k).ntiles < 3LL * k)) k /= 2;
     return k;
   };
-  std::vector<std::vector<int>> plans;
-  double best = 1e300;
-  auto attempt = [&](auto&& k_of, double* ms) -> int32_t {
-    std::vector<int> p(n);
-    for (size_t j = 0; j < n; ++j) p[j] = limit(j, k_of(j));
-    if (std::find(plans.begin(), plans.end(), p) != plans.end()) return E3D_OK;
-    plans.push_back(p);
-    float t2 = 0.f, t10 = 0.f;
-    int32_t rc = batch_time(b, p, step, 2, &t2);
-    if (!rc) rc = batch_time(b, p, step, 10, &t10);
-    if (rc) return rc;
-    *ms = (double)t10 - t2;
-    if (*ms < best) {
-      best = *ms;
-      kjob = p;
-    }
-    return E3D_OK;
-  };
-  int32_t rc = E3D_OK;
-  // Many blocks first: where few solves leave most blocks idle, the long runs with
-  // few of them are not made.
-  double ms = 0.0;
-  for (int k = 64; k >= 1 && ms < 1.5 * best; k /= 2)
-    if ((rc = attempt([&](size_t) { return k; }, &ms))) return rc;
-  // A few solves: an even share of the blocks each, beyond the powers of two that
-  // are close together (25 blocks, not 16 or 32, for six solves).
-  const int share = B / (int)n;
-  if (share > 16 && (rc = attempt([&](size_t) { return std::min(share, kMaxParts); }, &ms))) return rc;
-  for (int per : {16384, 32768, 65536, 131072}) {
-    rc = attempt(
-        [&](size_t j) {
-          const long long ns = b->rves[(size_t)b->jobs[j].rve].ns;
-          int k = 1;
-          while (k < 64 && (long long)per * k * 3 < ns * 2) k *= 2;  // nearest power of two
-          return k;
-        },
-        &ms);
-    if (rc) return rc;
-  }
-  return E3D_OK;
+  return pick_parts(
+      n, B, kMaxParts, limit, [&](size_t j) { return b->rves[(size_t)b->jobs[j].rve].ns; },
+      [&](const std::vector<int>& p, double* ms) -> int {
+        float t2 = 0.f, t10 = 0.f;
+        int32_t rc = batch_time(b, p, step, 2, &t2);
+        if (!rc) rc = batch_time(b, p, step, 10, &t10);
+        *ms = (double)t10 - t2;
+        return rc;
+      },
+      kjob);
 }
 
 }  // namespace
