@@ -141,7 +141,7 @@ struct e3d_handle {
   // row maxima of z, h0 and h1 (a stand-alone apply's x: in the last two)
   double* norms = nullptr;
   int4* fxtab = nullptr;
-  unsigned long long* phsums = nullptr;  // strain sums over each phase, then the exponent
+  unsigned long long* phsums = nullptr;  // gradient sums over each phase, then a StressInfo
   unsigned* mz = nullptr;
   unsigned* mh0 = nullptr;
   unsigned* mh1 = nullptr;
@@ -456,7 +456,7 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
       (rc = dalloc(h, &h->cs32, kCs32Stride * (size_t)np)) || (rc = dalloc(h, &h->dk, 576 * (size_t)np)) ||
       (rc = dalloc(h, &h->dkd, kDkdStride * (size_t)np)) || (rc = dalloc(h, &h->norms, 3 * (size_t)np)) ||
       (rc = dalloc(h, &h->fxtab, kFxStride * (size_t)np)) || (rc = dalloc(h, &h->mz, 2 * tile_rows)) ||
-      (rc = dalloc(h, &h->phsums, 12 * (size_t)np + 1)) ||
+      (rc = dalloc(h, &h->phsums, kPhaseSums * (size_t)np + sizeof(StressInfo) / 8)) ||
       (rc = dalloc(h, &h->mh0, tile_rows)) || (rc = dalloc(h, &h->mh1, tile_rows)) || (rc = dalloc(h, &h->u, n3)) || (rc = dalloc(h, &h->g, n3)) ||
       (rc = dalloc(h, &h->b, n3)) || (rc = dalloc(h, &h->z, n3)) || (rc = dalloc(h, &h->h0, n3)) ||
       (rc = dalloc(h, &h->h1, n3)) || (rc = dalloc(h, &h->Ah, n3)) || (rc = dalloc(h, &h->minv, 6 * ns)) ||
@@ -954,11 +954,12 @@ int32_t e3d_stress(e3d_handle_t* h, double strav[6], double epsav[6]) {
   const int np = h->prob.nphase;
   const unsigned tiles = (unsigned)h->Gx.ntiles;
   const int pgrid = (int)std::min<long long>(std::min(reduction_grid(h), h->partial_n / 12), h->Gx.ntiles);
-  int* info = reinterpret_cast<int*>(h->phsums + 12 * (size_t)np);
-  E3D_CUDA(cudaMemsetAsync(h->phsums, 0, 12 * sizeof(unsigned long long) * np, h->stream));
-  tile_max_kernel<<<tiles, kFxThreads, 0, h->stream>>>(h->Gx, h->u, h->mh0, h->mh1);
+  StressInfo* info = reinterpret_cast<StressInfo*>(h->phsums + kPhaseSums * (size_t)np);
+  E3D_CUDA(cudaMemsetAsync(h->phsums, 0, sizeof(unsigned long long) * kPhaseSums * np + sizeof(StressInfo), h->stream));
+  component_max_kernel<<<(unsigned)std::min<long long>(8LL * h->num_sms, blocks_for(h->G.ns, 256)), 256, 0, h->stream>>>(
+      h->G.ns, h->u, info);
   E3D_LAUNCHED(h);
-  stress_sums_kernel<<<tiles, kFxThreads, 0, h->stream>>>(h->Gx, h->J, h->pix, h->cmod, np, h->u, h->mh0, h->phsums, info,
+  stress_sums_kernel<<<tiles, kFxThreads, 0, h->stream>>>(h->Gx, h->J, h->pix, h->cmod, np, h->u, h->phsums, info,
                                                           h->partial, pgrid);
   E3D_LAUNCHED(h);
   stress_total_kernel<<<1, 256, 0, h->stream>>>(np, h->phsums, info, h->cmod, h->partial, pgrid, h->scalars);

@@ -2444,17 +2444,37 @@ __device__ __forceinline__ void voxel_strain(const GridDims& G, const JumpParams
 }
 
 // Volume sums of stress and strain (src/elas3dxtal_pcg.f90:2149-2408).  The stress
-// of a voxel is C(phase) . strain, so only the strains are summed over the voxels,
-// phase by phase: 72 additions a voxel instead of 130 FP64 operations.  They are
-// 64-bit integers as in the fixed-point stencil, with one exponent for the whole of
-// u (maxima in mx) and the periodic jumps, and their sums, in two words of 64 bits,
-// are exact and so do not depend on the order in which threads add a run of voxels
-// of one phase to its sums.  300^3: 6.55 ms voxel by voxel in FP64, 0.85 with the
-// maxima and the final sums.
-// sums[12 p + 2 i]: low halves of component i (first-order Hadamard sum, four times
-// the strain) over phase p; sums[12 p + 2 i + 1]: high halves.  info: the exponent.
+// of a voxel is C(phase) . strain, so only the gradients are summed over the voxels,
+// phase by phase: 81 additions a voxel instead of 130 FP64 operations.  They are
+// 64-bit integers as in the fixed-point stencil, with one exponent for each component
+// of u (its largest value over the grid) and the periodic jumps of it, and their sums,
+// in two words of 64 bits, are exact and so do not depend on the order in which
+// threads add a run of voxels of one phase to its sums.  300^3: 6.55 ms voxel by
+// voxel in FP64, 1.03 with the maxima and the final sums.
+// Of phase p, from word kPhaseSums * p: low and high halves of the nine sums (component
+// c, direction d: 2 * (3 c + d); first-order Hadamard sums, four times the gradient).
+// info: the exponents.
 // Values that are not finite or out of the exponents' range: FP64, voxel by voxel,
 // to the partials of pgrid blocks.
+constexpr int kPhaseSums = 18;
+struct StressInfo {
+  int kx[3];           // kx[0] == kFxGeneral: the FP64 sums
+  unsigned largest[3];  // size_word of each component's largest value
+};
+
+static __global__ void __launch_bounds__(256) component_max_kernel(long long ns, const double* __restrict__ u,
+                                                                   StressInfo* __restrict__ info) {
+  unsigned w[3] = {0, 0, 0};
+  for (long long m = (long long)blockIdx.x * 256 + threadIdx.x; m < ns; m += (long long)gridDim.x * 256)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) w[c] = max(w[c], size_word(__ldcg(u + m + c * ns)));
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const unsigned v = __reduce_max_sync(0xffffffffu, w[c]);
+    if ((threadIdx.x & 31) == 0 && v) atomicMax(&info->largest[c], v);
+  }
+}
+
 static __device__ __noinline__ void stress_general(const GridDims& G, const JumpParams& J, const int32_t* __restrict__ pix,
                                                    const double* __restrict__ cmod, int nphase,
                                                    const double* __restrict__ u, double* partial, int pgrid, double* red) {
@@ -2482,28 +2502,26 @@ static __device__ __noinline__ void stress_general(const GridDims& G, const Jump
 
 static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
     GridDims G, JumpParams J, const int32_t* __restrict__ pix, const double* __restrict__ cmod, int nphase,
-    const double* __restrict__ u, const unsigned* __restrict__ mx, unsigned long long* __restrict__ sums,
-    int* __restrict__ info, double* partial, int pgrid) {
+    const double* __restrict__ u, unsigned long long* __restrict__ sums, StressInfo* __restrict__ info,
+    double* partial, int pgrid) {
   constexpr int kHalo = TILE_X + kFxRows + 1, kRow = TILE_X + 1, cst = kRow * (kFxRows + 1);
   __shared__ long long node[2][3][cst];
   __shared__ double raw[3][kFxThreads + kHalo];
   __shared__ double red[kFxThreads / 32];
-  __shared__ unsigned mred[kFxThreads / 32];
   const int tid = threadIdx.x;
-  unsigned b = 0;
-  for (long long i = tid; i < G.ntiles * kFxRows; i += kFxThreads) b = max(b, mx[i]);
-  b = __reduce_max_sync(0xffffffffu, b);
-  if ((tid & 31) == 0) mred[tid >> 5] = b;
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < kFxThreads / 32; ++i) b = max(b, mred[i]);
   const double n3[3] = {(double)G.nx, (double)G.ny, (double)G.nz};
-  double big = b ? __hiloint2double((int)b + 1, 0) : 0.0;
-  for (int c = 0; c < 3; ++c)
+  int kx[3];
+  bool general = false;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const unsigned w = info->largest[c];
+    double big = w ? __hiloint2double((int)w + 1, 0) : 0.0;
     for (int d = 0; d < 3; ++d) big = fx_max(big, fabs(J.E[c][d] * n3[d]));
-  const int kx = b >= 0x7ff00000u ? kFxGeneral : fx_exponent_below(big);
-  if (blockIdx.x == 0 && tid == 0) *info = kx;
-  if (kx == kFxGeneral) {
+    kx[c] = w >= 0x7ff00000u ? kFxGeneral : fx_exponent_below(big);
+    general = general || kx[c] == kFxGeneral;
+  }
+  if (blockIdx.x == 0 && tid < 3) info->kx[tid] = general ? kFxGeneral : tid == 0 ? kx[0] : tid == 1 ? kx[1] : kx[2];
+  if (general) {
     stress_general(G, J, pix, cmod, nphase, u, partial, pgrid, red);
     return;
   }
@@ -2541,12 +2559,12 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
     cp_async_wait<0>();
     if (active) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) node[buf][c][ty * kRow + tx] = fx_from_double(raw[c][tid], kx);
+      for (int c = 0; c < 3; ++c) node[buf][c][ty * kRow + tx] = fx_from_double(raw[c][tid], kx[c]);
     }
     if (tid < nhalo) {
 #pragma unroll
       for (int c = 0; c < 3; ++c)
-        node[buf][c][E3D_IDX(hly * kRow + hlx, cst)] = fx_from_double(raw[c][kFxThreads + tid], kx);
+        node[buf][c][E3D_IDX(hly * kRow + hlx, cst)] = fx_from_double(raw[c][kFxThreads + tid], kx[c]);
     }
   };
   // sum, x and y difference of the voxel's four nodes of a plane
@@ -2563,13 +2581,13 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
   };
   // what the periodic jumps add at the last voxel of x, y and z
   const bool jx = active && x0 + tx == G.nx - 1, jy = active && y0 + ty == G.ny - 1;
-  auto jump = [&](int c, int d) { return 4 * fx_from_double(J.E[c][d] * n3[d], kx); };
-  unsigned long long lo[6] = {};
-  long long hi[6] = {};
+  auto jump = [&](int c, int d) { return 4 * fx_from_double(J.E[c][d] * n3[d], kx[c]); };
+  unsigned long long lo[9] = {};
+  long long hi[9] = {};
   int cur = -1;
   // Adds the runs of the lanes with `ends` to their phases' sums and clears them.  The
   // lanes of one phase are added up first (in pieces of 26 bits, whose sums fit 32),
-  // and twelve lanes then add a word each: every thread by itself, all to the words
+  // and eighteen lanes then add a word each: every thread by itself, all to the words
   // of a few phases, took 158 us on a grid of 32^3, where this takes 9.5.
   auto flush = [&](bool ends) {
     const int lane = tid & 31;
@@ -2579,7 +2597,7 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
       const bool in = ends && cur == p;
       unsigned long long word = 0;
 #pragma unroll
-      for (int i = 0; i < 6; ++i) {
+      for (int i = 0; i < 9; ++i) {
         const unsigned l0 = __reduce_add_sync(0xffffffffu, in ? (unsigned)lo[i] & 0x3ffffffu : 0u),
                        l1 = __reduce_add_sync(0xffffffffu, in ? (unsigned)(lo[i] >> 26) : 0u),
                        h0 = __reduce_add_sync(0xffffffffu, in ? (unsigned)hi[i] & 0x3ffffffu : 0u);
@@ -2587,12 +2605,12 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
         if (lane == 2 * i) word = l0 + ((unsigned long long)l1 << 26);
         if (lane == 2 * i + 1) word = h0 + (unsigned long long)((long long)h1 * (1 << 26));
       }
-      if (lane < 12) atomicAdd(sums + 12 * (long long)E3D_IDX(p, nphase) + lane, word);
+      if (lane < kPhaseSums) atomicAdd(sums + kPhaseSums * (long long)E3D_IDX(p, nphase) + lane, word);
       left &= ~__ballot_sync(0xffffffffu, in);
     }
     if (ends) {
 #pragma unroll
-      for (int i = 0; i < 6; ++i) {
+      for (int i = 0; i < 9; ++i) {
         lo[i] = 0;
         hi[i] = 0;
       }
@@ -2613,24 +2631,20 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
     if (__any_sync(0xffffffffu, ph != cur && cur >= 0)) flush(ph != cur && cur >= 0);
     cur = ph;
     if (!active) continue;
-    long long Pn[3][3], X[3], Y[3], Z[3];
+    long long Pn[3][3];
     plane(buf, Pn);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      X[c] = Pn[c][1] + Po[c][1];
-      Y[c] = Pn[c][2] + Po[c][2];
-      Z[c] = Pn[c][0] - Po[c][0];
-      if (jx) X[c] += jump(c, 0);
-      if (jy) Y[c] += jump(c, 1);
-      if (k == G.nz - 1) Z[c] += jump(c, 2);
+      long long e[3] = {Pn[c][1] + Po[c][1], Pn[c][2] + Po[c][2], Pn[c][0] - Po[c][0]};
+      if (jx) e[0] += jump(c, 0);
+      if (jy) e[1] += jump(c, 1);
+      if (k == G.nz - 1) e[2] += jump(c, 2);
 #pragma unroll
-      for (int q = 0; q < 3; ++q) Po[c][q] = Pn[c][q];
-    }
-    const long long e[6] = {X[0], Y[1], Z[2], Z[0] + X[2], Z[1] + Y[2], Y[0] + X[1]};
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      lo[i] += (unsigned)e[i];
-      hi[i] += e[i] >> 32;
+      for (int d = 0; d < 3; ++d) {
+        Po[c][d] = Pn[c][d];
+        lo[3 * c + d] += (unsigned)e[d];
+        hi[3 * c + d] += e[d] >> 32;
+      }
     }
   }
   flush(cur >= 0);
@@ -2638,26 +2652,26 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
 
 // The six sums of stress and of strain, from the sums over the phases.
 static __global__ void __launch_bounds__(256) stress_total_kernel(int nphase, const unsigned long long* __restrict__ sums,
-                                                                  const int* __restrict__ info,
+                                                                  const StressInfo* __restrict__ info,
                                                                   const double* __restrict__ cmod,
                                                                   const double* __restrict__ partial, int pgrid,
                                                                   double* __restrict__ out) {
   __shared__ double red[8];
-  const int kx = *info;
   double acc[12];
   for (int t = 0; t < 12; ++t) acc[t] = 0.0;
-  if (kx == kFxGeneral) {
+  if (info->kx[0] == kFxGeneral) {
     for (int i = threadIdx.x; i < pgrid; i += 256)
       for (int t = 0; t < 12; ++t) acc[t] += partial[12 * (long long)i + t];
   } else {
     for (int p = threadIdx.x; p < nphase; p += 256) {
-      double eps[6];
-      for (int c = 0; c < 6; ++c) {
-        const unsigned long long* s = sums + 12 * (long long)p + 2 * c;
-        const __int128 t = ((__int128)(long long)s[1] << 32) + s[0];
-        eps[c] = ldexp(ldexp((double)(long long)(t >> 32), 32) + (double)(unsigned)t, -kx - 2);
-        acc[6 + c] += eps[c];
+      const unsigned long long* sum = sums + kPhaseSums * (long long)p;
+      double g[3][3];
+      for (int q = 0; q < 9; ++q) {
+        const __int128 t = ((__int128)(long long)sum[2 * q + 1] << 32) + sum[2 * q];
+        g[q / 3][q % 3] = ldexp(ldexp((double)(long long)(t >> 32), 32) + (double)(unsigned)t, -info->kx[q / 3] - 2);
       }
+      const double eps[6] = {g[0][0], g[1][1], g[2][2], g[0][2] + g[2][0], g[1][2] + g[2][1], g[0][1] + g[1][0]};
+      for (int c = 0; c < 6; ++c) acc[6 + c] += eps[c];
       for (int r = 0; r < 6; ++r) {
         double s = 0.0;
         for (int c = 0; c < 6; ++c) s += cmod[p + (long long)nphase * (r + 6 * c)] * eps[c];
