@@ -2452,11 +2452,11 @@ __device__ __forceinline__ void voxel_strain(const GridDims& G, const JumpParams
 // threads add a run of voxels of one phase to its sums.  300^3: 6.55 ms voxel by
 // voxel in FP64, 1.03 with the maxima and the final sums.
 // Of phase p, from word kPhaseSums * p: low and high halves of the nine sums (component
-// c, direction d: 2 * (3 c + d); first-order Hadamard sums, four times the gradient).
-// info: the exponents.
+// c, direction d: 2 * (3 c + d); first-order Hadamard sums, four times the gradient),
+// then the runs added, zero for a phase that has no voxel.  info: the exponents.
 // Values that are not finite or out of the exponents' range: FP64, voxel by voxel,
 // to the partials of pgrid blocks.
-constexpr int kPhaseSums = 18;
+constexpr int kPhaseSums = 19;
 struct StressInfo {
   int kx[3];           // kx[0] == kFxGeneral: the FP64 sums
   unsigned largest[3];  // size_word of each component's largest value
@@ -2587,7 +2587,7 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
   int cur = -1;
   // Adds the runs of the lanes with `ends` to their phases' sums and clears them.  The
   // lanes of one phase are added up first (in pieces of 26 bits, whose sums fit 32),
-  // and eighteen lanes then add a word each: every thread by itself, all to the words
+  // and nineteen lanes then add a word each: every thread by itself, all to the words
   // of a few phases, took 158 us on a grid of 32^3, where this takes 9.5.
   auto flush = [&](bool ends) {
     const int lane = tid & 31;
@@ -2605,6 +2605,7 @@ static __global__ void __launch_bounds__(kFxThreads) stress_sums_kernel(
         if (lane == 2 * i) word = l0 + ((unsigned long long)l1 << 26);
         if (lane == 2 * i + 1) word = h0 + (unsigned long long)((long long)h1 * (1 << 26));
       }
+      if (lane == 18) word = 1;
       if (lane < kPhaseSums) atomicAdd(sums + kPhaseSums * (long long)E3D_IDX(p, nphase) + lane, word);
       left &= ~__ballot_sync(0xffffffffu, in);
     }
@@ -2665,6 +2666,7 @@ static __global__ void __launch_bounds__(256) stress_total_kernel(int nphase, co
   } else {
     for (int p = threadIdx.x; p < nphase; p += 256) {
       const unsigned long long* sum = sums + kPhaseSums * (long long)p;
+      if (sum[18] == 0) continue;  // no voxel: its stiffness, whatever it is, counts for nothing
       double g[3][3];
       for (int q = 0; q < 9; ++q) {
         const __int128 t = ((__int128)(long long)sum[2 * q + 1] << 32) + sum[2 * q];

@@ -1,4 +1,5 @@
-"""Volume averages where one component of the displacement is much larger than the others."""
+"""Volume averages where one component of the displacement is much larger than the others,
+and with phases that no voxel has."""
 import numpy as np
 import pytest
 
@@ -31,3 +32,19 @@ def test_offset(shape, component, size):
     peak = 4 * np.abs(np.delete(u, component, 0)).max()  # of a voxel's strain
     assert np.abs(e - e_ref).max() <= TOL * peak
     assert np.abs(s - s_ref).max() <= TOL * peak * 3 * 240e9
+
+
+def test_phase_without_voxels():
+    shape, ng = (20, 9, 7), 5
+    pix, rod = E.micro_grains(*shape, ng, 5)
+    pix[pix == 3] = 2
+    rod = np.array(rod, dtype=np.float64)
+    u = W.random_field(pix.size, 12)
+    got = []
+    for r in (0.25, np.inf):
+        rod.reshape(-1, 3)[2] = r  # of the phase that is not there
+        with E.Elas3D(E.Problem(*shape, ng + 1, strain=(1e-3, 0, 0, 0, 0, 0), **MATERIAL)) as g:
+            g.upload(pix, rod).femat().set_u(u)
+            got.append(np.concatenate(g.stress()))
+    assert np.isfinite(got[1]).all()
+    assert np.array_equal(*got)
