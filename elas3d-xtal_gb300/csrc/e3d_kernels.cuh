@@ -1975,8 +1975,7 @@ static __global__ void pix_to_zero_based_kernel(long long ns, int nphase, int32_
 // Reference local node r (1..8 -> 0..7) to corner index a = ox + 2oy + 4oz.
 static __constant__ int kRefToCorner[8] = {0, 1, 3, 2, 4, 5, 7, 6};
 
-// Norms of a phase (fx_phase_norms) from its element matrix in shared memory,
-// one warp.
+// Norms of a phase (see fx_info) from its element matrix in shared memory, one warp.
 static __device__ __forceinline__ void fx_store_norms(const double (&col)[24][24], const double* csh, double* out) {
   const int lane = threadIdx.x;
   double d = 0.0, rows = 0.0, entry = 0.0;
@@ -2023,10 +2022,6 @@ __device__ __forceinline__ void invert3x3(const double (&a)[6], double (&ai)[6])
   ai[4] = c02 * inv_det;
   ai[5] = (-a[0] * a[5] + a[4] * a[3]) * inv_det;
 }
-
-// Block-Jacobi (src/elas3dxtal_pcg.f90:1498-1520): sum of the node's diagonal
-// 3x3 blocks over its 8 elements (reference order), inverted.  Stores the
-// symmetric inverse as 6 SoA planes (00 11 22 01 02 12) in FP64 and FP32.
 
 // The diagonal blocks of a phase, and the inverse of their sum: the block of a node
 // whose eight elements are all of this phase (as bjacobi_kernel forms it).
@@ -2295,7 +2290,7 @@ static __global__ void __launch_bounds__(kFematThreads) femat_c_kernel(GridDims 
 
 // Affine initial guess (src/elas3dxtal_pcg.f90:423-438).
 // FP64-issue-bound: a thread takes `chunk` nodes of a z column, whose x and y terms
-// are one sum, 4 FP64 instructions a node instead of 12 (AFFINE_FIGURES).
+// are one sum, 4 FP64 instructions a node instead of 12 (300^3: 609 -> 234 us).
 static __global__ void __launch_bounds__(256) affine_kernel(GridDims G, JumpParams J, int chunk, double* __restrict__ u) {
   const unsigned nxy = (unsigned)G.nx * (unsigned)G.ny, cols = (nxy + 255u) / 256u;
   const unsigned col = blockIdx.x % cols * 256u + threadIdx.x;
@@ -2313,6 +2308,9 @@ static __global__ void __launch_bounds__(256) affine_kernel(GridDims G, JumpPara
     u[m + 2 * G.ns] = c2 + z * ezz;
   }
 }
+// Block-Jacobi (src/elas3dxtal_pcg.f90:1498-1520): sum of the node's diagonal
+// 3x3 blocks over its 8 elements (reference order), inverted.  Stores the
+// symmetric inverse as 6 SoA planes (00 11 22 01 02 12) in FP64 and FP32.
 constexpr int kBjacobiPer = 4;
 static __global__ void __launch_bounds__(256) bjacobi_kernel(GridDims G, int per, const int32_t* __restrict__ pix,
                                                              const double* __restrict__ dkd, double* __restrict__ minv,
@@ -3069,7 +3067,8 @@ struct GridBarrier {
 };
 
 // Barrier among n blocks that run at the same time; `first` is true in exactly one
-// of them.  One atomic a block: the first adds 2^31 - (n - 1), the others 1, so that
+// of them.  The counting is that of cooperative groups' grid barrier, with a time limit
+// and an error exit.  One atomic a block: the first adds 2^31 - (n - 1), the others 1, so that
 // the n-th arrival flips the top bit and clears the rest.  Its latency is most of
 // an iteration's overhead on small grids: with a generation that the last block
 // raises after it has reset the count, and a pause of 128 ns between looks, an
@@ -3129,7 +3128,9 @@ static __device__ double reduce_broadcast(const double* partial, int n, double* 
 }
 
 // Phase B's stages in the per-thread-load persistent kernels.  More take L1 from
-// phase A's loads: 500^3 FP32 iteration 5.72 ms with two, 8.0 with four at V = 4.
+// phase A's loads: 500^3 FP32 iteration 5.72 ms with two, 8.0 with four at V = 4.  Odd
+// rows (V = 1) gain nothing from four either: 301 x 300 x 300 1.49 ms both, 499 x 500 x
+// 500 7.65 with two and 7.69 with four.
 constexpr int kPbStages = 2;
 
 // Dynamic shared memory of those kernels: phase B's stages, and in the same bytes

@@ -93,7 +93,7 @@ typedef struct e3d_serve_opts {
   float tol;
   int32_t max_active;       /* concurrent solves on the device (slots)           */
   int32_t round_iters;      /* PCG iterations per solve per engine round          */
-  int32_t parts;            /* blocks per solve (<= 64): 0 = by size              */
+  int32_t parts;            /* blocks per solve (<= 152): 0 = by size             */
   int32_t round_balance;    /* 1: a solve with fewer nodes per block runs up to
                                8x round_iters per round (same results, fewer
                                rounds); 0 (default): round_iters for every solve */
