@@ -146,14 +146,9 @@ struct e3d_handle {
   unsigned* mh0 = nullptr;
   unsigned* mh1 = nullptr;
   int* fxleave = nullptr;
+  double* partG = nullptr;
   int fx_kc = 0;
   bool fx_ok = false;   // the problem's tables allow it
-  // Whether the solve goes on in the form for uneven tiles, and how many iterations
-  // without one, in a row, end that; twice as many after each return to it.  A
-  // direction is uneven until it has spread from the grains' boundaries over the
-  // grid, some five iterations, or, in a problem that stays so, always.
-  bool fx_uneven = false;
-  int fx_even = 1;
   double* hx = nullptr;
   double* hy = nullptr;
   double* hd = nullptr;
@@ -169,7 +164,7 @@ struct e3d_handle {
   double gg0 = 0.0;
   bool uploaded = false, femat_done = false, energy_done = false, solve_ready = false, minv_ready = false;
   int pcg_grid = 0;
-  int pcg_grid_fx = 0, pcg_grid_uneven = 0;
+  int pcg_grid_fx = 0;
   int pcg_grid32 = 0;
   double ms_setup = 0.0, ms_iter = 0.0;
   JumpParams J{};
@@ -240,9 +235,9 @@ struct PcgForm {
   int threads, smem;
 };
 
-template <typename T, bool FX, int V, bool UNEVEN = false>
+template <typename T, bool FX, int V>
 PcgForm pcg_form_of() {
-  return {(const void*)pcg_persistent_kernel<T, false, FX, V, UNEVEN>, FX ? kFxThreads : NT, pcg_dyn_smem_bytes<T, FX, V>()};
+  return {(const void*)pcg_persistent_kernel<T, false, FX, V>, FX ? kFxThreads : NT, pcg_dyn_smem_bytes<T, FX, V>()};
 }
 
 // The form for a solve: phase B takes two nodes of a row at a time where every row
@@ -258,8 +253,6 @@ PcgForm pcg_form(const e3d_handle* h, bool fx) {
     return nx % 2 == 0 ? pcg_form_of<T, true, 2>() : pcg_form_of<T, true, 1>();
   }
 }
-
-PcgForm pcg_uneven_form() { return pcg_form_of<double, true, 1, true>(); }
 
 PcgForm pcg_ring_form() { return {(const void*)pcg_persistent_kernel<float, true, false, 1>, NT, kRingSmemBytes}; }
 
@@ -436,7 +429,6 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
     return fail(cuda_fail(e, "occupancy"));
   for (auto [form, grid] : {std::pair{pcg_form<double>(h, false), &h->pcg_grid},
                             std::pair{pcg_form<double>(h, true), &h->pcg_grid_fx},
-                            std::pair{pcg_uneven_form(), &h->pcg_grid_uneven},
                             std::pair{pcg_form<float>(h, false), &h->pcg_grid32}}) {
     int per_sm = 0;
     if ((e = pcg_blocks_per_sm(form, &per_sm)) != cudaSuccess) return fail(cuda_fail(e, "occupancy"));
@@ -447,7 +439,7 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
   if (p->precision == E3D_PREC_MIXED &&
       (e = pcg_blocks_per_sm(pcg_ring_form(), &per_sm_tma)) != cudaSuccess)
     return fail(cuda_fail(e, "occupancy (TMA)"));
-  h->partial_n = std::max({h->pcg_grid, h->pcg_grid_fx, h->pcg_grid_uneven, h->pcg_grid32, h->num_sms * 4}) * 12;
+  h->partial_n = std::max({h->pcg_grid, h->pcg_grid_fx, h->pcg_grid32, h->num_sms * 4}) * 12;
   const long long halo = h->G.ntiles * h->G.tz, halo_x = h->Gx.ntiles * h->Gx.tz;
   const size_t tile_rows = (size_t)h->Gx.ntiles * kFxRows;
   int32_t rc = E3D_OK;
@@ -465,7 +457,7 @@ int32_t e3d_create(e3d_handle_t** out, const e3d_problem_t* p) {
       (rc = dalloc(h, &h->hd, 3 * std::max(halo, halo_x))) || (rc = dalloc(h, &h->partial, (size_t)h->partial_n)) ||
       (rc = dalloc(h, &h->scalars, 64)) ||
       (rc = dalloc(h, &h->history, (size_t)std::max(p->max_iter, 1))) || (rc = dalloc(h, &h->st, 1)) ||
-      (rc = dalloc(h, &h->bar, 1)) || (rc = dalloc(h, &h->err, 1)) || (rc = dalloc(h, &h->fxleave, 1)))
+      (rc = dalloc(h, &h->bar, 1)) || (rc = dalloc(h, &h->err, 1)) || (rc = dalloc(h, &h->fxleave, 1)) || (rc = dalloc(h, &h->partG, kUnevenBlocks)))
     return fail(rc);
   if (p->precision == E3D_PREC_MIXED) {
     if ((rc = dalloc(h, &h->du32, n3)) || (rc = dalloc(h, &h->g32, n3)) || (rc = dalloc(h, &h->z32, n3)) ||
@@ -716,8 +708,6 @@ int32_t e3d_solve_begin(e3d_handle_t* h) {
   h->since_replace = 0;
   h->minv_ready = true;
   h->solve_ready = true;
-  h->fx_uneven = false;
-  h->fx_even = 1;
   return E3D_OK;
 }
 
@@ -774,7 +764,7 @@ PcgArgs<double> pcg_args<double>(e3d_handle* h) {
   P.mh0 = h->mh0;
   P.mh1 = h->mh1;
   P.fxleave = h->fxleave;
-  P.fxeven = h->fx_even;
+  P.partG = h->partG;
   return P;
 }
 
@@ -799,13 +789,12 @@ PcgArgs<float> pcg_args<float>(e3d_handle* h) {
   return P;
 }
 
+// it_limit: iterations of this launch; for the fixed-point form the iteration to stop at.
 template <typename T>
 int32_t launch_pcg(e3d_handle* h, int it_limit) {
   const bool tma = sizeof(T) == 4 && h->maps != nullptr;
   const bool fx = sizeof(T) == 8 && h->fx_ok;
-  const bool uneven = fx && h->fx_uneven;
-  const int grid = uneven           ? h->pcg_grid_uneven
-                   : fx             ? h->pcg_grid_fx
+  const int grid = fx               ? h->pcg_grid_fx
                    : sizeof(T) == 8 ? h->pcg_grid
                    : tma            ? h->pcg_grid32_tma
                                     : h->pcg_grid32;
@@ -822,12 +811,24 @@ int32_t launch_pcg(e3d_handle* h, int it_limit) {
   E3D_CUDA(cudaMemsetAsync(h->bar, 0, sizeof(GridBarrier), h->stream));
   if (fx) E3D_CUDA(cudaMemsetAsync(h->fxleave, 0, sizeof(int), h->stream));
   void* args[] = {&P};
-  const PcgForm F = tma ? pcg_ring_form() : uneven ? pcg_uneven_form() : pcg_form<T>(h, fx);
+  const PcgForm F = tma ? pcg_ring_form() : pcg_form<T>(h, fx);
   if constexpr (sizeof(T) == 8)
-    if (fx) P.A.g = h->Gx;
+    if (fx) {
+      P.A.g = h->Gx;
+      P.it_end = it_limit;
+    }
   cudaError_t e = cudaLaunchCooperativeKernel(F.fn, dim3(grid), dim3(F.threads), args, F.smem, h->stream);
   h->launches++;
   if (e != cudaSuccess) return cuda_fail(e, "cudaLaunchCooperativeKernel(pcg)");
+  return E3D_OK;
+}
+
+int32_t launch_uneven(e3d_handle* h) {
+  PcgArgs<double> P = pcg_args<double>(h);
+  P.A.g = h->Gx;
+  P.st = h->st;
+  pcg_uneven_kernel<<<kUnevenBlocks, kFxThreads, 0, h->stream>>>(P);
+  E3D_LAUNCHED(h);
   return E3D_OK;
 }
 
@@ -890,9 +891,19 @@ int32_t e3d_iterate(e3d_handle_t* h, int32_t n, e3d_solve_stats_t* st) {
   while (remaining > 0 && S.status == PCG_RUNNING) {
     int chunk = std::min(remaining, 256);
     if (mixed) chunk = std::min(chunk, R - h->since_replace);
-    const bool fx = !mixed && h->fx_ok;
     const int it0 = S.it;
-    rc = mixed ? launch_pcg<float>(h, chunk) : launch_pcg<double>(h, chunk);
+    if (mixed || !h->fx_ok) {
+      rc = mixed ? launch_pcg<float>(h, chunk) : launch_pcg<double>(h, chunk);
+    } else {
+      // Uneven directions come in the first iterations, until they have spread from the
+      // grains' boundaries over the grid, or, in a problem that stays so, always: once
+      // there is one, a few iterations are launched ahead of the host's look.
+      const bool pending = S.since_replace != 0;
+      if (pending) rc = launch_uneven(h);
+      if (!rc) rc = launch_pcg<double>(h, it0 + chunk);
+      for (int i = 0; pending && i < 3 && !rc; ++i)
+        if (!(rc = launch_uneven(h))) rc = launch_pcg<double>(h, it0 + chunk);
+    }
     if (rc) break;
     if ((rc = read_state(h, &S))) break;
     // a launch ends early when the solve stops or, in the mixed form with
@@ -907,13 +918,7 @@ int32_t e3d_iterate(e3d_handle_t* h, int32_t n, e3d_solve_stats_t* st) {
         if ((rc = read_state(h, &S))) break;
       }
     }
-    if (fx && h->fx_uneven) {
-      h->fx_uneven = S.since_replace < h->fx_even;
-    } else if (fx && S.status == PCG_RUNNING && done < chunk) {  // it left at an uneven tile
-      h->fx_uneven = true;
-      h->fx_even = std::min(2 * h->fx_even, 64);
-      continue;
-    }
+    if (!mixed && S.since_replace != 0) continue;  // phase A of the next iteration is done
     if (done == 0 && S.status == PCG_RUNNING) break;  // nothing advanced: do not spin
   }
   if (!rc && mixed) rc = fold_correction(h);  // u always holds the current iterate on return
@@ -1353,10 +1358,7 @@ extern "C" int32_t e3d_checkpoint_save(e3d_handle_t* h, const char* path) {
   H.gg0 = h->gg0;
   E3D_CUDA(cudaMemcpyAsync(&H.st, h->st, sizeof(PcgState), cudaMemcpyDeviceToHost, h->stream));
   E3D_CUDA(cudaStreamSynchronize(h->stream));
-  if (mixed)
-    H.st.since_replace = h->since_replace;
-  else  // a field that this form has no other use for
-    H.st.final_ready = 2 * h->fx_even + h->fx_uneven;
+  if (mixed) H.st.since_replace = h->since_replace;
   FILE* f = std::fopen(path, "wb");
   if (!f) return E3D_ERR_INPUT;
   const size_t n3 = 3 * (size_t)h->G.ns;
@@ -1399,7 +1401,6 @@ extern "C" int32_t e3d_checkpoint_load(e3d_handle_t* h, const char* path) {
   }
   const size_t n3 = 3 * (size_t)h->G.ns;
   PcgState S = H.st;
-  S.final_ready = 0;
   int32_t rc = ckpt_read(f, h->u, n3, h->stream);
   if (!rc) rc = ckpt_read(f, h->g, n3, h->stream);
   if (!mixed) {
@@ -1420,9 +1421,7 @@ extern "C" int32_t e3d_checkpoint_load(e3d_handle_t* h, const char* path) {
   rc = sync(h);
   if (rc) return rc;
   h->gg0 = H.gg0;
-  h->since_replace = mixed ? S.since_replace : 0;
-  h->fx_uneven = !mixed && (H.st.final_ready & 1);
-  h->fx_even = std::clamp(H.st.final_ready / 2, 1, 64);  // (zero in older files)
+  h->since_replace = S.since_replace;
   h->energy_done = true;
   h->minv_ready = true;
   h->solve_ready = true;

@@ -344,9 +344,11 @@ __device__ __forceinline__ void tile_sync() {
 // h_new . (K h_new) through hAh.
 //
 // TY: rows of a tile (and warps of a block, or, GROUPED, of a group of 128 threads).
+// from, planes: the part of the tile's planes to form.
 template <typename T, bool FUSED, bool POLD_SMEM = (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), bool DEFER_U = false,
           int TY = TILE_Y, bool GROUPED = false>
-__device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, TY>& sm, double& hAh) {
+__device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, TY>& sm, double& hAh, int from = 0,
+                           int planes = 0x7fffffff) {
   constexpr int TILE_Y = TY;
   static_assert(!GROUPED || TILE_X * TY == 128, "a group is 128 threads");
   const GridDims& G = A.g;
@@ -355,8 +357,8 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
   const int tix = (int)(tile % G.ntx);
   const int tiy = (int)((tile / G.ntx) % G.nty);
   const int tiz = (int)(tile / ((long long)G.ntx * G.nty));
-  const int x0 = tix * TILE_X, y0 = tiy * TILE_Y, z0 = tiz * G.tz;
-  const int wx = min(TILE_X, G.nx - x0), wy = min(TILE_Y, G.ny - y0), wz = min(G.tz, G.nz - z0);
+  const int x0 = tix * TILE_X, y0 = tiy * TILE_Y, z0 = tiz * G.tz + from;
+  const int wx = min(TILE_X, G.nx - x0), wy = min(TILE_Y, G.ny - y0), wz = min(planes, min(G.tz - from, G.nz - z0));
   const bool active = (tx < wx) && (ty < wy);
   const int xg = x0 + tx, yg = y0 + ty;
   const long long ns = G.ns;
@@ -578,7 +580,7 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
       }
       tile_sync<GROUPED>();
       if (ty < wy) {  // warp-uniform: every lane of the row takes part in the shuffles
-        const int lz = k - z0;
+        const int lz = k - z0 + from;
         T acc[3], pxv[3], hyv[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -636,7 +638,7 @@ __device__ void apply_tile(const ApplyArgs<T>& A, long long tile, ApplySmem<T, T
       }
       tile_sync<GROUPED>();
       if (active) {
-        const int lz = k - z0;
+        const int lz = k - z0 + from;
         const long long m = E3D_IDX((long long)xg + (long long)G.nx * yg + nxy * wrapi(k, G.nz), ns);
         T hxv[3], hyv[3], acc[3];
 #pragma unroll
@@ -1381,16 +1383,6 @@ static __device__ __noinline__ void apply_tile_general(const ApplyArgs<double>& 
   double dot = 0.0;
   apply_tile<double, false, false, false, kFxRows, GROUPED>(A, tile, sm, dot);
 }
-__device__ __forceinline__ unsigned tile_row_max(const GridDims& G, long long tile, const double* x);
-// The same, fused, with the row maxima of h_new; returns the thread's share of h . A h.
-static __device__ __noinline__ double apply_tile_general_fused(const ApplyArgs<double>& A, long long tile,
-                                                               ApplySmem<double, kFxRows>& sm, unsigned* mx) {
-  double dot = 0.0;
-  apply_tile<double, true, false, false, kFxRows>(A, tile, sm, dot);
-  const unsigned v = tile_row_max(A.g, tile, A.hnew);  // the thread's own stores
-  if (threadIdx.x % TILE_X == 0) mx[E3D_IDX(tile * kFxRows + threadIdx.x / TILE_X, A.g.ntiles * kFxRows)] = v;
-  return dot;
-}
 
 // Shared memory of apply_tile_ring: the in-plane force exchange of the ZS
 // planes of a step, double-buffered by step parity so one barrier per step
@@ -1695,11 +1687,13 @@ struct FxRowScan {
 
 // Row maxima of a tile of a nodal vector, one block a tile: the largest |value|
 // alone, for a solve's own vectors.
-__device__ __forceinline__ unsigned tile_row_max(const GridDims& G, long long tile, const double* x) {
+__device__ __forceinline__ unsigned tile_row_max(const GridDims& G, long long tile, const double* x, int from = 0,
+                                                 int planes = 0x7fffffff) {
   const int tx = threadIdx.x % TILE_X, ty = threadIdx.x / TILE_X;
   const int tix = (int)(tile % G.ntx), tiy = (int)((tile / G.ntx) % G.nty),
             tiz = (int)(tile / ((long long)G.ntx * G.nty));
-  const int xg = tix * TILE_X + tx, yg = tiy * kFxRows + ty, z0 = tiz * G.tz, z1 = min(G.nz, z0 + G.tz);
+  const int xg = tix * TILE_X + tx, yg = tiy * kFxRows + ty, z0 = tiz * G.tz + from;
+  const int z1 = min(G.nz, z0 + min(planes, G.tz - from));
   unsigned v = 0;
   if (xg < G.nx && yg < G.ny) {
     const long long nxy = (long long)G.nx * G.ny;
@@ -3056,7 +3050,8 @@ struct PcgState {
   double rel_at_replace;  // mixed form: rel_res of the last FP64 residual (set-up or replacement)
   double refine_drop;     // mixed form: replace once rel_res < refine_drop * rel_at_replace (0: never)
   int it, status, reset, resets, cur, max_iter, divergence_reset, refinements;
-  // FP32 forms: iterations since the last replacement; FP64: see UNEVEN below
+  // FP32 forms: iterations since the last replacement; fixed-point FP64: 1 where phase A
+  // lacks its uneven tiles (pcg_uneven_kernel)
   int since_replace;
   int final_ready;  // the job engine ended on a converged FP64 replacement
 };
@@ -3171,20 +3166,21 @@ struct PcgArgs {
   unsigned* mz;
   unsigned* mh0;
   unsigned* mh1;
-  int* fxleave;  // set where a tile needs the FP64 form (UNEVEN: to the iteration)
-  int fxeven;    // UNEVEN: iterations without such a tile, in a row, that end the launch
+  int* fxleave;  // set where a tile needs the FP64 form
+  double* partG;  // partial h . A h of those tiles, kUnevenBlocks of them
+  int it_end;     // the iteration to stop at
 };
+constexpr int kUnevenBlocks = 1216;  // eight an SM
 
 // TMA (FP32 only): phase A reads its node planes through the block's plane
 // ring (dynamic shared memory of kRingSmemBytes).  FX (FP64 only): phase A in
 // fixed point, each tile scaled by its own values.  V: nodes of a row a thread
 // takes at a time in phase B, what the rows' alignment allows.
-// UNEVEN (with FX): tiles that fixed point does not take go through the FP64 form,
-// instead of ending the launch, until there is none for some iterations (counted in
-// PcgState::since_replace).  A form of its own: with the FP64 form in the kernel,
-// in line or called, the fixed-point sweep has too few registers (an iteration at
-// 300^3 4.5 ms without, 6.6 with).
-template <typename T, bool TMA, bool FX, int V, bool UNEVEN = false>
+// Where tiles need the FP64 form, phase A ends the launch without them, before anything
+// but h_new and A h is written; pcg_uneven_kernel forms them, and the next launch goes
+// on with phase B.  In this kernel the FP64 form, in line or called, would leave the
+// fixed-point sweep too few registers (300^3: 6.6 ms an iteration instead of 4.5).
+template <typename T, bool TMA, bool FX, int V>
 __global__ void __launch_bounds__(FX ? kFxThreads : NT,
                                   FX               ? kFxBlocks
                                   : sizeof(T) == 4 ? (TMA && E3D_RING_ZS == 2 ? 1 : E3D_F32_BLOCKS_PER_SM)
@@ -3211,102 +3207,90 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
   if (s.status != PCG_RUNNING) return;
   const bool lead = threadIdx.x == 0;
   const GridDims& G = P.A.g;
-  const int it_end = min(s.it + P.it_limit, s.max_iter);
+  const int it_end = FX ? min(P.it_end, s.max_iter) : min(s.it + P.it_limit, s.max_iter);
+  if (FX && s.it >= P.it_end) return;  // launched ahead, and not needed
+  bool resume = FX && s.since_replace != 0;  // phase A is done
   constexpr bool kDeferU = sizeof(T) == 4 && !TMA;
   T lam_pending = T(0);  // kDeferU: du -= lam_pending * h_pending not yet applied
   const T* h_pending = nullptr;
-  if constexpr (FX) {  // row maxima of the vectors that this launch starts from
-    for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x) {
-      const unsigned z = tile_row_max(G, t, P.z);
-      const unsigned h = s.reset ? 0u : tile_row_max(G, t, s.cur ? P.h1 : P.h0);
-      if (threadIdx.x % TILE_X == 0) {
-        const int row = threadIdx.x / TILE_X;
-        P.mz[E3D_IDX(t * 2 * TY + row, G.ntiles * 2 * TY)] = z;
-        P.mz[E3D_IDX(t * 2 * TY + TY + row, G.ntiles * 2 * TY)] = 0u;
-        (s.cur ? P.mh1 : P.mh0)[E3D_IDX(t * TY + row, G.ntiles * TY)] = h;
+  if constexpr (FX) {
+    if (!resume) {  // row maxima of the vectors that this launch starts from
+      for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x) {
+        const unsigned z = tile_row_max(G, t, P.z);
+        const unsigned h = s.reset ? 0u : tile_row_max(G, t, s.cur ? P.h1 : P.h0);
+        if (threadIdx.x % TILE_X == 0) {
+          const int row = threadIdx.x / TILE_X;
+          P.mz[E3D_IDX(t * 2 * TY + row, G.ntiles * 2 * TY)] = z;
+          P.mz[E3D_IDX(t * 2 * TY + TY + row, G.ntiles * 2 * TY)] = 0u;
+          (s.cur ? P.mh1 : P.mh0)[E3D_IDX(t * TY + row, G.ntiles * TY)] = h;
+        }
       }
-    }
-    if (!grid_barrier(P.bar, P.err, P.timeout_ns)) {
-      if (blockIdx.x == 0 && lead) {
-        s.status = PCG_TIMEOUT;
-        *P.st = s;
+      if (!grid_barrier(P.bar, P.err, P.timeout_ns)) {
+        if (blockIdx.x == 0 && lead) {
+          s.status = PCG_TIMEOUT;
+          *P.st = s;
+        }
+        return;
       }
-      return;
     }
   }
   while (s.it < it_end) {
-    // ---- phase A: fused direction update + stencil + h.Ah
-    ApplyArgs<T> A = P.A;
     const int cur = s.cur;
-    A.x = cur ? P.h1 : P.h0;
-    A.hnew = cur ? P.h0 : P.h1;
-    A.zv = P.z;
-    A.y = P.Ah;
-    A.gamma = (T)s.gamma;
-    A.reset = s.reset;
-    if constexpr (kDeferU) {
-      A.du = P.u;
-      A.lam_prev = lam_pending;
-    }
-    double hAh_t = 0.0;
-    if constexpr (TMA) ring_begin(ring, G, cur ? P.maps->h1 : P.maps->h0, blockIdx.x, gridDim.x, G.ntiles);
-    bool general = false;  // UNEVEN: tiles left to the FP64 form
-    for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x) {
-      if constexpr (TMA) {
-        apply_tile_ring<E3D_RING_ZS>(A, t, sm, hAh_t, ring);
-      } else if constexpr (FX) {
-        const FxArgs F{P.fxtab, P.fxkc, cur ? P.mh0 : P.mh1};
-        const int kx = fx_tile_exponent(G, t, FxRowMaxFused{A.reset ? nullptr : cur ? P.mh1 : P.mh0, P.mz, A.gamma});
-        if (kx != kFxGeneral)
-          apply_tile_fx<true>(A, F, kx, t, *reinterpret_cast<FxSmem<true>*>(e3d_pcg_smem), hAh_t);
-        else if constexpr (UNEVEN)
-          general = true;
-        else if (lead)
-          *P.fxleave = 1;
-      } else {
-        apply_tile<T, true, (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), kDeferU>(A, t, sm, hAh_t);
+    if (!resume) {
+      // ---- phase A: fused direction update + stencil + h.Ah
+      ApplyArgs<T> A = P.A;
+      A.x = cur ? P.h1 : P.h0;
+      A.hnew = cur ? P.h0 : P.h1;
+      A.zv = P.z;
+      A.y = P.Ah;
+      A.gamma = (T)s.gamma;
+      A.reset = s.reset;
+      if constexpr (kDeferU) {
+        A.du = P.u;
+        A.lam_prev = lam_pending;
       }
-      __syncthreads();
-    }
-    if constexpr (UNEVEN) {
-      if (general) {
-        __shared__ ApplyArgs<double> sA;
-        if (lead) {
-          sA = A;
-          *P.fxleave = s.it + 1;
+      double hAh_t = 0.0;
+      if constexpr (TMA) ring_begin(ring, G, cur ? P.maps->h1 : P.maps->h0, blockIdx.x, gridDim.x, G.ntiles);
+      for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x) {
+        if constexpr (TMA) {
+          apply_tile_ring<E3D_RING_ZS>(A, t, sm, hAh_t, ring);
+        } else if constexpr (FX) {
+          const FxArgs F{P.fxtab, P.fxkc, cur ? P.mh0 : P.mh1};
+          const int kx = fx_tile_exponent(G, t, FxRowMaxFused{A.reset ? nullptr : cur ? P.mh1 : P.mh0, P.mz, A.gamma});
+          if (kx != kFxGeneral)
+            apply_tile_fx<true>(A, F, kx, t, *reinterpret_cast<FxSmem<true>*>(e3d_pcg_smem), hAh_t);
+          else if (threadIdx.x < TY) {
+            if (lead) *P.fxleave = 1;
+            F.mx[E3D_IDX(t * TY + threadIdx.x, G.ntiles * TY)] = 0u;  // raised by pcg_uneven_kernel
+          }
+        } else {
+          apply_tile<T, true, (sizeof(T) == 4 && E3D_F32_POLD_SMEM != 0), kDeferU>(A, t, sm, hAh_t);
         }
         __syncthreads();
-        const FxRowMaxFused R{sA.reset ? nullptr : cur ? P.mh1 : P.mh0, P.mz, sA.gamma};
-        for (long long t = blockIdx.x; t < G.ntiles; t += gridDim.x)
-          if (fx_tile_exponent(G, t, R) == kFxGeneral) {
-            hAh_t += apply_tile_general_fused(sA, t, *reinterpret_cast<ApplySmem<double, TY>*>(e3d_pcg_smem),
-                                              cur ? P.mh0 : P.mh1);
-            __syncthreads();
-          }
       }
-    }
-    {
-      const double bs = block_sum<NT>(hAh_t, red);
-      if (threadIdx.x == 0) P.partA[blockIdx.x] = bs;
-    }
-    if constexpr (TMA) fence_proxy_async_all();  // h_new stores before the next pass's TMA reads
-    if (!grid_barrier(P.bar, P.err, P.timeout_ns)) {
-      if (lead) s.status = PCG_TIMEOUT;
-      break;
-    }
-    if constexpr (FX && !UNEVEN) {
-      // a tile that needs the FP64 form: leave before anything but h_new and A h is
-      // written; the host goes on with the UNEVEN form
-      if (__ldcg(P.fxleave)) {
-        if (lead) s.since_replace = 0;
+      {
+        const double bs = block_sum<NT>(hAh_t, red);
+        if (threadIdx.x == 0) P.partA[blockIdx.x] = bs;
+      }
+      if constexpr (TMA) fence_proxy_async_all();  // h_new stores before the next pass's TMA reads
+      if (!grid_barrier(P.bar, P.err, P.timeout_ns)) {
+        if (lead) s.status = PCG_TIMEOUT;
         break;
       }
+      if constexpr (FX) {
+        if (__ldcg(P.fxleave)) {
+          if (lead) s.since_replace = 1;
+          break;
+        }
+      }
     }
-    if constexpr (UNEVEN)
-      if (lead) s.since_replace = __ldcg(P.fxleave) == s.it + 1 ? 0 : s.since_replace + 1;
     lam_pending = T(0);  // applied by this phase A
-    const double hAh = reduce_broadcast<NT>(P.partA, gridDim.x, red);
+    double hAh = reduce_broadcast<NT>(P.partA, gridDim.x, red);
+    if constexpr (FX)
+      if (resume) hAh += reduce_broadcast<NT>(P.partG, kUnevenBlocks, red);
+    resume = false;
     if (lead) {
+      if (FX) s.since_replace = 0;
       s.it += 1;
       s.cur ^= 1;
       s.hAh = hAh;
@@ -3371,8 +3355,6 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
     }
     __syncthreads();
     if (s.status != PCG_RUNNING) break;
-    if constexpr (UNEVEN)
-      if (s.since_replace >= P.fxeven) break;
   }
   __syncthreads();
   if (lead && s.status == PCG_RUNNING && s.it >= s.max_iter) s.status = PCG_MAXITER;
@@ -3382,6 +3364,47 @@ __global__ void __launch_bounds__(FX ? kFxThreads : NT,
     if (lam_pending != T(0)) flush_u_tiles<T>(G, blockIdx.x, gridDim.x, lam_pending, h_pending, P.u);
   if constexpr (TMA) ring_drain(ring);
   if (blockIdx.x == 0 && threadIdx.x == 0) *P.st = s;
+}
+
+// The tiles that phase A left out, in the FP64 form, where it did (else nothing): h_new,
+// A h, halos, row maxima of h_new and their share of h . A h.  Such tiles are few, so
+// each is cut into eight or fewer parts along z, of two planes at least, or the march
+// of one tile would be the time of all: a solve of 71 x 58 x 90, uneven for 12 of 140
+// iterations, 19.2 ms with whole tiles, 17.9 with these; 16.4 without any such tile.
+static __global__ void __launch_bounds__(kFxThreads, kFxBlocks) pcg_uneven_kernel(PcgArgs<double> P) {
+  __shared__ ApplySmem<double, kFxRows> sm;
+  __shared__ ApplyArgs<double> sA;
+  __shared__ double red[kFxThreads / 32];
+  const PcgState& s = *P.st;
+  if (s.status != PCG_RUNNING || s.since_replace == 0) return;
+  const int cur = s.cur;
+  if (threadIdx.x == 0) {
+    sA = P.A;
+    sA.x = cur ? P.h1 : P.h0;
+    sA.hnew = cur ? P.h0 : P.h1;
+    sA.zv = P.z;
+    sA.y = P.Ah;
+    sA.gamma = s.gamma;
+    sA.reset = s.reset;
+  }
+  __syncthreads();
+  const FxRowMaxFused R{sA.reset ? nullptr : cur ? P.mh1 : P.mh0, P.mz, sA.gamma};
+  unsigned* const mx = cur ? P.mh0 : P.mh1;
+  const int planes = max(2, (sA.g.tz + 7) / 8), parts = (sA.g.tz + planes - 1) / planes;
+  double dot = 0.0;
+  for (long long i = blockIdx.x; i < sA.g.ntiles * parts; i += gridDim.x) {
+    const long long t = i / parts;
+    const int from = (int)(i % parts) * planes;
+    if (from >= sA.g.nz - t / ((long long)sA.g.ntx * sA.g.nty) * sA.g.tz) continue;  // the last chunk is shorter
+    if (fx_tile_exponent(sA.g, t, R) != kFxGeneral) continue;
+    apply_tile<double, true, false, false, kFxRows>(sA, t, sm, dot, from, planes);
+    const unsigned v = tile_row_max(sA.g, t, sA.hnew, from, planes);  // the thread's own stores
+    if (threadIdx.x % TILE_X == 0)
+      atomicMax(mx + E3D_IDX(t * kFxRows + threadIdx.x / TILE_X, sA.g.ntiles * kFxRows), v);
+    __syncthreads();
+  }
+  dot = block_sum<kFxThreads>(dot, red);
+  if (threadIdx.x == 0) P.partG[blockIdx.x] = dot;
 }
 
 // PCG set-up (src/elas3dxtal_pcg.f90:1527-1567): z = Minv g, partial z.g.
