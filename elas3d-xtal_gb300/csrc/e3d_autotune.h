@@ -7,15 +7,16 @@ namespace e3d {
 
 // n solves on `blocks` blocks, at most most_parts for one of them.  limit(j, k): the
 // blocks that solve j can use of k; nodes(j): its nodes; time(plan, ms): milliseconds
-// of some iterations of the batch with plan[j] blocks for solve j, returns a status.
+// of some iterations of the batch with plan[j] blocks for solve j, returns a status;
+// warm(plan): the shortest such run.
 // The plan that took least goes to best_plan.
 //
 // The first run in a process takes longer (the driver sets the kernel's stack up), so
 // one goes ahead of those that count: without it six solves of 64^3 got 64 blocks
 // each, 80 ms a batch where 25 take 61.  A time that is not positive counts for
 // nothing.
-template <typename Limit, typename Nodes, typename Time>
-int pick_parts(size_t n, int blocks, int most_parts, Limit&& limit, Nodes&& nodes, Time&& time,
+template <typename Limit, typename Nodes, typename Warm, typename Time>
+int pick_parts(size_t n, int blocks, int most_parts, Limit&& limit, Nodes&& nodes, Warm&& warm, Time&& time,
                std::vector<int>& best_plan) {
   std::vector<std::vector<int>> plans;
   double best = 1e300, ms = 0.0;
@@ -24,7 +25,7 @@ int pick_parts(size_t n, int blocks, int most_parts, Limit&& limit, Nodes&& node
     for (size_t j = 0; j < n; ++j) p[j] = limit(j, k_of(j));
     if (std::find(plans.begin(), plans.end(), p) != plans.end()) return 0;
     if (plans.empty())
-      if (int rc = time(p, &ms)) return rc;
+      if (int rc = warm(p)) return rc;
     plans.push_back(p);
     if (int rc = time(p, &ms)) return rc;
     if (ms > 0.0 && ms < best) {

@@ -441,6 +441,10 @@ int32_t batch_autotune(e3d_batch* b, std::vector<int>& kjob) {
   };
   return pick_parts(
       n, B, kMaxParts, limit, [&](size_t j) { return b->rves[(size_t)b->jobs[j].rve].ns; },
+      [&](const std::vector<int>& p) -> int {
+        float t = 0.f;
+        return batch_time(b, p, step, 1, &t);
+      },
       [&](const std::vector<int>& p, double* ms) -> int {
         float t2 = 0.f, t10 = 0.f;
         int32_t rc = batch_time(b, p, step, 2, &t2);

@@ -26,6 +26,7 @@ extern "C" double pick(int n, const long long* nodes, int blocks, double cold, i
   std::vector<int> best(n, 1);
   const int rc = e3d::pick_parts(
       n, blocks, 152, [](size_t, int k) { return k; }, [&](size_t j) { return nodes[j]; },
+      [&](const std::vector<int>&) { return ++*calls == fail_at ? 7 : 0; },
       [&](const std::vector<int>& p, double* ms) {
         *ms = model(p) + (*calls == 0 ? cold : 0.0);
         return ++*calls == fail_at ? 7 : 0;
