@@ -148,7 +148,9 @@ int32_t e3d_solve_begin(e3d_handle_t* h);
 int32_t e3d_iterate(e3d_handle_t* h, int32_t n, e3d_solve_stats_t* st);
 
 /* stress_OpenMP (:2149-2408): volume-averaged stress (Pa) and engineering
- * strain, Voigt xx, yy, zz, xz, yz, xy. */
+ * strain, Voigt xx, yy, zz, xz, yz, xy.  The sums over a phase's voxels are exact, of
+ * displacements held to 2^-57 of their component's largest (or FP64, voxel by voxel,
+ * where values are not finite or beyond 2^+-400). */
 int32_t e3d_stress(e3d_handle_t* h, double strav[6], double epsav[6]);
 
 /* stress_fullfield_OpenMP compute part (:2723-2833): sigma(ns,6) (SoA) and
