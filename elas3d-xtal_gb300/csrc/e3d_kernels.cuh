@@ -1076,7 +1076,7 @@ __device__ __forceinline__ int fx_exponent(unsigned hi) {
 // held to 2^-(56 - s) of itself.  Error of K.x there over that of the FP64 form,
 // measured with s from the typical size to the peak: 0.6 at s = 2, 1 at 4, 7 at 7, 57
 // at 10 (1.6e-15 of the part's own size).  Random vectors, the directions of a
-// solve from its fifth iteration on and displacements stay within these; a few
+// solve from its third to twelfth iteration on and displacements stay within these; a few
 // entries far above the rest, a direction that has not reached all of the grid
 // yet, and a rigid offset of one component do not: such a tile takes the FP64 form.
 constexpr unsigned kFxRow = 5;         // a row of the tile over all its planes
@@ -1718,15 +1718,16 @@ static __global__ void __launch_bounds__(kFxThreads) tile_max_kernel(GridDims G,
   const long long nxy = (long long)G.nx * G.ny;
   const double* col = x + E3D_IDX(active ? xg + (long long)G.nx * yg + nxy * z0 : 0, G.ns);
   FxRowScan scan;
-#pragma unroll 4
-  for (int z = z0; z < z1; ++z, col += nxy) {
-    unsigned a = 0, b = 0, c = 0;
-    if (active) {
-      a = size_word(__ldcg(col));
-      b = size_word(__ldcg(col + G.ns));
-      c = size_word(__ldcg(col + 2 * G.ns));
-    }
-    scan.plane(a, b, c);
+  constexpr int kAhead = 4;  // planes loaded before the first is scanned: the scan holds loads behind it back
+  for (int z = z0; z < z1; z += kAhead) {
+    double v[kAhead][3];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[j][c] = active && z + j < z1 ? __ldcg(col + j * nxy + c * G.ns) : 0.0;
+    col += kAhead * nxy;
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) scan.plane(size_word(v[j][0]), size_word(v[j][1]), size_word(v[j][2]));
   }
   unsigned vm, vl;
   scan.finish(vm, vl);
